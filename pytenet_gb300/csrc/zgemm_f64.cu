@@ -5,30 +5,39 @@
 // pytenet/chain_ops.py (apply_local_hamiltonian, the environment steps, the bond
 // contraction) and of the sweep (pytenet/tdvp.py:84,112) becomes one call.
 //
-// Tiling: 64x64 output tile per CTA of 8 warps (2 x 4), warp tile 32x16 = 4x2
-// DMMA fragments; K advances in slabs of 16 complex values staged through shared
-// memory as separate re/im planes (pitch 68 doubles: the 16-lane halves of a
-// fragment load hit 16 distinct 8-byte banks). A complex fragment product is four
-// real DMMAs: re += ar*br - ai*bi, im += ar*bi + ai*br.
-// Transposition and conjugation are folded into the global->shared load, so no
-// operand is ever materialised transposed. Skinny problems (fewer tiles than SMs)
-// split K across CTAs and reduce the FP64 partials in a second, deterministic pass.
+// What bounds it: an SM executes two FP64 FMAs per cycle whatever the instruction, so a
+// DMMA (256 FMAs) occupies its sub-partition for 512 cycles and the four DMMAs of a
+// complex 8 x 8 x 4 step for 2048. Next to that the operands cost nothing (1 KB per
+// step), so nothing is staged through shared memory: a warp owns one 8 x 8 block of C
+// and loads its fragments straight from L2 / L1 into registers, two steps ahead. What
+// matters is that no sub-partition multiplies padding or idles: the unit of work is one
+// warp's block (not a 64 x 64 tile), and blocks that are too few for the chip's 608
+// sub-partitions split K over the four warps of a CTA and over the CTAs of a cluster,
+// summed through (distributed) shared memory in a fixed order: no partial sums in
+// global memory, no second launch.
+// Measured against the 64 x 64 x 16 shared-memory tiles this replaces (one call of
+// H_eff . A, its two GEMMs): see choose_shape.
+// Transposition and conjugation are folded into the loads.
 //
-// Block sparsity: a K slab whose A part (64 x 16) or B part (16 x 64) of this tile is
-// entirely zero contributes nothing and its DMMAs are skipped (the barrier after the
-// shared-memory store votes on it). Tensors with quantum numbers hold zero blocks
-// (pytenet/block_sparse_util.py:47-64), and after the first block QR every bond is
-// ordered by quantum number, so their blocks line up with tiles and slabs; dense data
-// pays two barrier votes per slab.
+// Block sparsity: a K step whose A fragment (8 x 4) or B fragment (4 x 8) is entirely
+// zero contributes nothing and its DMMAs are skipped (a warp vote; not when the other
+// fragment holds an infinity or NaN, whose product with zero is NaN). Tensors with
+// quantum numbers hold zero blocks (pytenet/block_sparse_util.py:47-64), which after
+// the first block QR line up with these fragments.
 #include "ptn_common.cuh"
+#include <cooperative_groups.h>
 #include <algorithm>
+#include <cmath>
+
+namespace cg = cooperative_groups;
 
 namespace ptn {
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16;
-constexpr int PITCH = 68;
-constexpr int THREADS = 256;
+constexpr int FB = 8;              // rows and columns of a warp's block
+constexpr int WARPS = 4;
+constexpr int THREADS = 32 * WARPS;
+constexpr int MAX_CLUSTER = 8;
 
 enum { OP_N = 0, OP_T = 1, OP_C = 2, OP_H = 3 };
 
@@ -44,203 +53,127 @@ struct OpTraits {
   static constexpr bool conj = (OP == OP_C || OP == OP_H);
 };
 
-// whether any of a thread's four loaded entries is non-zero
-__device__ __forceinline__ bool nonzero4(const double2 (&r)[4]) {
-  bool nz = false;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) nz |= (r[i].x != 0.0) | (r[i].y != 0.0);
-  return nz;
-}
-
-// Load op(A)[m0 + m][k0 + k] for the 64x16 tile into registers.
-template <int OA>
-__device__ __forceinline__ void load_a(double2 (&ra)[4], const double2* __restrict__ A, long lda,
-                                       int M, int m0, int k0, int kend) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int m, k;
-    if (!OpTraits<OA>::trans) { k = tid & 15; m = (tid >> 4) + 16 * i; }
-    else                      { m = tid & 63; k = (tid >> 6) + 4 * i; }
-    const int gm = m0 + m, gk = k0 + k;
-    double2 v = make_double2(0.0, 0.0);
-    if (gm < M && gk < kend)
-      v = OpTraits<OA>::trans ? A[(long)gk * lda + gm] : A[(long)gm * lda + gk];
-    if (OpTraits<OA>::conj) v.y = -v.y;
-    ra[i] = v;
-  }
-}
-
-template <int OA>
-__device__ __forceinline__ void store_a(const double2 (&ra)[4], double (*sre)[PITCH],
-                                        double (*sim)[PITCH]) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int m, k;
-    if (!OpTraits<OA>::trans) { k = tid & 15; m = (tid >> 4) + 16 * i; }
-    else                      { m = tid & 63; k = (tid >> 6) + 4 * i; }
-    sre[k][m] = ra[i].x;
-    sim[k][m] = ra[i].y;
-  }
-}
-
-// Load op(B)[k0 + k][n0 + n] for the 16x64 tile.
-template <int OB>
-__device__ __forceinline__ void load_b(double2 (&rb)[4], const double2* __restrict__ B, long ldb,
-                                       int N, int n0, int k0, int kend) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int n, k;
-    if (!OpTraits<OB>::trans) { n = tid & 63; k = (tid >> 6) + 4 * i; }
-    else                      { k = tid & 15; n = (tid >> 4) + 16 * i; }
-    const int gn = n0 + n, gk = k0 + k;
-    double2 v = make_double2(0.0, 0.0);
-    if (gn < N && gk < kend)
-      v = OpTraits<OB>::trans ? B[(long)gn * ldb + gk] : B[(long)gk * ldb + gn];
-    if (OpTraits<OB>::conj) v.y = -v.y;
-    rb[i] = v;
-  }
-}
-
-template <int OB>
-__device__ __forceinline__ void store_b(const double2 (&rb)[4], double (*sre)[PITCH],
-                                        double (*sim)[PITCH]) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int n, k;
-    if (!OpTraits<OB>::trans) { n = tid & 63; k = (tid >> 6) + 4 * i; }
-    else                      { k = tid & 15; n = (tid >> 4) + 16 * i; }
-    sre[k][n] = rb[i].x;
-    sim[k][n] = rb[i].y;
-  }
-}
-
 struct KArgs {
-  int M, N, K, batch, splits, kchunk;
+  int M, N, K;
+  int kchunk;                       // K entries per part (a multiple of 4)
   double2 alpha, beta;
   const double2* A; long lda, sA;
   const double2* B; long ldb, sB;
   double2* C; long ldc, sC;
-  double2* part;   // split-K partials [batch][splits][M][N], or null
   const int* skip;
 };
 
-template <int OA, int OB>
-__global__ void __launch_bounds__(THREADS) zgemm_dmma_kernel(const KArgs p) {
-  if (p.skip != nullptr && *p.skip != 0) return;
-  __shared__ __align__(16) double sa_re[BK][PITCH];
-  __shared__ __align__(16) double sa_im[BK][PITCH];
-  __shared__ __align__(16) double sb_re[BK][PITCH];
-  __shared__ __align__(16) double sb_im[BK][PITCH];
-
-  const int bz = blockIdx.z;
-  const int b = bz / p.splits, split = bz % p.splits;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int kbeg = split * p.kchunk;
-  const int kend = min(p.K, kbeg + p.kchunk);
-  const double2* A = p.A + (long)b * p.sA;
-  const double2* B = p.B + (long)b * p.sB;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
-  const int fr = lane >> 2, fc = lane & 3;
-
-  double acc[4][2][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int t = 0; t < 4; ++t) acc[i][j][t] = 0.0;
-
-  double2 ra[4], rb[4];
-  if (kbeg < kend) {
-    load_a<OA>(ra, A, p.lda, p.M, m0, kbeg, kend);
-    load_b<OB>(rb, B, p.ldb, p.N, n0, kbeg, kend);
-  }
-  for (int k0 = kbeg; k0 < kend; k0 += BK) {
-    __syncthreads();
-    store_a<OA>(ra, sa_re, sa_im);
-    store_b<OB>(rb, sb_re, sb_im);
-    // barrier with a vote: does this slab have a non-zero entry in A's and in B's part
-    const int live_a = __syncthreads_or(nonzero4(ra));
-    const int live_b = __syncthreads_or(nonzero4(rb));
-    const bool live = live_a != 0 && live_b != 0;
-    if (k0 + BK < kend) {
-      load_a<OA>(ra, A, p.lda, p.M, m0, k0 + BK, kend);
-      load_b<OB>(rb, B, p.ldb, p.N, n0, k0 + BK, kend);
-    }
-    if (!live) continue;
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      double are[4], aim[4], bre[2], bim[2];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        are[i] = sa_re[kk + fc][wm + i * 8 + fr];
-        aim[i] = sa_im[kk + fc][wm + i * 8 + fr];
-      }
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        bre[j] = sb_re[kk + fc][wn + j * 8 + fr];
-        bim[j] = sb_im[kk + fc][wn + j * 8 + fr];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const double naim = -aim[i];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          dmma(acc[i][j][0], acc[i][j][1], are[i], bre[j]);
-          dmma(acc[i][j][0], acc[i][j][1], naim, bim[j]);
-          dmma(acc[i][j][2], acc[i][j][3], are[i], bim[j]);
-          dmma(acc[i][j][2], acc[i][j][3], aim[i], bre[j]);
-        }
-      }
-    }
-  }
-
-  // epilogue: fragment element (fr, 2*fc + e)
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + wm + i * 8 + fr;
-    if (gm >= p.M) continue;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int gn = n0 + wn + j * 8 + 2 * fc + e;
-        if (gn >= p.N) continue;
-        const double2 v = make_double2(acc[i][j][e], acc[i][j][2 + e]);
-        if (p.part != nullptr) {
-          p.part[(((long)b * p.splits + split) * p.M + gm) * p.N + gn] = v;
-        } else {
-          double2* cp = p.C + (long)b * p.sC + (long)gm * p.ldc + gn;
-          double2 out = cmul(p.alpha, v);
-          if (p.beta.x != 0.0 || p.beta.y != 0.0) out = cadd(out, cmul(p.beta, *cp));
-          *cp = out;
-        }
-      }
-    }
-  }
+// op(X)[r][k] of a fragment lane, zero outside
+template <int OP>
+__device__ __forceinline__ double2 frag_a(const double2* __restrict__ A, long lda, int r, int k,
+                                          int M, int kend) {
+  double2 v = make_double2(0.0, 0.0);
+  if (r < M && k < kend) v = OpTraits<OP>::trans ? A[(long)k * lda + r] : A[(long)r * lda + k];
+  if (OpTraits<OP>::conj) v.y = -v.y;
+  return v;
 }
 
-__global__ void splitk_reduce_kernel(const KArgs p) {
-  if (p.skip != nullptr && *p.skip != 0) return;
-  const long total = (long)p.batch * p.M * p.N;
-  for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long)gridDim.x * blockDim.x) {
-    const long b = idx / ((long)p.M * p.N);
-    const long mn = idx - b * (long)p.M * p.N;
-    const int gm = (int)(mn / p.N), gn = (int)(mn % p.N);
-    double2 s = make_double2(0.0, 0.0);
-    for (int k = 0; k < p.splits; ++k) s = cadd(s, p.part[((b * p.splits + k) * p.M) * (long)p.N + mn]);
-    double2* cp = p.C + b * p.sC + (long)gm * p.ldc + gn;
-    double2 out = cmul(p.alpha, s);
-    if (p.beta.x != 0.0 || p.beta.y != 0.0) out = cadd(out, cmul(p.beta, *cp));
-    *cp = out;
+template <int OP>
+__device__ __forceinline__ double2 frag_b(const double2* __restrict__ B, long ldb, int c, int k,
+                                          int N, int kend) {
+  double2 v = make_double2(0.0, 0.0);
+  if (c < N && k < kend) v = OpTraits<OP>::trans ? B[(long)c * ldb + k] : B[(long)k * ldb + c];
+  if (OpTraits<OP>::conj) v.y = -v.y;
+  return v;
+}
+
+// 1: has a non-zero entry; 2: has an infinity or NaN
+__device__ __forceinline__ unsigned entry_class(double2 v) {
+  const unsigned hx = (unsigned)__double2hiint(v.x) & 0x7FF00000u;
+  const unsigned hy = (unsigned)__double2hiint(v.y) & 0x7FF00000u;
+  return ((v.x != 0.0 || v.y != 0.0) ? 1u : 0u) |
+         ((hx == 0x7FF00000u || hy == 0x7FF00000u) ? 2u : 0u);
+}
+
+// KW = 1: the CTA's four warps own a 2 x 2 group of blocks; KW = 4: they share one
+// block, a quarter of the K part each. gridDim.y (= the cluster's y extent) splits K too.
+template <int OA, int OB, int KW>
+__global__ void __launch_bounds__(THREADS) zgemm_dmma_kernel(const KArgs p) {
+  if (p.skip != nullptr && *p.skip != 0) return;   // uniform over the launch
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int fr = lane >> 2, fc = lane & 3;
+  const int parts = gridDim.y, part = blockIdx.y;
+  constexpr int CB = KW == 1 ? 2 * FB : FB;        // CTA block edge
+  const int nct = (p.N + CB - 1) / CB;
+  const int m0 = (int)(blockIdx.x / nct) * CB + (KW == 1 ? (warp >> 1) * FB : 0);
+  const int n0 = (int)(blockIdx.x % nct) * CB + (KW == 1 ? (warp & 1) * FB : 0);
+  const double2* A = p.A + (long)blockIdx.z * p.sA;
+  const double2* B = p.B + (long)blockIdx.z * p.sB;
+  const int kp = (KW == 1) ? part : part * KW + warp;
+  const int kbeg = kp * p.kchunk;
+  const int kend = min(p.K, kbeg + p.kchunk);
+  const int r = m0 + fr, c = n0 + fr;
+
+  double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+  if (m0 < p.M && n0 < p.N && kbeg < kend) {
+    double2 a0 = frag_a<OA>(A, p.lda, r, kbeg + fc, p.M, kend);
+    double2 b0 = frag_b<OB>(B, p.ldb, c, kbeg + fc, p.N, kend);
+    double2 a1 = frag_a<OA>(A, p.lda, r, kbeg + 4 + fc, p.M, kend);
+    double2 b1 = frag_b<OB>(B, p.ldb, c, kbeg + 4 + fc, p.N, kend);
+    for (int k = kbeg; k < kend; k += 4) {
+      const double2 a = a0, b = b0;
+      a0 = a1;
+      b0 = b1;
+      a1 = frag_a<OA>(A, p.lda, r, k + 8 + fc, p.M, kend);
+      b1 = frag_b<OB>(B, p.ldb, c, k + 8 + fc, p.N, kend);
+      const unsigned ca = entry_class(a), cb = entry_class(b);
+      const bool za = !__any_sync(0xffffffffu, ca & 1u), zb = !__any_sync(0xffffffffu, cb & 1u);
+      if ((za || zb) && !__any_sync(0xffffffffu, (ca | cb) & 2u)) continue;
+      dmma(re[0], re[1], a.x, b.x);
+      dmma(im[0], im[1], a.x, b.y);
+      dmma(re[0], re[1], -a.y, b.y);
+      dmma(im[0], im[1], a.y, b.x);
+    }
   }
+
+  // sum the K parts in a fixed order: the warps' quarters, then the cluster's CTAs
+  __shared__ double2 s_part[WARPS][2 * 32];
+  if (KW == 1 && parts == 1) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int gm = m0 + fr, gn = n0 + 2 * fc + e;
+      if (gm < p.M && gn < p.N) {
+        double2* cp = p.C + (long)blockIdx.z * p.sC + (long)gm * p.ldc + gn;
+        double2 out = cmul(p.alpha, make_double2(re[e], im[e]));
+        if (p.beta.x != 0.0 || p.beta.y != 0.0) out = cadd(out, cmul(p.beta, *cp));
+        *cp = out;
+      }
+    }
+    return;
+  }
+  s_part[warp][2 * lane] = make_double2(re[0], im[0]);
+  s_part[warp][2 * lane + 1] = make_double2(re[1], im[1]);
+  if (parts > 1) cg::this_cluster().sync();
+  else __syncthreads();
+  // entries of the CTA's blocks, spread over the cluster's CTAs
+  constexpr int ENT = (KW == 1 ? WARPS : 1) * 64;
+  for (int e = part * THREADS + (int)threadIdx.x; e < ENT; e += parts * THREADS) {
+    const int wb = e >> 6, x = e & 63;             // block of the CTA, entry of the block
+    double2 s = make_double2(0.0, 0.0);
+    for (int q = 0; q < parts; ++q) {
+#pragma unroll
+      for (int w = 0; w < KW; ++w) {
+        const double2* src = &s_part[KW == 1 ? wb : w][x];
+        const double2 v = parts > 1 ? *cg::this_cluster().map_shared_rank(src, q) : *src;
+        s = (q == 0 && w == 0) ? v : cadd(s, v);
+      }
+    }
+    const int bm = (int)(blockIdx.x / nct) * CB + (wb >> 1) * FB;
+    const int bn = (int)(blockIdx.x % nct) * CB + (wb & 1) * FB;
+    const int gm = bm + (x >> 3), gn = bn + (x & 7);
+    if (gm < p.M && gn < p.N) {
+      double2* cp = p.C + (long)blockIdx.z * p.sC + (long)gm * p.ldc + gn;
+      double2 out = cmul(p.alpha, s);
+      if (p.beta.x != 0.0 || p.beta.y != 0.0) out = cadd(out, cmul(p.beta, *cp));
+      *cp = out;
+    }
+  }
+  if (parts > 1) cg::this_cluster().sync();   // no CTA leaves while its shared memory is read
 }
 
 int op_code(char c) {
@@ -253,90 +186,116 @@ int op_code(char c) {
   }
 }
 
-template <int OA>
-void launch_b(int ob, dim3 grid, cudaStream_t st, const KArgs& k) {
-  switch (ob) {
-    case OP_N: zgemm_dmma_kernel<OA, OP_N><<<grid, THREADS, 0, st>>>(k); break;
-    case OP_T: zgemm_dmma_kernel<OA, OP_T><<<grid, THREADS, 0, st>>>(k); break;
-    case OP_C: zgemm_dmma_kernel<OA, OP_C><<<grid, THREADS, 0, st>>>(k); break;
-    default:   zgemm_dmma_kernel<OA, OP_H><<<grid, THREADS, 0, st>>>(k); break;
-  }
+struct Shape {
+  int kw;       // K parts inside a CTA (1: four blocks per CTA, 4: one)
+  int parts;    // CTAs of a cluster that split K
+  int kchunk;   // K entries per part
+};
+
+// Launch shape: the split of K that finishes first under a plain model: 2048 cycles per
+// K step of a block and one block per sub-partition at a time (counted in whole turns
+// while there are few), plus what a CTA's and a cluster's sum cost. Measured on the two
+// GEMMs of H_eff . A (64 x 64 x 16 tiles with split K through global memory before):
+//   bonds 250 x 256, chi 5   1207 + 1485 us -> 1201 + 1423 us (1.01 TF/s)
+//   bonds <= 28 (README run)   83 +  213 us ->    4 +    5 us, mean over a time step
+//   bonds <= 24, U(1) (DMRG)   87 +  289 us ->    4 +    5 us, mean over a sweep
+// PTN_TUNE_ZGEMM_SPLIT_WAVES 0 keeps K within a CTA, other values allow clusters.
+Shape choose_shape(int M, int N, int K, int batch) {
+  const long subp = 4L * num_sms();
+  const long steps = std::max(1, (K + 3) / 4);
+  const bool clusters = tune(PTN_TUNE_ZGEMM_SPLIT_WAVES) != 0;
+  Shape best{1, 1, 0};
+  double best_cost = -1.0;
+  for (int kw : {1, 4})
+    for (int parts = 1; parts <= (clusters ? MAX_CLUSTER : 1); parts *= 2) {
+      const long np = (long)kw * parts;
+      if (np > 1 && steps < np) continue;
+      const long per = (steps + np - 1) / np;
+      const long edge = kw == 1 ? 2 * FB : FB;
+      const long ctas = ((M + edge - 1) / edge) * ((N + edge - 1) / edge) * (long)batch * parts;
+      const double turns = (double)ctas * WARPS / subp;
+      const double whole = turns < 8.0 ? std::ceil(turns) : turns;
+      const double cost = whole * (per * 2048.0 + (kw > 1 ? 300.0 : 0.0) + (parts > 1 ? 1200.0 : 0.0));
+      if (best_cost < 0.0 || cost < best_cost) {
+        best_cost = cost;
+        best = Shape{kw, parts, 0};
+      }
+    }
+  const long np = (long)best.kw * best.parts;
+  best.kchunk = (int)((steps + np - 1) / np * 4);
+  return best;
 }
 
-// K splits for skinny problems: up to PTN_TUNE_ZGEMM_SPLIT_WAVES waves of CTAs (at
-// most 32 splits of at least 4 K slabs), choosing the count with the fewest
-// waves x (K slabs per CTA + a fixed per-CTA cost of about SLAB_OVERHEAD slabs).
-int choose_splits(int M, int N, int K, int batch) {
-  constexpr int SLAB_OVERHEAD = 4;
-  const long tiles = (long)((M + BM - 1) / BM) * ((N + BN - 1) / BN) * batch;
-  const long sms = num_sms();
-  const int waves = tune(PTN_TUNE_ZGEMM_SPLIT_WAVES);
-  if (waves == 0 || tiles >= (long)waves * sms || K < 8 * BK) return 1;
-  const long slabs = (K + BK - 1) / BK;
-  long s_cap = ((long)waves * sms + tiles - 1) / tiles;
-  s_cap = std::min<long>(s_cap, std::max(1, K / (4 * BK)));
-  s_cap = std::min<long>(s_cap, 32);
-  int best = 1;
-  long best_cost = -1;
-  for (long s = 1; s <= s_cap; ++s) {
-    const long w = (tiles * s + sms - 1) / sms;
-    const long cost = w * ((slabs + s - 1) / s + SLAB_OVERHEAD);
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best = (int)s;
-    }
+template <int OA, int OB>
+cudaError_t launch_ab(const Shape& s, const KArgs& k, int batch, cudaStream_t st) {
+  const long edge = s.kw == 1 ? 2 * FB : FB;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(((k.M + edge - 1) / edge) * ((k.N + edge - 1) / edge)),
+                     (unsigned)s.parts, (unsigned)batch);
+  cfg.blockDim = dim3(THREADS);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = s.parts;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = s.parts > 1 ? 1 : 0;
+  if (s.kw == 1) return cudaLaunchKernelEx(&cfg, zgemm_dmma_kernel<OA, OB, 1>, k);
+  return cudaLaunchKernelEx(&cfg, zgemm_dmma_kernel<OA, OB, 4>, k);
+}
+
+template <int OA>
+cudaError_t launch_b(int ob, const Shape& s, const KArgs& k, int batch, cudaStream_t st) {
+  switch (ob) {
+    case OP_N: return launch_ab<OA, OP_N>(s, k, batch, st);
+    case OP_T: return launch_ab<OA, OP_T>(s, k, batch, st);
+    case OP_C: return launch_ab<OA, OP_C>(s, k, batch, st);
+    default: return launch_ab<OA, OP_H>(s, k, batch, st);
   }
-  return best;
 }
 
 }  // namespace
 
 void note_launches(int n);
 
+// K is split inside the launch (clusters): no scratch in global memory
 size_t zgemm_workspace_bytes(int M, int N, int K, int batch) {
-  const int s = choose_splits(M, N, K, batch);
-  return s > 1 ? (size_t)s * batch * (size_t)M * N * sizeof(double2) : 0;
+  (void)M;
+  (void)N;
+  (void)K;
+  (void)batch;
+  return 0;
 }
 
 ptn_status zgemm(const GemmArgs& g, void* ws, size_t ws_bytes, cudaStream_t st) {
+  (void)ws;
+  (void)ws_bytes;
   const int oa = op_code(g.opA), ob = op_code(g.opB);
   PTN_CHECK_ARG(oa >= 0 && ob >= 0, "zgemm: bad op (%c, %c)", g.opA, g.opB);
   PTN_CHECK_ARG(g.M >= 0 && g.N >= 0 && g.K >= 0 && g.batch >= 1, "zgemm: bad sizes");
   if (g.M == 0 || g.N == 0) return PTN_OK;
   KArgs k;
-  k.M = g.M; k.N = g.N; k.K = g.K; k.batch = g.batch;
+  k.M = g.M; k.N = g.N; k.K = g.K;
   k.alpha = g.alpha; k.beta = g.beta;
   k.A = g.A; k.lda = g.lda; k.sA = g.sA;
   k.B = g.B; k.ldb = g.ldb; k.sB = g.sB;
   k.C = g.C; k.ldc = g.ldc; k.sC = g.sC;
   k.skip = g.skip;
-  int splits = choose_splits(g.M, g.N, g.K, g.batch);
-  while (splits > 1 && (size_t)splits * g.batch * (size_t)g.M * g.N * sizeof(double2) > ws_bytes)
-    splits /= 2;
-  if (splits < 1) splits = 1;
-  k.splits = splits;
-  k.kchunk = ((g.K + splits - 1) / splits + BK - 1) / BK * BK;
-  if (k.kchunk == 0) k.kchunk = BK;
-  k.part = splits > 1 ? static_cast<double2*>(ws) : nullptr;
-  dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, g.batch * splits);
-  PTN_CHECK_ARG(grid.y <= 65535 && grid.z <= 65535, "zgemm: grid too large");
+  const Shape s = choose_shape(g.M, g.N, g.K, g.batch);
+  k.kchunk = s.kchunk;
+  PTN_CHECK_ARG(g.batch <= 65535, "zgemm: grid too large");
   const int prof = prof_begin(st, PROF_ZGEMM_F64, 8.0 * g.M * g.N * (double)g.K * g.batch,
                               16.0 * g.batch * ((double)g.M * g.K + (double)g.K * g.N + 2.0 * g.M * g.N));
+  cudaError_t e;
   switch (oa) {
-    case OP_N: launch_b<OP_N>(ob, grid, st, k); break;
-    case OP_T: launch_b<OP_T>(ob, grid, st, k); break;
-    case OP_C: launch_b<OP_C>(ob, grid, st, k); break;
-    default:   launch_b<OP_H>(ob, grid, st, k); break;
+    case OP_N: e = launch_b<OP_N>(ob, s, k, g.batch, st); break;
+    case OP_T: e = launch_b<OP_T>(ob, s, k, g.batch, st); break;
+    case OP_C: e = launch_b<OP_C>(ob, s, k, g.batch, st); break;
+    default: e = launch_b<OP_H>(ob, s, k, g.batch, st); break;
   }
-  PTN_LAUNCH_CHECK();
+  PTN_CUDA_TRY(e);
   note_launches(1);
-  if (splits > 1) {
-    const long total = (long)g.batch * g.M * g.N;
-    const int blocks = (int)std::min<long>((total + 255) / 256, 4L * num_sms());
-    splitk_reduce_kernel<<<blocks, 256, 0, st>>>(k);
-    PTN_LAUNCH_CHECK();
-    note_launches(1);
-  }
   prof_end(st, prof);
   return PTN_OK;
 }
