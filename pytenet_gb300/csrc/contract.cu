@@ -15,6 +15,8 @@
 // intermediate once) and skips the zero entries of W, which for the XXZ MPO are
 // ~90% of the (chi d)^2 matrix.
 #include "ptn_common.cuh"
+#include "mpo_stage.cuh"
+#include "rns.cuh"
 #include <algorithm>
 
 namespace ptn {
@@ -23,88 +25,45 @@ void note_launches(int n);
 
 namespace {
 
-// out[x, q, y] = sum_p M[q, p] in[x, p, y]; M given by (ldq, ldp) strides into w.
-// One CTA per (x, 128-wide y chunk); thread q compacts the nonzeros of row q of M in
-// shared memory, the P input rows of the chunk are staged there too.
-// Bound: HBM / L2 for large tensors, latency for small ones, and close behind both the
-// FP64 units (two operations per SM and cycle), so entries are applied by kind: an MPO
-// entry is real nearly always (two operations instead of four), often exactly 1 (one
-// addition), and the first entry of a row starts the sum instead of being added to zero.
-// Measured at bonds 512 x 512, chi 5: 65 -> 37 us; at bonds <= 28: 15.9 -> 6.3 us (one
-// thread scanned W before, and every entry took four FMAs).
-enum { ENTRY_COMPLEX = 0, ENTRY_REAL = 1, ENTRY_ONE = 2 };
-
-__device__ __forceinline__ double2 entry_mul(int kind, double2 v, double2 x) {
-  if (kind == ENTRY_ONE) return x;
-  if (kind == ENTRY_REAL) return make_double2(v.x * x.x, v.x * x.y);
-  return cmul(v, x);
-}
-
-__device__ __forceinline__ double2 entry_fma(int kind, double2 v, double2 x, double2 acc) {
-  if (kind == ENTRY_ONE) return cadd(acc, x);
-  if (kind == ENTRY_REAL) return make_double2(fma(v.x, x.x, acc.x), fma(v.x, x.y, acc.y));
-  return cfma(v, x, acc);
-}
-
-__global__ void mpo_stage_kernel(const double2* __restrict__ in, double2* __restrict__ out,
-                                 const double2* __restrict__ w, long ldq, long ldp, int X, int P,
-                                 int Q, int Y, const int* skip) {
+__global__ void __launch_bounds__(STAGE_Y)
+    mpo_stage_kernel(const double2* __restrict__ in, double2* __restrict__ out,
+                     const double2* __restrict__ w, long ldq, long ldp, int X, int P, int Q, int Y,
+                     const int* skip) {
   if (skip != nullptr && *skip != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* sin = reinterpret_cast<double2*>(smem_raw);             // [P][128]
-  double2* sval = sin + (size_t)P * 128;                            // [Q][P] row q: its nonzeros
+  double2* sin = reinterpret_cast<double2*>(smem_raw);             // [P][STAGE_Y]
+  double2* sval = sin + (size_t)P * STAGE_Y;                        // [Q][P] row q: its nonzeros
   int* sidx = reinterpret_cast<int*>(sval + (size_t)P * Q);         // [Q][P] 4 * p + kind
-  __shared__ int scount[64];
+  __shared__ int scount[STAGE_MAX];
 
   const int x = blockIdx.y;
-  const int y0 = blockIdx.x * 128;
-  const int ty = threadIdx.x;   // 128 threads
-  const int y = y0 + ty;
-  for (int e = ty; e < P * Q; e += 128) sval[e] = w[(e / P) * ldq + (e % P) * ldp];
+  const int ty = threadIdx.x;
+  const int y = blockIdx.x * STAGE_Y + ty;
+  stage_load_w(w, ldq, ldp, P, Q, sval);
   for (int p = 0; p < P; ++p)
-    sin[p * 128 + ty] = (y < Y) ? in[((long)x * P + p) * Y + y] : make_double2(0.0, 0.0);
+    sin[p * STAGE_Y + ty] = (y < Y) ? in[((long)x * P + p) * Y + y] : make_double2(0.0, 0.0);
   __syncthreads();
-  if (ty < Q) {
-    double2* row = sval + ty * P;
-    int* idx = sidx + ty * P;
-    int nz = 0;
-    for (int p = 0; p < P; ++p) {
-      const double2 v = row[p];
-      if (v.x != 0.0 || v.y != 0.0) {
-        row[nz] = v;
-        idx[nz] = 4 * p + (v.y != 0.0 ? ENTRY_COMPLEX : v.x != 1.0 ? ENTRY_REAL : ENTRY_ONE);
-        ++nz;
-      }
-    }
-    scount[ty] = nz;
-  }
+  stage_compact(P, Q, sval, sidx, scount);
   __syncthreads();
   if (y >= Y) return;
-  for (int q = 0; q < Q; ++q) {
-    const double2* row = sval + q * P;
-    const int* idx = sidx + q * P;
-    const int nz = scount[q];
-    double2 acc = make_double2(0.0, 0.0);
-    if (nz > 0) acc = entry_mul(idx[0] & 3, row[0], sin[(idx[0] >> 2) * 128 + ty]);
-    for (int e = 1; e < nz; ++e) acc = entry_fma(idx[e] & 3, row[e], sin[(idx[e] >> 2) * 128 + ty], acc);
-    out[((long)x * Q + q) * Y + y] = acc;
-  }
+  for (int q = 0; q < Q; ++q)
+    out[((long)x * Q + q) * Y + y] = stage_row(q, P, sin + ty, sval, sidx, scount);
 }
 
 ptn_status mpo_stage(const double2* in, double2* out, const double2* w, long ldq, long ldp, int X,
                      int P, int Q, int Y, const int* skip, cudaStream_t st) {
-  PTN_CHECK_ARG(P <= 64 && Q <= 64, "MPO stage: chi*d must be <= 64 (got %d, %d)", P, Q);
+  PTN_CHECK_ARG(P <= STAGE_MAX && Q <= STAGE_MAX, "MPO stage: chi*d must be <= 64 (got %d, %d)", P, Q);
   if (X == 0 || Y == 0) return PTN_OK;
-  const size_t smem = (size_t)P * 128 * sizeof(double2) + (size_t)P * Q * (sizeof(double2) + sizeof(int));
+  const size_t smem = stage_smem(P, Q);
   static bool attr_done = false;
   if (!attr_done) {
     PTN_CUDA_TRY(cudaFuncSetAttribute(mpo_stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      64 * 128 * 16 + 64 * 64 * 20));
+                                      (int)stage_smem(STAGE_MAX, STAGE_MAX)));
     attr_done = true;
   }
-  dim3 grid((Y + 127) / 128, X);
+  dim3 grid((Y + STAGE_Y - 1) / STAGE_Y, X);
   PTN_CHECK_ARG(X <= 65535, "MPO stage: X too large");
-  mpo_stage_kernel<<<grid, 128, smem, st>>>(in, out, w, ldq, ldp, X, P, Q, Y, skip);
+  mpo_stage_kernel<<<grid, STAGE_Y, smem, st>>>(in, out, w, ldq, ldp, X, P, Q, Y, skip);
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;
@@ -135,6 +94,22 @@ GemmArgs gemm_args(char oa, char ob, int M, int N, int K, const double2* A, long
 
 }  // namespace
 
+// ------------------------------------------------------------------ choice of kernels
+// The FP64 form takes the residue planes where both GEMMs do (rns_wanted), the DMMA kernel
+// otherwise, or when the workspace is smaller than the query asks for.
+bool heff_f64_rns(int Dl, int d, int Dr, int cl, int cr) {
+  return rns_wanted((long)Dl * d, (long)cr * Dr, Dr) && rns_wanted(Dl, (long)d * Dr, (long)Dl * cl);
+}
+
+bool bond_f64_rns(int Dl, int Dr, int chi) {
+  return rns_wanted(Dl, (long)chi * Dr, Dr) && rns_wanted(Dl, Dr, (long)Dl * chi);
+}
+
+static bool env_f64_rns(int Dl, int d, int Dr, int cl, int cr) {
+  return rns_wanted((long)Dl * cl, (long)d * Dr, Dl) && rns_wanted(Dr, (long)cr * Dr, (long)Dl * d) &&
+         rns_wanted((long)Dl * d, (long)cr * Dr, Dr) && rns_wanted((long)Dl * cl, Dl, (long)d * Dr);
+}
+
 // ------------------------------------------------------------------ workspace layout
 // [T1 | T2 | split-K partials]
 struct ContractWs {
@@ -154,6 +129,8 @@ static size_t heff_gemm_ws(int Dl, int d, int Dr, int chil, int chir) {
 }
 
 size_t heff_workspace_bytes_f64(int Dl, int d, int Dr, int chil, int chir) {
+  if (heff_f64_rns(Dl, d, Dr, chil, chir))
+    return heff_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir);
   const size_t t = align256(heff_t_elems(Dl, d, Dr, chil, chir) * sizeof(double2));
   return 2 * t + align256(heff_gemm_ws(Dl, d, Dr, chil, chir));
 }
@@ -187,6 +164,7 @@ ptn_status heff_apply_f64(const double2* a, const double2* w, const double2* l, 
 }
 
 size_t bond_workspace_bytes_f64(int Dl, int Dr, int chi) {
+  if (bond_f64_rns(Dl, Dr, chi)) return bond_workspace_bytes_rns(RNS_FP64, Dl, Dr, chi);
   const size_t t = align256((size_t)Dl * chi * Dr * sizeof(double2));
   const size_t g = std::max(zgemm_workspace_bytes(Dl, chi * Dr, Dr, 1),
                             zgemm_workspace_bytes(Dl, Dr, Dl * chi, 1));
@@ -209,6 +187,8 @@ ptn_status bond_apply_f64(const double2* cm, const double2* l, const double2* r,
 }
 
 size_t env_workspace_bytes_f64(int Dl, int d, int Dr, int chil, int chir) {
+  if (env_f64_rns(Dl, d, Dr, chil, chir))
+    return env_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir);
   const size_t te = (size_t)std::max(Dl * chil * d * Dr, Dl * d * chir * Dr);
   const size_t t = align256(te * sizeof(double2));
   size_t g = zgemm_workspace_bytes(Dl * chil, d * Dr, Dl, 1);
@@ -221,6 +201,9 @@ size_t env_workspace_bytes_f64(int Dl, int d, int Dr, int chil, int chir) {
 ptn_status env_left_f64(const double2* a, const double2* b, const double2* w, const double2* l,
                         double2* lnext, int Dl, int d, int Dr, int chil, int chir, void* ws,
                         size_t ws_bytes, cudaStream_t st) {
+  if (env_f64_rns(Dl, d, Dr, chil, chir) &&
+      ws_bytes >= env_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir))
+    return env_left_rns(RNS_FP64, a, b, w, l, lnext, Dl, d, Dr, chil, chir, ws, ws_bytes, st);
   const size_t te = (size_t)std::max(Dl * chil * d * Dr, Dl * d * chir * Dr);
   PTN_CHECK_ARG(ws_bytes >= 2 * align256(te * sizeof(double2)), "env_left: workspace too small");
   ContractWs c = carve(ws, te, ws_bytes);
@@ -238,6 +221,9 @@ ptn_status env_left_f64(const double2* a, const double2* b, const double2* w, co
 ptn_status env_right_f64(const double2* a, const double2* b, const double2* w, const double2* r,
                          double2* rnext, int Dl, int d, int Dr, int chil, int chir, void* ws,
                          size_t ws_bytes, cudaStream_t st) {
+  if (env_f64_rns(Dl, d, Dr, chil, chir) &&
+      ws_bytes >= env_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir))
+    return env_right_rns(RNS_FP64, a, b, w, r, rnext, Dl, d, Dr, chil, chir, ws, ws_bytes, st);
   const size_t te = (size_t)std::max(Dl * chil * d * Dr, Dl * d * chir * Dr);
   PTN_CHECK_ARG(ws_bytes >= 2 * align256(te * sizeof(double2)), "env_right: workspace too small");
   ContractWs c = carve(ws, te, ws_bytes);
@@ -295,6 +281,13 @@ ptn_status ptn_heff_apply(const ptn_c128* a, const ptn_c128* w, const ptn_c128* 
                           const ptn_c128* r, ptn_c128* out, int Dl, int d, int Dr, int chil,
                           int chir, int prec, void* ws, size_t ws_bytes, void* stream) {
   PTN_CHECK_ARG(Dl > 0 && d > 0 && Dr > 0 && chil > 0 && chir > 0, "heff: bad dims");
+  if (prec == PTN_PREC_FP64 && heff_f64_rns(Dl, d, Dr, chil, chir) &&
+      ws_bytes >= heff_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir)) {
+    PTN_TRY(heff_prepare_rns(RNS_FP64, D2(l), D2(r), Dl, d, Dr, chil, chir, ws, ws_bytes,
+                             as_stream(stream)));
+    return heff_apply_rns(RNS_FP64, D2(a), D2(out), D2(w), D2(l), D2(r), Dl, d, Dr, chil, chir, ws,
+                          nullptr, as_stream(stream));
+  }
   if (prec == PTN_PREC_FP64)
     return heff_apply_f64(D2(a), D2(w), D2(l), D2(r), D2(out), Dl, d, Dr, chil, chir, ws, ws_bytes,
                           nullptr, as_stream(stream));
@@ -306,6 +299,12 @@ ptn_status ptn_bond_apply(const ptn_c128* c, const ptn_c128* l, const ptn_c128* 
                           int Dl, int Dr, int chi, int prec, void* ws, size_t ws_bytes,
                           void* stream) {
   PTN_CHECK_ARG(Dl > 0 && Dr > 0 && chi > 0, "bond: bad dims");
+  if (prec == PTN_PREC_FP64 && bond_f64_rns(Dl, Dr, chi) &&
+      ws_bytes >= bond_workspace_bytes_rns(RNS_FP64, Dl, Dr, chi)) {
+    PTN_TRY(bond_prepare_rns(RNS_FP64, D2(l), D2(r), Dl, Dr, chi, ws, ws_bytes, as_stream(stream)));
+    return bond_apply_rns(RNS_FP64, D2(c), D2(out), D2(l), D2(r), Dl, Dr, chi, ws, nullptr,
+                          as_stream(stream));
+  }
   if (prec == PTN_PREC_FP64)
     return bond_apply_f64(D2(c), D2(l), D2(r), D2(out), Dl, Dr, chi, ws, ws_bytes, nullptr,
                           as_stream(stream));

@@ -1,0 +1,1115 @@
+// Complex GEMM in a residue number system on the 5th-generation tensor cores (tcgen05).
+//
+// C = A B over complex FP64 is computed exactly in integers and rounded once:
+//   - every row of A and every column of B is scaled by its own power of two and rounded
+//     to Gaussian integers of `bits` bits (53 or 54 in the FP64 form, 40 and more in the
+//     mixed form);
+//   - the integer product is formed modulo nm small pairwise coprime numbers p and put
+//     together by the Chinese remainder theorem (Ozaki, Uchino and Imamura, "Ozaki Scheme
+//     II", 2025, use it for real matrices). All prime factors of the moduli are 1 mod 4,
+//     so -1 has a square root j modulo p and the Gaussian integers modulo p split into two
+//     independent copies of the integers modulo p: z = x + i y -> (x + j y, x - j y). A
+//     complex product therefore costs two real ones per modulus (not four), conjugation
+//     swaps the copies, and the copies of all moduli are 2 nm independent real GEMMs;
+//   - residues are held centred (|r| <= 256, exact in BF16); a chunk of KC = 256 terms
+//     sums to less than 2^24, so the FP32 accumulators hold exact integers whatever the
+//     signs; each chunk is reduced modulo p while the next one runs;
+//   - T / P (P the product of the moduli) is the fractional part of sum_p s_p w_p with
+//     s_p = u + v or u - v and w_p a 96-bit constant, so the reconstruction is a sum of
+//     small times wide integers that wraps by itself, one 64 x 64 product by P and one
+//     rounding. Error of a result before that rounding: 2^-bits max|A row| max|B column|
+//     per term, from the rounding of the operands alone.
+//
+// Why: the FP64 units of this part do two FMAs per SM and cycle (1.0 TF/s measured for
+// the DMMA kernel, zgemm_f64.cu); 28 BF16 products at the tensor cores' rate are some 40
+// times faster. Rows that hold an infinity or NaN, or numbers near the ends of the FP64
+// range, are multiplied entry by entry in FP64 by the reconstruction kernel.
+#include "rns.cuh"
+#include "mpo_stage.cuh"
+#include <cuda.h>
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <mutex>
+
+namespace ptn {
+
+void note_launches(int n);
+
+namespace {
+
+typedef __nv_bfloat16 bf16;
+typedef unsigned long long u64;
+typedef unsigned __int128 u128;
+
+// ------------------------------------------------------------------ constants
+constexpr int NMOD = RNS_FP64;
+constexpr int MOD[NMOD] = {509, 505, 493, 481, 461, 457, 449, 433, 421, 409, 401, 397, 389, 373};
+constexpr int PIECES = 5, PBITS = 11;     // |T| < 2^55 in five 11-bit pieces
+constexpr int MAX_BITS = 54;
+constexpr int KC = 256;                   // terms per exact FP32 sum: 256 * 255^2 < 2^24
+static_assert((long)KC * 255 * 255 < (1L << 24), "chunk sums are exact in FP32");
+
+constexpr int mod_pos(long a, int p) { return (int)(((a % p) + p) % p); }
+constexpr int mod_centred(long a, int p) {
+  const int r = mod_pos(a, p);
+  return r > p / 2 ? r - p : r;
+}
+constexpr int mod_inv(long a, int p) {
+  for (int x = 1; x < p; ++x)
+    if (mod_pos(a, p) * (long)x % p == 1) return x;
+  return 0;
+}
+constexpr int sqrt_minus_one(int p) {
+  for (long x = 1; x < p; ++x)
+    if (x * x % p == p - 1) return (int)x;
+  return 0;
+}
+
+template <int NM>
+struct RnsConst {
+  float p[NM], inv[NM];
+  float cx[NM][PIECES], cy[NM][PIECES];   // 2^(11 i) and j 2^(11 i) modulo p, centred
+  unsigned wx[NM][3], wy[NM][3];          // 2^96 w_p of the real / imaginary part, low first
+  u64 off_x_hi, off_y_hi;                 // 512 sum_p w_p modulo 1 (64 + 32 bits)
+  unsigned off_x_lo, off_y_lo;
+  u64 pm;                                 // P, top 64 bits
+  int pe;                                 // floor(log2 P)
+};
+
+template <int NM>
+constexpr RnsConst<NM> make_const() {
+  RnsConst<NM> c{};
+  u128 P = 1;
+  for (int i = 0; i < NM; ++i) P *= (u128)MOD[i];
+  u128 ox = 0, oy = 0;
+  for (int i = 0; i < NM; ++i) {
+    const int p = MOD[i];
+    const int j = sqrt_minus_one(p);
+    c.p[i] = (float)p;
+    c.inv[i] = 1.0f / (float)p;
+    long pw = 1;
+    for (int q = 0; q < PIECES; ++q) {
+      c.cx[i][q] = (float)mod_centred(pw, p);
+      c.cy[i][q] = (float)mod_centred(pw * j, p);
+      pw = (pw << PBITS) % p;
+    }
+    const int m = mod_inv((long)((P / (u128)p) % (u128)p), p);   // (P / p)^-1 modulo p
+    const long ax = (long)m * mod_inv(2, p) % p, ay = (long)m * mod_inv(2L * j, p) % p;
+    const u128 w0 = ((u128)ax << 96) / (u128)p, w1 = ((u128)ay << 96) / (u128)p;
+    for (int q = 0; q < 3; ++q) {
+      c.wx[i][q] = (unsigned)(w0 >> (32 * q));
+      c.wy[i][q] = (unsigned)(w1 >> (32 * q));
+    }
+    ox += 512 * w0;
+    oy += 512 * w1;
+  }
+  c.off_x_lo = (unsigned)ox;
+  c.off_x_hi = (u64)(ox >> 32);
+  c.off_y_lo = (unsigned)oy;
+  c.off_y_hi = (u64)(oy >> 32);
+  int e = 0;
+  while ((P >> (e + 1)) != 0) ++e;
+  c.pe = e;
+  c.pm = (u64)(e >= 63 ? P >> (e - 63) : P << (63 - e));
+  return c;
+}
+
+constexpr bool moduli_ok() {
+  for (int i = 0; i < NMOD; ++i) {
+    if (sqrt_minus_one(MOD[i]) == 0 || MOD[i] % 2 == 0) return false;
+    for (int k = 0; k < i; ++k) {
+      int a = MOD[i], b = MOD[k];
+      while (b != 0) {
+        const int t = a % b;
+        a = b;
+        b = t;
+      }
+      if (a != 1) return false;
+    }
+  }
+  return true;
+}
+static_assert(moduli_ok(), "moduli: odd, pairwise coprime, -1 a square");
+
+__constant__ RnsConst<RNS_FP64> c_fp64 = make_const<RNS_FP64>();
+__constant__ RnsConst<RNS_MIXED> c_mixed = make_const<RNS_MIXED>();
+
+template <int NM>
+__device__ __forceinline__ const RnsConst<NM>& rns_const() {
+  if constexpr (NM == RNS_FP64) return c_fp64;
+  else return c_mixed;
+}
+
+constexpr float MAGIC = 12582912.0f;   // 1.5 2^23: adding it rounds to an integer
+
+// v modulo p, centred, for an integer |v| <= 2^24 (off centre by one at most)
+__device__ __forceinline__ float reduce_mod(float v, float p, float inv) {
+  const float q = fmaf(v, inv, MAGIC) - MAGIC;
+  return fmaf(-q, p, v);
+}
+
+__device__ __forceinline__ int biased_exp(double x) {
+  const long long b = __double_as_longlong(x);
+  const int E = (int)((b >> 52) & 0x7FF);
+  return E != 0 ? E : ((b << 1) != 0 ? 1 : 0);   // subnormals count as exponent 1
+}
+
+// rows whose products are formed in FP64 entry by entry: infinities, NaNs, numbers so
+// small that entries of the row or products may be subnormal
+constexpr int EXP_TINY = 200;
+__device__ __forceinline__ bool special(int E) { return E == 2047 || (E != 0 && E < EXP_TINY); }
+
+// ------------------------------------------------------------------ conversion
+constexpr int TR = 32, TK = 64;        // conversion tile: rows x terms
+constexpr int TP = TK + 1;
+
+// tile of the view in shared memory; threads (32, 8), coalesced along the unit stride
+__device__ __forceinline__ void load_tile(double2 (*tile)[TP], const RnsView& v, int R, int K,
+                                          int r0, int k0) {
+  const int lane = threadIdx.x, w = threadIdx.y;
+  const double2 zero = make_double2(0.0, 0.0);
+  if (v.sk == 1) {
+    for (int rr = w; rr < TR; rr += 8)
+#pragma unroll
+      for (int h = 0; h < TK; h += 32) {
+        const int r = r0 + rr, k = k0 + h + lane;
+        tile[rr][h + lane] = (r < R && k < K) ? v.src[(long)r * v.sr + k] : zero;
+      }
+  } else {
+    for (int kk = w; kk < TK; kk += 8) {
+      const int r = r0 + lane, k = k0 + kk;
+      tile[lane][kk] = (r < R && k < K) ? v.src[(long)r * v.sr + (long)k * v.sk] : zero;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) k_row_exp(const RnsView v, int R, int K, int* __restrict__ e,
+                                                 const int* skip) {
+  if (skip != nullptr && *skip != 0) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2 (*tile)[TP] = reinterpret_cast<double2 (*)[TP]>(smem_raw);
+  const int r0 = blockIdx.x * TR, k0 = blockIdx.y * TK;
+  load_tile(tile, v, R, K, r0, k0);
+  __syncthreads();
+  for (int rr = threadIdx.y; rr < TR; rr += 8) {
+    int m = 0;
+#pragma unroll
+    for (int h = 0; h < TK; h += 32) {
+      const double2 z = tile[rr][h + threadIdx.x];
+      m = max(m, max(biased_exp(z.x), biased_exp(z.y)));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (threadIdx.x == 0 && r0 + rr < R && m > 0) atomicMax(&e[r0 + rr], m);
+  }
+}
+
+// pieces of T = round(x 2^(bits - e)), |x| < 2^e = 2^(E - 1022), as signed floats
+__device__ __forceinline__ void pieces_of(double x, int E, int bits, float (&f)[PIECES]) {
+  const long long b = __double_as_longlong(x);
+  const int Ex = (int)((b >> 52) & 0x7FF);
+  u64 T = 0;
+  if (Ex != 0) {
+    const u64 mant = ((u64)b & ((1ULL << 52) - 1)) | (1ULL << 52);
+    const int rs = E - Ex + 53 - bits;
+    if (rs <= 0) T = mant << (-rs);
+    else if (rs < 55) T = (mant + (1ULL << (rs - 1))) >> rs;
+  }
+  const unsigned sign = (unsigned)((u64)b >> 32) & 0x80000000u;
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const unsigned q = (unsigned)(T >> (PBITS * i)) & ((1u << PBITS) - 1u);
+    const float g = __uint_as_float(q | 0x4B000000u) - 8388608.0f;
+    f[i] = __uint_as_float(__float_as_uint(g) ^ sign);
+  }
+}
+
+// Residues of two neighbouring terms in all planes. 18 FP32 operations per term and
+// modulus: x and y as five pieces times small constants, two reductions.
+template <int NM>
+__device__ __forceinline__ void convert_pair(const double2 (&z)[2], int E, int bits,
+                                             bf16* __restrict__ row, long plane) {
+  const RnsConst<NM>& c = rns_const<NM>();
+  float px[2][PIECES], py[2][PIECES];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    pieces_of(z[q].x, E, bits, px[q]);
+    pieces_of(z[q].y, E, bits, py[q]);
+  }
+#pragma unroll
+  for (int i = 0; i < NM; ++i) {
+    const float p = c.p[i], inv = c.inv[i];
+    float u[2], w[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      float sx = px[q][0], sy = py[q][0] * c.cy[i][0];
+#pragma unroll
+      for (int t = 1; t < PIECES; ++t) {
+        sx = fmaf(px[q][t], c.cx[i][t], sx);
+        sy = fmaf(py[q][t], c.cy[i][t], sy);
+      }
+      u[q] = reduce_mod(sx + sy, p, inv);
+      w[q] = reduce_mod(sx - sy, p, inv);
+    }
+    *reinterpret_cast<__nv_bfloat162*>(row + (2L * i) * plane) = __floats2bfloat162_rn(u[0], u[1]);
+    *reinterpret_cast<__nv_bfloat162*>(row + (2L * i + 1) * plane) =
+        __floats2bfloat162_rn(w[0], w[1]);
+  }
+}
+
+// Residue planes of a tile of any view (row exponents known). Bound: the FP32 pipe, then
+// the writes (4 nm bytes per entry). A lane holds two neighbouring terms, so a warp writes
+// 128 contiguous bytes per plane and row.
+template <int NM>
+__global__ void __launch_bounds__(256) k_convert(const RnsView v, int R, int K,
+                                                 const int* __restrict__ e, int bits,
+                                                 bf16* __restrict__ dst, long Kp, long plane,
+                                                 const int* skip) {
+  if (skip != nullptr && *skip != 0) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2 (*tile)[TP] = reinterpret_cast<double2 (*)[TP]>(smem_raw);
+  const int r0 = blockIdx.x * TR, k0 = blockIdx.y * TK;
+  load_tile(tile, v, R, K, r0, k0);
+  __syncthreads();
+  const int k = k0 + 2 * threadIdx.x;
+  if (k >= Kp) return;
+  for (int rr = threadIdx.y; rr < TR; rr += 8) {
+    const int r = r0 + rr;
+    if (r >= R) break;
+    const int E = e[r];
+    const bool live = E != 0 && !special(E);
+    double2 z[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      z[q] = live ? tile[rr][2 * threadIdx.x + q] : make_double2(0.0, 0.0);
+      if (v.conj) z[q].y = -z[q].y;
+    }
+    convert_pair<NM>(z, E, bits, dst + (long)r * Kp + k, plane);
+  }
+}
+
+// Views with contiguous rows: one warp finds the exponent of its row and converts it (the
+// second read hits L1 / L2): one launch instead of a memset, a maximum pass and a
+// conversion. Also zeroes clear[0 .. nclear) for a later kernel of the stream.
+template <int NM>
+__global__ void __launch_bounds__(128) k_convert_rows(const RnsView v, int R, int K,
+                                                      int* __restrict__ e, int bits,
+                                                      bf16* __restrict__ dst, long Kp, long plane,
+                                                      int* __restrict__ clear, int nclear,
+                                                      const int* skip) {
+  if (skip != nullptr && *skip != 0) return;
+  for (int i = blockIdx.x * 128 + threadIdx.x; i < nclear; i += gridDim.x * 128) clear[i] = 0;
+  const int lane = threadIdx.x & 31;
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (r >= R) return;
+  const double2* src = v.src + (long)r * v.sr;
+  int E = 0;
+  for (int k = lane; k < K; k += 32) {
+    const double2 z = src[k];
+    E = max(E, max(biased_exp(z.x), biased_exp(z.y)));
+  }
+  E = __reduce_max_sync(0xffffffffu, E);
+  if (lane == 0) e[r] = E;
+  const bool live = E != 0 && !special(E);
+  for (int k = 2 * lane; k < Kp; k += 64) {
+    double2 z[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      z[q] = (live && k + q < K) ? src[k + q] : make_double2(0.0, 0.0);
+      if (v.conj) z[q].y = -z[q].y;
+    }
+    convert_pair<NM>(z, E, bits, dst + (long)r * Kp + k, plane);
+  }
+}
+
+// ------------------------------------------------------------------ GEMM
+constexpr int BM = 128, BK = 64;
+constexpr int A_STAGE = BM * BK * 2;
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 64 + 32 * EPI_WARPS;
+constexpr long WAIT_LIMIT = 1L << 22;
+constexpr int KB_CHUNK = KC / BK;
+
+template <int BN>
+struct Tile {
+  static constexpr int B_STAGE = BN * BK * 2;
+  static constexpr int STAGE = A_STAGE + B_STAGE;
+  static constexpr int STAGES = BN == 256 ? 4 : 6;
+  static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+  static constexpr int TMEM = 2 * BN;       // two accumulators (a power of two)
+  static constexpr int COLS = BN / 2;       // columns per epilogue warp
+  // kind::f16 instruction descriptor: FP32 accumulate (bit 4), A and B BF16 (bits 7, 10),
+  // both K-major, N >> 3 at bit 17, M >> 4 at bit 24
+  static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) |
+                                    ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+  static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+__device__ __forceinline__ void mbar_init(u64* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect_tx(u64* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
+               "r"(bytes)
+               : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(u64* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// bounded wait on the phase with parity `parity` that also gives up once another role
+// raised the CTA's abort flag (null: none); false on expiry
+__device__ __forceinline__ bool mbar_wait(u64* bar, uint32_t parity, const int* abort_flag) {
+  const uint32_t a = smem_u32(bar);
+  for (long it = 0; it < WAIT_LIMIT; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(a), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (abort_flag != nullptr && *(volatile const int*)abort_flag) return false;
+  }
+  return false;
+}
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* tm, int x, int y, int z,
+                                            u64* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// shared-memory matrix descriptor: K-major, 128-byte swizzle (layout type 2), 8-row
+// groups 1024 B apart
+__device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
+  uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
+__device__ __forceinline__ void umma(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc,
+                                     uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+      "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+      : "memory");
+}
+
+__device__ __forceinline__ void umma_commit(u64* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                   smem_u32(bar))
+               : "memory");
+}
+
+// 32 lanes x 16 columns of tensor memory
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15},"
+      " [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+}
+
+__device__ __forceinline__ void tmem_wait_ld() {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// keeps every use of v after the preceding tcgen05.wait::ld
+template <int N>
+__device__ __forceinline__ void after_wait(uint32_t (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(v[i]));
+}
+
+struct GemmP {
+  int M, N;
+  int nkb;                   // K blocks of BK
+  int gx, gy, units;         // N tiles, M tiles, tiles over all planes
+  unsigned short* res;       // residues + 256: [plane][M][ldr]
+  long ldr, rplane;
+  int* err;
+  const int* skip;
+};
+
+// All 2 nm real GEMMs in one launch. A persistent CTA walks the tiles u = blockIdx.x,
+// + gridDim.x, ... (N tile fastest, then M tile, then plane). Warp 0 lane 0 issues TMA
+// (a ring of STAGES K blocks), warp 1 lane 0 tcgen05.mma; a chunk of KC terms fills one of
+// two accumulators in tensor memory while warps 2..9 (warp w: lanes 32 (w % 4).., half of
+// the columns) read the other one, reduce it modulo p and add it up in registers, so the
+// drain of a chunk hides behind the next chunk's MMAs, across tiles too. Every wait is
+// bounded: on expiry an error code is set, the copies in flight land and TMEM is freed.
+template <int BN>
+__global__ void __launch_bounds__(THREADS, 1)
+    k_rns_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+               const GemmP g) {
+  if (g.skip != nullptr && *g.skip != 0) return;   // uniform: before any barrier or allocation
+  typedef Tile<BN> T;
+  extern __shared__ uint8_t smem_raw8[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw8) + 1023) &
+                                             ~uintptr_t(1023));
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + T::STAGES * A_STAGE;
+  u64* full = reinterpret_cast<u64*>(smem + T::STAGES * T::STAGE);
+  u64* empty = full + T::STAGES;
+  u64* tfull = empty + T::STAGES;    // [2] a chunk's accumulator is complete
+  u64* tempty = tfull + 2;           // [2] the epilogue has read it
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(tempty + 2);
+  int* abort_flag = reinterpret_cast<int*>(tslot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nch = (g.nkb + KB_CHUNK - 1) / KB_CHUNK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < T::STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tfull[b], 1);
+      mbar_init(&tempty[b], EPI_WARPS);
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tslot)),
+                 "r"(T::TMEM)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tslot;
+
+  if (warp == 0 && lane == 0) {
+    // ---------------- TMA producer
+    int i = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
+      const int n0 = (u % g.gx) * BN, m0 = ((u / g.gx) % g.gy) * BM, pl = u / (g.gx * g.gy);
+      for (int kb = 0; kb < g.nkb; ++kb, ++i) {
+        const int s = i % T::STAGES;
+        if (i >= T::STAGES && !mbar_wait(&empty[s], ((uint32_t)(i / T::STAGES) & 1u) ^ 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        mbar_expect_tx(&full[s], T::STAGE);
+        tma_load_3d(sA + s * A_STAGE, &tmA, kb * BK, m0, pl, &full[s]);
+        tma_load_3d(sB + s * T::B_STAGE, &tmB, kb * BK, n0, pl, &full[s]);
+      }
+    }
+    if (!ok) {
+      atomicExch(g.err, 1);
+      *(volatile int*)abort_flag = 1;
+      // let the copies still in flight land before the CTA retires (bounded)
+      for (int q = max(0, i - T::STAGES); q < i; ++q)
+        mbar_wait(&full[q % T::STAGES], (uint32_t)(q / T::STAGES) & 1u, nullptr);
+    }
+  } else if (warp == 1 && lane == 0) {
+    // ---------------- MMA issuer
+    int i = 0, ch = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
+      for (int kb = 0; kb < g.nkb; ++kb, ++i) {
+        const int kin = kb % KB_CHUNK;
+        const int b = ch & 1;
+        if (kin == 0 && ch >= 2) {
+          if (!mbar_wait(&tempty[b], ((uint32_t)(ch >> 1) & 1u) ^ 1u, abort_flag)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        const int s = i % T::STAGES;
+        if (!mbar_wait(&full[s], (uint32_t)(i / T::STAGES) & 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a0 = smem_u32(sA + s * A_STAGE), b0 = smem_u32(sB + s * T::B_STAGE);
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          umma(tmem + (uint32_t)(b * BN), sdesc(a0 + k * 32), sdesc(b0 + k * 32), T::IDESC,
+               (kin == 0 && k == 0) ? 0u : 1u);
+        umma_commit(&empty[s]);
+        if (kin == KB_CHUNK - 1 || kb == g.nkb - 1) {
+          umma_commit(&tfull[b]);
+          ++ch;
+        }
+      }
+    }
+    if (!ok) {
+      atomicExch(g.err, 2);
+      *(volatile int*)abort_flag = 1;
+    }
+    // every MMA issued is complete before the CTA may free its tensor memory: the last
+    // stage commits are waited for here (bounded)
+    for (int q = max(0, i - T::STAGES); q < i; ++q)
+      mbar_wait(&empty[q % T::STAGES], (uint32_t)(q / T::STAGES) & 1u, nullptr);
+  } else if (warp >= 2) {
+    // ---------------- epilogue
+    const int quad = warp & 3, half = (warp - 2) >> 2;
+    const uint32_t tl = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(half * T::COLS);
+    int ch = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
+      const int n0 = (u % g.gx) * BN + half * T::COLS, pl = u / (g.gx * g.gy);
+      const int row = ((u / g.gx) % g.gy) * BM + 32 * quad + lane;
+      const float p = c_fp64.p[pl >> 1], inv = c_fp64.inv[pl >> 1];
+      float acc[T::COLS];
+      for (int c = 0; c < nch; ++c, ++ch) {
+        const int b = ch & 1;
+        if (!mbar_wait(&tfull[b], (uint32_t)(ch >> 1) & 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int c0 = 0; c0 < T::COLS; c0 += 16) {
+          uint32_t v[16];
+          __syncwarp();
+          tmem_ld16(tl + (uint32_t)(b * BN + c0), v);
+          tmem_wait_ld();
+          after_wait(v);
+          if (c0 + 16 == T::COLS) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[b]);
+          }
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float r = reduce_mod(__uint_as_float(v[j]), p, inv);
+            acc[c0 + j] = c == 0 ? r : acc[c0 + j] + r;
+          }
+        }
+      }
+      if (!ok) break;
+      if (row < g.M) {
+        unsigned short* dst = g.res + (long)pl * g.rplane + (long)row * g.ldr + n0;
+#pragma unroll
+        for (int c0 = 0; c0 < T::COLS; c0 += 8) {
+          if (n0 + c0 >= g.N) break;
+          unsigned q[4];
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) {
+            float r0 = acc[c0 + j], r1 = acc[c0 + j + 1];
+            if (nch > 1) {
+              r0 = reduce_mod(r0, p, inv);
+              r1 = reduce_mod(r1, p, inv);
+            }
+            // the low half of the magic sum's bits is the residue + 256
+            q[j >> 1] = __byte_perm(__float_as_uint(r0 + (MAGIC + 256.0f)),
+                                    __float_as_uint(r1 + (MAGIC + 256.0f)), 0x5410);
+          }
+          *reinterpret_cast<uint4*>(dst + c0) = make_uint4(q[0], q[1], q[2], q[3]);
+        }
+      }
+    }
+    if (!ok && !*(volatile int*)abort_flag) {
+      atomicExch(g.err, 3);
+      *(volatile int*)abort_flag = 1;
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::TMEM)
+                 : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ reconstruction
+// |F| P 2^sh as FP64 for the signed 96-bit fraction F = hi 2^-64 + lo 2^-96 of P; ok is
+// cleared when the result leaves the normal range. Integer arithmetic: an FP64 operation
+// costs this part as much as 64 integer ones.
+__device__ __forceinline__ double finish(u64 hi, unsigned lo, u64 pm, int pe, int sh, bool& ok) {
+  const u64 sign = hi & (1ULL << 63);
+  if (sign) {
+    lo = 0u - lo;
+    hi = ~hi + (lo == 0u ? 1ULL : 0ULL);
+  }
+  if (hi == 0) {
+    if (lo == 0) return 0.0;
+    hi = (u64)lo << 32;
+    lo = 0;
+    sh -= 64;
+  }
+  const int lz = __clzll((long long)hi);
+  u64 m = hi << lz;
+  if (lz > 0) m |= ((u64)lo << 32) >> (64 - lz);
+  u64 q = __umul64hi(m, pm);
+  int x = pe + 1023 - lz + sh;      // biased exponent when q has its top bit set
+  if (!(q >> 63)) {
+    q <<= 1;
+    --x;
+  }
+  const u64 r = (q >> 11) + ((q >> 10) & 1ULL);
+  if (x < 1 || x > 2045) {
+    ok = false;
+    return 0.0;
+  }
+  return __longlong_as_double((long long)(sign | (((u64)x << 52) + (r - (1ULL << 52)))));
+}
+
+struct ReconP {
+  int M, N, K;
+  const unsigned short* res;
+  long ldr, rplane;
+  const int *ea, *eb;
+  int sh0;                // -2 bits - 2 * 1022
+  RnsView va, vb;
+  const int* skip;
+};
+
+__device__ __noinline__ double2 direct_product(const RnsView& va, const RnsView& vb, int K, int m,
+                                               int n) {
+  double2 s = make_double2(0.0, 0.0);
+  for (int k = 0; k < K; ++k) {
+    double2 a = va.src[(long)m * va.sr + (long)k * va.sk];
+    double2 b = vb.src[(long)n * vb.sr + (long)k * vb.sk];
+    if (va.conj) a.y = -a.y;
+    if (vb.conj) b.y = -b.y;
+    s = cfma(a, b, s);
+  }
+  return s;
+}
+
+
+// the 2 NM residues of elements n and n + 1 of a row, packed (low half first); second =
+// false: of n alone. 32-bit loads where n is even.
+template <int NM>
+__device__ __forceinline__ void load_residues(const unsigned short* __restrict__ src, long rplane,
+                                              bool second, unsigned (&ru)[NM], unsigned (&rv)[NM]) {
+  if ((reinterpret_cast<uintptr_t>(src) & 3) == 0) {   // the leading dimension is even
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+      ru[i] = *reinterpret_cast<const unsigned*>(src + (2L * i) * rplane);
+      rv[i] = *reinterpret_cast<const unsigned*>(src + (2L * i + 1) * rplane);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+      const unsigned short* a = src + (2L * i) * rplane;
+      const unsigned short* b = a + rplane;
+      ru[i] = a[0] | (second ? (unsigned)a[1] << 16 : 0u);
+      rv[i] = b[0] | (second ? (unsigned)b[1] << 16 : 0u);
+    }
+  }
+}
+
+// element (m, n) of the product from its residues (low or high half: q = 0 or 1)
+template <int NM>
+__device__ __forceinline__ double2 element(const ReconP& g, int m, int n, int q,
+                                           const unsigned (&ru)[NM], const unsigned (&rv)[NM]) {
+  const RnsConst<NM>& c = rns_const<NM>();
+  const int Ea = g.ea[m], Eb = g.eb[n];
+  u64 x0 = 0, x1 = 0, y0 = 0, y1 = 0;
+  unsigned x2 = 0, y2 = 0;
+#pragma unroll
+  for (int i = 0; i < NM; ++i) {
+    const unsigned u = q ? ru[i] >> 16 : ru[i] & 0xFFFFu, v = q ? rv[i] >> 16 : rv[i] & 0xFFFFu;
+    const unsigned s = u + v, d = u - v + 512u;
+    x0 += (u64)s * c.wx[i][0];
+    x1 += (u64)s * c.wx[i][1];
+    x2 += s * c.wx[i][2];
+    y0 += (u64)d * c.wy[i][0];
+    y1 += (u64)d * c.wy[i][1];
+    y2 += d * c.wy[i][2];
+  }
+  x1 += x0 >> 32;
+  y1 += y0 >> 32;
+  const unsigned xl = (unsigned)x0, yl = (unsigned)y0;
+  u64 xh = x1 + ((u64)x2 << 32), yh = y1 + ((u64)y2 << 32);
+  xh -= c.off_x_hi + (xl < c.off_x_lo ? 1ULL : 0ULL);
+  yh -= c.off_y_hi + (yl < c.off_y_lo ? 1ULL : 0ULL);
+  bool ok = !special(Ea) && !special(Eb);
+  double2 z = make_double2(0.0, 0.0);
+  if (ok && Ea != 0 && Eb != 0) {
+    const int sh = Ea + Eb + g.sh0;
+    z.x = finish(xh, xl - c.off_x_lo, c.pm, c.pe, sh, ok);
+    z.y = finish(yh, yl - c.off_y_lo, c.pm, c.pe, sh, ok);
+  }
+  if (!ok) z = direct_product(g.va, g.vb, g.K, m, n);
+  return z;
+}
+
+// alpha z; alpha = 1 matters to infinities and NaNs alone (0 * inf), as in the DMMA kernel
+__device__ __forceinline__ double2 scaled(double2 alpha, double2 z) {
+  const bool one = alpha.x == 1.0 && alpha.y == 0.0;
+  if (one && biased_exp(z.x) != 2047 && biased_exp(z.y) != 2047) return z;
+  return cmul(alpha, z);
+}
+
+// Bound: the integer pipe (about 10 operations per residue pair), then reading 4 nm bytes
+// of residues per element, from L2 where the product fits it.
+template <int NM>
+__global__ void __launch_bounds__(256) k_reconstruct(const ReconP g, double2 alpha, double2 beta,
+                                                     double2* __restrict__ out, long ldc) {
+  if (g.skip != nullptr && *g.skip != 0) return;
+  const int np = (g.N + 1) >> 1;
+  const long total = (long)g.M * np;
+  for (long idx = blockIdx.x * 256L + threadIdx.x; idx < total; idx += gridDim.x * 256L) {
+    const int m = (int)(idx / np), n = 2 * (int)(idx % np);
+    unsigned ru[NM], rv[NM];
+    load_residues<NM>(g.res + (long)m * g.ldr + n, g.rplane, n + 1 < g.N, ru, rv);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (n + q >= g.N) break;
+      double2 z = element<NM>(g, m, n + q, q, ru, rv);
+      double2* o = out + (long)m * ldc + n + q;
+      z = scaled(alpha, z);
+      if (beta.x != 0.0 || beta.y != 0.0) z = cadd(z, cmul(beta, *o));
+      *o = z;
+    }
+  }
+}
+
+// Reconstruction fused with the MPO stage (mpo_stage.cuh): the product's element
+// ((x, p / pin), (p % pin, y)) is stage input (x, p, y), put together straight into the
+// shared-memory rows of the stage; the stage output goes to `out` and the exponents of the
+// rows it forms as the next operand to e2 (zeroed before). by_x false: rows (q % eq, y);
+// true: rows (x, q / eq). One CTA per (x, 128-wide y chunk). Saves writing and reading the
+// product in FP64 and a maximum pass over the stage output.
+template <int NM>
+__global__ void __launch_bounds__(128)
+    k_reconstruct_stage(const ReconP g, const double2* __restrict__ w, long ldq, long ldp, int P,
+                        int pin, int Q, int Y, double2* __restrict__ out, int* __restrict__ e2,
+                        int eq, int by_x) {
+  if (g.skip != nullptr && *g.skip != 0) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* sin = reinterpret_cast<double2*>(smem_raw);
+  double2* sval = sin + (size_t)P * STAGE_Y;
+  int* sidx = reinterpret_cast<int*>(sval + (size_t)P * Q);
+  __shared__ int scount[STAGE_MAX];
+  const int x = blockIdx.y, y0 = blockIdx.x * STAGE_Y, ty = threadIdx.x;
+  stage_load_w(w, ldq, ldp, P, Q, sval);
+  const int pair = 2 * (ty & 63);
+  for (int p = ty >> 6; p < P; p += 2) {
+    const int y = y0 + pair;
+    if (y < Y) {
+      const int m = x * (P / pin) + p / pin, n = (p % pin) * Y + y;
+      unsigned ru[NM], rv[NM];
+      load_residues<NM>(g.res + (long)m * g.ldr + n, g.rplane, y + 1 < Y, ru, rv);
+      const double2 one = make_double2(1.0, 0.0);
+      sin[p * STAGE_Y + pair] = scaled(one, element<NM>(g, m, n, 0, ru, rv));
+      if (y + 1 < Y)
+        sin[p * STAGE_Y + pair + 1] = scaled(one, element<NM>(g, m, n + 1, 1, ru, rv));
+    }
+  }
+  __syncthreads();
+  stage_compact(P, Q, sval, sidx, scount);
+  __syncthreads();
+  const int y = y0 + ty;
+  const int na = by_x ? Q / eq : eq, nb = by_x ? eq : Q / eq;
+  for (int a = 0; a < na; ++a) {
+    int E = 0;
+    if (y < Y)
+      for (int b = 0; b < nb; ++b) {
+        const int q = by_x ? a * eq + b : b * eq + a;
+        const double2 z = stage_row(q, P, sin + ty, sval, sidx, scount);
+        out[((long)x * Q + q) * Y + y] = z;
+        E = max(E, max(biased_exp(z.x), biased_exp(z.y)));
+      }
+    if (by_x) {
+      E = __reduce_max_sync(0xffffffffu, E);
+      if ((ty & 31) == 0 && E > 0) atomicMax(&e2[x * na + a], E);
+    } else if (E > 0) {
+      int* dst = e2 + (long)a * Y + y;
+      if (*(volatile int*)dst < E) atomicMax(dst, E);
+    }
+  }
+}
+
+// ------------------------------------------------------------------ tensor maps
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
+                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_fn() {
+  static EncodeTiledFn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault,
+                                         &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<EncodeTiledFn>(f);
+  });
+  return fn;
+}
+
+// map over the planes [2 nm][rows][Kp] of logical extent (kc, rows, 2 nm), box (BK,
+// box_rows, 1): terms beyond kc and rows beyond the last read as zero
+bool make_map(CUtensorMap* out, const RnsOperand& o, int box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)o.kc, (cuuint64_t)o.rows, (cuuint64_t)(2 * o.nm)};
+  cuuint64_t strides[2] = {(cuuint64_t)o.Kp * 2, (cuuint64_t)o.plane() * 2};
+  cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, o.p, dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// sticky error code of the kernels (bounded waits that expired)
+__device__ int g_rns_err;
+
+int* err_flag() {
+  static int* flag = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* a = nullptr;
+    if (cudaGetSymbolAddress(&a, g_rns_err) == cudaSuccess) flag = static_cast<int*>(a);
+  });
+  return flag;
+}
+
+long residue_ld(long N) { return (N + 7) / 8 * 8; }
+
+template <int BN>
+ptn_status launch_gemm(const RnsOperand& A, const RnsOperand& B, GemmP g, cudaStream_t st) {
+  CUtensorMap ma, mb;
+  if (!make_map(&ma, A, BM) || !make_map(&mb, B, BN)) {
+    set_error("rns_gemm: cuTensorMapEncodeTiled failed");
+    return PTN_CUDA_ERROR;
+  }
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(k_rns_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                Tile<BN>::SMEM);
+  });
+  PTN_CUDA_TRY(attr);
+  g.gx = (g.N + BN - 1) / BN;
+  g.gy = (g.M + BM - 1) / BM;
+  const long units = (long)g.gx * g.gy * 2 * A.nm;
+  PTN_CHECK_ARG(units <= INT_MAX / 2, "rns_gemm: too many tiles");
+  g.units = (int)units;
+  const int grid = (int)std::min<long>(units, num_sms());
+  k_rns_gemm<BN><<<grid, THREADS, Tile<BN>::SMEM, st>>>(ma, mb, g);
+  PTN_LAUNCH_CHECK();
+  return PTN_OK;
+}
+
+// cycles of a launch with N tiles of bn columns: whole turns of the SMs, the MMAs of a tile
+// (half a cycle per column and 16 terms, at least what reading the operands from shared
+// memory takes) and a fixed cost per tile
+double tile_cost(int bn, long M, long N, long K, int planes) {
+  const long units = ((N + bn - 1) / bn) * ((M + BM - 1) / BM) * planes;
+  const long turns = (units + num_sms() - 1) / num_sms();
+  const double k16 = (double)((K + 15) / 16);
+  return turns * (k16 * std::max(bn / 2.0, 32.0 + bn / 4.0) + 300.0 + bn);
+}
+
+constexpr double plog2(int nm) {
+  double s = 1.0;   // log2 of the product, by halving
+  double l = 0.0;
+  for (int i = 0; i < nm; ++i) {
+    s *= MOD[i];
+    while (s >= 2.0) {
+      s *= 0.5;
+      l += 1.0;
+    }
+  }
+  return l;         // floor(log2 P)
+}
+
+}  // namespace
+
+size_t rns_plane_bytes(long rows, long kc, int nm) {
+  return (size_t)(2 * nm) * rows * ((kc + 7) / 8 * 8) * sizeof(bf16);
+}
+
+size_t rns_out_bytes(long M, long N, int nm) {
+  return (size_t)(2 * nm) * M * residue_ld(N) * sizeof(unsigned short);
+}
+
+RnsOperand rns_operand(void* planes, void* exps, long rows, long kc, int nm) {
+  RnsOperand o;
+  o.p = static_cast<bf16*>(planes);
+  o.e = static_cast<int*>(exps);
+  o.rows = (int)rows;
+  o.kc = (int)kc;
+  o.nm = nm;
+  o.Kp = (kc + 7) / 8 * 8;
+  return o;
+}
+
+// |sum of K terms| <= K 2^(2 bits + 1) has to stay below 0.49 P; 0.49 P > 2^(floor(log2 P) - 2)
+int rns_bits(long K, int nm) {
+  int lk = 0;
+  while ((1L << lk) < K) ++lk;
+  const int room = (int)plog2(nm) - 2 - 1 - lk;
+  const int bits = std::min(MAX_BITS, room / 2);
+  return bits >= (nm == RNS_FP64 ? 53 : 39) ? bits : 0;
+}
+
+// The fixed cost of the path (conversions, planes, reconstruction: about 33 us for a single
+// GEMM) meets the DMMA kernel's 1 TF/s near 4e6 complex products. Measured, the GEMMs of
+// H_eff at bond D and MPO bond 5 alone (DMMA -> residues):
+//   D = 64: 30.5 us;  80: 50 -> 34;  128: 184 -> 40;  256: 1416 -> 74;  512: 11269 -> 246
+// and a Lanczos step (operands of the operator converted once):
+//   D = 80: 147 -> 86 us;  128: 436 -> 82;  256: 2924 -> 149;  512: 22967 -> 453
+bool rns_wanted(long M, long N, long K) {
+  if (std::min(M, std::min(N, K)) < 32 || M > INT_MAX / 2 || N > INT_MAX / 2) return false;
+  return (double)M * N * K >= 4.0e6 && rns_bits(K, RNS_FP64) != 0;
+}
+
+template <int NM>
+static void launch_convert(const RnsView& v, const RnsOperand& d, int bits, bool rows, dim3 grid,
+                           int smem, int* clear, int nclear, const int* skip, cudaStream_t st) {
+  if (rows)
+    k_convert_rows<NM><<<(d.rows + 3) / 4, 128, 0, st>>>(v, d.rows, d.kc, d.e, bits, d.p, d.Kp,
+                                                         d.plane(), clear, nclear, skip);
+  else
+    k_convert<NM><<<grid, dim3(32, 8), smem, st>>>(v, d.rows, d.kc, d.e, bits, d.p, d.Kp,
+                                                   d.plane(), skip);
+}
+
+ptn_status rns_convert(const RnsView& v, const RnsOperand& d, bool have_exp, const int* skip,
+                       cudaStream_t st, int* clear, int nclear) {
+  const int bits = rns_bits(d.kc, d.nm);
+  PTN_CHECK_ARG(bits != 0, "rns_convert: products of %d terms are too long", d.kc);
+  const dim3 grid((unsigned)((d.rows + TR - 1) / TR), (unsigned)((d.kc + TK - 1) / TK));
+  PTN_CHECK_ARG(grid.y <= 65535, "rns_convert: too many columns");
+  constexpr int smem = TR * TP * sizeof(double2);
+  const bool rows = v.sk == 1 && !have_exp;
+  int launches = 1;
+  if (!rows) {
+    if (nclear > 0) PTN_CUDA_TRY(cudaMemsetAsync(clear, 0, (size_t)nclear * sizeof(int), st));
+    if (!have_exp) {
+      PTN_CUDA_TRY(cudaMemsetAsync(d.e, 0, (size_t)d.rows * sizeof(int), st));
+      k_row_exp<<<grid, dim3(32, 8), smem, st>>>(v, d.rows, d.kc, d.e, skip);
+      ++launches;
+    }
+  }
+  if (d.nm == RNS_FP64) launch_convert<RNS_FP64>(v, d, bits, rows, grid, smem, clear, nclear, skip, st);
+  else launch_convert<RNS_MIXED>(v, d, bits, rows, grid, smem, clear, nclear, skip, st);
+  PTN_LAUNCH_CHECK();
+  note_launches(launches);
+  return PTN_OK;
+}
+
+// the integer products of all planes -> res, and what their reconstruction needs
+static ptn_status multiply(const RnsOperand& A, const RnsView& va, const RnsOperand& B,
+                           const RnsView& vb, void* res, const int* skip, cudaStream_t st,
+                           ReconP* r) {
+  const int M = A.rows, N = B.rows, K = A.kc;
+  PTN_CHECK_ARG(M > 0 && N > 0 && K > 0 && B.kc == K && A.nm == B.nm, "rns_gemm: bad operands");
+  const int bits = rns_bits(K, A.nm);
+  PTN_CHECK_ARG(bits != 0, "rns_gemm: products of %d terms are too long", K);
+  GemmP g;
+  g.M = M;
+  g.N = N;
+  g.nkb = (K + BK - 1) / BK;
+  g.gx = g.gy = g.units = 0;
+  g.res = static_cast<unsigned short*>(res);
+  g.ldr = residue_ld(N);
+  g.rplane = (long)M * g.ldr;
+  g.err = err_flag();
+  g.skip = skip;
+  PTN_CHECK_ARG(g.err != nullptr, "rns_gemm: error flag lookup failed");
+  const int planes = 2 * A.nm;
+  const int prof = prof_begin(st, PROF_TC_GEMM, 8.0 * M * (double)N * K,
+                              2.0 * planes * ((double)M * K + (double)N * K + (double)M * N));
+  const double c64 = tile_cost(64, M, N, K, planes), c128 = tile_cost(128, M, N, K, planes),
+               c256 = tile_cost(256, M, N, K, planes);
+  if (c256 <= c128 && c256 <= c64) PTN_TRY(launch_gemm<256>(A, B, g, st));
+  else if (c128 <= c64) PTN_TRY(launch_gemm<128>(A, B, g, st));
+  else PTN_TRY(launch_gemm<64>(A, B, g, st));
+  prof_end(st, prof);
+  note_launches(1);
+  r->M = M;
+  r->N = N;
+  r->K = K;
+  r->res = g.res;
+  r->ldr = g.ldr;
+  r->rplane = g.rplane;
+  r->ea = A.e;
+  r->eb = B.e;
+  r->sh0 = -2 * bits - 2 * 1022;
+  r->va = va;
+  r->vb = vb;
+  r->skip = skip;
+  return PTN_OK;
+}
+
+ptn_status rns_gemm(const RnsOperand& A, const RnsView& va, const RnsOperand& B, const RnsView& vb,
+                    double2 alpha, double2 beta, double2* out, long ldc, void* res,
+                    const int* skip, cudaStream_t st) {
+  ReconP r;
+  PTN_TRY(multiply(A, va, B, vb, res, skip, st, &r));
+  const long pairs = (long)r.M * ((r.N + 1) / 2);
+  const int blocks = (int)std::min<long>((pairs + 255) / 256, 16L * num_sms());
+  if (A.nm == RNS_FP64) k_reconstruct<RNS_FP64><<<blocks, 256, 0, st>>>(r, alpha, beta, out, ldc);
+  else k_reconstruct<RNS_MIXED><<<blocks, 256, 0, st>>>(r, alpha, beta, out, ldc);
+  PTN_LAUNCH_CHECK();
+  note_launches(1);
+  return PTN_OK;
+}
+
+template <int NM>
+static ptn_status launch_stage(const ReconP& r, const RnsStage& s, cudaStream_t st) {
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(k_reconstruct_stage<NM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)stage_smem(STAGE_MAX, STAGE_MAX));
+  });
+  PTN_CUDA_TRY(attr);
+  const dim3 grid((s.Y + STAGE_Y - 1) / STAGE_Y, s.X);
+  k_reconstruct_stage<NM><<<grid, STAGE_Y, stage_smem(s.P, s.Q), st>>>(
+      r, s.w, s.ldq, s.ldp, s.P, s.pin, s.Q, s.Y, s.out, s.e2, s.eq, s.by_x ? 1 : 0);
+  PTN_LAUNCH_CHECK();
+  note_launches(1);
+  return PTN_OK;
+}
+
+ptn_status rns_gemm_stage(const RnsOperand& A, const RnsView& va, const RnsOperand& B,
+                          const RnsView& vb, const RnsStage& s, void* res, const int* skip,
+                          cudaStream_t st) {
+  PTN_CHECK_ARG(s.P <= STAGE_MAX && s.Q <= STAGE_MAX, "MPO stage: chi*d must be <= 64 (got %d, %d)",
+                s.P, s.Q);
+  PTN_CHECK_ARG(s.X <= 65535, "MPO stage: X too large");
+  ReconP r;
+  PTN_TRY(multiply(A, va, B, vb, res, skip, st, &r));
+  return A.nm == RNS_FP64 ? launch_stage<RNS_FP64>(r, s, st) : launch_stage<RNS_MIXED>(r, s, st);
+}
+
+int rns_error_and_reset() {
+  int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_rns_err, sizeof(int)) != cudaSuccess) return -1;
+  if (v != 0) {
+    const int zero = 0;
+    cudaMemcpyToSymbol(g_rns_err, &zero, sizeof(int));
+  }
+  return v;
+}
+
+}  // namespace ptn

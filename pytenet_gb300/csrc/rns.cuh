@@ -1,0 +1,97 @@
+// Complex GEMM in a residue number system on the tensor cores (kernels: rns.cu): the
+// operand type and the launches the contractions are built from.
+#pragma once
+
+#include "ptn_common.cuh"
+#include <cuda_bf16.h>
+
+namespace ptn {
+
+// moduli of the FP64 form and of the mixed form
+constexpr int RNS_FP64 = 14;
+constexpr int RNS_MIXED = 11;
+
+// element (r, k) of a complex operand: src[r * sr + k * sk], conjugated if `conj`
+struct RnsView {
+  const double2* src;
+  long sr, sk;
+  int conj;
+};
+
+// a complex operand with `rows` rows and kc columns as 2 * nm residue planes
+// [plane][rows][Kp] (BF16, Kp a multiple of 8), and the biased exponent of the largest
+// component of every row (0: no non-zero entry)
+struct RnsOperand {
+  __nv_bfloat16* p;
+  int* e;
+  int rows, kc, nm;
+  long Kp;
+  long plane() const { return (long)rows * Kp; }
+};
+
+// bytes of the planes / exponents / GEMM residues, each to be 256-byte aligned
+size_t rns_plane_bytes(long rows, long kc, int nm);
+size_t rns_out_bytes(long M, long N, int nm);
+RnsOperand rns_operand(void* planes, void* exps, long rows, long kc, int nm);
+
+// bits that a row-scaled value keeps in products of K complex terms, or 0 when K is too
+// long for the precision of the form
+int rns_bits(long K, int nm);
+
+// whether the FP64 form of C (M x N) = A B (K terms) takes the residue planes
+bool rns_wanted(long M, long N, long K);
+
+// view -> residue planes for products over all kc terms. `have_exp`: the row exponents are
+// in d.e already (from rns_gemm_stage). Also zeroes clear[0 .. nclear).
+ptn_status rns_convert(const RnsView& v, const RnsOperand& d, bool have_exp, const int* skip,
+                       cudaStream_t st, int* clear = nullptr, int nclear = 0);
+
+// out[m * ldc + n] = alpha sum_k A[m, k] B[n, k] + beta out[m * ldc + n]; va / vb are the
+// views the operands came from (rows with infinities, NaNs or numbers near the ends of the
+// FP64 range are multiplied from them directly), res the residue buffer
+ptn_status rns_gemm(const RnsOperand& A, const RnsView& va, const RnsOperand& B, const RnsView& vb,
+                    double2 alpha, double2 beta, double2* out, long ldc, void* res,
+                    const int* skip, cudaStream_t st);
+
+// MPO stage on a product: out[x, q, y] = sum_p W[q, p] in[x, p, y] (W at w[q * ldq + p * ldp]),
+// in[x, p, y] = element ((x, p / pin), (p % pin, y)) of the product. e2 (zeroed before) takes
+// the row exponents of the output as an operand with rows (q % eq, y), or (x, q / eq) if by_x.
+struct RnsStage {
+  const double2* w;
+  long ldq, ldp;
+  int X, P, pin, Q, Y;
+  double2* out;
+  int* e2;
+  int eq;
+  bool by_x;
+};
+ptn_status rns_gemm_stage(const RnsOperand& A, const RnsView& va, const RnsOperand& B,
+                          const RnsView& vb, const RnsStage& s, void* res, const int* skip,
+                          cudaStream_t st);
+
+// Contractions through residue planes (rns_ops.cu), nm = RNS_FP64 or RNS_MIXED. The views
+// of an operator's l and r stay in use between prepare and the applies.
+size_t heff_workspace_bytes_rns(int nm, int Dl, int d, int Dr, int cl, int cr);
+ptn_status heff_prepare_rns(int nm, const double2* l, const double2* r, int Dl, int d, int Dr,
+                            int cl, int cr, void* ws, size_t ws_bytes, cudaStream_t st);
+ptn_status heff_apply_rns(int nm, const double2* x, double2* y, const double2* w, const double2* l,
+                          const double2* r, int Dl, int d, int Dr, int cl, int cr, void* ws,
+                          const int* skip, cudaStream_t st);
+size_t bond_workspace_bytes_rns(int nm, int Dl, int Dr, int chi);
+ptn_status bond_prepare_rns(int nm, const double2* l, const double2* r, int Dl, int Dr, int chi,
+                            void* ws, size_t ws_bytes, cudaStream_t st);
+ptn_status bond_apply_rns(int nm, const double2* x, double2* y, const double2* l, const double2* r,
+                          int Dl, int Dr, int chi, void* ws, const int* skip, cudaStream_t st);
+size_t env_workspace_bytes_rns(int nm, int Dl, int d, int Dr, int cl, int cr);
+ptn_status env_left_rns(int nm, const double2* a, const double2* b, const double2* w,
+                        const double2* l, double2* lnext, int Dl, int d, int Dr, int cl, int cr,
+                        void* ws, size_t ws_bytes, cudaStream_t st);
+ptn_status env_right_rns(int nm, const double2* a, const double2* b, const double2* w,
+                         const double2* r, double2* rnext, int Dl, int d, int Dr, int cl, int cr,
+                         void* ws, size_t ws_bytes, cudaStream_t st);
+
+// whether the FP64 form of a contraction takes the residue planes (contract.cu)
+bool heff_f64_rns(int Dl, int d, int Dr, int cl, int cr);
+bool bond_f64_rns(int Dl, int Dr, int chi);
+
+}  // namespace ptn

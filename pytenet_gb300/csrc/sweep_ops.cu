@@ -7,6 +7,7 @@
 // their skip predicate, so after a Lanczos breakdown the remaining launches of
 // the (possibly graph-captured) sequence retire immediately on the device.
 #include "ptn_common.cuh"
+#include "rns.cuh"
 #include <algorithm>
 
 namespace ptn {
@@ -54,13 +55,29 @@ struct LocalOp {
 
   long n() const { return site ? (long)Dl * d * Dr : (long)Dl * Dr; }
 
+  // FP64 through residue planes, converted once per local step; a workspace smaller than
+  // the query asks for leaves the DMMA kernel
+  bool f64_rns() const {
+    if (prec != PTN_PREC_FP64) return false;
+    return site ? heff_f64_rns(Dl, d, Dr, chil, chir) &&
+                      ws_bytes >= heff_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir)
+                : bond_f64_rns(Dl, Dr, chil) &&
+                      ws_bytes >= bond_workspace_bytes_rns(RNS_FP64, Dl, Dr, chil);
+  }
+
   ptn_status prepare(cudaStream_t st) const {
+    if (f64_rns())
+      return site ? heff_prepare_rns(RNS_FP64, l, r, Dl, d, Dr, chil, chir, ws, ws_bytes, st)
+                  : bond_prepare_rns(RNS_FP64, l, r, Dl, Dr, chil, ws, ws_bytes, st);
     if (prec == PTN_PREC_FP64) return PTN_OK;
     return site ? heff_prepare_mixed(w, l, r, Dl, d, Dr, chil, chir, ws, ws_bytes, st)
                 : bond_prepare_mixed(l, r, Dl, Dr, chil, ws, ws_bytes, st);
   }
 
   ptn_status apply(const double2* x, double2* y, const int* skip, cudaStream_t st) const {
+    if (f64_rns())
+      return site ? heff_apply_rns(RNS_FP64, x, y, w, l, r, Dl, d, Dr, chil, chir, ws, skip, st)
+                  : bond_apply_rns(RNS_FP64, x, y, l, r, Dl, Dr, chil, ws, skip, st);
     if (prec == PTN_PREC_FP64)
       return site ? heff_apply_f64(x, w, l, r, y, Dl, d, Dr, chil, chir, ws, ws_bytes, skip, st)
                   : bond_apply_f64(x, l, r, y, Dl, Dr, chil, ws, ws_bytes, skip, st);

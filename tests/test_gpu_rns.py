@@ -1,0 +1,150 @@
+"""FP64 GEMM in the residue number system (csrc/rns.cu): against products formed in extended
+precision and against the DMMA kernel, over the edges of its tiles, all operand forms, rows
+that leave the FP64 range, and operands whose products all have one sign.
+
+Bound: an operand row is rounded to 53 bits or more of its largest component, so one of K
+terms is off by at most 4 * 2^-53 max|A row| max|B column| and a result by K times that,
+plus its own rounding; the tolerance is twice that."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def zgemm(A, B, opa="N", opb="N", alpha=1.0, beta=0.0, C=None, rns=True):
+    """op(A) op(B) through ptn_zgemm; rns=False: no workspace, so the DMMA kernel."""
+    import torch
+    from pytenet_gb300 import _lib
+    from pytenet_gb300.device import to_dev, to_host, ptr, stream_ptr, zeros
+    L = _lib.load()
+    M, K = A.shape if opa in "NC" else A.shape[::-1]
+    N = B.shape[1] if opb in "NC" else B.shape[0]
+    dA, dB = to_dev(A), to_dev(B)
+    dC = zeros((M, N)) if C is None else to_dev(C).clone()
+    wsb = L.ptn_zgemm_workspace_bytes(M, N, K, 1)
+    assert not rns or wsb > 0, "the shape should take the residue planes"
+    ws = torch.empty(max(wsb, 256), dtype=torch.uint8, device="cuda")
+    _lib.check(L.ptn_zgemm(opa.encode(), opb.encode(), M, N, K, _lib.cval(alpha), ptr(dA),
+                           A.shape[1], 0, ptr(dB), B.shape[1], 0, _lib.cval(beta), ptr(dC), N, 0,
+                           1, ptr(ws), wsb if rns else 0, stream_ptr()))
+    out = to_host(dC)
+    assert L.ptn_tc_error() == 0
+    return out
+
+
+def crandn(rng, *s):
+    return rng.standard_normal(s) + 1j * rng.standard_normal(s)
+
+
+def exact(A, B, rows, cols):
+    """Rows x columns of A B in extended precision."""
+    a, b = A[rows].astype(np.clongdouble), B[:, cols].astype(np.clongdouble)
+    return np.stack([(a[i][:, None] * b).sum(axis=0) for i in range(len(rows))])
+
+
+def errors(C, A, B, rng, count=24):
+    rows = np.unique(np.r_[0, A.shape[0] - 1, rng.integers(0, A.shape[0], count)])
+    cols = np.unique(np.r_[0, B.shape[1] - 1, rng.integers(0, B.shape[1], count)])
+    ref = exact(A, B, rows, cols)
+    scale = (np.abs(A[rows]).max(axis=1)[:, None] * np.abs(B[:, cols]).max(axis=0)[None, :])
+    err = np.abs(C[np.ix_(rows, cols)].astype(np.clongdouble) - ref)
+    tol = 2 * (4 * A.shape[1] * scale * 2.0 ** -53 + 2.0 ** -53 * np.abs(ref).astype(float))
+    return err, tol
+
+
+@pytest.mark.parametrize("mnk", [(128, 256, 128), (129, 257, 200), (500, 1280, 256), (130, 66, 700),
+                                 (1024, 33, 321), (64, 128, 512), (33, 4100, 255), (300, 300, 257),
+                                 (250, 512, 1280), (37, 70, 8192)])
+def test_matches_extended_precision(mnk):
+    M, N, K = mnk
+    rng = np.random.default_rng(M + 3 * N + 7 * K)
+    A, B = crandn(rng, M, K), crandn(rng, K, N)
+    err, tol = errors(zgemm(A, B), A, B, rng)
+    assert np.all(err <= tol), (err / tol).max()
+    err0, _ = errors(zgemm(A, B, rns=False), A, B, np.random.default_rng(1))
+    rms, rms0 = (float(np.sqrt((e.astype(float) ** 2).mean())) for e in (err, err0))
+    print(f"{mnk}: rms error {rms:.2e}, DMMA kernel {rms0:.2e}")
+    assert rms <= 1.1 * rms0
+
+
+@pytest.mark.parametrize("opa", list("NTCH"))
+@pytest.mark.parametrize("opb", list("NTCH"))
+def test_operand_forms(opa, opb):
+    rng = np.random.default_rng(5)
+    M, N, K = 141, 203, 167
+    f = {"N": lambda x: x, "T": lambda x: x.T, "C": np.conj, "H": lambda x: x.conj().T}
+    A = crandn(rng, *((M, K) if opa in "NC" else (K, M)))
+    B = crandn(rng, *((K, N) if opb in "NC" else (N, K)))
+    C0 = crandn(rng, M, N)
+    al, be = 0.7 - 0.2j, -1.3 + 0.4j
+    got = zgemm(A, B, opa, opb, al, be, C0)
+    ref = al * (f[opa](A) @ f[opb](B)) + be * C0
+    assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("kind", ["constant", "positive", "alternating", "powers"])
+def test_one_signed_sums_are_exact(kind):
+    """Every product of one sign: the largest chunk sums there can be."""
+    rng = np.random.default_rng(6)
+    M, N, K = 140, 150, 1500
+    if kind == "constant":
+        A, B = np.full((M, K), 0.7123 + 0.4567j), np.full((K, N), 0.9876 - 0.1j)
+    elif kind == "positive":
+        A = rng.uniform(0.5, 1, (M, K)) + 1j * rng.uniform(0.5, 1, (M, K))
+        B = rng.uniform(0.5, 1, (K, N)) + 0j
+    elif kind == "alternating":
+        s = (-1.0) ** np.arange(K)
+        A, B = np.full((M, K), 0.999) * s + 0j, (np.full((K, N), 0.999) * s[:, None]) + 0j
+    else:
+        A = 2.0 ** rng.integers(-30, 1, (M, K)) + 0j
+        B = 2.0 ** rng.integers(-30, 1, (K, N)) + 0j
+    err, tol = errors(zgemm(A, B), A, B, rng)
+    assert np.all(err <= tol), (err / tol).max()
+
+
+def test_scales_zeros_and_range_ends():
+    """Rows and columns of very different size, zero rows, and rows whose entries or results
+    leave the normal range: as the DMMA kernel gives them."""
+    rng = np.random.default_rng(7)
+    M, N, K = 160, 170, 180
+    A, B = crandn(rng, M, K), crandn(rng, K, N)
+    A[3] = 0
+    B[:, 5] = 0
+    A[10] *= 1e-150
+    B[:, 11] *= 1e140
+    A[20] *= 1e-300
+    B[:, 21] *= 1e-300
+    A[30] *= 1e-320 / 1e-10 * 1e-10
+    A[40] *= 1e300
+    B[:, 41] *= 1e300
+    got, ref = zgemm(A, B), zgemm(A, B, rns=False)
+    assert np.all(got[3] == 0) and np.all(got[:, 5] == 0)
+    with np.errstate(over="ignore", invalid="ignore"):
+        scale = np.abs(A).max(axis=1)[:, None] * np.abs(B).max(axis=0)[None, :] * K
+    fin = np.isfinite(ref.real) & np.isfinite(ref.imag)
+    assert np.array_equal(fin, np.isfinite(got.real) & np.isfinite(got.imag))
+    ok = fin & np.isfinite(scale)
+    d = np.abs(np.where(ok, got, 0) - np.where(ok, ref, 0))
+    assert np.all(d <= np.where(ok, 1e-14 * scale, 0) + 1e-321)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_infinities_and_nans(bad):
+    """An infinity or NaN makes the same results infinite or NaN as in the DMMA kernel and
+    leaves every other result alone."""
+    rng = np.random.default_rng(8)
+    M, N, K = 140, 130, 256
+    A, B = crandn(rng, M, K), crandn(rng, K, N)
+    A[0] = 0
+    clean = zgemm(A, B)
+    A[7, 3] = bad
+    B[9, 15] = 1j * bad
+    got, ref = zgemm(A, B), zgemm(A, B, rns=False)
+    for part in (np.real, np.imag):
+        g, r = part(got), part(ref)
+        assert np.array_equal(np.isnan(g), np.isnan(r)) and np.array_equal(np.isinf(g), np.isinf(r))
+    same = np.ones((M, N), bool)
+    same[7] = False
+    same[:, 15] = False
+    assert np.array_equal(got[same], clean[same])
