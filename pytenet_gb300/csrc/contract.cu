@@ -71,11 +71,6 @@ ptn_status mpo_stage(const double2* in, double2* out, const double2* w, long ldq
 
 }  // namespace
 
-ptn_status mpo_stage_f64(const double2* in, double2* out, const double2* w, long ldq, long ldp, int X,
-                         int P, int Q, int Y, const int* skip, cudaStream_t st) {
-  return mpo_stage(in, out, w, ldq, ldp, X, P, Q, Y, skip, st);
-}
-
 namespace {
 
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -96,18 +91,30 @@ GemmArgs gemm_args(char oa, char ob, int M, int N, int K, const double2* A, long
 
 // ------------------------------------------------------------------ choice of kernels
 // The FP64 form takes the residue planes where both GEMMs do (rns_wanted), the DMMA kernel
-// otherwise, or when the workspace is smaller than the query asks for.
-bool heff_f64_rns(int Dl, int d, int Dr, int cl, int cr) {
-  return rns_wanted((long)Dl * d, (long)cr * Dr, Dr) && rns_wanted(Dl, (long)d * Dr, (long)Dl * cl);
+// otherwise, or when the workspace is smaller than the query asks for; the mixed form takes
+// its (fewer) planes unless a product is too long for them.
+static int form(int prec, bool wanted, long k1, long k2) {
+  if (prec == PTN_PREC_FP64) return wanted ? RNS_FP64 : 0;
+  return rns_bits(k1, RNS_MIXED) != 0 && rns_bits(k2, RNS_MIXED) != 0 ? RNS_MIXED : 0;
 }
 
-bool bond_f64_rns(int Dl, int Dr, int chi) {
-  return rns_wanted(Dl, (long)chi * Dr, Dr) && rns_wanted(Dl, Dr, (long)Dl * chi);
+int heff_form(int prec, int Dl, int d, int Dr, int cl, int cr) {
+  return form(prec, rns_wanted((long)Dl * d, (long)cr * Dr, Dr) &&
+                        rns_wanted(Dl, (long)d * Dr, (long)Dl * cl), Dr, (long)Dl * cl);
 }
 
-static bool env_f64_rns(int Dl, int d, int Dr, int cl, int cr) {
-  return rns_wanted((long)Dl * cl, (long)d * Dr, Dl) && rns_wanted(Dr, (long)cr * Dr, (long)Dl * d) &&
-         rns_wanted((long)Dl * d, (long)cr * Dr, Dr) && rns_wanted((long)Dl * cl, Dl, (long)d * Dr);
+int bond_form(int prec, int Dl, int Dr, int chi) {
+  return form(prec, rns_wanted(Dl, (long)chi * Dr, Dr) && rns_wanted(Dl, Dr, (long)Dl * chi), Dr,
+              (long)Dl * chi);
+}
+
+static int env_form(int prec, int Dl, int d, int Dr, int cl, int cr) {
+  return form(prec,
+              rns_wanted((long)Dl * cl, (long)d * Dr, Dl) &&
+                  rns_wanted(Dr, (long)cr * Dr, (long)Dl * d) &&
+                  rns_wanted((long)Dl * d, (long)cr * Dr, Dr) &&
+                  rns_wanted((long)Dl * cl, Dl, (long)d * Dr),
+              std::max(Dl, Dr), (long)std::max(Dl, Dr) * d);
 }
 
 // ------------------------------------------------------------------ workspace layout
@@ -129,8 +136,6 @@ static size_t heff_gemm_ws(int Dl, int d, int Dr, int chil, int chir) {
 }
 
 size_t heff_workspace_bytes_f64(int Dl, int d, int Dr, int chil, int chir) {
-  if (heff_f64_rns(Dl, d, Dr, chil, chir))
-    return heff_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir);
   const size_t t = align256(heff_t_elems(Dl, d, Dr, chil, chir) * sizeof(double2));
   return 2 * t + align256(heff_gemm_ws(Dl, d, Dr, chil, chir));
 }
@@ -164,7 +169,6 @@ ptn_status heff_apply_f64(const double2* a, const double2* w, const double2* l, 
 }
 
 size_t bond_workspace_bytes_f64(int Dl, int Dr, int chi) {
-  if (bond_f64_rns(Dl, Dr, chi)) return bond_workspace_bytes_rns(RNS_FP64, Dl, Dr, chi);
   const size_t t = align256((size_t)Dl * chi * Dr * sizeof(double2));
   const size_t g = std::max(zgemm_workspace_bytes(Dl, chi * Dr, Dr, 1),
                             zgemm_workspace_bytes(Dl, Dr, Dl * chi, 1));
@@ -187,8 +191,6 @@ ptn_status bond_apply_f64(const double2* cm, const double2* l, const double2* r,
 }
 
 size_t env_workspace_bytes_f64(int Dl, int d, int Dr, int chil, int chir) {
-  if (env_f64_rns(Dl, d, Dr, chil, chir))
-    return env_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir);
   const size_t te = (size_t)std::max(Dl * chil * d * Dr, Dl * d * chir * Dr);
   const size_t t = align256(te * sizeof(double2));
   size_t g = zgemm_workspace_bytes(Dl * chil, d * Dr, Dl, 1);
@@ -201,9 +203,6 @@ size_t env_workspace_bytes_f64(int Dl, int d, int Dr, int chil, int chir) {
 ptn_status env_left_f64(const double2* a, const double2* b, const double2* w, const double2* l,
                         double2* lnext, int Dl, int d, int Dr, int chil, int chir, void* ws,
                         size_t ws_bytes, cudaStream_t st) {
-  if (env_f64_rns(Dl, d, Dr, chil, chir) &&
-      ws_bytes >= env_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir))
-    return env_left_rns(RNS_FP64, a, b, w, l, lnext, Dl, d, Dr, chil, chir, ws, ws_bytes, st);
   const size_t te = (size_t)std::max(Dl * chil * d * Dr, Dl * d * chir * Dr);
   PTN_CHECK_ARG(ws_bytes >= 2 * align256(te * sizeof(double2)), "env_left: workspace too small");
   ContractWs c = carve(ws, te, ws_bytes);
@@ -221,9 +220,6 @@ ptn_status env_left_f64(const double2* a, const double2* b, const double2* w, co
 ptn_status env_right_f64(const double2* a, const double2* b, const double2* w, const double2* r,
                          double2* rnext, int Dl, int d, int Dr, int chil, int chir, void* ws,
                          size_t ws_bytes, cudaStream_t st) {
-  if (env_f64_rns(Dl, d, Dr, chil, chir) &&
-      ws_bytes >= env_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir))
-    return env_right_rns(RNS_FP64, a, b, w, r, rnext, Dl, d, Dr, chil, chir, ws, ws_bytes, st);
   const size_t te = (size_t)std::max(Dl * chil * d * Dr, Dl * d * chir * Dr);
   PTN_CHECK_ARG(ws_bytes >= 2 * align256(te * sizeof(double2)), "env_right: workspace too small");
   ContractWs c = carve(ws, te, ws_bytes);
@@ -246,79 +242,68 @@ using namespace ptn;
 static inline const double2* D2(const ptn_c128* p) { return reinterpret_cast<const double2*>(p); }
 static inline double2* D2(ptn_c128* p) { return reinterpret_cast<double2*>(p); }
 
-namespace ptn {
-size_t heff_workspace_bytes_mixed(int Dl, int d, int Dr, int chil, int chir);
-size_t bond_workspace_bytes_mixed(int Dl, int Dr, int chi);
-ptn_status heff_apply_mixed_entry(const double2*, const double2*, const double2*, const double2*,
-                                  double2*, int, int, int, int, int, void*, size_t, cudaStream_t);
-ptn_status bond_apply_mixed_entry(const double2*, const double2*, const double2*, double2*, int,
-                                  int, int, void*, size_t, cudaStream_t);
-size_t env_workspace_bytes_mixed(int Dl, int d, int Dr, int cl, int cr);
-ptn_status env_left_mixed(const double2*, const double2*, const double2*, const double2*, double2*,
-                          int, int, int, int, int, void*, size_t, cudaStream_t);
-ptn_status env_right_mixed(const double2*, const double2*, const double2*, const double2*, double2*,
-                           int, int, int, int, int, void*, size_t, cudaStream_t);
-}  // namespace ptn
-
 extern "C" {
 
 size_t ptn_heff_workspace_bytes(int Dl, int d, int Dr, int chil, int chir, int prec) {
-  return prec == PTN_PREC_FP64 ? heff_workspace_bytes_f64(Dl, d, Dr, chil, chir)
-                               : heff_workspace_bytes_mixed(Dl, d, Dr, chil, chir);
+  const int nm = heff_form(prec, Dl, d, Dr, chil, chir);
+  return nm != 0 ? heff_workspace_bytes_rns(nm, Dl, d, Dr, chil, chir)
+                 : heff_workspace_bytes_f64(Dl, d, Dr, chil, chir);
 }
 
 size_t ptn_bond_workspace_bytes(int Dl, int Dr, int chi, int prec) {
-  return prec == PTN_PREC_FP64 ? bond_workspace_bytes_f64(Dl, Dr, chi)
-                               : bond_workspace_bytes_mixed(Dl, Dr, chi);
+  const int nm = bond_form(prec, Dl, Dr, chi);
+  return nm != 0 ? bond_workspace_bytes_rns(nm, Dl, Dr, chi) : bond_workspace_bytes_f64(Dl, Dr, chi);
 }
 
 size_t ptn_env_workspace_bytes(int Dl, int d, int Dr, int chil, int chir, int prec) {
-  return prec == PTN_PREC_FP64 ? env_workspace_bytes_f64(Dl, d, Dr, chil, chir)
-                               : env_workspace_bytes_mixed(Dl, d, Dr, chil, chir);
+  const int nm = env_form(prec, Dl, d, Dr, chil, chir);
+  return nm != 0 ? env_workspace_bytes_rns(nm, Dl, d, Dr, chil, chir)
+                 : env_workspace_bytes_f64(Dl, d, Dr, chil, chir);
+}
+
+// the FP64 form falls back to the DMMA kernels on a workspace smaller than the query's
+static int fitting(int nm, int prec, size_t ws_bytes, size_t need) {
+  return prec == PTN_PREC_FP64 && ws_bytes < need ? 0 : nm;
 }
 
 ptn_status ptn_heff_apply(const ptn_c128* a, const ptn_c128* w, const ptn_c128* l,
                           const ptn_c128* r, ptn_c128* out, int Dl, int d, int Dr, int chil,
                           int chir, int prec, void* ws, size_t ws_bytes, void* stream) {
   PTN_CHECK_ARG(Dl > 0 && d > 0 && Dr > 0 && chil > 0 && chir > 0, "heff: bad dims");
-  if (prec == PTN_PREC_FP64 && heff_f64_rns(Dl, d, Dr, chil, chir) &&
-      ws_bytes >= heff_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir)) {
-    PTN_TRY(heff_prepare_rns(RNS_FP64, D2(l), D2(r), Dl, d, Dr, chil, chir, ws, ws_bytes,
-                             as_stream(stream)));
-    return heff_apply_rns(RNS_FP64, D2(a), D2(out), D2(w), D2(l), D2(r), Dl, d, Dr, chil, chir, ws,
-                          nullptr, as_stream(stream));
-  }
-  if (prec == PTN_PREC_FP64)
+  const int nm = fitting(heff_form(prec, Dl, d, Dr, chil, chir), prec, ws_bytes,
+                         ptn_heff_workspace_bytes(Dl, d, Dr, chil, chir, prec));
+  if (nm == 0)
     return heff_apply_f64(D2(a), D2(w), D2(l), D2(r), D2(out), Dl, d, Dr, chil, chir, ws, ws_bytes,
                           nullptr, as_stream(stream));
-  return heff_apply_mixed_entry(D2(a), D2(w), D2(l), D2(r), D2(out), Dl, d, Dr, chil, chir, ws,
-                                ws_bytes, as_stream(stream));
+  PTN_TRY(heff_prepare_rns(nm, D2(l), D2(r), Dl, d, Dr, chil, chir, ws, ws_bytes,
+                           as_stream(stream)));
+  return heff_apply_rns(nm, D2(a), D2(out), D2(w), D2(l), D2(r), Dl, d, Dr, chil, chir, ws, nullptr,
+                        as_stream(stream));
 }
 
 ptn_status ptn_bond_apply(const ptn_c128* c, const ptn_c128* l, const ptn_c128* r, ptn_c128* out,
                           int Dl, int Dr, int chi, int prec, void* ws, size_t ws_bytes,
                           void* stream) {
   PTN_CHECK_ARG(Dl > 0 && Dr > 0 && chi > 0, "bond: bad dims");
-  if (prec == PTN_PREC_FP64 && bond_f64_rns(Dl, Dr, chi) &&
-      ws_bytes >= bond_workspace_bytes_rns(RNS_FP64, Dl, Dr, chi)) {
-    PTN_TRY(bond_prepare_rns(RNS_FP64, D2(l), D2(r), Dl, Dr, chi, ws, ws_bytes, as_stream(stream)));
-    return bond_apply_rns(RNS_FP64, D2(c), D2(out), D2(l), D2(r), Dl, Dr, chi, ws, nullptr,
-                          as_stream(stream));
-  }
-  if (prec == PTN_PREC_FP64)
+  const int nm = fitting(bond_form(prec, Dl, Dr, chi), prec, ws_bytes,
+                         ptn_bond_workspace_bytes(Dl, Dr, chi, prec));
+  if (nm == 0)
     return bond_apply_f64(D2(c), D2(l), D2(r), D2(out), Dl, Dr, chi, ws, ws_bytes, nullptr,
                           as_stream(stream));
-  return bond_apply_mixed_entry(D2(c), D2(l), D2(r), D2(out), Dl, Dr, chi, ws, ws_bytes,
-                                as_stream(stream));
+  PTN_TRY(bond_prepare_rns(nm, D2(l), D2(r), Dl, Dr, chi, ws, ws_bytes, as_stream(stream)));
+  return bond_apply_rns(nm, D2(c), D2(out), D2(l), D2(r), Dl, Dr, chi, ws, nullptr,
+                        as_stream(stream));
 }
 
 ptn_status ptn_env_step_left(const ptn_c128* a, const ptn_c128* b, const ptn_c128* w,
                              const ptn_c128* l, ptn_c128* l_next, int Dl, int d, int Dr, int chil,
                              int chir, int prec, void* ws, size_t ws_bytes, void* stream) {
   PTN_CHECK_ARG(Dl > 0 && d > 0 && Dr > 0 && chil > 0 && chir > 0, "env_left: bad dims");
-  if (prec != PTN_PREC_FP64)
-    return env_left_mixed(D2(a), D2(b), D2(w), D2(l), D2(l_next), Dl, d, Dr, chil, chir, ws,
-                          ws_bytes, as_stream(stream));
+  const int nm = fitting(env_form(prec, Dl, d, Dr, chil, chir), prec, ws_bytes,
+                         ptn_env_workspace_bytes(Dl, d, Dr, chil, chir, prec));
+  if (nm != 0)
+    return env_left_rns(nm, D2(a), D2(b), D2(w), D2(l), D2(l_next), Dl, d, Dr, chil, chir, ws,
+                        ws_bytes, as_stream(stream));
   return env_left_f64(D2(a), D2(b), D2(w), D2(l), D2(l_next), Dl, d, Dr, chil, chir, ws, ws_bytes,
                       as_stream(stream));
 }
@@ -327,9 +312,11 @@ ptn_status ptn_env_step_right(const ptn_c128* a, const ptn_c128* b, const ptn_c1
                               const ptn_c128* r, ptn_c128* r_next, int Dl, int d, int Dr, int chil,
                               int chir, int prec, void* ws, size_t ws_bytes, void* stream) {
   PTN_CHECK_ARG(Dl > 0 && d > 0 && Dr > 0 && chil > 0 && chir > 0, "env_right: bad dims");
-  if (prec != PTN_PREC_FP64)
-    return env_right_mixed(D2(a), D2(b), D2(w), D2(r), D2(r_next), Dl, d, Dr, chil, chir, ws,
-                           ws_bytes, as_stream(stream));
+  const int nm = fitting(env_form(prec, Dl, d, Dr, chil, chir), prec, ws_bytes,
+                         ptn_env_workspace_bytes(Dl, d, Dr, chil, chir, prec));
+  if (nm != 0)
+    return env_right_rns(nm, D2(a), D2(b), D2(w), D2(r), D2(r_next), Dl, d, Dr, chil, chir, ws,
+                         ws_bytes, as_stream(stream));
   return env_right_f64(D2(a), D2(b), D2(w), D2(r), D2(r_next), Dl, d, Dr, chil, chir, ws, ws_bytes,
                        as_stream(stream));
 }

@@ -1,8 +1,8 @@
-// Mixed-precision form of the site / bond operators and of the environment steps
-// (pytenet/chain_ops.py:16-99, 237-317): the two GEMMs of every contraction run on
-// the tensor cores as exact fixed-point BF16 digit products (tc_gemm.cu); the MPO
-// stage, the digit levels, the split-K sums and everything outside the
-// contractions are FP64.
+// The digit GEMM's entry (ptn_zgemm_split_bf16), which absorbs the bond matrix into the next
+// site in the mixed form: conversion of both operands to BF16 digits, exact digit products
+// on the tensor cores (tc_gemm.cu). The contractions of the mixed form run in the residue
+// number system (rns_ops.cu); this product acts on the state itself once per site, so its
+// results stay the ones it always gave, bit for bit.
 //
 // Operand conversion ("digits"): a complex matrix view (element (r, k) at
 // src[r * sr + k * sk]) becomes five BF16 digit planes plus one power-of-two
@@ -11,17 +11,6 @@
 // fixed-point integer round(x 2^(39 - e)) from the IEEE fields and cuts it into
 // five balanced base-256 digits with integer arithmetic only, stored k-contiguously. "Plain" operands keep
 // re/im interleaved along K; "embedded" operands store z as [[Re, -Im], [Im, Re]].
-//
-// Data flow of H_eff . x (site tensors (Dl, d, Dr), MPO bonds cl / cr):
-//   prepare (once per local step):  R -> Rt  (plain, rows (wr, r2), K = r0)
-//                                   L -> Le  (embedded, n = l2, K = (l0, wl))
-//   apply:  x -> Xe (embedded, n = (l0, t), K = r0)
-//           GEMM 1: T1^T[(wr,r2)][(l0,t)] = Rt . Xe^T, written as T1[(l0,t)][(wr,r2)]
-//           MPO stage (FP64): T2[l0,(wl,s),r2]
-//           T2 -> T2s (plain, rows (s, r2), K = (l0, wl))
-//           GEMM 2: out^T[(s,r2)][l2] = T2s . Le^T, written as out[l2][(s,r2)]
-// Every GEMM computes the transpose of the wanted product so that the epilogue
-// thread of output row m writes consecutive addresses with its neighbours.
 #include "ptn_common.cuh"
 #include <cuda_bf16.h>
 #include <algorithm>
@@ -35,8 +24,6 @@ ptn_status tc_gemm(const void* Aslices, long aplane, const int* ea, const void* 
                    bool accumulate, void* ws, size_t ws_bytes, const int* skip, cudaStream_t st,
                    const unsigned char* fa, const unsigned char* fb, int fk);
 size_t tc_gemm_workspace_bytes(int M, int Ncomplex, int Kcomplex);
-ptn_status mpo_stage_f64(const double2* in, double2* out, const double2* w, long ldq, long ldp, int X,
-                         int P, int Q, int Y, const int* skip, cudaStream_t st);
 
 namespace {
 
@@ -189,22 +176,6 @@ struct Carver {
   }
 };
 
-// The split-K scratch of the digit GEMMs is the last piece of every workspace
-// layout: give the GEMMs all that the caller's workspace has left (the GEMM picks
-// its K splits to fit, never below what exact accumulation needs), so a workspace
-// sized under other tuning-knob values still works.
-template <class W>
-void use_rest(W& w, void* ws, size_t ws_bytes) {
-  const size_t off = (size_t)(static_cast<char*>(w.gws) - static_cast<char*>(ws));
-  w.gbytes = ws_bytes > off ? ws_bytes - off : 0;
-}
-
-// bytes a layout needs before its GEMM scratch
-template <class W>
-size_t before_gemm(const Carver& c, const W& w) {
-  return c.off - al(w.gbytes);
-}
-
 // BF16 digit planes of a complex matrix with `rows` rows (2 * rows real rows when
 // embedded) and kc complex columns, plus the per-row exponents
 struct Digits {
@@ -258,239 +229,7 @@ ptn_status gemm(const Digits& A, const Digits& Be, double2* out, long ldm, long 
                  flags ? A.f : nullptr, flags ? Be.f : nullptr, (int)A.fk());
 }
 
-// ---------------------------------------------------------------- H_eff (site)
-struct HeffWs {
-  Digits Rt, Le, Xe, T2s;
-  double2 *T1, *T2;
-  void* gws;
-  size_t gbytes;
-};
-
-HeffWs heff_ws(Carver& c, int Dl, int d, int Dr, int cl, int cr) {
-  HeffWs w;
-  w.Rt = take_digits(c, (long)cr * Dr, Dr, false);
-  w.Le = take_digits(c, Dl, (long)Dl * cl, true);
-  w.Xe = take_digits(c, (long)Dl * d, Dr, true);
-  w.T2s = take_digits(c, (long)d * Dr, (long)Dl * cl, false);
-  w.T1 = static_cast<double2*>(c.take((size_t)Dl * d * cr * Dr * sizeof(double2)));
-  w.T2 = static_cast<double2*>(c.take((size_t)Dl * cl * d * Dr * sizeof(double2)));
-  w.gbytes = std::max(tc_gemm_workspace_bytes(cr * Dr, Dl * d, Dr),
-                      tc_gemm_workspace_bytes(d * Dr, Dl, Dl * cl));
-  w.gws = c.take(w.gbytes);
-  return w;
-}
-
-// ---------------------------------------------------------------- zero-site (bond)
-struct BondWs {
-  Digits Rt, Le, Xe, T1s;
-  double2* T1;
-  void* gws;
-  size_t gbytes;
-};
-
-BondWs bond_ws(Carver& c, int Dl, int Dr, int chi) {
-  BondWs w;
-  w.Rt = take_digits(c, (long)chi * Dr, Dr, false);
-  w.Le = take_digits(c, Dl, (long)Dl * chi, true);
-  w.Xe = take_digits(c, Dl, Dr, true);
-  w.T1s = take_digits(c, Dr, (long)Dl * chi, false);
-  w.T1 = static_cast<double2*>(c.take((size_t)Dl * chi * Dr * sizeof(double2)));
-  w.gbytes = std::max(tc_gemm_workspace_bytes(chi * Dr, Dl, Dr),
-                      tc_gemm_workspace_bytes(Dr, Dl, Dl * chi));
-  w.gws = c.take(w.gbytes);
-  return w;
-}
-
-// ---------------------------------------------------------------- environments
-struct EnvWs {
-  Digits S1, E1, S2, E2;
-  double2 *T1, *T2;
-  void* gws;
-  size_t gbytes;
-};
-
-EnvWs env_left_ws(Carver& c, int Dl, int d, int Dr, int cl, int cr) {
-  EnvWs w;
-  w.S1 = take_digits(c, (long)d * Dr, Dl, false);           // conj(B)^T, rows (t, rb), K = l2
-  w.E1 = take_digits(c, (long)Dl * cl, Dl, true);           // L, n = (l0, wl), K = l2
-  w.S2 = take_digits(c, (long)cr * Dr, (long)Dl * d, false); // T2^T, rows (wr, rb), K = (l0, s)
-  w.E2 = take_digits(c, Dr, (long)Dl * d, true);            // A, n = ra, K = (l0, s)
-  w.T1 = static_cast<double2*>(c.take((size_t)Dl * cl * d * Dr * sizeof(double2)));
-  w.T2 = static_cast<double2*>(c.take((size_t)Dl * d * cr * Dr * sizeof(double2)));
-  w.gbytes = std::max(tc_gemm_workspace_bytes(d * Dr, Dl * cl, Dl),
-                      tc_gemm_workspace_bytes(cr * Dr, Dr, Dl * d));
-  w.gws = c.take(w.gbytes);
-  return w;
-}
-
-EnvWs env_right_ws(Carver& c, int Dl, int d, int Dr, int cl, int cr) {
-  EnvWs w;
-  w.S1 = take_digits(c, (long)cr * Dr, Dr, false);          // R^T, rows (wr, r2), K = r0
-  w.E1 = take_digits(c, (long)Dl * d, Dr, true);            // A, n = (l0, s), K = r0
-  w.S2 = take_digits(c, Dl, (long)d * Dr, false);           // conj(B), rows lb, K = (t, r2)
-  w.E2 = take_digits(c, (long)Dl * cl, (long)d * Dr, true); // T2, n = (l0, wl), K = (t, r2)
-  w.T1 = static_cast<double2*>(c.take((size_t)Dl * d * cr * Dr * sizeof(double2)));
-  w.T2 = static_cast<double2*>(c.take((size_t)Dl * cl * d * Dr * sizeof(double2)));
-  w.gbytes = std::max(tc_gemm_workspace_bytes(cr * Dr, Dl * d, Dr),
-                      tc_gemm_workspace_bytes(Dl, Dl * cl, d * Dr));
-  w.gws = c.take(w.gbytes);
-  return w;
-}
-
 }  // namespace
-
-// ================================================================ site operator
-size_t heff_workspace_bytes_mixed(int Dl, int d, int Dr, int chil, int chir) {
-  Carver c(nullptr);
-  heff_ws(c, Dl, d, Dr, chil, chir);
-  return c.off;
-}
-
-ptn_status heff_prepare_mixed(const double2* w, const double2* l, const double2* r, int Dl, int d,
-                              int Dr, int chil, int chir, void* ws, size_t ws_bytes,
-                              cudaStream_t st) {
-  (void)w;
-  {
-    Carver q(nullptr);
-    const HeffWs hq = heff_ws(q, Dl, d, Dr, chil, chir);
-    PTN_CHECK_ARG(ws_bytes >= before_gemm(q, hq), "mixed heff: workspace too small");
-  }
-  Carver c(ws);
-  HeffWs h = heff_ws(c, Dl, d, Dr, chil, chir);
-  // Rt: (m = (wr, r2), k = r0) = R[r0][(wr, r2)]
-  PTN_TRY(to_digits(r, 1, (long)chir * Dr, h.Rt, false, nullptr, st));
-  // Le: (n = l2, k = (l0, wl)) = L[(l0, wl)][l2]
-  PTN_TRY(to_digits(l, 1, Dl, h.Le, false, nullptr, st));
-  return PTN_OK;
-}
-
-ptn_status heff_apply_mixed(const double2* x, double2* y, const double2* w, int Dl, int d, int Dr,
-                            int chil, int chir, void* ws, size_t ws_bytes, const int* skip,
-                            cudaStream_t st) {
-  Carver c(ws);
-  HeffWs h = heff_ws(c, Dl, d, Dr, chil, chir);
-  use_rest(h, ws, ws_bytes);
-  // Xe: (n = (l0, t), k = r0) = x[(l0, t)][r0]
-  PTN_TRY(to_digits(x, Dr, 1, h.Xe, false, skip, st));
-  // T1[(l0,t)][(wr,r2)] via T1^T = Rt . Xe^T
-  PTN_TRY(gemm(h.Rt, h.Xe, h.T1, 1, (long)chir * Dr, h.gws, h.gbytes, skip, st));
-  // T2[l0][(wl, s)][r2] = sum_(t, wr) W[(wl, s), (t, wr)] T1[l0][(t, wr)][r2]
-  PTN_TRY(mpo_stage_f64(h.T1, h.T2, w, (long)d * chir, 1, Dl, d * chir, chil * d, Dr, skip, st));
-  // T2s: (m = (s, r2), k = (l0, wl)) = T2[(l0, wl)][(s, r2)]
-  PTN_TRY(to_digits(h.T2, 1, (long)d * Dr, h.T2s, false, skip, st));
-  // out^T[(s, r2)][l2] = T2s . Le^T -> out[l2][(s, r2)]
-  PTN_TRY(gemm(h.T2s, h.Le, y, 1, (long)d * Dr, h.gws, h.gbytes, skip, st));
-  return PTN_OK;
-}
-
-ptn_status heff_apply_mixed_entry(const double2* a, const double2* w, const double2* l,
-                                  const double2* r, double2* out, int Dl, int d, int Dr, int chil,
-                                  int chir, void* ws, size_t ws_bytes, cudaStream_t st) {
-  PTN_TRY(heff_prepare_mixed(w, l, r, Dl, d, Dr, chil, chir, ws, ws_bytes, st));
-  return heff_apply_mixed(a, out, w, Dl, d, Dr, chil, chir, ws, ws_bytes, nullptr, st);
-}
-
-// ================================================================ bond operator
-size_t bond_workspace_bytes_mixed(int Dl, int Dr, int chi) {
-  Carver c(nullptr);
-  bond_ws(c, Dl, Dr, chi);
-  return c.off;
-}
-
-ptn_status bond_prepare_mixed(const double2* l, const double2* r, int Dl, int Dr, int chi, void* ws,
-                              size_t ws_bytes, cudaStream_t st) {
-  {
-    Carver q(nullptr);
-    const BondWs bq = bond_ws(q, Dl, Dr, chi);
-    PTN_CHECK_ARG(ws_bytes >= before_gemm(q, bq), "mixed bond: workspace too small");
-  }
-  Carver c(ws);
-  BondWs b = bond_ws(c, Dl, Dr, chi);
-  PTN_TRY(to_digits(r, 1, (long)chi * Dr, b.Rt, false, nullptr, st));
-  PTN_TRY(to_digits(l, 1, Dl, b.Le, false, nullptr, st));
-  return PTN_OK;
-}
-
-ptn_status bond_apply_mixed(const double2* x, double2* y, int Dl, int Dr, int chi, void* ws,
-                            size_t ws_bytes, const int* skip, cudaStream_t st) {
-  Carver c(ws);
-  BondWs b = bond_ws(c, Dl, Dr, chi);
-  use_rest(b, ws, ws_bytes);
-  // Xe: (n = l0, k = r0) = C[l0][r0]
-  PTN_TRY(to_digits(x, Dr, 1, b.Xe, false, skip, st));
-  // T1[l0][(w, r2)] via T1^T = Rt . Xe^T
-  PTN_TRY(gemm(b.Rt, b.Xe, b.T1, 1, (long)chi * Dr, b.gws, b.gbytes, skip, st));
-  // T1s: (m = r2, k = (l0, w)) = T1[(l0, w)][r2]
-  PTN_TRY(to_digits(b.T1, 1, Dr, b.T1s, false, skip, st));
-  // out^T[r2][l2] = T1s . Le^T -> out[l2][r2]
-  PTN_TRY(gemm(b.T1s, b.Le, y, 1, Dr, b.gws, b.gbytes, skip, st));
-  return PTN_OK;
-}
-
-ptn_status bond_apply_mixed_entry(const double2* cm, const double2* l, const double2* r,
-                                  double2* out, int Dl, int Dr, int chi, void* ws, size_t ws_bytes,
-                                  cudaStream_t st) {
-  PTN_TRY(bond_prepare_mixed(l, r, Dl, Dr, chi, ws, ws_bytes, st));
-  return bond_apply_mixed(cm, out, Dl, Dr, chi, ws, ws_bytes, nullptr, st);
-}
-
-// ================================================================ environments
-size_t env_workspace_bytes_mixed(int Dl, int d, int Dr, int cl, int cr) {
-  Carver a(nullptr), b(nullptr);
-  env_left_ws(a, Dl, d, Dr, cl, cr);
-  env_right_ws(b, Dl, d, Dr, cl, cr);
-  return std::max(a.off, b.off);
-}
-
-// l_next[ra, wr, rb] = sum A[l0,s,ra] W[wl,t,s,wr] L[l0,wl,l2] conj(B[l2,t,rb])
-ptn_status env_left_mixed(const double2* a, const double2* b, const double2* w, const double2* l,
-                          double2* lnext, int Dl, int d, int Dr, int cl, int cr, void* ws,
-                          size_t ws_bytes, cudaStream_t st) {
-  Carver c(ws);
-  EnvWs e = env_left_ws(c, Dl, d, Dr, cl, cr);
-  PTN_CHECK_ARG(ws_bytes >= before_gemm(c, e), "mixed env: workspace too small");
-  use_rest(e, ws, ws_bytes);
-  // S1: (m = (t, rb), k = l2) = conj(B[l2][(t, rb)])
-  PTN_TRY(to_digits(b, 1, (long)d * Dr, e.S1, true, nullptr, st));
-  // E1: (n = (l0, wl), k = l2) = L[(l0, wl)][l2]
-  PTN_TRY(to_digits(l, Dl, 1, e.E1, false, nullptr, st));
-  // T1^T[(t, rb)][(l0, wl)] -> T1[(l0, wl)][(t, rb)]
-  PTN_TRY(gemm(e.S1, e.E1, e.T1, 1, (long)d * Dr, e.gws, e.gbytes, nullptr, st));
-  // T2[l0][(s, wr)][rb] = sum_(wl, t) W[wl,t,s,wr] T1[l0][(wl, t)][rb]   (stage matrix W^T)
-  PTN_TRY(mpo_stage_f64(e.T1, e.T2, w, 1, (long)d * cr, Dl, cl * d, d * cr, Dr, nullptr, st));
-  // S2: (m = (wr, rb), k = (l0, s)) = T2[(l0, s)][(wr, rb)]
-  PTN_TRY(to_digits(e.T2, 1, (long)cr * Dr, e.S2, false, nullptr, st));
-  // E2: (n = ra, k = (l0, s)) = A[(l0, s)][ra]
-  PTN_TRY(to_digits(a, 1, Dr, e.E2, false, nullptr, st));
-  // l_next^T[(wr, rb)][ra] = S2 . E2^T -> l_next[ra][(wr, rb)]
-  PTN_TRY(gemm(e.S2, e.E2, lnext, 1, (long)cr * Dr, e.gws, e.gbytes, nullptr, st));
-  return PTN_OK;
-}
-
-// r_next[la, wl, lb] = sum A[la,s,r0] W[wl,t,s,wr] R[r0,wr,r2] conj(B[lb,t,r2])
-ptn_status env_right_mixed(const double2* a, const double2* b, const double2* w, const double2* r,
-                           double2* rnext, int Dl, int d, int Dr, int cl, int cr, void* ws,
-                           size_t ws_bytes, cudaStream_t st) {
-  Carver c(ws);
-  EnvWs e = env_right_ws(c, Dl, d, Dr, cl, cr);
-  PTN_CHECK_ARG(ws_bytes >= before_gemm(c, e), "mixed env: workspace too small");
-  use_rest(e, ws, ws_bytes);
-  // S1: (m = (wr, r2), k = r0) = R[r0][(wr, r2)]
-  PTN_TRY(to_digits(r, 1, (long)cr * Dr, e.S1, false, nullptr, st));
-  // E1: (n = (l0, s), k = r0) = A[(l0, s)][r0]
-  PTN_TRY(to_digits(a, Dr, 1, e.E1, false, nullptr, st));
-  // T1^T[(wr, r2)][(l0, s)] -> T1[(l0, s)][(wr, r2)]
-  PTN_TRY(gemm(e.S1, e.E1, e.T1, 1, (long)cr * Dr, e.gws, e.gbytes, nullptr, st));
-  // T2[l0][(wl, t)][r2] = sum_(s, wr) W[(wl, t), (s, wr)] T1[l0][(s, wr)][r2]
-  PTN_TRY(mpo_stage_f64(e.T1, e.T2, w, (long)d * cr, 1, Dl, d * cr, cl * d, Dr, nullptr, st));
-  // E2: (n = (l0, wl), k = (t, r2)) = T2[(l0, wl)][(t, r2)]
-  PTN_TRY(to_digits(e.T2, (long)d * Dr, 1, e.E2, false, nullptr, st));
-  // S2: (m = lb, k = (t, r2)) = conj(B[lb][(t, r2)])
-  PTN_TRY(to_digits(b, (long)d * Dr, 1, e.S2, true, nullptr, st));
-  // r_next^T[lb][(l0, wl)] = S2 . E2^T -> r_next[(l0, wl)][lb]
-  PTN_TRY(gemm(e.S2, e.E2, rnext, 1, Dl, e.gws, e.gbytes, nullptr, st));
-  return PTN_OK;
-}
 
 // ================================================================ plain GEMM entry
 size_t zgemm_split_workspace_bytes(int M, int N, int K) {

@@ -90,8 +90,12 @@ ptn_status env_right_rns(int nm, const double2* a, const double2* b, const doubl
                          const double2* r, double2* rnext, int Dl, int d, int Dr, int cl, int cr,
                          void* ws, size_t ws_bytes, cudaStream_t st);
 
-// whether the FP64 form of a contraction takes the residue planes (contract.cu)
-bool heff_f64_rns(int Dl, int d, int Dr, int cl, int cr);
-bool bond_f64_rns(int Dl, int Dr, int chi);
+// moduli of a contraction's residue planes at precision `prec`, 0: the DMMA kernels (contract.cu)
+int heff_form(int prec, int Dl, int d, int Dr, int cl, int cr);
+int bond_form(int prec, int Dl, int Dr, int chi);
+
+// C = alpha op(A) op(B) + beta C through residue planes (alignment of ws: any)
+size_t zgemm_rns_workspace_bytes(int nm, long M, long N, long K);
+ptn_status zgemm_rns(int nm, const GemmArgs& g, void* ws, cudaStream_t st);
 
 }  // namespace ptn

@@ -1,6 +1,6 @@
 // Site / bond operators and environment steps (pytenet/chain_ops.py:16-99, 237-317) with both
 // GEMMs of every contraction in the residue number system (rns.cu): the FP64 form where the
-// problem is large enough for it (contract.cu decides), the mixed form always.
+// problem is large enough for it (contract.cu decides), the mixed form nearly always.
 //
 // Data flow of H_eff . x (site tensors (Dl, d, Dr), MPO bonds cl / cr); an operand is a set
 // of residue planes, rows x terms:
@@ -226,6 +226,30 @@ ptn_status env_right_rns(int nm, const double2* a, const double2* b, const doubl
   PTN_TRY(rns_gemm_stage(e.a1, v1, e.b1, v2, s, e.res, nullptr, st));
   PTN_TRY(rns_convert(v3, e.a2, true, nullptr, st));
   return rns_gemm(e.a2, v3, e.b2, v4, ONE, ZERO, rnext, Dl, e.res, nullptr, st);
+}
+
+// ================================================================ plain GEMM
+size_t zgemm_rns_workspace_bytes(int nm, long M, long N, long K) {
+  Carver c(nullptr);
+  c.operand(M, K, nm);
+  c.operand(N, K, nm);
+  c.take(rns_out_bytes(M, N, nm));
+  return c.off + 256;
+}
+
+ptn_status zgemm_rns(int nm, const GemmArgs& g, void* ws, cudaStream_t st) {
+  Carver c(reinterpret_cast<void*>(al(reinterpret_cast<uintptr_t>(ws))));
+  const RnsOperand A = c.operand(g.M, g.K, nm);
+  const RnsOperand B = c.operand(g.N, g.K, nm);
+  void* res = c.take(0);
+  // op(A) by rows, op(B) by columns
+  const bool ta = g.opA == 'T' || g.opA == 'H', tb = g.opB == 'T' || g.opB == 'H';
+  const bool ca = g.opA == 'C' || g.opA == 'H', cb = g.opB == 'C' || g.opB == 'H';
+  const RnsView va = ta ? RnsView{g.A, 1, g.lda, ca} : RnsView{g.A, g.lda, 1, ca};
+  const RnsView vb = tb ? RnsView{g.B, g.ldb, 1, cb} : RnsView{g.B, 1, g.ldb, cb};
+  PTN_TRY(rns_convert(va, A, false, g.skip, st));
+  PTN_TRY(rns_convert(vb, B, false, g.skip, st));
+  return rns_gemm(A, va, B, vb, g.alpha, g.beta, g.C, g.ldc, res, g.skip, st);
 }
 
 }  // namespace ptn

@@ -30,20 +30,6 @@ ptn_status heff_apply_f64(const double2*, const double2*, const double2*, const 
 ptn_status bond_apply_f64(const double2*, const double2*, const double2*, double2*, int, int, int,
                           void*, size_t, const int*, cudaStream_t);
 
-// mixed-precision operator (BF16-digit tcgen05 contractions), see mixed.cu
-size_t heff_workspace_bytes_mixed(int Dl, int d, int Dr, int chil, int chir);
-size_t bond_workspace_bytes_mixed(int Dl, int Dr, int chi);
-ptn_status heff_prepare_mixed(const double2* w, const double2* l, const double2* r, int Dl, int d,
-                              int Dr, int chil, int chir, void* ws, size_t ws_bytes,
-                              cudaStream_t st);
-ptn_status heff_apply_mixed(const double2* x, double2* y, const double2* w, int Dl, int d, int Dr,
-                            int chil, int chir, void* ws, size_t ws_bytes, const int* skip,
-                            cudaStream_t st);
-ptn_status bond_prepare_mixed(const double2* l, const double2* r, int Dl, int Dr, int chi, void* ws,
-                              size_t ws_bytes, cudaStream_t st);
-ptn_status bond_apply_mixed(const double2* x, double2* y, int Dl, int Dr, int chi, void* ws,
-                            size_t ws_bytes, const int* skip, cudaStream_t st);
-
 namespace {
 
 struct LocalOp {
@@ -55,34 +41,30 @@ struct LocalOp {
 
   long n() const { return site ? (long)Dl * d * Dr : (long)Dl * Dr; }
 
-  // FP64 through residue planes, converted once per local step; a workspace smaller than
-  // the query asks for leaves the DMMA kernel
-  bool f64_rns() const {
-    if (prec != PTN_PREC_FP64) return false;
-    return site ? heff_f64_rns(Dl, d, Dr, chil, chir) &&
-                      ws_bytes >= heff_workspace_bytes_rns(RNS_FP64, Dl, d, Dr, chil, chir)
-                : bond_f64_rns(Dl, Dr, chil) &&
-                      ws_bytes >= bond_workspace_bytes_rns(RNS_FP64, Dl, Dr, chil);
+  // moduli of the residue planes (the operator's are converted once per local step), or 0:
+  // the DMMA kernels, also where the workspace is smaller than the FP64 query asks for
+  int form() const {
+    const int nm = site ? heff_form(prec, Dl, d, Dr, chil, chir) : bond_form(prec, Dl, Dr, chil);
+    if (nm == 0 || prec != PTN_PREC_FP64) return nm;
+    const size_t need = site ? heff_workspace_bytes_rns(nm, Dl, d, Dr, chil, chir)
+                             : bond_workspace_bytes_rns(nm, Dl, Dr, chil);
+    return ws_bytes >= need ? nm : 0;
   }
 
   ptn_status prepare(cudaStream_t st) const {
-    if (f64_rns())
-      return site ? heff_prepare_rns(RNS_FP64, l, r, Dl, d, Dr, chil, chir, ws, ws_bytes, st)
-                  : bond_prepare_rns(RNS_FP64, l, r, Dl, Dr, chil, ws, ws_bytes, st);
-    if (prec == PTN_PREC_FP64) return PTN_OK;
-    return site ? heff_prepare_mixed(w, l, r, Dl, d, Dr, chil, chir, ws, ws_bytes, st)
-                : bond_prepare_mixed(l, r, Dl, Dr, chil, ws, ws_bytes, st);
+    const int nm = form();
+    if (nm == 0) return PTN_OK;
+    return site ? heff_prepare_rns(nm, l, r, Dl, d, Dr, chil, chir, ws, ws_bytes, st)
+                : bond_prepare_rns(nm, l, r, Dl, Dr, chil, ws, ws_bytes, st);
   }
 
   ptn_status apply(const double2* x, double2* y, const int* skip, cudaStream_t st) const {
-    if (f64_rns())
-      return site ? heff_apply_rns(RNS_FP64, x, y, w, l, r, Dl, d, Dr, chil, chir, ws, skip, st)
-                  : bond_apply_rns(RNS_FP64, x, y, l, r, Dl, Dr, chil, ws, skip, st);
-    if (prec == PTN_PREC_FP64)
+    const int nm = form();
+    if (nm == 0)
       return site ? heff_apply_f64(x, w, l, r, y, Dl, d, Dr, chil, chir, ws, ws_bytes, skip, st)
                   : bond_apply_f64(x, l, r, y, Dl, Dr, chil, ws, ws_bytes, skip, st);
-    return site ? heff_apply_mixed(x, y, w, Dl, d, Dr, chil, chir, ws, ws_bytes, skip, st)
-                : bond_apply_mixed(x, y, Dl, Dr, chil, ws, ws_bytes, skip, st);
+    return site ? heff_apply_rns(nm, x, y, w, l, r, Dl, d, Dr, chil, chir, ws, skip, st)
+                : bond_apply_rns(nm, x, y, l, r, Dl, Dr, chil, ws, skip, st);
   }
 };
 
@@ -124,13 +106,14 @@ using namespace ptn;
 extern "C" {
 
 size_t ptn_site_step_workspace_bytes(int Dl, int d, int Dr, int chil, int chir, int prec) {
-  return prec == PTN_PREC_FP64 ? heff_workspace_bytes_f64(Dl, d, Dr, chil, chir)
-                               : heff_workspace_bytes_mixed(Dl, d, Dr, chil, chir);
+  const int nm = heff_form(prec, Dl, d, Dr, chil, chir);
+  return nm != 0 ? heff_workspace_bytes_rns(nm, Dl, d, Dr, chil, chir)
+                 : heff_workspace_bytes_f64(Dl, d, Dr, chil, chir);
 }
 
 size_t ptn_bond_step_workspace_bytes(int Dl, int Dr, int chi, int prec) {
-  return prec == PTN_PREC_FP64 ? bond_workspace_bytes_f64(Dl, Dr, chi)
-                               : bond_workspace_bytes_mixed(Dl, Dr, chi);
+  const int nm = bond_form(prec, Dl, Dr, chi);
+  return nm != 0 ? bond_workspace_bytes_rns(nm, Dl, Dr, chi) : bond_workspace_bytes_f64(Dl, Dr, chi);
 }
 
 ptn_status ptn_expm_site(ptn_c128* a, const ptn_c128* w, const ptn_c128* l, const ptn_c128* r,

@@ -260,47 +260,9 @@ cudaError_t launch_b(int ob, const Shape& s, const KArgs& k, int batch, cudaStre
 
 void note_launches(int n);
 
-namespace {
-
-inline size_t al(size_t b) { return (b + 255) & ~size_t(255); }
-
-// residue planes of both operands, their row exponents, the residues of the product
-size_t rns_workspace(long M, long N, long K) {
-  return 256 + al(rns_plane_bytes(M, K, RNS_FP64)) + al(rns_plane_bytes(N, K, RNS_FP64)) +
-         al(M * sizeof(int)) + al(N * sizeof(int)) + al(rns_out_bytes(M, N, RNS_FP64));
-}
-
-RnsView operand_view(const double2* src, long ld, bool trans, bool conj) {
-  return trans ? RnsView{src, 1, ld, conj} : RnsView{src, ld, 1, conj};
-}
-
-// C = alpha op(A) op(B) + beta C through the residue planes
-ptn_status zgemm_rns(const GemmArgs& g, int oa, int ob, void* ws, cudaStream_t st) {
-  char* p = reinterpret_cast<char*>(al(reinterpret_cast<uintptr_t>(ws)));
-  auto take = [&](size_t bytes) {
-    void* q = p;
-    p += al(bytes);
-    return q;
-  };
-  void* pa = take(rns_plane_bytes(g.M, g.K, RNS_FP64));
-  void* pb = take(rns_plane_bytes(g.N, g.K, RNS_FP64));
-  void* ea = take(g.M * sizeof(int));
-  void* eb = take(g.N * sizeof(int));
-  const RnsOperand A = rns_operand(pa, ea, g.M, g.K, RNS_FP64);
-  const RnsOperand B = rns_operand(pb, eb, g.N, g.K, RNS_FP64);
-  const bool ta = oa == OP_T || oa == OP_H, tb = ob == OP_T || ob == OP_H;
-  const RnsView va = operand_view(g.A, g.lda, ta, oa == OP_C || oa == OP_H);
-  const RnsView vb = operand_view(g.B, g.ldb, !tb, ob == OP_C || ob == OP_H);
-  PTN_TRY(rns_convert(va, A, false, g.skip, st));
-  PTN_TRY(rns_convert(vb, B, false, g.skip, st));
-  return rns_gemm(A, va, B, vb, g.alpha, g.beta, g.C, g.ldc, p, g.skip, st);
-}
-
-}  // namespace
-
 // the DMMA kernel splits K inside the launch (clusters) and needs no scratch
 size_t zgemm_workspace_bytes(int M, int N, int K, int batch) {
-  return batch == 1 && rns_wanted(M, N, K) ? rns_workspace(M, N, K) : 0;
+  return batch == 1 && rns_wanted(M, N, K) ? zgemm_rns_workspace_bytes(RNS_FP64, M, N, K) : 0;
 }
 
 ptn_status zgemm(const GemmArgs& g, void* ws, size_t ws_bytes, cudaStream_t st) {
@@ -310,8 +272,8 @@ ptn_status zgemm(const GemmArgs& g, void* ws, size_t ws_bytes, cudaStream_t st) 
   if (g.M == 0 || g.N == 0) return PTN_OK;
   // a smaller workspace than the query asks for: the DMMA kernel
   if (g.batch == 1 && rns_wanted(g.M, g.N, g.K) && ws != nullptr &&
-      ws_bytes >= rns_workspace(g.M, g.N, g.K))
-    return zgemm_rns(g, oa, ob, ws, st);
+      ws_bytes >= zgemm_rns_workspace_bytes(RNS_FP64, g.M, g.N, g.K))
+    return zgemm_rns(RNS_FP64, g, ws, st);
   KArgs k;
   k.M = g.M; k.N = g.N; k.K = g.K;
   k.alpha = g.alpha; k.beta = g.beta;

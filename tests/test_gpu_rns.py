@@ -148,3 +148,22 @@ def test_infinities_and_nans(bad):
     same[7] = False
     same[:, 15] = False
     assert np.array_equal(got[same], clean[same])
+
+
+@pytest.mark.parametrize("dims", [(32, 2, 40, 3, 5), (33, 3, 37, 5, 4), (129, 2, 65, 5, 5), (40, 2, 1100, 3, 3)])
+def test_mixed_contractions_in_residues(dims):
+    """The mixed form of every contraction (40 bits and more per operand row) on odd bonds, a
+    physical dimension of 3, unequal MPO bonds and rows longer than one CTA converts: within
+    2^-38 of the row maxima per term, by the bound of the FP64 planes at 40 bits."""
+    import pytenet_gb300 as ptg
+    Dl, d, Dr, cl, cr = dims
+    rng = np.random.default_rng(sum(dims))
+    a, b = crandn(rng, Dl, d, Dr), crandn(rng, Dl, d, Dr)
+    w = rng.standard_normal((cl, d, d, cr))
+    w[np.abs(w) < 0.7] = 0.0
+    l, r = crandn(rng, Dl, cl, Dl), crandn(rng, Dr, cr, Dr)
+    for fn, args, tr in ((ptg.apply_local_hamiltonian, (a, w, l, r), None),
+                         (ptg.contraction_operator_step_left, (a, b, w, l), None),
+                         (ptg.contraction_operator_step_right, (a, b, w, r), None)):
+        got, ref = fn(*args, precision="mixed"), fn(*args, precision="fp64")
+        assert np.linalg.norm(got - ref) < 1e-11 * np.linalg.norm(ref), fn.__name__
