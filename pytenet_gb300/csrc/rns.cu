@@ -26,11 +26,14 @@
 // range, are multiplied entry by entry in FP64 by the reconstruction kernel.
 #include "rns.cuh"
 #include "mpo_stage.cuh"
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <algorithm>
 #include <climits>
 #include <cmath>
 #include <mutex>
+
+namespace cg = cooperative_groups;
 
 namespace ptn {
 
@@ -132,14 +135,20 @@ constexpr bool moduli_ok() {
 }
 static_assert(moduli_ok(), "moduli: odd, pairwise coprime, -1 a square");
 
-__constant__ RnsConst<RNS_FP64> c_fp64 = make_const<RNS_FP64>();
-__constant__ RnsConst<RNS_MIXED> c_mixed = make_const<RNS_MIXED>();
-
-template <int NM>
-__device__ __forceinline__ const RnsConst<NM>& rns_const() {
-  if constexpr (NM == RNS_FP64) return c_fp64;
-  else return c_mixed;
+// p and 1 / p by run-time index (the GEMM's epilogue); the other kernels unroll over the
+// moduli and take every constant as an immediate operand
+struct ModTable {
+  float p[NMOD], inv[NMOD];
+};
+constexpr ModTable make_table() {
+  ModTable t{};
+  for (int i = 0; i < NMOD; ++i) {
+    t.p[i] = (float)MOD[i];
+    t.inv[i] = 1.0f / (float)MOD[i];
+  }
+  return t;
 }
+__constant__ ModTable c_mod = make_table();
 
 constexpr float MAGIC = 12582912.0f;   // 1.5 2^23: adding it rounds to an integer
 
@@ -161,49 +170,6 @@ constexpr int EXP_TINY = 200;
 __device__ __forceinline__ bool special(int E) { return E == 2047 || (E != 0 && E < EXP_TINY); }
 
 // ------------------------------------------------------------------ conversion
-constexpr int TR = 32, TK = 64;        // conversion tile: rows x terms
-constexpr int TP = TK + 1;
-
-// tile of the view in shared memory; threads (32, 8), coalesced along the unit stride
-__device__ __forceinline__ void load_tile(double2 (*tile)[TP], const RnsView& v, int R, int K,
-                                          int r0, int k0) {
-  const int lane = threadIdx.x, w = threadIdx.y;
-  const double2 zero = make_double2(0.0, 0.0);
-  if (v.sk == 1) {
-    for (int rr = w; rr < TR; rr += 8)
-#pragma unroll
-      for (int h = 0; h < TK; h += 32) {
-        const int r = r0 + rr, k = k0 + h + lane;
-        tile[rr][h + lane] = (r < R && k < K) ? v.src[(long)r * v.sr + k] : zero;
-      }
-  } else {
-    for (int kk = w; kk < TK; kk += 8) {
-      const int r = r0 + lane, k = k0 + kk;
-      tile[lane][kk] = (r < R && k < K) ? v.src[(long)r * v.sr + (long)k * v.sk] : zero;
-    }
-  }
-}
-
-__global__ void __launch_bounds__(256) k_row_exp(const RnsView v, int R, int K, int* __restrict__ e,
-                                                 const int* skip) {
-  if (skip != nullptr && *skip != 0) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2 (*tile)[TP] = reinterpret_cast<double2 (*)[TP]>(smem_raw);
-  const int r0 = blockIdx.x * TR, k0 = blockIdx.y * TK;
-  load_tile(tile, v, R, K, r0, k0);
-  __syncthreads();
-  for (int rr = threadIdx.y; rr < TR; rr += 8) {
-    int m = 0;
-#pragma unroll
-    for (int h = 0; h < TK; h += 32) {
-      const double2 z = tile[rr][h + threadIdx.x];
-      m = max(m, max(biased_exp(z.x), biased_exp(z.y)));
-    }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if (threadIdx.x == 0 && r0 + rr < R && m > 0) atomicMax(&e[r0 + rr], m);
-  }
-}
-
 // pieces of T = round(x 2^(bits - e)), |x| < 2^e = 2^(E - 1022), as signed floats
 __device__ __forceinline__ void pieces_of(double x, int E, int bits, float (&f)[PIECES]) {
   const long long b = __double_as_longlong(x);
@@ -229,7 +195,7 @@ __device__ __forceinline__ void pieces_of(double x, int E, int bits, float (&f)[
 template <int NM>
 __device__ __forceinline__ void convert_pair(const double2 (&z)[2], int E, int bits,
                                              bf16* __restrict__ row, long plane) {
-  const RnsConst<NM>& c = rns_const<NM>();
+  constexpr RnsConst<NM> c = make_const<NM>();
   float px[2][PIECES], py[2][PIECES];
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
@@ -257,40 +223,104 @@ __device__ __forceinline__ void convert_pair(const double2 (&z)[2], int E, int b
   }
 }
 
-// Residue planes of a tile of any view (row exponents known). Bound: the FP32 pipe, then
-// the writes (4 nm bytes per entry). A lane holds two neighbouring terms, so a warp writes
-// 128 contiguous bytes per plane and row.
+// Residue planes of a view with any strides: a CTA takes 8 rows (128 contiguous bytes per
+// term of a transposed view) and part of the terms into shared memory; the CTAs of a
+// cluster share the rows' terms and exchange the row maxima, so the view is read once and
+// nothing is zeroed before. `have_exp`: the exponents are in e (no exchange). Bound: the
+// FP32 pipe, then the writes (4 nm bytes per entry). A lane holds two neighbouring terms,
+// so a warp (one row) writes 128 contiguous bytes per plane.
+// Measured, 1280 x 250: 23.5 us in three launches (memset, maximum, conversion) -> 12.0.
+constexpr int CR = 8;              // rows of a CTA
+constexpr int CK_MAX = 1024;       // most terms of a CTA (128 KB)
+
 template <int NM>
-__global__ void __launch_bounds__(256) k_convert(const RnsView v, int R, int K,
-                                                 const int* __restrict__ e, int bits,
+__global__ void __launch_bounds__(256) k_convert(const RnsView v, int R, int K, int chunk,
+                                                 int* __restrict__ e, int have_exp, int bits,
                                                  bf16* __restrict__ dst, long Kp, long plane,
+                                                 int* __restrict__ clear, int nclear,
                                                  const int* skip) {
-  if (skip != nullptr && *skip != 0) return;
+  if (skip != nullptr && *skip != 0) return;   // uniform over the launch
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2 (*tile)[TP] = reinterpret_cast<double2 (*)[TP]>(smem_raw);
-  const int r0 = blockIdx.x * TR, k0 = blockIdx.y * TK;
-  load_tile(tile, v, R, K, r0, k0);
+  double2* tile = reinterpret_cast<double2*>(smem_raw);   // [CR][chunk + 1]
+  __shared__ int s_max[CR];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r0 = blockIdx.x * CR, k0 = blockIdx.y * chunk, ld = chunk + 1;
+  const int kn = min(chunk, K - k0);           // terms of this CTA (the last may have fewer)
+  for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * 256 + tid; i < nclear;
+       i += gridDim.x * gridDim.y * 256)
+    clear[i] = 0;
+  if (tid < CR) s_max[tid] = 0;
+  if (v.sk == 1) {
+    const int r = r0 + warp;
+    for (int k = lane; k < chunk; k += 32)
+      tile[warp * ld + k] = (r < R && k < kn) ? v.src[(long)r * v.sr + k0 + k] : make_double2(0.0, 0.0);
+  } else {
+    const int rr = tid & 7, r = r0 + rr;
+    for (int k = tid >> 3; k < chunk; k += 32)
+      tile[rr * ld + k] = (r < R && k < kn) ? v.src[(long)r * v.sr + (long)(k0 + k) * v.sk]
+                                            : make_double2(0.0, 0.0);
+  }
   __syncthreads();
-  const int k = k0 + 2 * threadIdx.x;
-  if (k >= Kp) return;
-  for (int rr = threadIdx.y; rr < TR; rr += 8) {
-    const int r = r0 + rr;
-    if (r >= R) break;
-    const int E = e[r];
-    const bool live = E != 0 && !special(E);
+  const double2* row = tile + warp * ld;
+  const int r = r0 + warp;
+  int E;
+  if (have_exp) {
+    E = r < R ? e[r] : 0;
+  } else {
+    E = 0;
+    for (int k = lane; k < kn; k += 32) E = max(E, max(biased_exp(row[k].x), biased_exp(row[k].y)));
+    E = __reduce_max_sync(0xffffffffu, E);
+    if (gridDim.y > 1) {
+      cg::cluster_group cluster = cg::this_cluster();
+      if (lane == 0) s_max[warp] = E;
+      cluster.sync();
+      E = lane < (int)gridDim.y ? *cluster.map_shared_rank(&s_max[warp], lane) : 0;
+      E = __reduce_max_sync(0xffffffffu, E);
+      cluster.sync();   // no CTA leaves while its maxima are read
+    }
+    if (lane == 0 && blockIdx.y == 0 && r < R) e[r] = E;
+  }
+  if (r >= R) return;
+  const bool live = E != 0 && !special(E);
+  const int kend = (int)min((long)chunk, Kp - k0);
+  for (int k = 2 * lane; k < kend; k += 64) {
     double2 z[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      z[q] = live ? tile[rr][2 * threadIdx.x + q] : make_double2(0.0, 0.0);
+      z[q] = live ? row[k + q] : make_double2(0.0, 0.0);
       if (v.conj) z[q].y = -z[q].y;
     }
-    convert_pair<NM>(z, E, bits, dst + (long)r * Kp + k, plane);
+    convert_pair<NM>(z, E, bits, dst + (long)r * Kp + k0 + k, plane);
   }
 }
 
-// Views with contiguous rows: one warp finds the exponent of its row and converts it (the
-// second read hits L1 / L2): one launch instead of a memset, a maximum pass and a
-// conversion. Also zeroes clear[0 .. nclear) for a later kernel of the stream.
+// The exponents alone, for rows too long for a cluster (e zeroed before).
+__global__ void __launch_bounds__(256) k_row_exp(const RnsView v, int R, int K, int* __restrict__ e,
+                                                 const int* skip) {
+  if (skip != nullptr && *skip != 0) return;
+  __shared__ int s_max[32];
+  const int rr = v.sk == 1 ? (int)threadIdx.x >> 5 : (int)threadIdx.x & 7;
+  const int kk = v.sk == 1 ? (int)threadIdx.x & 31 : (int)threadIdx.x >> 3;
+  if (threadIdx.x < CR) s_max[threadIdx.x] = 0;
+  __syncthreads();
+  const int r = blockIdx.x * CR + rr;
+  int m = 0;
+  if (r < R)
+    for (long k = blockIdx.y * (long)CK_MAX + kk; k < min((long)K, (blockIdx.y + 1) * (long)CK_MAX); k += 32) {
+      const double2 z = v.src[(long)r * v.sr + k * v.sk];
+      m = max(m, max(biased_exp(z.x), biased_exp(z.y)));
+    }
+  atomicMax(&s_max[rr], m);
+  __syncthreads();
+  if (threadIdx.x < CR && blockIdx.x * CR + threadIdx.x < R && s_max[threadIdx.x] > 0)
+    atomicMax(&e[blockIdx.x * CR + threadIdx.x], s_max[threadIdx.x]);
+}
+
+// Views with contiguous rows of at most ROW_MAX terms: one warp finds the exponent of its
+// row and converts it (the second read hits L1 / L2). Also zeroes clear[0 .. nclear) for a
+// later kernel of the stream.
+constexpr int ROW_MAX = 512;
+
 template <int NM>
 __global__ void __launch_bounds__(128) k_convert_rows(const RnsView v, int R, int K,
                                                       int* __restrict__ e, int bits,
@@ -576,7 +606,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (int u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
       const int n0 = (u % g.gx) * BN + half * T::COLS, pl = u / (g.gx * g.gy);
       const int row = ((u / g.gx) % g.gy) * BM + 32 * quad + lane;
-      const float p = c_fp64.p[pl >> 1], inv = c_fp64.inv[pl >> 1];
+      const float p = c_mod.p[pl >> 1], inv = c_mod.inv[pl >> 1];
       float acc[T::COLS];
       for (int c = 0; c < nch; ++c, ++ch) {
         const int b = ch & 1;
@@ -724,7 +754,7 @@ __device__ __forceinline__ void load_residues(const unsigned short* __restrict__
 template <int NM>
 __device__ __forceinline__ double2 element(const ReconP& g, int m, int n, int q,
                                            const unsigned (&ru)[NM], const unsigned (&rv)[NM]) {
-  const RnsConst<NM>& c = rns_const<NM>();
+  constexpr RnsConst<NM> c = make_const<NM>();
   const int Ea = g.ea[m], Eb = g.eb[n];
   u64 x0 = 0, x1 = 0, y0 = 0, y1 = 0;
   unsigned x2 = 0, y2 = 0;
@@ -982,38 +1012,72 @@ bool rns_wanted(long M, long N, long K) {
 }
 
 template <int NM>
-static void launch_convert(const RnsView& v, const RnsOperand& d, int bits, bool rows, dim3 grid,
-                           int smem, int* clear, int nclear, const int* skip, cudaStream_t st) {
-  if (rows)
-    k_convert_rows<NM><<<(d.rows + 3) / 4, 128, 0, st>>>(v, d.rows, d.kc, d.e, bits, d.p, d.Kp,
-                                                         d.plane(), clear, nclear, skip);
-  else
-    k_convert<NM><<<grid, dim3(32, 8), smem, st>>>(v, d.rows, d.kc, d.e, bits, d.p, d.Kp,
-                                                   d.plane(), skip);
+static ptn_status launch_convert(const RnsView& v, const RnsOperand& d, bool have_exp, int bits,
+                                 int* clear, int nclear, const int* skip, cudaStream_t st) {
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(k_convert<NM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                CR * (CK_MAX + 1) * (int)sizeof(double2));
+  });
+  PTN_CUDA_TRY(attr);
+  // terms per CTA: enough CTAs for the chip, multiples of 64, at most 8 CTAs to a row where
+  // the maxima are exchanged
+  const long groups = (d.rows + CR - 1) / CR;
+  const long want = std::max<long>(1, 2L * num_sms() / groups);
+  const long blocks64 = (d.kc + 63) / 64;
+  long parts = std::min(want, blocks64);
+  parts = std::max(parts, ((long)d.kc + CK_MAX - 1) / CK_MAX);
+  if (!have_exp) parts = std::min(parts, 8L);
+  const long chunk = (blocks64 + parts - 1) / parts * 64;
+  parts = (d.kc + chunk - 1) / chunk;
+  if (chunk > CK_MAX) {   // longer than a cluster takes: the exponents in a pass of their own
+    PTN_CUDA_TRY(cudaMemsetAsync(d.e, 0, (size_t)d.rows * sizeof(int), st));
+    const dim3 ge((unsigned)groups, (unsigned)((d.kc + CK_MAX - 1) / CK_MAX));
+    PTN_CHECK_ARG(ge.y <= 65535, "rns_convert: too many columns");
+    k_row_exp<<<ge, 256, 0, st>>>(v, d.rows, d.kc, d.e, skip);
+    PTN_LAUNCH_CHECK();
+    note_launches(1);
+    return launch_convert<NM>(v, d, true, bits, clear, nclear, skip, st);
+  }
+  PTN_CHECK_ARG(parts <= 65535, "rns_convert: too many columns");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)groups, (unsigned)parts);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = CR * (size_t)(chunk + 1) * sizeof(double2);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = (unsigned)parts;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = have_exp ? 0 : 1;
+  PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_convert<NM>, v, d.rows, d.kc, (int)chunk, d.e,
+                                  have_exp ? 1 : 0, bits, d.p, d.Kp, d.plane(), clear, nclear, skip));
+  note_launches(1);
+  return PTN_OK;
+}
+
+template <int NM>
+static ptn_status convert(const RnsView& v, const RnsOperand& d, bool have_exp, int bits,
+                          int* clear, int nclear, const int* skip, cudaStream_t st) {
+  if (v.sk != 1 || have_exp || d.kc > ROW_MAX)
+    return launch_convert<NM>(v, d, have_exp, bits, clear, nclear, skip, st);
+  k_convert_rows<NM><<<(d.rows + 3) / 4, 128, 0, st>>>(v, d.rows, d.kc, d.e, bits, d.p, d.Kp,
+                                                       d.plane(), clear, nclear, skip);
+  PTN_LAUNCH_CHECK();
+  note_launches(1);
+  return PTN_OK;
 }
 
 ptn_status rns_convert(const RnsView& v, const RnsOperand& d, bool have_exp, const int* skip,
                        cudaStream_t st, int* clear, int nclear) {
   const int bits = rns_bits(d.kc, d.nm);
   PTN_CHECK_ARG(bits != 0, "rns_convert: products of %d terms are too long", d.kc);
-  const dim3 grid((unsigned)((d.rows + TR - 1) / TR), (unsigned)((d.kc + TK - 1) / TK));
-  PTN_CHECK_ARG(grid.y <= 65535, "rns_convert: too many columns");
-  constexpr int smem = TR * TP * sizeof(double2);
-  const bool rows = v.sk == 1 && !have_exp;
-  int launches = 1;
-  if (!rows) {
-    if (nclear > 0) PTN_CUDA_TRY(cudaMemsetAsync(clear, 0, (size_t)nclear * sizeof(int), st));
-    if (!have_exp) {
-      PTN_CUDA_TRY(cudaMemsetAsync(d.e, 0, (size_t)d.rows * sizeof(int), st));
-      k_row_exp<<<grid, dim3(32, 8), smem, st>>>(v, d.rows, d.kc, d.e, skip);
-      ++launches;
-    }
-  }
-  if (d.nm == RNS_FP64) launch_convert<RNS_FP64>(v, d, bits, rows, grid, smem, clear, nclear, skip, st);
-  else launch_convert<RNS_MIXED>(v, d, bits, rows, grid, smem, clear, nclear, skip, st);
-  PTN_LAUNCH_CHECK();
-  note_launches(launches);
-  return PTN_OK;
+  return d.nm == RNS_FP64
+             ? convert<RNS_FP64>(v, d, have_exp, bits, clear, nclear, skip, st)
+             : convert<RNS_MIXED>(v, d, have_exp, bits, clear, nclear, skip, st);
 }
 
 // the integer products of all planes -> res, and what their reconstruction needs
