@@ -11,22 +11,37 @@
 // t = sign(zeta) / (|zeta| + sqrt(1 + zeta^2)), cs = 1 / sqrt(1 + t^2), sn = cs t
 // zeroes it: w_j <- cs w_j - sn w_k, w_k <- sn w_j + cs w_k. The same unitary column
 // operations accumulate in V (r x r, starting at I). Pairs follow the round-robin
-// (circle) order, r/2 disjoint pairs per round, one warp per pair; a sweep is
-// r - 1 rounds; sweeps repeat until no pair has |c| > tol sqrt(a b)
-// (tol = p * eps), at most MAX_SWEEPS of them. Then s_j = |w_j|, the columns are
-// sorted by decreasing s (ties by index, LAPACK's order), U = W / s, and
-// A = U diag(s) V^H (for a wide A the roles of U and V swap).
+// (circle) order, r/2 disjoint pairs per round; a sweep is r - 1 rounds; sweeps repeat
+// until no pair has |c| > tol sqrt(a b) (tol = p * eps), at most MAX_SWEEPS of them.
+// Then s_j = |w_j|, the columns are sorted by decreasing s (ties by index, LAPACK's
+// order), U = W / s, and A = U diag(s) V^H (for a wide A the roles of U and V swap).
+//
+// From PRE_MIN columns on, the sweeps start from the singular vectors found by the same
+// iteration in FP32 (mixed-precision Jacobi: Gao, Ma and Shao 2022): V32 is made unitary in
+// FP64 by a Newton-Schulz step and then improved twice for all pairs at once by GEMMs: with
+// G = W^H W, W = A V, the first-order rotation V (I + X), X_ij = G_ij / (G_jj - G_ii), leaves
+// the square of the off-diagonal part (pairs too close for that are left to the sweeps), and
+// two more Newton-Schulz steps make it unitary. The FP64 sweeps, whose stopping rule and so
+// whose accuracy stay as they are, then mostly verify: one sweep instead of nine or ten.
+// What bounds the iteration: an FP64 instruction of a warp takes 64 cycles of its
+// sub-partition; the FP32 sweeps cost only their rounds' latency (L2 round trip, cluster
+// barrier).
 //
 // Singular vectors of one singular value are unique only up to a phase (or a
 // unitary mix for repeated values): they need not equal LAPACK's, while the
 // singular values, the products U diag(s) V^H and every quantity built from a
 // truncated split agree to rounding.
 //
-// One CTA per matrix: for the block sizes of quantum-number blocks and of the
-// two-site steps at moderate bond dimension (hundreds); larger dense blocks take
-// O(r^2 p) FP64 work per sweep on a single SM.
+// One cluster of up to 16 CTAs per matrix: a round's pairs are spread over the CTAs, four
+// warps to a pair; the columns stay in global memory (L2), a cluster barrier ends a round.
+// Measured, 128 x 96: 75.6 ms (one CTA, FP64 sweeps only) -> 2.45 ms (FP32 sweeps 1.57,
+// GEMMs 0.25, FP64 sweeps 0.57).
 #include "ptn_common.cuh"
+#include <cooperative_groups.h>
 #include <algorithm>
+#include <mutex>
+
+namespace cg = cooperative_groups;
 
 namespace ptn {
 
@@ -34,17 +49,388 @@ void note_launches(int n);
 
 namespace {
 
-constexpr int ST = 256;           // threads per CTA
-constexpr int NWARP = ST / 32;
+constexpr int GROUP = 128;        // threads that share a pair
+constexpr int NGROUP = 4;         // groups per CTA
+constexpr int ST = GROUP * NGROUP;
 constexpr int MAX_SWEEPS = 60;
+constexpr int PRE_SWEEPS = 15;    // at most that many FP32 sweeps
+constexpr int PRE_MIN = 32;       // columns from which the FP32 sweeps pay
+constexpr int NS = 5;             // Newton-Schulz steps: one, and two after each refinement
+// Largest first-order rotation times the column count, by step: |X| <= X_NORM, so V is off
+// unitary by X_NORM^2 at most, and every Newton-Schulz step takes an error e to 0.75 e^2
+// (0.1: 1e-2 -> 8e-5 -> 4e-9; 1e-3: 1e-6 -> 8e-13 -> below rounding).
+constexpr int REFINE = 2;
+constexpr double X_NORM[REFINE] = {0.1, 1e-3};
+constexpr int REG = 4;            // column entries a thread keeps in registers
 
-__device__ __forceinline__ double warp_sum(double x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
+template <typename T>
+struct Cplx;
+template <>
+struct Cplx<double> {
+  typedef double2 type;
+};
+template <>
+struct Cplx<float> {
+  typedef float2 type;
+};
+
+// four values summed over the warp with seven additions: value q ends in the lanes with
+// (lane & 3) == q
+template <typename T>
+__device__ __forceinline__ T warp_sum4(T v0, T v1, T v2, T v3) {
+  const int lane = threadIdx.x & 31;
+  const bool h1 = lane & 1, h2 = lane & 2;
+  // lanes exchange the half they do not keep
+  const T a = (h1 ? v1 : v0) + __shfl_xor_sync(0xffffffffu, h1 ? v0 : v1, 1);
+  const T b = (h1 ? v3 : v2) + __shfl_xor_sync(0xffffffffu, h1 ? v2 : v3, 1);
+  T c = (h2 ? b : a) + __shfl_xor_sync(0xffffffffu, h2 ? a : b, 2);
+  c += __shfl_xor_sync(0xffffffffu, c, 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 8);
+  c += __shfl_xor_sync(0xffffffffu, c, 16);
+  return c;
 }
 
-// W (p x r) and V (r x r) are column-major scratch; u, vh row-major outputs.
+// Rotation of a pair: x' = cs x - g y, y' = sn x + h y
+template <typename T>
+struct Rot {
+  T cs, sn, gr, gi, hr, hi;
+  int on;
+};
+
+// off: |c| / sqrt(a b) as far as FP32 tells. FP32 form.
+__device__ __forceinline__ Rot<float> rotation(float aa, float bb, float cr, float ci, float tol,
+                                               float& off) {
+  Rot<float> R;
+  R.on = 0;
+  off = 0.0f;
+  // columns below 1e-15 of the largest entry: beyond what FP32 resolves (and their products
+  // near the end of its range)
+  if (!(aa > 1e-30f && bb > 1e-30f)) return R;
+  const float mx = fmaxf(fabsf(cr), fabsf(ci)), ab = sqrtf(aa) * sqrtf(bb);
+  if (!(mx > 0.5f * tol * ab)) return R;
+  const float ur = cr / mx, ui = ci / mx, ul = rsqrtf(ur * ur + ui * ui);
+  const float ac = mx / ul;
+  off = ac / ab;
+  R.on = ac > tol * ab;
+  if (!R.on) return R;
+  const float pr = ur * ul, pi = -ui * ul;
+  const float z = (bb - aa) / (2.0f * ac);
+  const float t = copysignf(1.0f, z) / (fabsf(z) + sqrtf(1.0f + z * z));
+  R.cs = rsqrtf(1.0f + t * t);
+  R.sn = R.cs * t;
+  R.gr = R.sn * pr;
+  R.gi = R.sn * pi;
+  R.hr = R.cs * pr;
+  R.hi = R.cs * pi;
+  return R;
+}
+
+__device__ __forceinline__ int exp_of(double x) {
+  return (int)((__double_as_longlong(x) >> 52) & 0x7FF) - 1023;
+}
+
+// x 2^-h as a float (0 below, infinity above its range), integer work only
+__device__ __forceinline__ float scaled_float(double x, int h) {
+  const long long b = __double_as_longlong(x);
+  const int e = (int)((b >> 52) & 0x7FF) - h - 1023 + 127;
+  const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
+  if (((b >> 52) & 0x7FF) == 0 || e <= 0) return __uint_as_float(sign);
+  if (e >= 255) return __uint_as_float(sign | 0x7F800000u);
+  return __uint_as_float(sign | ((unsigned)e << 23) | ((unsigned)(b >> 29) & 0x7FFFFFu));
+}
+
+// 1 / sqrt(x^2 + y^2) to FP64 accuracy from an FP32 seed (one third-order step), for sums
+// near 1 .. 2
+__device__ __forceinline__ double inv_norm(double x, double y) {
+  const double d = fma(x, x, y * y);
+  const double s = (double)rsqrtf((float)d);
+  const double e = fma(-d * s, s, 1.0);
+  return fma(s * e, fma(e, 0.375, 0.5), s);
+}
+
+// FP64 throughout: columns of very different size, or near the lower end of the range
+__device__ __noinline__ Rot<double> rotation_fp64(double aa, double bb, double cr, double ci,
+                                                  double tol, float& off) {
+  Rot<double> R;
+  const double ac = sqrt(cr * cr + ci * ci), ab = sqrt(aa) * sqrt(bb);
+  R.on = ac > 0.0 && ac > tol * ab;
+  off = R.on ? (float)fmax(ac / ab, 1e-30) : 0.0f;
+  if (!R.on) return R;
+  const double pr = cr / ac, pi = -ci / ac;
+  const double z = (bb - aa) / (2.0 * ac);
+  const double t = copysign(1.0, z) / (fabs(z) + sqrt(1.0 + z * z));
+  R.cs = 1.0 / sqrt(1.0 + t * t);
+  R.sn = R.cs * t;
+  R.gr = R.sn * pr;
+  R.gi = R.sn * pi;
+  R.hr = R.cs * pr;
+  R.hi = R.cs * pi;
+  return R;
+}
+
+// FP64 form, by a whole warp (all lanes get the result). The angle and the phase need only
+// FP32 accuracy (an angle off by 1e-7 leaves 1e-7 of c, as good as another sweep); the
+// rotation itself is unitary to FP64 accuracy: lane 0 forms cs = (1 + t^2)^-1/2, lane 1 the
+// modulus of the FP32 phase, with the same instructions. FP64 divisions and square roots
+// would take 64 cycles for every one of their dozens of steps.
+__device__ __forceinline__ Rot<double> rotation(double aa, double bb, double cr, double ci,
+                                                double tol, float& off) {
+  Rot<double> R;
+  const int ea = exp_of(aa), eb = exp_of(bb), h = (ea + eb) >> 1;
+  R.on = 0;
+  off = 0.0f;
+  if (ea == 1024 || eb == 1024) return R;            // overflow, NaN: left alone
+  if (ea < -960 || eb < -960) return rotation_fp64(aa, bb, cr, ci, tol, off);
+  const float fr = scaled_float(cr, h), fi = scaled_float(ci, h);
+  const float ab = scaled_float(aa, ea) * scaled_float(bb, eb) * ((ea + eb) & 1 ? 2.0f : 1.0f);
+  const float c2v = fr * fr + fi * fi;
+  off = c2v > 0.0f ? sqrtf(c2v / ab) : 0.0f;
+  R.on = off > (float)tol;
+  if (!R.on) return R;
+  const int lane = threadIdx.x & 31;
+  const float rc = rsqrtf(c2v);
+  const double pr = (double)(fr * rc), pi = (double)(-fi * rc);
+  const double diff = bb - aa;
+  const float z = scaled_float(diff, h) * 0.5f * rc;
+  if (!(fabsf(z) < 1e15f)) return rotation_fp64(aa, bb, cr, ci, tol, off);
+  const double t = (double)(copysignf(1.0f, z) / (fabsf(z) + sqrtf(1.0f + z * z)));
+  const double v = inv_norm(lane == 0 ? t : pr, lane == 0 ? 1.0 : pi);
+  R.cs = __shfl_sync(0xffffffffu, v, 0);
+  const double s = __shfl_sync(0xffffffffu, v, 1);
+  R.sn = R.cs * t;
+  const double qr = pr * s, qi = pi * s;
+  R.gr = R.sn * qr;
+  R.gi = R.sn * qi;
+  R.hr = R.cs * qr;
+  R.hi = R.cs * qi;
+  return R;
+}
+
+template <typename T, typename T2>
+__device__ __forceinline__ void rotate(const Rot<T>& R, T2& x, T2& y) {
+  T2 u, v;
+  u.x = R.cs * x.x;
+  u.x = fma(-R.gr, y.x, u.x);
+  u.x = fma(R.gi, y.y, u.x);
+  u.y = R.cs * x.y;
+  u.y = fma(-R.gr, y.y, u.y);
+  u.y = fma(-R.gi, y.x, u.y);
+  v.x = R.sn * x.x;
+  v.x = fma(R.hr, y.x, v.x);
+  v.x = fma(-R.hi, y.y, v.x);
+  v.y = R.sn * x.y;
+  v.y = fma(R.hr, y.y, v.y);
+  v.y = fma(R.hi, y.x, v.y);
+  x = u;
+  y = v;
+}
+
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(GROUP) : "memory");
+}
+
+// The sweeps over W (p x r) and V (r x r), column-major in global memory, by a cluster;
+// returns the number of sweeps. A sweep in which no pair was further from orthogonal than
+// `last` is the last one (0: a sweep without rotations is).
+template <typename T>
+__device__ int sweeps(typename Cplx<T>::type* __restrict__ W, typename Cplx<T>::type* __restrict__ V,
+                      int p, int r, T tol, float last, int max_sweeps) {
+  typedef typename Cplx<T>::type T2;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int g = tid / GROUP, gt = tid % GROUP, gw = gt >> 5;
+  __shared__ T s_sum[NGROUP][4][4];
+  __shared__ Rot<T> s_rot[NGROUP];
+  __shared__ int s_off[2];          // largest off-orthogonality of a sweep (float bits)
+  if (tid < 2) s_off[tid] = 0;
+  const int rr = r + (r & 1);       // an odd count plays against an absent column
+  cluster.sync();
+  int sweep = 0;
+  for (; sweep < max_sweeps; ++sweep) {
+    int worst = 0;
+    for (int q = 0; q < rr - 1; ++q) {
+      for (int t = rank + cs * g; t < rr / 2; t += cs * NGROUP) {
+        int j = t == 0 ? 0 : 1 + (q + t) % (rr - 1);
+        int k = t == 0 ? 1 + q : 1 + (q + rr - 1 - t) % (rr - 1);
+        if (j > k) {
+          const int x = j;
+          j = k;
+          k = x;
+        }
+        if (k >= r) continue;
+        T2* wj = W + (long)j * p;
+        T2* wk = W + (long)k * p;
+        T2* vj = V + (long)j * r;
+        T2* vk = V + (long)k * r;
+        T2 x[REG], y[REG], a, b;
+        T aa = 0, bb = 0, cr = 0, ci = 0;
+#pragma unroll
+        for (int e = 0; e < REG; ++e) {
+          const int i = gt + e * GROUP;
+          if (i < p) {
+            x[e] = __ldcg(wj + i);
+            y[e] = __ldcg(wk + i);
+          } else {
+            x[e].x = x[e].y = y[e].x = y[e].y = 0;
+          }
+        }
+        if (gt < r) {
+          a = __ldcg(vj + gt);
+          b = __ldcg(vk + gt);
+        }
+        auto gram = [&](const T2& u, const T2& v) {
+          aa = fma(u.x, u.x, fma(u.y, u.y, aa));
+          bb = fma(v.x, v.x, fma(v.y, v.y, bb));
+          cr = fma(u.x, v.x, fma(u.y, v.y, cr));   // conj(u) v
+          ci = fma(u.x, v.y, fma(-u.y, v.x, ci));
+        };
+#pragma unroll
+        for (int e = 0; e < REG; ++e)
+          if (e * GROUP < p) gram(x[e], y[e]);
+        for (int i = gt + REG * GROUP; i < p; i += GROUP) gram(__ldcg(wj + i), __ldcg(wk + i));
+        const T sum = warp_sum4(aa, bb, cr, ci);
+        if (lane < 4) s_sum[g][gw][lane] = sum;
+        group_sync(g);
+        if (gw == (g & 3)) {   // one warp per sub-partition forms its group's rotation
+          T v = 0;
+          if (lane < 4)
+            v = (s_sum[g][0][lane] + s_sum[g][1][lane]) + (s_sum[g][2][lane] + s_sum[g][3][lane]);
+          float off;
+          const Rot<T> R = rotation(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1),
+                                    __shfl_sync(0xffffffffu, v, 2), __shfl_sync(0xffffffffu, v, 3),
+                                    tol, off);
+          if (lane == 0) s_rot[g] = R;
+          if (R.on) worst = max(worst, __float_as_int(off));
+        }
+        group_sync(g);
+        const Rot<T> R = s_rot[g];
+        if (!R.on) continue;
+#pragma unroll
+        for (int e = 0; e < REG; ++e) {
+          const int i = gt + e * GROUP;
+          if (e * GROUP < p) rotate(R, x[e], y[e]);
+          if (i < p) {
+            __stcg(wj + i, x[e]);
+            __stcg(wk + i, y[e]);
+          }
+        }
+        for (int i = gt + REG * GROUP; i < p; i += GROUP) {
+          T2 u = __ldcg(wj + i), v = __ldcg(wk + i);
+          rotate(R, u, v);
+          __stcg(wj + i, u);
+          __stcg(wk + i, v);
+        }
+        if (gt < r) {
+          rotate(R, a, b);
+          __stcg(vj + gt, a);
+          __stcg(vk + gt, b);
+        }
+        for (int i = gt + GROUP; i < r; i += GROUP) {
+          T2 u = __ldcg(vj + i), v = __ldcg(vk + i);
+          rotate(R, u, v);
+          __stcg(vj + i, u);
+          __stcg(vk + i, v);
+        }
+      }
+      cluster.sync();
+    }
+    // the largest off-orthogonality of the sweep, over the cluster
+    if (worst > 0 && lane == 0)
+      for (int c = 0; c < cs; ++c) atomicMax(cluster.map_shared_rank(&s_off[sweep & 1], c), worst);
+    if (tid == 0) s_off[(sweep + 1) & 1] = 0;
+    cluster.sync();
+    const float off = __int_as_float(s_off[sweep & 1]);
+    if (off <= last) break;
+    // everyone has read it before the next but one sweep clears it
+  }
+  cluster.sync();
+  return sweep;
+}
+
+// biased exponent of the largest component of A (2047: an infinity or NaN), by the cluster
+__device__ int largest_exponent(const double2* __restrict__ a, int m, int n, long lda) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  __shared__ int s_max;
+  if (threadIdx.x == 0) s_max = 0;
+  cluster.sync();
+  int e = 0;
+  for (long q = rank * (long)ST + threadIdx.x; q < (long)m * n; q += (long)cs * ST) {
+    const double2 z = a[(q / n) * lda + q % n];
+    e = max(e, max((int)((__double_as_longlong(z.x) >> 52) & 0x7FF),
+                   (int)((__double_as_longlong(z.y) >> 52) & 0x7FF)));
+  }
+  e = __reduce_max_sync(0xffffffffu, e);
+  if ((threadIdx.x & 31) == 0)
+    for (int c = 0; c < cs; ++c) atomicMax(cluster.map_shared_rank(&s_max, c), e);
+  cluster.sync();
+  return s_max;
+}
+
+// Y = I + X from G = W^H W (r x r, row-major), see the top of the file
+__global__ void svd_first_order_kernel(const double2* __restrict__ G, int r, double2* __restrict__ Y,
+                                       double xmax, const int* __restrict__ bad) {
+  if (*bad != 0) return;
+  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < (long)r * r;
+       e += (long)gridDim.x * blockDim.x) {
+    const int i = (int)(e / r), j = (int)(e % r);
+    double2 y = c2(i == j ? 1.0 : 0.0, 0.0);
+    if (i != j) {
+      const double2 g = G[e];
+      const double d = G[(long)j * r + j].x - G[(long)i * r + i].x;
+      // both pairs (i, j) and (j, i) decide alike: G is Hermitian bit for bit only up to
+      // rounding, so the test is made on the element above the diagonal
+      const double2 t = i < j ? g : G[(long)j * r + i];
+      if (fabs(t.x) + fabs(t.y) <= xmax * fabs(d) && d != 0.0) y = c2(g.x / d, g.y / d);
+    }
+    Y[e] = y;
+  }
+}
+
+// FP32 sweeps on A scaled to entries below 1: V32 as FP64 to Vd (column-major), identities
+// to the NS buffers G (for the Newton-Schulz steps), *bad = 1 when A holds an infinity or NaN (the
+// GEMMs and the FP64 sweeps then start from A itself).
+__global__ void __launch_bounds__(ST) svd_pre_kernel(const double2* __restrict__ a, int m, int n,
+                                                     long lda, float2* __restrict__ W,
+                                                     float2* __restrict__ V,
+                                                     double2* __restrict__ Vd,
+                                                     double2* __restrict__ G,
+                                                     int* __restrict__ bad) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x;
+  const bool wide = m < n;
+  const int p = wide ? n : m, r = wide ? m : n;
+  const long step = (long)cs * ST, first = rank * (long)ST + tid;
+  const int e = largest_exponent(a, m, n, lda);
+  if (rank == 0 && tid == 0) *bad = e == 2047 ? 1 : 0;
+  if (e != 2047) {
+    for (long q = first; q < (long)p * r; q += step) {
+      const int j = (int)(q / p), i = (int)(q % p);
+      double2 z = wide ? a[(long)j * lda + i] : a[(long)i * lda + j];
+      if (wide) z.y = -z.y;
+      __stcg(W + q, make_float2(scaled_float(z.x, e - 1022), scaled_float(z.y, e - 1022)));
+    }
+    for (long q = first; q < (long)r * r; q += step)
+      __stcg(V + q, make_float2(q / r == q % r ? 1.0f : 0.0f, 0.0f));
+    cluster.sync();
+    sweeps<float>(W, V, p, r, 1e-6f, 3e-4f, PRE_SWEEPS);
+  }
+  for (long q = first; q < (long)r * r; q += step) {
+    const double2 one = c2(q / r == q % r ? 1.0 : 0.0, 0.0);
+#pragma unroll
+    for (int t = 0; t < NS; ++t) G[(long)t * r * r + q] = one;
+    if (e != 2047) {
+      const float2 v = __ldcg(V + q);
+      Vd[q] = c2(v.x, v.y);
+    }
+  }
+  cluster.sync();
+}
+
+// W (p x r) and V (r x r) are column-major scratch; u, vh row-major outputs. `pre`: W and V
+// hold the start of the sweeps unless *bad.
 __global__ void __launch_bounds__(ST) svd_jacobi_kernel(const double2* __restrict__ a, int m, int n,
                                                        long lda, double2* __restrict__ W,
                                                        double2* __restrict__ V,
@@ -52,124 +438,76 @@ __global__ void __launch_bounds__(ST) svd_jacobi_kernel(const double2* __restric
                                                        int* __restrict__ pos, double2* __restrict__ u,
                                                        long ldu, double* __restrict__ s,
                                                        double2* __restrict__ vh, long ldvh,
-                                                       int* __restrict__ sweeps_out) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+                                                       int* __restrict__ sweeps_out, int pre,
+                                                       const int* __restrict__ bad) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = rank * (ST / 32) + (tid >> 5), nwarp = cs * (ST / 32);
   const bool wide = m < n;
   const int p = wide ? n : m, r = wide ? m : n;
-  for (long e = tid; e < (long)p * r; e += ST) {
-    const int j = (int)(e / p), i = (int)(e % p);
-    W[e] = wide ? cconj(a[(long)j * lda + i]) : a[(long)i * lda + j];
-  }
-  for (long e = tid; e < (long)r * r; e += ST) V[e] = c2((e / r == e % r) ? 1.0 : 0.0, 0.0);
-  __shared__ int s_rot;
-  __syncthreads();
-  const double tol = (double)p * 2.220446049250313e-16;
-  const int rr = r + (r & 1);   // an odd count plays against an absent column
-  int sweep = 0;
-  for (; sweep < MAX_SWEEPS; ++sweep) {
-    if (tid == 0) s_rot = 0;
-    __syncthreads();
-    for (int q = 0; q < rr - 1; ++q) {
-      for (int t = warp; t < rr / 2; t += NWARP) {
-        int j, k;
-        if (t == 0) {
-          j = 0;
-          k = 1 + q;
-        } else {
-          j = 1 + (q + t) % (rr - 1);
-          k = 1 + (q + rr - 1 - t) % (rr - 1);
-        }
-        if (j > k) {
-          const int x = j;
-          j = k;
-          k = x;
-        }
-        if (k >= r) continue;
-        double2* wj = W + (long)j * p;
-        double2* wk = W + (long)k * p;
-        double aa = 0.0, bb = 0.0, cr = 0.0, ci = 0.0;
-        for (int i = lane; i < p; i += 32) {
-          const double2 x = wj[i], y = wk[i];
-          aa = fma(x.x, x.x, fma(x.y, x.y, aa));
-          bb = fma(y.x, y.x, fma(y.y, y.y, bb));
-          cr = fma(x.x, y.x, fma(x.y, y.y, cr));   // conj(x) y
-          ci = fma(x.x, y.y, fma(-x.y, y.x, ci));
-        }
-        aa = warp_sum(aa);
-        bb = warp_sum(bb);
-        cr = warp_sum(cr);
-        ci = warp_sum(ci);
-        const double ac = sqrt(cr * cr + ci * ci);
-        if (!(ac > 0.0) || !(ac > tol * sqrt(aa) * sqrt(bb))) continue;
-        const double2 ph = c2(cr / ac, -ci / ac);   // e^{-i phi}
-        const double zeta = (bb - aa) / (2.0 * ac);
-        const double tt = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-        const double cs = 1.0 / sqrt(1.0 + tt * tt), sn = cs * tt;
-        for (int i = lane; i < p; i += 32) {
-          const double2 x = wj[i], y = cmul(wk[i], ph);
-          wj[i] = c2(cs * x.x - sn * y.x, cs * x.y - sn * y.y);
-          wk[i] = c2(sn * x.x + cs * y.x, sn * x.y + cs * y.y);
-        }
-        double2* vj = V + (long)j * r;
-        double2* vk = V + (long)k * r;
-        for (int i = lane; i < r; i += 32) {
-          const double2 x = vj[i], y = cmul(vk[i], ph);
-          vj[i] = c2(cs * x.x - sn * y.x, cs * x.y - sn * y.y);
-          vk[i] = c2(sn * x.x + cs * y.x, sn * x.y + cs * y.y);
-        }
-        if (lane == 0) atomicAdd(&s_rot, 1);
-      }
-      __syncthreads();
+  const long step = (long)cs * ST, first = rank * (long)ST + tid;
+  // entries whose squares would leave the FP64 range: W carries a power of two
+  const int ea = largest_exponent(a, m, n, lda);
+  const int shift = (ea != 0 && ea != 2047 && abs(ea - 1023) > 400) ? 1023 - ea : 0;
+  if (!pre || *bad != 0) {
+    for (long e = first; e < (long)p * r; e += step) {
+      const int j = (int)(e / p), i = (int)(e % p);
+      double2 z = wide ? cconj(a[(long)j * lda + i]) : a[(long)i * lda + j];
+      if (shift != 0) z = c2(ldexp(z.x, shift), ldexp(z.y, shift));
+      __stcg(W + e, z);
     }
-    const int rot = s_rot;
-    __syncthreads();
-    if (rot == 0) break;
+    for (long e = first; e < (long)r * r; e += step)
+      __stcg(V + e, c2((e / r == e % r) ? 1.0 : 0.0, 0.0));
+  } else if (shift != 0) {
+    for (long e = first; e < (long)p * r; e += step)
+      __stcg(W + e, c2(ldexp(W[e].x, shift), ldexp(W[e].y, shift)));
   }
+  cluster.sync();
+  const double tol = (double)p * 2.220446049250313e-16;
+  const int sweep = sweeps<double>(W, V, p, r, tol, 0.0f, MAX_SWEEPS);
   // singular values, their order, the outputs
-  for (int j = warp; j < r; j += NWARP) {
+  for (int j = warp; j < r; j += nwarp) {
     const double2* wj = W + (long)j * p;
     double acc = 0.0;
-    for (int i = lane; i < p; i += 32) acc = fma(wj[i].x, wj[i].x, fma(wj[i].y, wj[i].y, acc));
+    for (int i = lane; i < p; i += 32) {
+      const double2 z = __ldcg(wj + i);
+      acc = fma(z.x, z.x, fma(z.y, z.y, acc));
+    }
     acc = warp_sum(acc);
-    if (lane == 0) sig[j] = sqrt(acc);
+    if (lane == 0) __stcg(sig + j, sqrt(acc));
   }
-  __syncthreads();
-  for (int j = tid; j < r; j += ST) {
-    const double sj = sig[j];
+  cluster.sync();
+  for (int j = (int)first; j < r; j += (int)step) {
+    const double sj = __ldcg(sig + j);
     int c = 0;
-    for (int i = 0; i < r; ++i) c += (sig[i] > sj || (sig[i] == sj && i < j)) ? 1 : 0;
-    pos[j] = c;
-    s[c] = sj;
+    for (int i = 0; i < r; ++i) {
+      const double si = __ldcg(sig + i);
+      c += (si > sj || (si == sj && i < j)) ? 1 : 0;
+    }
+    __stcg(pos + j, c);
+    s[c] = shift != 0 ? ldexp(sj, -shift) : sj;
   }
-  __syncthreads();
-  if (!wide) {
-    // U[i][pos j] = w_j[i] / s_j (i < m), Vh[pos j][c] = conj(V[c][j]) (c < n)
-    for (long e = tid; e < (long)r * p; e += ST) {
-      const int j = (int)(e / p), i = (int)(e % p);
-      const double sj = sig[j];
-      const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
-      const double2 x = W[e];
-      u[(long)i * ldu + pos[j]] = c2(x.x * inv, x.y * inv);
+  cluster.sync();
+  // tall: U[i][pos j] = w_j[i] / s_j, Vh[pos j][c] = conj(V[c][j]); wide: A^H = U_w diag(s)
+  // V^H, so U[i][pos j] = V[i][j], Vh[pos j][c] = conj(w_j[c]) / s_j. One warp per column.
+  for (int j = warp; j < r; j += nwarp) {
+    const double sj = __ldcg(sig + j);
+    const int c = __ldcg(pos + j);
+    const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
+    for (int i = lane; i < p; i += 32) {
+      const double2 x = __ldcg(W + (long)j * p + i);
+      if (!wide) u[(long)i * ldu + c] = c2(x.x * inv, x.y * inv);
+      else vh[(long)c * ldvh + i] = c2(x.x * inv, -x.y * inv);
     }
-    for (long e = tid; e < (long)r * r; e += ST) {
-      const int j = (int)(e / r), c = (int)(e % r);
-      vh[(long)pos[j] * ldvh + c] = cconj(V[e]);
-    }
-  } else {
-    // A^H = W-side U_w diag(s) V^H: U[i][pos j] = V[i][j] (i < m), Vh[pos j][c] = conj(w_j[c]) / s_j
-    for (long e = tid; e < (long)r * r; e += ST) {
-      const int j = (int)(e / r), i = (int)(e % r);
-      u[(long)i * ldu + pos[j]] = V[e];
-    }
-    for (long e = tid; e < (long)r * p; e += ST) {
-      const int j = (int)(e / p), c = (int)(e % p);
-      const double sj = sig[j];
-      const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
-      const double2 x = W[e];
-      vh[(long)pos[j] * ldvh + c] = c2(x.x * inv, -x.y * inv);
+    for (int i = lane; i < r; i += 32) {
+      const double2 x = __ldcg(V + (long)j * r + i);
+      if (!wide) vh[(long)c * ldvh + i] = cconj(x);
+      else u[(long)i * ldu + c] = x;
     }
   }
-  if (tid == 0 && sweeps_out != nullptr) *sweeps_out = sweep + (sweep == MAX_SWEEPS ? 1 : 0);
+  if (rank == 0 && tid == 0 && sweeps_out != nullptr)
+    *sweeps_out = sweep + (sweep == MAX_SWEEPS ? 1 : 0);
 }
 
 // a[i][j] *= s[j] (side 0: columns) or s[i] (side 1: rows), row-major with ld
@@ -189,10 +527,73 @@ inline size_t al(size_t b) { return (b + 255) & ~size_t(255); }
 
 }  // namespace
 
+// largest cluster the kernels can be launched with (16, else 8, else 1); decided once
+static int svd_cluster_max() {
+  static int best = 1;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    for (const void* f : {(const void*)svd_pre_kernel, (const void*)svd_jacobi_kernel})
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        cudaGetLastError();
+    for (int c : {16, 8}) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(c);
+      cfg.blockDim = dim3(ST);
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = c;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int na = 0, nb = 0;
+      if (cudaOccupancyMaxActiveClusters(&na, svd_pre_kernel, &cfg) == cudaSuccess &&
+          cudaOccupancyMaxActiveClusters(&nb, svd_jacobi_kernel, &cfg) == cudaSuccess && na > 0 &&
+          nb > 0) {
+        best = c;
+        break;
+      }
+      cudaGetLastError();
+    }
+  });
+  return best;
+}
+
+struct SvdWs {
+  double2 *W, *V;
+  double* sig;
+  int *pos, *bad;
+  // FP32 start
+  float2 *W32, *V32;
+  double2 *V0, *G, *H, *Y;   // V's second buffer, NS identities, W^H W, I + X
+};
+
+static size_t svd_layout(void* base, long p, long r, SvdWs* w) {
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    void* q = base ? static_cast<char*>(base) + off : nullptr;
+    off += al(bytes);
+    return q;
+  };
+  w->W = static_cast<double2*>(take((size_t)p * r * sizeof(double2)));
+  w->V = static_cast<double2*>(take((size_t)r * r * sizeof(double2)));
+  w->sig = static_cast<double*>(take((size_t)r * sizeof(double)));
+  w->pos = static_cast<int*>(take((size_t)(r + 1) * sizeof(int)));
+  w->bad = w->pos ? w->pos + r : nullptr;
+  if (r >= PRE_MIN) {
+    w->W32 = static_cast<float2*>(take((size_t)p * r * sizeof(float2)));
+    w->V32 = static_cast<float2*>(take((size_t)r * r * sizeof(float2)));
+    w->V0 = static_cast<double2*>(take((size_t)r * r * sizeof(double2)));
+    w->G = static_cast<double2*>(take((size_t)NS * r * r * sizeof(double2)));
+    w->H = static_cast<double2*>(take((size_t)r * r * sizeof(double2)));
+    w->Y = static_cast<double2*>(take((size_t)r * r * sizeof(double2)));
+  }
+  return off;
+}
+
 size_t svd_workspace_bytes(int m, int n) {
-  const long p = std::max(m, n), r = std::min(m, n);
-  return al((size_t)p * r * sizeof(double2)) + al((size_t)r * r * sizeof(double2)) +
-         al((size_t)r * sizeof(double)) + al((size_t)r * sizeof(int));
+  SvdWs w;
+  return svd_layout(nullptr, std::max(m, n), std::min(m, n), &w);
 }
 
 ptn_status svd(const double2* a, int m, int n, long lda, double2* u, long ldu, double* s,
@@ -200,16 +601,70 @@ ptn_status svd(const double2* a, int m, int n, long lda, double2* u, long ldu, d
   PTN_CHECK_ARG(m > 0 && n > 0, "svd: empty matrix (%d x %d)", m, n);
   PTN_CHECK_ARG(lda >= n && ldu >= std::min(m, n) && ldvh >= n, "svd: bad leading dimensions");
   PTN_CHECK_ARG(ws_bytes >= svd_workspace_bytes(m, n), "svd: workspace too small");
-  const long p = std::max(m, n), r = std::min(m, n);
-  char* c = static_cast<char*>(ws);
-  double2* W = reinterpret_cast<double2*>(c);
-  c += al((size_t)p * r * sizeof(double2));
-  double2* V = reinterpret_cast<double2*>(c);
-  c += al((size_t)r * r * sizeof(double2));
-  double* sig = reinterpret_cast<double*>(c);
-  c += al((size_t)r * sizeof(double));
-  int* pos = reinterpret_cast<int*>(c);
-  svd_jacobi_kernel<<<1, ST, 0, st>>>(a, m, n, lda, W, V, sig, pos, u, ldu, s, vh, ldvh, sweeps);
+  const int p = std::max(m, n), r = std::min(m, n);
+  const bool wide = m < n, pre = r >= PRE_MIN;
+  SvdWs w;
+  svd_layout(ws, p, r, &w);
+  // one pair per CTA while the cluster allows
+  int cs = 1;
+  while (cs < svd_cluster_max() && cs < (r + 1) / 2) cs *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cs);
+  cfg.blockDim = dim3(ST);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (pre) {
+    PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, svd_pre_kernel, a, m, n, lda, w.W32, w.V32, w.V0, w.G,
+                                    w.bad));
+    note_launches(1);
+    // the buffers hold V^T and W^T row-major (V and W column by column)
+    double2* V = w.V0;
+    double2* V2 = w.V;
+    auto mult = [&](char oa, char ob, int M, int N, int K, const double2* A, long la,
+                    const double2* B, long lb, double2* C, double al, double be) {
+      GemmArgs g;
+      g.M = M; g.N = N; g.K = K; g.opA = oa; g.opB = ob;
+      g.alpha = make_double2(al, 0.0); g.beta = make_double2(be, 0.0);
+      g.A = A; g.lda = la; g.sA = 0;
+      g.B = B; g.ldb = lb; g.sB = 0;
+      g.C = C; g.ldc = N; g.sC = 0;
+      g.batch = 1; g.skip = w.bad;
+      return zgemm(g, nullptr, 0, st);
+    };
+    auto newton_schulz = [&](int t) -> ptn_status {   // V <- V (3 I - V^H V) / 2
+      double2* G = w.G + (long)t * r * r;
+      PTN_TRY(mult('C', 'T', r, r, r, V, r, V, r, G, -0.5, 1.5));
+      PTN_TRY(mult('T', 'N', r, r, r, G, r, V, r, V2, 1.0, 0.0));
+      std::swap(V, V2);
+      return PTN_OK;
+    };
+    auto times_a = [&]() {   // W = A V (tall) or A^H V (wide)
+      return mult('N', wide ? 'C' : 'T', r, p, r, V, r, a, lda, w.W, 1.0, 0.0);
+    };
+    PTN_TRY(newton_schulz(0));
+    PTN_TRY(times_a());
+    for (int t = 0; t < REFINE; ++t) {
+      PTN_TRY(mult('C', 'T', r, r, p, w.W, p, w.W, p, w.H, 1.0, 0.0));
+      svd_first_order_kernel<<<std::min(4 * num_sms(), (r * r + 127) / 128), 128, 0, st>>>(
+          w.H, r, w.Y, X_NORM[t] / r, w.bad);
+      PTN_LAUNCH_CHECK();
+      note_launches(1);
+      PTN_TRY(mult('T', 'N', r, r, r, w.Y, r, V, r, V2, 1.0, 0.0));   // V (I + X)
+      std::swap(V, V2);
+      PTN_TRY(newton_schulz(2 * t + 1));
+      PTN_TRY(newton_schulz(2 * t + 2));
+      PTN_TRY(times_a());
+    }
+    w.V = V;
+  }
+  PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, svd_jacobi_kernel, a, m, n, lda, w.W, w.V, w.sig, w.pos, u,
+                                  ldu, s, vh, ldvh, sweeps, pre ? 1 : 0, (const int*)w.bad));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;

@@ -248,3 +248,33 @@ def test_compress_density_matches_reference(ptg):
     print("compress density bonds", [len(q) for q in psi.qbonds], "state", np.abs(v - vr).max())
     assert np.abs(v - vr).max() < 1e-10 * max(1.0, np.abs(vr).max())
     assert abs(np.linalg.norm(v) - 1.0) < 1e-12
+
+
+@pytest.mark.parametrize("kind", ["gauss", "graded", "rank", "tiny", "repeated"])
+@pytest.mark.parametrize("mn", [(31, 31), (32, 32), (33, 70), (128, 96), (97, 160), (600, 40)])
+def test_svd_from_fp32_start(mn, kind):
+    """Around the size from which the sweeps start from FP32 singular vectors, an odd column
+    count, more rows than a thread keeps in registers, and spectra that FP32 cannot resolve:
+    orthogonality and reconstruction to p eps per column pair (the stopping rule), every
+    singular value to the absolute accuracy of numpy's."""
+    m, n = mn
+    r = min(m, n)
+    rng = np.random.default_rng(m + n)
+    a = orc.crandn((m, n), rng)
+    if kind in ("graded", "rank", "repeated"):
+        u, _, vh = np.linalg.svd(a, full_matrices=False)
+        s = {"graded": 10.0 ** np.linspace(0, -14, r), "rank": np.r_[np.ones(r // 2), np.zeros(r - r // 2)],
+             "repeated": np.r_[np.full(r - 3, 2.0), 1.0, 1.0, 0.5]}[kind]
+        a = (u * s) @ vh
+    if kind == "tiny":
+        a *= 1e-200
+    u, s, vh, sweeps = dev_svd(a)
+    assert sweeps < 60
+    s_ref = np.linalg.svd(a, compute_uv=False)
+    tol = 16 * max(m, n) * np.finfo(float).eps
+    assert np.all(np.diff(s) <= 0)
+    assert np.abs(s - s_ref).max() <= tol * s_ref[0]
+    assert np.linalg.norm((u * s) @ vh - a) <= tol * np.linalg.norm(a) * np.sqrt(r)
+    keep = s > 1e-13 * s[0]
+    for x in (u[:, keep], vh[keep].conj().T):
+        assert np.abs(x.conj().T @ x - np.eye(keep.sum())).max() <= tol * np.sqrt(r)
