@@ -977,230 +977,259 @@ __global__ void __launch_bounds__(P6W * 32) qr_panel6_kernel(double2* __restrict
   cluster.sync();   // no CTA leaves while its shared memory may still be read
 }
 
-__device__ __forceinline__ void cluster_arrive() {
-  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+// 1 / sqrt(d) and 1 / d from an FP32 seed and one third-order step, seed and scaling by
+// integer work on the IEEE fields: five and three FP64 instructions (64 cycles each on this
+// part) where the division and square root sequences take several times that. Subnormal, zero and
+// non-finite arguments take the CUDA functions.
+__device__ __forceinline__ double seed_scale(float y, int e) {   // y 2^e for a normal float y
+  const unsigned b = __float_as_uint(y);
+  const int x = (int)(b >> 23) - 127 + 1023 + e;
+  return __longlong_as_double(((long long)x << 52) | ((long long)(b & 0x7FFFFFu) << 29));
 }
 
-// Panel, fourth form (default): the layout of qr_panel6_kernel (two warps per 32-row
-// group, even / odd columns) with a shorter instruction path per column:
-//  - one product per row and column, conj(v) x_c, for every column: on the rows
-//    where a masked operand would differ, v is zero, so the dot products (c > jj)
-//    and the conjugated Gram entries (c < jj) come out of the same select-free loop;
-//  - the products go to shared memory (rows x 17 complex, conflict-free) and
-//    thread (column, 8-row block) sums them: one pass instead of a shuffle
-//    reduce-scatter with selects;
-//  - after the gather, the next pivot column is updated first and its norm partial
-//    published; the cluster barrier that guards it is split (arrive now, wait at the
-//    next pivot), so the other updates run while the barrier completes.
-// Dynamic shared memory: xs[NB][R] and the product buffer [R][17], R = 32 x row groups.
-__global__ void __launch_bounds__(P6W * 32) qr_panel7_kernel(double2* __restrict__ a, long lda, int m,
-                                                             int j0, int jb,
-                                                             double2* __restrict__ Tout,
-                                                             double2* __restrict__ V, long ldv) {
+__device__ __forceinline__ double fast_rsqrt(double d) {
+  const long long b = __double_as_longlong(d);
+  const int E = (int)((b >> 52) & 0x7FF);
+  if (b <= 0 || E == 0 || E == 0x7FF) return 1.0 / sqrt(d);
+  const int e = E - 1023, odd = e & 1;
+  const float m = __uint_as_float(((unsigned)(127 + odd) << 23) | ((unsigned)(b >> 29) & 0x7FFFFFu));
+  const double y = seed_scale(rsqrtf(m), -(e - odd) / 2);
+  const double r = fma(-(d * y), y, 1.0);
+  return fma(y * r, fma(r, 0.375, 0.5), y);
+}
+
+__device__ __forceinline__ double fast_recip(double d) {   // d > 0
+  const long long b = __double_as_longlong(d);
+  const int E = (int)((b >> 52) & 0x7FF);
+  if (b <= 0 || E < 2 || E > 2040) return 1.0 / d;
+  const float m = __uint_as_float(0x3F800000u | ((unsigned)(b >> 29) & 0x7FFFFFu));
+  const double y = seed_scale(__frcp_rn(m), -(E - 1023));
+  const double r = fma(-d, y, 1.0);
+  return fma(y, fma(r, r, r), y);
+}
+
+// Panel, default form: ONE cluster-wide reduction per column. The sums over the rows below
+// the pivot of conj(x_j) x_c for every column c (c = j: the norm) and the pivot row are all
+// that the reflector and its application need: with v = (1, scal x_j),
+//   beta = -sign(Re alpha) sqrt(|alpha|^2 + sum_j),   row j of R: r_c = (conj(alpha) a_jc +
+//   sum_c) / beta,   a_ic -= (scal x_j)_i (a_jc - r_c)
+// (the last factor is conj(tau) v^H a_c), so nothing waits for the scaled vector before it
+// is multiplied with the other columns, and every CTA forms the same scalars from the same
+// sums. For c < j the sums are entries of the Gram matrix of the finished reflectors, from
+// which one CTA of the cluster grows T column by column while the scalars are formed.
+// What bounds it: FP64 issue. An FP64 instruction takes a warp 64 cycles of its
+// sub-partition, so rows are held row-major and a thread sums several rows of one column
+// (no products through shared memory), finished columns drop out of the update by
+// halving the column width of the thread grid, and square root and reciprocals are
+// Newton steps on an FP32 seed.
+// Measured (panels of a 1024 x 512 matrix, 16 CTAs, mean over its 32): 127 us per 16 columns
+// with two reductions per column and the scaled vector multiplied -> 85 us; the whole QR
+// 8.25 -> 6.57 ms.
+// Dynamic shared memory: xs[rows of the CTA][NB].
+constexpr int P8T = 256;
+constexpr int P8_ROWS = 768;   // most rows per CTA: 192 KB
+
+__global__ void __launch_bounds__(P8T) qr_panel8_kernel(double2* __restrict__ a, long lda, int m,
+                                                        int j0, int jb, double2* __restrict__ Tout,
+                                                        double2* __restrict__ V, long ldv) {
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const int cs = (int)cluster.num_blocks();
+  const int rank = (int)cluster.block_rank(), cs = (int)cluster.num_blocks();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ng = (int)(blockDim.x >> 6);   // row groups
-  const int nw = 2 * ng;
-  const int R = 32 * ng;                   // rows held by this CTA
-  const int ch = warp & 1, rg = warp >> 1;
+  const int c16 = tid & 15, b16 = tid >> 4;
   extern __shared__ double2 dyn[];
-  double2* xs = dyn;                       // xs[c * R + row]
-  double2* qs = dyn + NB * R;              // qs[row * 17 + c]
-  __shared__ double s_wn[P6W / 2];
-  __shared__ double2 s_wv[P6W][NB];        // per-warp column sums
-  __shared__ double2 s_alpha;
-  __shared__ double2 s_vec[NB];            // CTA column sums (read remotely)
-  __shared__ double2 s_tau[NB];
-  __shared__ double2 s_scal;
-  __shared__ double s_beta;
+  double2* xs = dyn;                        // xs[row * NB + c]
+  __shared__ double2 s_part[P8T / 32][NB];  // per-warp sums
+  __shared__ double2 s_pub[2][NB];          // this CTA's sums (read remotely), by column parity
+  __shared__ double2 s_row[2][NB];          // the pivot row, in its owner
+  __shared__ double2 s_gat[P8T / 32][NB];   // sums of two ranks per warp
+  __shared__ double2 s_prow[NB];
+  __shared__ double2 s_r[NB], s_u[NB];      // row of R; scal times the update factors
+  __shared__ double2 s_S[NB][NB + 1];       // Gram entries of the reflectors, [c][j], c < j
+  __shared__ double2 s_T[NB][NB + 1];
+  __shared__ double2 s_tau[NB], s_scal;
+  __shared__ double s_beta, s_ib;
   __shared__ int s_apply;
-  __shared__ double2 s_upd[NB];
-  __shared__ double2 s_G[NB][NB];
 
   const int mp = m - j0;
   const int chunk = (mp + cs - 1) / cs;
-  const int rb = j0 + rank * chunk;
-  const int re = min(m, rb + chunk);
-  const int lr = rg * 32 + lane;
-  const int i = rb + lr;
-  const bool mine = i < re;
-
-#pragma unroll
-  for (int t = 0; t < NB / 2; ++t) {
-    const int c = 2 * t + ch;
-    xs[c * R + lr] = (mine && c < jb) ? a[(long)i * lda + j0 + c] : c2(0.0, 0.0);
+  const int rb = j0 + rank * chunk;                 // first row of this CTA
+  const int nr = max(0, min(m, rb + chunk) - rb);   // its rows
+  for (int e = tid; e < nr * NB; e += P8T) {
+    const int c = e & (NB - 1);
+    xs[e] = c < jb ? a[(long)(rb + (e >> 4)) * lda + j0 + c] : c2(0.0, 0.0);
   }
-  for (int e = tid; e < NB * NB; e += blockDim.x) s_G[e / NB][e % NB] = c2(0.0, 0.0);
-
-  // norm partial of pivot column p (its set's warps) and the pivot entry
-  auto publish_norm = [&](int p) {
-    if (ch == (p & 1)) {
-      const double2 x = xs[p * R + lr];
-      double acc = (mine && i > j0 + p) ? fma(x.x, x.x, x.y * x.y) : 0.0;
+  for (int e = tid; e < NB * (NB + 1); e += P8T) {
+    (&s_S[0][0])[e] = c2(0.0, 0.0);
+    (&s_T[0][0])[e] = c2(0.0, 0.0);
+  }
+  const bool make_t = rank == cs - 1;   // the CTA with the fewest rows
+  // column q of T from columns < q (threads 128 .. 255: eight per row)
+  auto t_column = [&](int q) {
+    const int t = tid - 128;
+    const int row = t >> 3, g = t & 7;
+    double2 s = c2(0.0, 0.0);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) s_wn[rg] = acc;
-      if (i == j0 + p) s_alpha = x;
+    for (int h = 0; h < 2; ++h) {
+      const int k = g + 8 * h;
+      if (k < q && k >= row) s = cfma(s_T[row][k], s_S[k][q], s);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    if (g == 0) {
+      const double2 tau = s_tau[q];
+      if (row < q) s_T[row][q] = cmul(c2(-tau.x, -tau.y), s);
+      if (row == q) s_T[row][q] = tau;
     }
   };
-  publish_norm(0);
-  cluster_arrive();
 
 #pragma unroll 1
-  for (int jj = 0; jj < jb; ++jj) {
-    const int col = j0 + jj;
-    const int owner = jj / chunk;
-    const int oh = jj & 1;
-    cluster_wait();
-    // ---- warp 0: the reflector scalars (fixed summation order)
-    if (warp == 0) {
-      const int np = cs * ng;
-      double v = 0.0;
-      if (lane < np) v = cluster.map_shared_rank(s_wn, lane / ng)[lane % ng];
-      if (lane + 32 < np) v += cluster.map_shared_rank(s_wn, (lane + 32) / ng)[(lane + 32) % ng];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      const double xn2 = v;
-      const double2 alpha = *cluster.map_shared_rank(&s_alpha, owner);
-      const bool apply = !(xn2 == 0.0 && alpha.y == 0.0);
-      double beta = 0.0, dx = 0.0, d2 = 1.0;
-      if (apply) {
-        beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
-        dx = alpha.x - beta;
-        d2 = dx * dx + alpha.y * alpha.y;
-      }
-      const double rec = 1.0 / ((lane == 0) ? (apply ? beta : 1.0) : d2);
-      const double ib = __shfl_sync(0xffffffffu, rec, 0);
-      const double id2 = __shfl_sync(0xffffffffu, rec, 1);
-      if (lane == 0) {
-        double2 tau = c2(0.0, 0.0), scal = c2(0.0, 0.0);
-        if (apply) {
-          tau = c2((beta - alpha.x) * ib, -alpha.y * ib);
-          scal = c2(dx * id2, -alpha.y * id2);
-        }
-        s_tau[jj] = tau;
-        s_scal = scal;
-        s_beta = beta;
-        s_apply = apply ? 1 : 0;
-      }
-    }
+  for (int j = 0; j < jb; ++j) {
+    const int par = j & 1;
+    const int owner = j / chunk;
+    const int first = j0 + j + 1 - rb;          // first row below the pivot, local
     __syncthreads();
-    const bool apply = s_apply != 0;
-    const double2 xj = xs[jj * R + lr];
-    double2 xjn = xj;
-    if (apply && mine && i > col) xjn = cmul(xj, s_scal);
-    if (apply && i == col) xjn = c2(s_beta, 0.0);
-    const double2 vcur = (mine && i >= col) ? ((i == col) ? c2(1.0, 0.0) : xjn) : c2(0.0, 0.0);
-    const double2 vc = cconj(vcur);
-    // ---- products conj(v) x_c of this row, own set
-#pragma unroll
-    for (int t = 0; t < NB / 2; ++t) {
-      const int c = 2 * t + ch;
-      qs[lr * 17 + c] = cmul(vc, xs[c * R + lr]);
-    }
-    __syncthreads();
-    // ---- column sums: thread (c, 8-row block), the two blocks of a warp, per warp
+    // ---- sums over the own rows below the pivot
     {
-      const int c = tid & 15, p = tid >> 4;
-      const double2* src = qs + (8 * p) * 17 + c;
-      double2 s01 = cadd(src[0 * 17], src[1 * 17]), s23 = cadd(src[2 * 17], src[3 * 17]);
-      double2 s45 = cadd(src[4 * 17], src[5 * 17]), s67 = cadd(src[6 * 17], src[7 * 17]);
-      double2 s = cadd(cadd(s01, s23), cadd(s45, s67));
-      s = cadd(s, c2(__shfl_xor_sync(0xffffffffu, s.x, 16), __shfl_xor_sync(0xffffffffu, s.y, 16)));
-      if (lane < 16) s_wv[warp][c] = s;
+      double2 s = c2(0.0, 0.0);
+      int lr = b16;
+      if (lr < first) lr += (first - lr + 15) / 16 * 16;
+      for (; lr < nr; lr += 16) s = cfma(cconj(xs[lr * NB + j]), xs[lr * NB + c16], s);
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
+      if (lane < 16) s_part[warp][c16] = s;
     }
     __syncthreads();
-    if (tid < NB) {
-      double2 s = s_wv[0][tid];
-      for (int w = 1; w < nw; ++w) s = cadd(s, s_wv[w][tid]);
-      s_vec[tid] = s;
+    if (warp == 0) {
+      const int w = (lane >> 4) * 4;
+      double2 s = cadd(cadd(s_part[w][c16], s_part[w + 1][c16]),
+                       cadd(s_part[w + 2][c16], s_part[w + 3][c16]));
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
+      if (lane < 16) s_pub[par][c16] = s;
+    } else if (warp == 1 && rank == owner && lane < 16) {
+      s_row[par][c16] = xs[(j0 + j - rb) * NB + c16];
     }
     cluster.sync();
-    // ---- row group 0, one warp per set: gather four ranks per lane, then the quarters
-    if (rg == 0) {
-      const int t = lane & 7, rq = lane >> 3;
-      const int c = 2 * t + ch;
-      double2 vals[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int rr = rq * 4 + k;
-        vals[k] = (rr < cs) ? cluster.map_shared_rank(s_vec, rr)[c] : c2(0.0, 0.0);
+    // ---- gather: thread (column, rank)
+    {
+      double2 s = c2(0.0, 0.0);
+      if (b16 < cs) s = cluster.map_shared_rank(&s_pub[par][0], b16)[c16];
+      if (cs > 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
       }
-      double2 tot = cadd(cadd(vals[0], vals[1]), cadd(vals[2], vals[3]));
-      tot = cadd(tot, c2(__shfl_xor_sync(0xffffffffu, tot.x, 8), __shfl_xor_sync(0xffffffffu, tot.y, 8)));
-      tot = cadd(tot, c2(__shfl_xor_sync(0xffffffffu, tot.x, 16), __shfl_xor_sync(0xffffffffu, tot.y, 16)));
-      if (rq == 0) {
-        if (rank == 0 && c < jj) s_G[c][jj] = cconj(tot);   // v_c^H v_jj
-        s_upd[c] = (apply && c > jj) ? cmul(cconj(s_tau[jj]), tot) : c2(0.0, 0.0);
-      }
+      if (lane < 16) s_gat[warp][c16] = s;
+      if (warp == 7 && lane >= 16) s_prow[c16] = cluster.map_shared_rank(&s_row[par][0], owner)[c16];
     }
     __syncthreads();
-    // ---- next pivot first: update, publish its norm, arrive; then the rest
-    auto upd = [&](int c) {
-      const double2 s = s_upd[c];
-      double2 x = xs[c * R + lr];
-      x.x = fma(-vcur.x, s.x, x.x);
-      x.x = fma(vcur.y, s.y, x.x);
-      x.y = fma(-vcur.x, s.y, x.y);
-      x.y = fma(-vcur.y, s.x, x.y);
-      xs[c * R + lr] = x;
-    };
-    if (ch == oh) xs[jj * R + lr] = xjn;   // the pivot column takes its reflector
-    if (jj + 1 < jb) {
-      if (ch != oh) upd(jj + 1);
-      publish_norm(jj + 1);
-      cluster_arrive();
-    }
-#pragma unroll 1
-    for (int t = (jj + 3 - ch) >> 1; 2 * t + ch < jb; ++t) upd(2 * t + ch);
-  }
-
-  // ---- write the panel back and the explicit V
-  if (mine) {
-#pragma unroll
-    for (int t = 0; t < NB / 2; ++t) {
-      const int c = 2 * t + ch;
-      if (c < jb) {
-        const int colc = j0 + c;
-        const double2 x = xs[c * R + lr];
-        a[(long)i * lda + colc] = x;
-        V[(long)i * ldv + colc] = (i < colc) ? c2(0.0, 0.0) : (i == colc) ? c2(1.0, 0.0) : x;
+    if (warp < 2) {
+      // all sums, in the lane of their column (both warps, to save an exchange)
+      const int w = (lane >> 4) * 4;
+      double2 tot = s_gat[w][c16];
+      if (cs > 2) {
+        tot = cadd(cadd(tot, s_gat[w + 1][c16]), cadd(s_gat[w + 2][c16], s_gat[w + 3][c16]));
+        tot.x += __shfl_xor_sync(0xffffffffu, tot.x, 16);
+        tot.y += __shfl_xor_sync(0xffffffffu, tot.y, 16);
+      } else {
+        tot.x = __shfl_sync(0xffffffffu, tot.x, c16);
+        tot.y = __shfl_sync(0xffffffffu, tot.y, c16);
       }
-    }
-  }
-  // ---- T (zlarft) on rank 0 from the Gram entries
-  if (rank == 0) {
-    __syncthreads();
-    if (warp == 0) {
-      double2 T[NB];
-#pragma unroll
-      for (int c = 0; c < NB; ++c) T[c] = c2(0.0, 0.0);
-#pragma unroll
-      for (int c = 0; c < NB; ++c) {
-        if (c < jb) {
-          double2 acc2 = c2(0.0, 0.0);
-#pragma unroll
-          for (int qq = 0; qq < NB; ++qq)
-            if (qq < c && lane <= qq) acc2 = cfma(T[qq], s_G[qq][c], acc2);
-          const double2 tc = s_tau[c];
-          if (lane < c) T[c] = cmul(c2(-tc.x, -tc.y), acc2);
-          if (lane == c) T[c] = tc;
+      const double2 prow = s_prow[c16];
+      const double2 alpha = s_prow[j];
+      const double xn2 = __shfl_sync(0xffffffffu, tot.x, j);
+      const bool apply = !(xn2 == 0.0 && alpha.y == 0.0);
+      if (warp == 0) {
+        // reflector scalars (every lane the same)
+        double beta = alpha.x, ib = 0.0;
+        double2 tau = c2(0.0, 0.0), scal = c2(0.0, 0.0);
+        if (apply) {
+          const double n2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn2));
+          const double y = fast_rsqrt(n2);
+          double nrm = n2 * y;
+          nrm = fma(0.5 * y, fma(-nrm, nrm, n2), nrm);
+          beta = -copysign(nrm, alpha.x);
+          ib = -copysign(y, alpha.x);
+        }
+        if (lane == 0) {
+          s_ib = ib;
+          s_beta = beta;
+          s_apply = apply ? 1 : 0;
+        }
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        if (apply) {
+          const double dx = alpha.x - beta;
+          const double id2 = fast_recip(fma(dx, dx, alpha.y * alpha.y));
+          scal = c2(dx * id2, -alpha.y * id2);
+          tau = c2((beta - alpha.x) * ib, -alpha.y * ib);
+        }
+        if (lane == 0) {
+          s_scal = scal;
+          s_tau[j] = tau;
+        }
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        // Gram entries v_c^H v_j, c < j
+        if (lane < j) s_S[lane][j] = cadd(cmul(cconj(tot), scal), cconj(prow));
+      } else {
+        // row of R and the update factors
+        const double2 t = cfma(cconj(alpha), prow, tot);
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        const double ib = s_ib;
+        const double2 r = c2(t.x * ib, t.y * ib);
+        const double2 w = csub(prow, r);
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        const double2 scal = s_scal;
+        if (lane < 16) {
+          s_r[c16] = apply ? (c16 > j ? r : c16 == j ? c2(s_beta, 0.0) : prow) : prow;
+          // column j takes scal x_j, the columns behind it x - x_j (scal w)
+          const double2 u = cmul(scal, w);
+          s_u[c16] = c16 == j ? scal : c2(-u.x, -u.y);
         }
       }
-      if (lane < NB)
-#pragma unroll
-        for (int c = 0; c < NB; ++c) Tout[lane * NB + c] = T[c];
+    } else if (warp >= 4 && make_t && j > 0) {
+      t_column(j - 1);
     }
+    __syncthreads();
+    if (s_apply != 0) {
+      // ---- update of the own rows; thread grid as wide as the columns still in work
+      const int lg = j < 8 ? 4 : j < 12 ? 3 : 2;
+      const int c = NB - (1 << lg) + (tid & ((1 << lg) - 1));
+      const int nb = P8T >> lg;
+      const double2 u = s_u[c];
+      for (int base = 0; base < nr; base += nb) {
+        const int lr = base + (tid >> lg);
+        const bool on = lr < nr && lr >= first && c >= j;
+        double2 xj = c2(0.0, 0.0), x = c2(0.0, 0.0);
+        if (on) {
+          xj = xs[lr * NB + j];
+          x = xs[lr * NB + c];
+        }
+        __syncwarp();   // column j is read before its thread replaces it
+        if (on) xs[lr * NB + c] = cfma(xj, u, c == j ? c2(0.0, 0.0) : x);
+      }
+      if (rank == owner && tid < 16) xs[(j0 + j - rb) * NB + tid] = s_r[tid];
+    }
+  }
+  __syncthreads();
+  // ---- the panel and the explicit V
+  for (int e = tid; e < nr * NB; e += P8T) {
+    const int c = e & (NB - 1);
+    if (c < jb) {
+      const int i = rb + (e >> 4), col = j0 + c;
+      const double2 x = xs[e];
+      a[(long)i * lda + col] = x;
+      V[(long)i * ldv + col] = i < col ? c2(0.0, 0.0) : i == col ? c2(1.0, 0.0) : x;
+    }
+  }
+  if (make_t) {
+    if (warp >= 4) t_column(jb - 1);
+    __syncthreads();
+    Tout[tid] = s_T[b16][c16];
   }
   cluster.sync();   // no CTA leaves while its shared memory may still be read
 }
-
-size_t panel7_smem_bytes(int ng) { return (size_t)(NB * 32 * ng + 32 * ng * 17) * sizeof(double2); }
 
 // partial[rb][j][c] = sum_{rows r of tile rb} conj(V[r][v0 + j]) C[r][c0 + c]
 // lane layout: tr = lane & 7 (row phase), 4 columns per warp, 8 warps -> 32 columns.
@@ -1639,11 +1668,11 @@ int panel_cluster_size() {
   if (cudaFuncSetAttribute(qr_panel6_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
       cudaSuccess)
     cudaGetLastError();
-  if (cudaFuncSetAttribute(qr_panel7_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+  if (cudaFuncSetAttribute(qr_panel8_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
       cudaSuccess)
     cudaGetLastError();
-  if (cudaFuncSetAttribute(qr_panel7_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)panel7_smem_bytes(P6W / 2)) != cudaSuccess)
+  if (cudaFuncSetAttribute(qr_panel8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           P8_ROWS * NB * (int)sizeof(double2)) != cudaSuccess)
     cudaGetLastError();
   for (int c : {16, 8}) {
     cudaLaunchConfig_t cfg = {};
@@ -1736,14 +1765,14 @@ ptn_status qr(double2* a, int m, int n, double2* q, long ldq, double2* r, long l
     while (cs < cs_max && cs * 32 < m - j0) cs *= 2;
     if (cap > 0) cs = std::min(cs, cap);
     const int chunk = cs > 1 ? (m - j0 + cs - 1) / cs : m - j0;
-    if (chunk <= QW * 32) {   // a cluster of one CTA is the single-CTA case
+    const int form = tune(PTN_TUNE_QR_PANEL);
+    if (chunk <= (form == 0 ? P8_ROWS : QW * 32)) {   // a cluster of one CTA is the single-CTA case
       cudaLaunchConfig_t cfg = {};
-      const int form = tune(PTN_TUNE_QR_PANEL);
       const int ngroups = (chunk + 31) / 32;
       cfg.gridDim = dim3(cs);
-      // warps the row chunk needs (two per 32-row group for the two-set panels)
-      cfg.blockDim = dim3((form == 0 || form == 3 ? 64 : 32) * ngroups);
-      cfg.dynamicSmemBytes = form == 0 ? panel7_smem_bytes(ngroups) : 0;
+      // warps the row chunk needs (two per 32-row group for the two-set panel)
+      cfg.blockDim = dim3(form == 0 ? P8T : (form == 3 ? 64 : 32) * ngroups);
+      cfg.dynamicSmemBytes = form == 0 ? (size_t)chunk * NB * sizeof(double2) : 0;
       cfg.stream = st;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1753,7 +1782,7 @@ ptn_status qr(double2* a, int m, int n, double2* q, long ldq, double2* r, long l
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       if (form == 0)
-        PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, qr_panel7_kernel, a, lda, m, j0, jb,
+        PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, qr_panel8_kernel, a, lda, m, j0, jb,
                                         w.T + (long)p * NB * NB, w.V, (long)k));
       else if (form == 3)
         PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, qr_panel6_kernel, a, lda, m, j0, jb,
