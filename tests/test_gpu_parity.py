@@ -353,3 +353,33 @@ def test_apply_mpo_golden(ptg):
     for x, y in zip(out.a, p1.a):
         assert x.shape == y.shape
         assert np.max(np.abs(x - y)) < 1e-13 * max(1.0, np.max(np.abs(y)))
+
+
+@pytest.mark.parametrize("mn", [(33, 33), (96, 40), (512, 256), (513, 129), (700, 257), (300, 640)])
+def test_qr_in_wide_blocks(ptg, mn):
+    """Q formed in blocks of 128 reflectors, from a workspace that held other numbers (NaN):
+    full blocks, partial ones, one column past a block, a wide matrix, and zero columns;
+    numpy.linalg.qr's factors to 1e-13 of the matrix norm times the block count."""
+    import torch
+    from pytenet_gb300 import _lib
+    from pytenet_gb300.device import empty, ptr, stream_ptr, to_dev, to_host
+    L = _lib.load()
+    m, n = mn
+    k = min(m, n)
+    rng = np.random.default_rng(m + n)
+    for zero in (False, True):
+        a = orc.crandn((m, n), rng)
+        if zero:
+            a[:, n // 2] = 0
+            a[:, 3] = 0
+        wsb = L.ptn_qr_workspace_bytes(m, n)
+        ws = torch.full((wsb,), 255, dtype=torch.uint8, device="cuda")   # NaN everywhere
+        da, q, r = to_dev(a), empty((m, k)), empty((k, n))
+        _lib.check(L.ptn_qr(ptr(da), m, n, ptr(q), k, ptr(r), n, ptr(ws), wsb, stream_ptr()))
+        q, r = to_host(q), to_host(r)
+        q_ref, r_ref = np.linalg.qr(a)
+        tol = 1e-13 * np.linalg.norm(a, 2) * (1 + k // 128)
+        assert np.abs(q @ r - a).max() <= tol
+        assert np.abs(q.conj().T @ q - np.eye(k)).max() <= 1e-13 * (1 + k // 128)
+        if not zero or m > n:
+            assert np.abs(r - r_ref).max() <= 10 * tol and np.abs(q - q_ref).max() <= 1e-10
