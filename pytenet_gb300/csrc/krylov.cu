@@ -21,8 +21,12 @@
 // to coefficients c_k and one combination pass out = sum_k c_k V[k].
 #include "ptn_common.cuh"
 #include "mlp_common.cuh"
+#include <cooperative_groups.h>
 #include <cfloat>
 #include <algorithm>
+#include <mutex>
+
+namespace cg = cooperative_groups;
 
 namespace ptn {
 
@@ -46,6 +50,30 @@ __device__ __forceinline__ double reduce_partials(const double* part, int nb, do
   double v = 0.0;
   for (int i = threadIdx.x; i < nb; i += blockDim.x) v += part[i];
   return block_sum(v, sh);
+}
+
+// state of a new run, by one CTA
+__device__ __forceinline__ void start_state(KState* st, double nrm, bool ok, int maxiter, int nb) {
+  for (int i = threadIdx.x; i < PTN_KRYLOV_MAXITER; i += blockDim.x) {
+    st->s.alpha[i] = 0.0;
+    st->s.beta[i] = 0.0;
+    st->s.coef[i].re = 0.0;
+    st->s.coef[i].im = 0.0;
+  }
+  if (threadIdx.x == 0) {
+    st->s.nrm = nrm;
+    st->s.m_used = 1;
+    st->s.stopped = ok ? 0 : 1;
+    st->s.maxiter = maxiter;
+    st->s.status = ok ? PTN_OK : PTN_NAN;
+    st->s.beta_next = 0.0;
+    st->s.eval0 = 0.0;
+    st->s.resid = 0.0;
+    st->s.m_target = 0;
+    st->coef_ready = 0;
+    st->bar = 0;
+    st->nblocks = nb;
+  }
 }
 
 __global__ void __launch_bounds__(VT) k_norm_partial(KState* st, const double2* __restrict__ x,
@@ -74,28 +102,7 @@ __global__ void __launch_bounds__(VT) k_start_finish(KState* st, const double2* 
       v0[i] = make_double2(v.x * inv, v.y * inv);
     }
   }
-  if (blockIdx.x == 0) {
-    for (int i = threadIdx.x; i < PTN_KRYLOV_MAXITER; i += blockDim.x) {
-      st->s.alpha[i] = 0.0;
-      st->s.beta[i] = 0.0;
-      st->s.coef[i].re = 0.0;
-      st->s.coef[i].im = 0.0;
-    }
-    if (threadIdx.x == 0) {
-      st->s.nrm = nrm;
-      st->s.m_used = 1;
-      st->s.stopped = ok ? 0 : 1;
-      st->s.maxiter = maxiter;
-      st->s.status = ok ? PTN_OK : PTN_NAN;
-      st->s.beta_next = 0.0;
-      st->s.eval0 = 0.0;
-      st->s.resid = 0.0;
-      st->s.m_target = 0;
-      st->coef_ready = 0;
-      st->bar = 0;
-      st->nblocks = nb;
-    }
-  }
+  if (blockIdx.x == 0) start_state(st, nrm, ok, maxiter, nb);
 }
 
 // partial Re <w, v> = sum w.x v.x + w.y v.y
@@ -296,6 +303,132 @@ __global__ void __launch_bounds__(FT, 2) k_lanczos_fused(KState* st, double2* __
     if (i < n) w[i] = make_double2(x[r].x * inv, x[r].y * inv);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->s.alpha[j] = alpha;
+    st->s.beta[j] = bnext;
+    st->s.m_used = j + 2;
+  }
+}
+
+// ------------------------------------------------------------------ small vectors
+// The same passes by ONE cluster, for vectors of at most SMALL_MAX entries: start (norm,
+// scaling), step (dot, update, norm, test, scaling) and the final pass (dot, residual norm)
+// are one launch each instead of two, three and three. What bounds the separate passes at
+// these sizes is the launches and the two-phase sums; here the vector stays in registers
+// (FS entries per thread) and the sums cross the cluster through distributed shared memory,
+// summed by every CTA in rank order. Above SMALL_MAX the FP64 work of 16 SMs outweighs it.
+// Measured (Lanczos step, graph replay): n = 512: 10.9 -> 7.7 us; n = 1568: 12.5 -> 10.3;
+// n = 16384: 13.1 -> 12.3.
+constexpr int CT = 512;              // threads per CTA
+constexpr int FS = 2;                // entries per thread
+constexpr int CLUSTER_MAX = 16;
+constexpr long SMALL_MAX = (long)CT * FS * CLUSTER_MAX;
+enum { SMALL_START = 0, SMALL_STEP = 1, SMALL_LAST = 2 };
+
+// sum over the cluster, valid in every thread; slot: 33 + CLUSTER_MAX doubles of this phase
+__device__ __forceinline__ double cluster_sum(double v, double* sh, double* part) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = (int)cluster.num_blocks();
+  v = block_sum(v, sh);
+  if (cs == 1) return v;
+  if (threadIdx.x == 0) *part = v;
+  cluster.sync();
+  const int lane = threadIdx.x & 31;
+  double t = lane < cs ? *cluster.map_shared_rank(part, lane) : 0.0;
+#pragma unroll
+  for (int o = CLUSTER_MAX / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return __shfl_sync(0xffffffffu, t, 0);
+}
+
+// SMALL_START: w is the start vector, vj receives w / |w|. SMALL_STEP: w (= A v_j) becomes
+// v_{j+1}. SMALL_LAST: alpha_j and the residual norm alone.
+template <int MODE>
+__global__ void __launch_bounds__(CT) k_lanczos_small(KState* st, double2* __restrict__ w,
+                                                      double2* __restrict__ vj,
+                                                      const double2* __restrict__ vjm1, long n,
+                                                      int j, double thresh, int maxiter) {
+  if (MODE != SMALL_START && st->s.stopped) return;   // set by earlier launches: uniform
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ double sh[33], part[2];
+  const long T = (long)gridDim.x * CT;
+  const long base = blockIdx.x * (long)CT + threadIdx.x;
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  double2 x[FS], a[FS], b[FS];
+  const double beta = (MODE != SMALL_START && j > 0) ? st->s.beta[j - 1] : 0.0;
+  double acc = 0.0;
+#pragma unroll
+  for (int r = 0; r < FS; ++r) {
+    const long i = base + r * T;
+    x[r] = a[r] = b[r] = make_double2(0.0, 0.0);
+    if (i < n) {
+      x[r] = w[i];
+      if (MODE != SMALL_START) {
+        a[r] = vj[i];
+        if (j > 0) b[r] = vjm1[i];
+        acc = fma(x[r].x, a[r].x, acc);
+        acc = fma(x[r].y, a[r].y, acc);
+      }
+    }
+  }
+  double alpha = 0.0;
+  if (MODE != SMALL_START) {
+    alpha = cluster_sum(acc, sh, &part[0]);
+    acc = 0.0;
+  }
+#pragma unroll
+  for (int r = 0; r < FS; ++r) {
+    if (base + r * T < n) {
+      if (MODE != SMALL_START) {
+        double2 t = make_double2(alpha * a[r].x, alpha * a[r].y);
+        if (j > 0) {
+          t.x += beta * b[r].x;
+          t.y += beta * b[r].y;
+        }
+        x[r].x -= t.x;
+        x[r].y -= t.y;
+      }
+      acc = fma(x[r].x, x[r].x, acc);
+      acc = fma(x[r].y, x[r].y, acc);
+    }
+  }
+  const double bnext = sqrt(cluster_sum(acc, sh, &part[1]));
+  // no CTA leaves while its partial sums are read
+  if (cluster.num_blocks() > 1) cluster.sync();
+  if (MODE == SMALL_START) {
+    const bool ok = bnext > 0.0 && isfinite(bnext);
+    const double inv = ok ? 1.0 / bnext : 0.0;
+    if (ok)
+#pragma unroll
+      for (int r = 0; r < FS; ++r) {
+        const long i = base + r * T;
+        if (i < n) vj[i] = make_double2(x[r].x * inv, x[r].y * inv);
+      }
+    if (blockIdx.x == 0) start_state(st, bnext, ok, maxiter, gridDim.x);
+    return;
+  }
+  if (MODE == SMALL_LAST) {
+    if (lead) {
+      st->s.alpha[j] = alpha;
+      st->s.beta_next = bnext;
+    }
+    return;
+  }
+  if (bnext < thresh) {
+    if (lead) {
+      st->s.alpha[j] = alpha;
+      st->s.beta_next = bnext;
+      st->s.m_used = j + 1;
+      st->s.stopped = 1;
+      st->s.breakdowns += 1;
+    }
+    return;
+  }
+  const double inv = 1.0 / bnext;
+#pragma unroll
+  for (int r = 0; r < FS; ++r) {
+    const long i = base + r * T;
+    if (i < n) w[i] = make_double2(x[r].x * inv, x[r].y * inv);
+  }
+  if (lead) {
     st->s.alpha[j] = alpha;
     st->s.beta[j] = bnext;
     st->s.m_used = j + 2;
@@ -731,12 +864,71 @@ const int32_t* krylov_stop_flag(const void* state) {
   return &static_cast<const KState*>(state)->s.stopped;
 }
 
+// CTAs of the one-cluster passes for vectors of n entries, 0: not taken
+static int small_blocks(long n) {
+  if (n > SMALL_MAX) return 0;
+  static int best = 0;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    const void* f[3] = {(const void*)k_lanczos_small<SMALL_START>,
+                        (const void*)k_lanczos_small<SMALL_STEP>,
+                        (const void*)k_lanczos_small<SMALL_LAST>};
+    bool ok = true;
+    for (const void* k : f)
+      ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    for (int c : {16, 8}) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(c);
+      cfg.blockDim = dim3(CT);
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = c;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int k = 0;
+      if (cudaOccupancyMaxActiveClusters(&k, k_lanczos_small<SMALL_STEP>, &cfg) == cudaSuccess && k > 0) {
+        best = c;
+        break;
+      }
+      cudaGetLastError();
+    }
+  });
+  int cs = 1;
+  while (cs < CLUSTER_MAX && (long)cs * CT < n) cs *= 2;   // one entry per thread if possible
+  if (cs > best) cs = best;
+  return (long)cs * CT * FS >= n ? cs : 0;
+}
+
+template <int MODE>
+static ptn_status launch_small(int cs, KState* s, double2* w, double2* vj, const double2* vjm1, long n,
+                               int j, double thresh, int maxiter, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cs);
+  cfg.blockDim = dim3(CT);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_lanczos_small<MODE>, s, w, vj, vjm1, n, j, thresh, maxiter));
+  note_launches(1);
+  return PTN_OK;
+}
+
 ptn_status krylov_start(void* state, const double2* vstart, double2* V, long n, int maxiter,
                         cudaStream_t st) {
   PTN_CHECK_ARG(n > 0, "krylov: empty vector");
   PTN_CHECK_ARG(maxiter >= 1 && maxiter <= PTN_KRYLOV_MAXITER,
                 "krylov: numiter must be in [1, %d]", PTN_KRYLOV_MAXITER);
   KState* s = static_cast<KState*>(state);
+  if (const int cs = small_blocks(n))
+    return launch_small<SMALL_START>(cs, s, const_cast<double2*>(vstart), V, V, n, 0, 0.0, maxiter, st);
   const int nb = vec_blocks(n);
   k_norm_partial<<<nb, VT, 0, st>>>(s, vstart, n);
   k_start_finish<<<nb, VT, 0, st>>>(s, vstart, V, n, maxiter);
@@ -780,6 +972,8 @@ ptn_status krylov_step(void* state, double2* V, long n, int j, cudaStream_t st) 
   double2* w = V + (long)(j + 1) * n;
   const double2* vj = V + (long)j * n;
   const double2* vjm1 = j > 0 ? V + (long)(j - 1) * n : vj;
+  if (const int cs = small_blocks(n))
+    return launch_small<SMALL_STEP>(cs, s, w, const_cast<double2*>(vj), vjm1, n, j, thresh, 0, st);
   const int fb = fused_blocks(n);
   if (fb > 0) {
     cudaLaunchConfig_t cfg = {};
@@ -812,6 +1006,10 @@ ptn_status krylov_last(void* state, const double2* V, const double2* w, long n, 
   const int nb = vec_blocks(n);
   const double2* vj = V + (long)j * n;
   const double2* vjm1 = j > 0 ? V + (long)(j - 1) * n : vj;
+  // always with the residual norm: it costs the small form nothing
+  if (const int cs = small_blocks(n))
+    return launch_small<SMALL_LAST>(cs, s, const_cast<double2*>(w), const_cast<double2*>(vj), vjm1, n,
+                                    j, 0.0, 0, st);
   k_dot_partial<<<nb, VT, 0, st>>>(s, w, vj, n);
   int launches = 1;
   if (resid) {
