@@ -15,6 +15,7 @@
 // intermediate once) and skips the zero entries of W, which for the XXZ MPO are
 // ~90% of the (chi d)^2 matrix.
 #include "ptn_common.cuh"
+#include "launch.cuh"
 #include "mpo_stage.cuh"
 #include "rns.cuh"
 #include <algorithm>
@@ -29,6 +30,7 @@ __global__ void __launch_bounds__(STAGE_Y)
     mpo_stage_kernel(const double2* __restrict__ in, double2* __restrict__ out,
                      const double2* __restrict__ w, long ldq, long ldp, int X, int P, int Q, int Y,
                      const int* skip) {
+  grid_wait();
   if (skip != nullptr && *skip != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* sin = reinterpret_cast<double2*>(smem_raw);             // [P][STAGE_Y]
@@ -63,7 +65,8 @@ ptn_status mpo_stage(const double2* in, double2* out, const double2* w, long ldq
   }
   dim3 grid((Y + STAGE_Y - 1) / STAGE_Y, X);
   PTN_CHECK_ARG(X <= 65535, "MPO stage: X too large");
-  mpo_stage_kernel<<<grid, STAGE_Y, smem, st>>>(in, out, w, ldq, ldp, X, P, Q, Y, skip);
+  PTN_CUDA_TRY(launch(mpo_stage_kernel, dim3(grid), dim3(STAGE_Y), smem, st, in, out, w, ldq, ldp,
+      X, P, Q, Y, skip));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;

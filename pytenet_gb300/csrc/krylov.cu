@@ -20,6 +20,7 @@
 // expm_krylov (krylov.py:122-136) and eigh_krylov (krylov.py:110-119) then reduce
 // to coefficients c_k and one combination pass out = sum_k c_k V[k].
 #include "ptn_common.cuh"
+#include "launch.cuh"
 #include "mlp_common.cuh"
 #include <cooperative_groups.h>
 #include <cfloat>
@@ -78,6 +79,7 @@ __device__ __forceinline__ void start_state(KState* st, double nrm, bool ok, int
 
 __global__ void __launch_bounds__(VT) k_norm_partial(KState* st, const double2* __restrict__ x,
                                                      long n) {
+  grid_wait();
   __shared__ double sh[33];
   double acc = 0.0;
   for (long i = blockIdx.x * (long)VT + threadIdx.x; i < n; i += (long)gridDim.x * VT) {
@@ -91,6 +93,7 @@ __global__ void __launch_bounds__(VT) k_norm_partial(KState* st, const double2* 
 
 __global__ void __launch_bounds__(VT) k_start_finish(KState* st, const double2* __restrict__ x,
                                                      double2* __restrict__ v0, long n, int maxiter) {
+  grid_wait();
   __shared__ double sh[33];
   const int nb = gridDim.x;
   const double nrm = sqrt(reduce_partials(st->part_a, nb, sh));
@@ -108,6 +111,7 @@ __global__ void __launch_bounds__(VT) k_start_finish(KState* st, const double2* 
 // partial Re <w, v> = sum w.x v.x + w.y v.y
 __global__ void __launch_bounds__(VT) k_dot_partial(KState* st, const double2* __restrict__ w,
                                                     const double2* __restrict__ v, long n) {
+  grid_wait();
   if (st->s.stopped) return;
   __shared__ double sh[33];
   double acc = 0.0;
@@ -126,6 +130,7 @@ __global__ void __launch_bounds__(VT) k_update(KState* st, double2* __restrict__
                                                const double2* __restrict__ vj,
                                                const double2* __restrict__ vjm1, long n, int j,
                                                int inplace) {
+  grid_wait();
   if (st->s.stopped) return;
   __shared__ double sh[33];
   const double alpha = reduce_partials(st->part_a, gridDim.x, sh);
@@ -155,6 +160,7 @@ __global__ void __launch_bounds__(VT) k_update(KState* st, double2* __restrict__
 
 __global__ void __launch_bounds__(VT) k_scale(KState* st, double2* __restrict__ w, long n, int j,
                                               double thresh) {
+  grid_wait();
   if (st->s.stopped) return;
   __shared__ double sh[33];
   const double beta = sqrt(reduce_partials(st->part_b, gridDim.x, sh));
@@ -346,6 +352,7 @@ __global__ void __launch_bounds__(CT) k_lanczos_small(KState* st, double2* __res
                                                       double2* __restrict__ vj,
                                                       const double2* __restrict__ vjm1, long n,
                                                       int j, double thresh, int maxiter) {
+  grid_wait();
   if (MODE != SMALL_START && st->s.stopped) return;   // set by earlier launches: uniform
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ double sh[33], part[2];
@@ -437,6 +444,7 @@ __global__ void __launch_bounds__(CT) k_lanczos_small(KState* st, double2* __res
 
 // final alpha; beta_next comes from the partials of a non-writing update pass
 __global__ void k_last_alpha(KState* st, int j) {
+  grid_wait();
   if (st->s.stopped) return;
   __shared__ double sh[33];
   const double alpha = reduce_partials(st->part_a, st->nblocks, sh);
@@ -444,6 +452,7 @@ __global__ void k_last_alpha(KState* st, int j) {
 }
 
 __global__ void k_last_resid(KState* st) {
+  grid_wait();
   if (st->s.stopped) return;
   __shared__ double sh[33];
   const double b = sqrt(reduce_partials(st->part_b, st->nblocks, sh));
@@ -594,6 +603,7 @@ __device__ double2 expm_e1_warp(const double* alpha, const double* beta, int m, 
 // mode 0: expm coefficients c = nrm U exp(dt Lambda) U^T e_1;
 // mode 1: lowest Ritz vector coefficients c = U[:, argmin], eval0 = min eigenvalue.
 __global__ void k_tridiag(KState* st, double dt_re, double dt_im, int mode) {
+  grid_wait();
   const int lane = threadIdx.x;  // one warp
   if (st->s.status != PTN_OK) return;
   const int m = st->s.m_used;
@@ -677,6 +687,7 @@ __device__ double2 last_coef(const double* alpha, const double* beta, int m, dou
 
 // after iteration 0: features of this local step, and the predicted depth
 __global__ void k_predict(KState* st, DepthArgs a, int Dl, int Dr, double dt_abs, int numiter) {
+  grid_wait();
   __shared__ float x[12];
   const int lane = threadIdx.x;
   if (st->s.status != PTN_OK) return;
@@ -718,6 +729,7 @@ __global__ void k_predict(KState* st, DepthArgs a, int Dl, int Dr, double dt_abs
 // after step j: from the learned depth on, accept the first depth whose residual
 // estimate is small (a prediction one short costs one more check, not the full depth)
 __global__ void k_depth_check(KState* st, int j, double dt_re, double dt_im, double tol) {
+  grid_wait();
   if (st->s.stopped || st->s.m_target != j + 1) return;
   const int m = j + 1;
   const double nrm = st->s.nrm;
@@ -742,6 +754,7 @@ __global__ void k_depth_check(KState* st, int j, double dt_re, double dt_im, dou
 
 // after the coefficients: history of this slot and, optionally, a training record
 __global__ void k_record(KState* st, DepthArgs a, double dt_re, double dt_im) {
+  grid_wait();
   if (threadIdx.x != 0 || st->s.status != PTN_OK) return;
   const int m = st->s.m_used;
   const double dta = sqrt(dt_re * dt_re + dt_im * dt_im);
@@ -815,6 +828,7 @@ __global__ void k_tridiag_eig(const KState* st, double* evals, double* evecs) {
 
 __global__ void __launch_bounds__(VT) k_combine(const KState* st, const double2* __restrict__ V,
                                                 long n, double2* __restrict__ out) {
+  grid_wait();
   if (st->s.status != PTN_OK) return;
   const int m = st->s.m_used;
   for (long i = blockIdx.x * (long)VT + threadIdx.x; i < n; i += (long)gridDim.x * VT) {
@@ -837,23 +851,24 @@ int vec_blocks(long n) {
 
 ptn_status depth_predict(void* state, const void* args, int Dl, int Dr, double dt_abs, int numiter,
                          cudaStream_t st) {
-  k_predict<<<1, 32, 0, st>>>(static_cast<KState*>(state), *static_cast<const DepthArgs*>(args), Dl,
-                              Dr, dt_abs, numiter);
+  PTN_CUDA_TRY(launch(k_predict, dim3(1), dim3(32), 0, st, static_cast<KState*>(state),
+      *static_cast<const DepthArgs*>(args), Dl, Dr, dt_abs, numiter));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;
 }
 
 ptn_status depth_check(void* state, int j, double dt_re, double dt_im, double tol, cudaStream_t st) {
-  k_depth_check<<<1, 32, 0, st>>>(static_cast<KState*>(state), j, dt_re, dt_im, tol);
+  PTN_CUDA_TRY(launch(k_depth_check, dim3(1), dim3(32), 0, st, static_cast<KState*>(state), j,
+      dt_re, dt_im, tol));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;
 }
 
 ptn_status depth_record(void* state, const void* args, double dt_re, double dt_im, cudaStream_t st) {
-  k_record<<<1, 32, 0, st>>>(static_cast<KState*>(state), *static_cast<const DepthArgs*>(args), dt_re,
-                             dt_im);
+  PTN_CUDA_TRY(launch(k_record, dim3(1), dim3(32), 0, st, static_cast<KState*>(state),
+      *static_cast<const DepthArgs*>(args), dt_re, dt_im));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;
@@ -905,18 +920,8 @@ static int small_blocks(long n) {
 template <int MODE>
 static ptn_status launch_small(int cs, KState* s, double2* w, double2* vj, const double2* vjm1, long n,
                                int j, double thresh, int maxiter, cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cs);
-  cfg.blockDim = dim3(CT);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_lanczos_small<MODE>, s, w, vj, vjm1, n, j, thresh, maxiter));
+  const LaunchShape shape{dim3(cs), dim3(CT), 0, dim3(cs, 1, 1)};
+  PTN_CUDA_TRY(launch_shape(k_lanczos_small<MODE>, shape, st, s, w, vj, vjm1, n, j, thresh, maxiter));
   note_launches(1);
   return PTN_OK;
 }
@@ -930,8 +935,8 @@ ptn_status krylov_start(void* state, const double2* vstart, double2* V, long n, 
   if (const int cs = small_blocks(n))
     return launch_small<SMALL_START>(cs, s, const_cast<double2*>(vstart), V, V, n, 0, 0.0, maxiter, st);
   const int nb = vec_blocks(n);
-  k_norm_partial<<<nb, VT, 0, st>>>(s, vstart, n);
-  k_start_finish<<<nb, VT, 0, st>>>(s, vstart, V, n, maxiter);
+  PTN_CUDA_TRY(launch(k_norm_partial, dim3(nb), dim3(VT), 0, st, s, vstart, n));
+  PTN_CUDA_TRY(launch(k_start_finish, dim3(nb), dim3(VT), 0, st, s, vstart, V, n, maxiter));
   PTN_LAUNCH_CHECK();
   note_launches(2);
   return PTN_OK;
@@ -992,9 +997,9 @@ ptn_status krylov_step(void* state, double2* V, long n, int j, cudaStream_t st) 
     note_launches(1);
     return PTN_OK;
   }
-  k_dot_partial<<<nb, VT, 0, st>>>(s, w, vj, n);
-  k_update<<<nb, VT, 0, st>>>(s, w, vj, vjm1, n, j, 1);
-  k_scale<<<nb, VT, 0, st>>>(s, w, n, j, thresh);
+  PTN_CUDA_TRY(launch(k_dot_partial, dim3(nb), dim3(VT), 0, st, s, w, vj, n));
+  PTN_CUDA_TRY(launch(k_update, dim3(nb), dim3(VT), 0, st, s, w, vj, vjm1, n, j, 1));
+  PTN_CUDA_TRY(launch(k_scale, dim3(nb), dim3(VT), 0, st, s, w, n, j, thresh));
   PTN_LAUNCH_CHECK();
   note_launches(3);
   return PTN_OK;
@@ -1010,14 +1015,15 @@ ptn_status krylov_last(void* state, const double2* V, const double2* w, long n, 
   if (const int cs = small_blocks(n))
     return launch_small<SMALL_LAST>(cs, s, const_cast<double2*>(w), const_cast<double2*>(vj), vjm1, n,
                                     j, 0.0, 0, st);
-  k_dot_partial<<<nb, VT, 0, st>>>(s, w, vj, n);
+  PTN_CUDA_TRY(launch(k_dot_partial, dim3(nb), dim3(VT), 0, st, s, w, vj, n));
   int launches = 1;
   if (resid) {
-    k_update<<<nb, VT, 0, st>>>(s, const_cast<double2*>(w), vj, vjm1, n, j, 0);
-    k_last_resid<<<1, 256, 0, st>>>(s);
+    PTN_CUDA_TRY(launch(k_update, dim3(nb), dim3(VT), 0, st, s, const_cast<double2*>(w), vj, vjm1,
+        n, j, 0));
+    PTN_CUDA_TRY(launch(k_last_resid, dim3(1), dim3(256), 0, st, s));
     launches += 2;
   } else {
-    k_last_alpha<<<1, 256, 0, st>>>(s, j);
+    PTN_CUDA_TRY(launch(k_last_alpha, dim3(1), dim3(256), 0, st, s, j));
     launches += 1;
   }
   PTN_LAUNCH_CHECK();
@@ -1026,7 +1032,8 @@ ptn_status krylov_last(void* state, const double2* V, const double2* w, long n, 
 }
 
 ptn_status krylov_coef(void* state, double dt_re, double dt_im, int mode, cudaStream_t st) {
-  k_tridiag<<<1, 32, 0, st>>>(static_cast<KState*>(state), dt_re, dt_im, mode);
+  PTN_CUDA_TRY(launch(k_tridiag, dim3(1), dim3(32), 0, st, static_cast<KState*>(state), dt_re,
+      dt_im, mode));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;
@@ -1041,7 +1048,8 @@ ptn_status krylov_tridiag_eig(const void* state, double* evals, double* evecs, c
 
 ptn_status krylov_combine(const void* state, const double2* V, long n, double2* out,
                           cudaStream_t st) {
-  k_combine<<<vec_blocks(n), VT, 0, st>>>(static_cast<const KState*>(state), V, n, out);
+  PTN_CUDA_TRY(launch(k_combine, dim3(vec_blocks(n)), dim3(VT), 0, st, static_cast<const
+      KState*>(state), V, n, out));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;

@@ -20,6 +20,7 @@
 // then Q = H_1 ... H_k [I; 0] is formed backwards with the same block update
 // (using T instead of T^H).
 #include "ptn_common.cuh"
+#include "launch.cuh"
 #include "rns.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -1033,6 +1034,7 @@ constexpr int P8_ROWS = 768;   // most rows per CTA: 192 KB
 __global__ void __launch_bounds__(P8T) qr_panel8_kernel(double2* __restrict__ a, long lda, int m,
                                                         int j0, int jb, double2* __restrict__ Tout,
                                                         double2* __restrict__ V, long ldv) {
+  grid_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), cs = (int)cluster.num_blocks();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1434,6 +1436,7 @@ __global__ void __launch_bounds__(128) larfb_tw1_kernel(double2* __restrict__ pa
                                                         int nc, int jb,
                                                         const double2* __restrict__ T,
                                                         int conjT) {
+  grid_wait();
   __shared__ double2 sT[NB][NB];
   __shared__ double2 sp[8][NB];
   __shared__ double2 sw[NB];
@@ -1489,6 +1492,7 @@ __global__ void __launch_bounds__(LW * 32) larfb_apply_kernel(double2* __restric
                                                               const double2* __restrict__ V, long ldv,
                                                               int r0, int m, int c0, int nc, int v0,
                                                               int jb, const double2* __restrict__ W2) {
+  grid_wait();
   constexpr int PH = 32 / TC;
   constexpr int RT = LW * RPW * PH;       // rows of one CTA
   __shared__ double2 sv[RT * NB];
@@ -1608,14 +1612,20 @@ ptn_status larfb_rt(double2* C, long ldc, const double2* V, long ldv, int r0, in
     case 2: larfb_vhc_kernel<2, TC><<<gp, LW * 32, 0, st>>>(C, ldc, V, ldv, r0, m, c0, nc, v0, jb, part); break;
     default: larfb_vhc_kernel<1, TC><<<gp, LW * 32, 0, st>>>(C, ldc, V, ldv, r0, m, c0, nc, v0, jb, part); break;
   }
-  larfb_tw1_kernel<<<nc, 128, 0, st>>>(part, nsplit, nc, jb, T, conjT ? 1 : 0);
+  PTN_CUDA_TRY(launch(larfb_tw1_kernel, dim3(nc), dim3(128), 0, st, part, nsplit, nc, jb, T, conjT
+      ? 1 : 0));
   const dim3 ga((unsigned)ctiles, (unsigned)splits(ra));
   switch (ra) {
-    case 16: larfb_apply_kernel<16, TC><<<ga, LW * 32, 0, st>>>(C, ldc, V, ldv, r0, m, c0, nc, v0, jb, part); break;
-    case 8: larfb_apply_kernel<8, TC><<<ga, LW * 32, 0, st>>>(C, ldc, V, ldv, r0, m, c0, nc, v0, jb, part); break;
-    case 4: larfb_apply_kernel<4, TC><<<ga, LW * 32, 0, st>>>(C, ldc, V, ldv, r0, m, c0, nc, v0, jb, part); break;
-    case 2: larfb_apply_kernel<2, TC><<<ga, LW * 32, 0, st>>>(C, ldc, V, ldv, r0, m, c0, nc, v0, jb, part); break;
-    default: larfb_apply_kernel<1, TC><<<ga, LW * 32, 0, st>>>(C, ldc, V, ldv, r0, m, c0, nc, v0, jb, part); break;
+    case 16: PTN_CUDA_TRY(launch(larfb_apply_kernel<16, TC>, dim3(ga), dim3(LW * 32), 0, st, C,
+        ldc, V, ldv, r0, m, c0, nc, v0, jb, part)); break;
+    case 8: PTN_CUDA_TRY(launch(larfb_apply_kernel<8, TC>, dim3(ga), dim3(LW * 32), 0, st, C, ldc,
+        V, ldv, r0, m, c0, nc, v0, jb, part)); break;
+    case 4: PTN_CUDA_TRY(launch(larfb_apply_kernel<4, TC>, dim3(ga), dim3(LW * 32), 0, st, C, ldc,
+        V, ldv, r0, m, c0, nc, v0, jb, part)); break;
+    case 2: PTN_CUDA_TRY(launch(larfb_apply_kernel<2, TC>, dim3(ga), dim3(LW * 32), 0, st, C, ldc,
+        V, ldv, r0, m, c0, nc, v0, jb, part)); break;
+    default: PTN_CUDA_TRY(launch(larfb_apply_kernel<1, TC>, dim3(ga), dim3(LW * 32), 0, st, C, ldc,
+        V, ldv, r0, m, c0, nc, v0, jb, part)); break;
   }
   PTN_LAUNCH_CHECK();
   note_launches(3);
@@ -1909,8 +1919,10 @@ ptn_status qr(double2* a, int m, int n, double2* q, long ldq, double2* r, long l
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       if (form == 0)
-        PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, qr_panel8_kernel, a, lda, m, j0, jb,
-                                        w.T + (long)p * NB * NB, w.V, (long)k));
+        PTN_CUDA_TRY(launch_shape(qr_panel8_kernel,
+                                  LaunchShape{cfg.gridDim, cfg.blockDim, cfg.dynamicSmemBytes,
+                                              dim3(cs, 1, 1)},
+                                  st, a, lda, m, j0, jb, w.T + (long)p * NB * NB, w.V, (long)k));
       else if (form == 3)
         PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, qr_panel6_kernel, a, lda, m, j0, jb,
                                         w.T + (long)p * NB * NB, w.V, (long)k));

@@ -25,6 +25,7 @@
 // times faster. Rows that hold an infinity or NaN, or numbers near the ends of the FP64
 // range, are multiplied entry by entry in FP64 by the reconstruction kernel.
 #include "rns.cuh"
+#include "launch.cuh"
 #include "mpo_stage.cuh"
 #include <cooperative_groups.h>
 #include <cuda.h>
@@ -239,6 +240,7 @@ __global__ void __launch_bounds__(256) k_convert(const RnsView v, int R, int K, 
                                                  bf16* __restrict__ dst, long Kp, long plane,
                                                  int* __restrict__ clear, int nclear,
                                                  const int* skip) {
+  grid_wait();
   if (skip != nullptr && *skip != 0) return;   // uniform over the launch
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* tile = reinterpret_cast<double2*>(smem_raw);   // [CR][chunk + 1]
@@ -327,6 +329,7 @@ __global__ void __launch_bounds__(128) k_convert_rows(const RnsView v, int R, in
                                                       bf16* __restrict__ dst, long Kp, long plane,
                                                       int* __restrict__ clear, int nclear,
                                                       const int* skip) {
+  grid_wait();
   if (skip != nullptr && *skip != 0) return;
   for (int i = blockIdx.x * 128 + threadIdx.x; i < nclear; i += gridDim.x * 128) clear[i] = 0;
   const int lane = threadIdx.x & 31;
@@ -489,6 +492,7 @@ template <int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     k_rns_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const GemmP g) {
+  grid_wait();
   if (g.skip != nullptr && *g.skip != 0) return;   // uniform: before any barrier or allocation
   typedef Tile<BN> T;
   extern __shared__ uint8_t smem_raw8[];
@@ -798,6 +802,7 @@ __device__ __forceinline__ double2 scaled(double2 alpha, double2 z) {
 template <int NM>
 __global__ void __launch_bounds__(256) k_reconstruct(const ReconP g, double2 alpha, double2 beta,
                                                      double2* __restrict__ out, long ldc) {
+  grid_wait();
   if (g.skip != nullptr && *g.skip != 0) return;
   const int np = (g.N + 1) >> 1;
   const long total = (long)g.M * np;
@@ -828,6 +833,7 @@ __global__ void __launch_bounds__(128)
     k_reconstruct_stage(const ReconP g, const double2* __restrict__ w, long ldq, long ldp, int P,
                         int pin, int Q, int Y, double2* __restrict__ out, int* __restrict__ e2,
                         int eq, int by_x) {
+  grid_wait();
   if (g.skip != nullptr && *g.skip != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* sin = reinterpret_cast<double2*>(smem_raw);
@@ -942,7 +948,7 @@ ptn_status launch_gemm(const RnsOperand& A, const RnsOperand& B, GemmP g, cudaSt
   PTN_CHECK_ARG(units <= INT_MAX / 2, "rns_gemm: too many tiles");
   g.units = (int)units;
   const int grid = (int)std::min<long>(units, num_sms());
-  k_rns_gemm<BN><<<grid, THREADS, Tile<BN>::SMEM, st>>>(ma, mb, g);
+  PTN_CUDA_TRY(launch(k_rns_gemm<BN>, dim3(grid), dim3(THREADS), Tile<BN>::SMEM, st, ma, mb, g));
   PTN_LAUNCH_CHECK();
   return PTN_OK;
 }
@@ -1041,20 +1047,11 @@ static ptn_status launch_convert(const RnsView& v, const RnsOperand& d, bool hav
     return launch_convert<NM>(v, d, true, bits, clear, nclear, skip, st);
   }
   PTN_CHECK_ARG(parts <= 65535, "rns_convert: too many columns");
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)groups, (unsigned)parts);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = CR * (size_t)(chunk + 1) * sizeof(double2);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 1;
-  at[0].val.clusterDim.y = (unsigned)parts;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = have_exp ? 0 : 1;
-  PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_convert<NM>, v, d.rows, d.kc, (int)chunk, d.e,
-                                  have_exp ? 1 : 0, bits, d.p, d.Kp, d.plane(), clear, nclear, skip));
+  LaunchShape shape{dim3((unsigned)groups, (unsigned)parts), dim3(256),
+                    CR * (size_t)(chunk + 1) * sizeof(double2)};
+  if (!have_exp) shape.cluster = dim3(1, (unsigned)parts, 1);
+  PTN_CUDA_TRY(launch_shape(k_convert<NM>, shape, st, v, d.rows, d.kc, (int)chunk, d.e,
+                            have_exp ? 1 : 0, bits, d.p, d.Kp, d.plane(), clear, nclear, skip));
   note_launches(1);
   return PTN_OK;
 }
@@ -1064,8 +1061,8 @@ static ptn_status convert(const RnsView& v, const RnsOperand& d, bool have_exp, 
                           int* clear, int nclear, const int* skip, cudaStream_t st) {
   if (v.sk != 1 || have_exp || d.kc > ROW_MAX)
     return launch_convert<NM>(v, d, have_exp, bits, clear, nclear, skip, st);
-  k_convert_rows<NM><<<(d.rows + 3) / 4, 128, 0, st>>>(v, d.rows, d.kc, d.e, bits, d.p, d.Kp,
-                                                       d.plane(), clear, nclear, skip);
+  PTN_CUDA_TRY(launch(k_convert_rows<NM>, dim3((d.rows + 3) / 4), dim3(128), 0, st, v, d.rows,
+      d.kc, d.e, bits, d.p, d.Kp, d.plane(), clear, nclear, skip));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;
@@ -1131,8 +1128,10 @@ ptn_status rns_gemm(const RnsOperand& A, const RnsView& va, const RnsOperand& B,
   PTN_TRY(multiply(A, va, B, vb, res, skip, st, &r));
   const long pairs = (long)r.M * ((r.N + 1) / 2);
   const int blocks = (int)std::min<long>((pairs + 255) / 256, 16L * num_sms());
-  if (A.nm == RNS_FP64) k_reconstruct<RNS_FP64><<<blocks, 256, 0, st>>>(r, alpha, beta, out, ldc);
-  else k_reconstruct<RNS_MIXED><<<blocks, 256, 0, st>>>(r, alpha, beta, out, ldc);
+  if (A.nm == RNS_FP64) PTN_CUDA_TRY(launch(k_reconstruct<RNS_FP64>, dim3(blocks), dim3(256), 0,
+      st, r, alpha, beta, out, ldc));
+  else PTN_CUDA_TRY(launch(k_reconstruct<RNS_MIXED>, dim3(blocks), dim3(256), 0, st, r, alpha,
+      beta, out, ldc));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;
@@ -1148,8 +1147,8 @@ static ptn_status launch_stage(const ReconP& r, const RnsStage& s, cudaStream_t 
   });
   PTN_CUDA_TRY(attr);
   const dim3 grid((s.Y + STAGE_Y - 1) / STAGE_Y, s.X);
-  k_reconstruct_stage<NM><<<grid, STAGE_Y, stage_smem(s.P, s.Q), st>>>(
-      r, s.w, s.ldq, s.ldp, s.P, s.pin, s.Q, s.Y, s.out, s.e2, s.eq, s.by_x ? 1 : 0);
+  PTN_CUDA_TRY(launch(k_reconstruct_stage<NM>, dim3(grid), dim3(STAGE_Y), stage_smem(s.P, s.Q), st,
+      r, s.w, s.ldq, s.ldp, s.P, s.pin, s.Q, s.Y, s.out, s.e2, s.eq, s.by_x ? 1 : 0));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;

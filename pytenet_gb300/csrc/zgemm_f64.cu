@@ -25,6 +25,7 @@
 // quantum numbers hold zero blocks (pytenet/block_sparse_util.py:47-64), which after
 // the first block QR line up with these fragments.
 #include "ptn_common.cuh"
+#include "launch.cuh"
 #include "rns.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -95,6 +96,7 @@ __device__ __forceinline__ unsigned entry_class(double2 v) {
 // block, a quarter of the K part each. gridDim.y (= the cluster's y extent) splits K too.
 template <int OA, int OB, int KW>
 __global__ void __launch_bounds__(THREADS) zgemm_dmma_kernel(const KArgs p) {
+  grid_wait();
   if (p.skip != nullptr && *p.skip != 0) return;   // uniform over the launch
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int fr = lane >> 2, fc = lane & 3;
@@ -230,20 +232,11 @@ Shape choose_shape(int M, int N, int K, int batch) {
 template <int OA, int OB>
 cudaError_t launch_ab(const Shape& s, const KArgs& k, int batch, cudaStream_t st) {
   const long edge = s.kw == 1 ? 2 * FB : FB;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(((k.M + edge - 1) / edge) * ((k.N + edge - 1) / edge)),
-                     (unsigned)s.parts, (unsigned)batch);
-  cfg.blockDim = dim3(THREADS);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = s.parts;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = s.parts > 1 ? 1 : 0;
-  if (s.kw == 1) return cudaLaunchKernelEx(&cfg, zgemm_dmma_kernel<OA, OB, 1>, k);
-  return cudaLaunchKernelEx(&cfg, zgemm_dmma_kernel<OA, OB, 4>, k);
+  LaunchShape shape{dim3((unsigned)(((k.M + edge - 1) / edge) * ((k.N + edge - 1) / edge)),
+                         (unsigned)s.parts, (unsigned)batch), dim3(THREADS), 0};
+  if (s.parts > 1) shape.cluster = dim3(1, (unsigned)s.parts, 1);
+  if (s.kw == 1) return launch_shape(zgemm_dmma_kernel<OA, OB, 1>, shape, st, k);
+  return launch_shape(zgemm_dmma_kernel<OA, OB, 4>, shape, st, k);
 }
 
 template <int OA>
