@@ -1,6 +1,5 @@
-// Device parts of the MPO stage out[x, q, y] = sum_p M[q, p] in[x, p, y], for CTAs of
-// STAGE_Y threads that each own one (x, STAGE_Y-wide y chunk): thread q compacts the
-// nonzeros of row q of M in shared memory, the P input rows of the chunk are staged there
+// Device parts of the MPO stage out[x, q, y] = sum_p M[q, p] in[x, p, y], for CTAs that
+// each own one (x, STAGE_Y-wide y chunk): thread q compacts the nonzeros of row q of M in shared memory, the P input rows of the chunk are staged there
 // too.
 // Bound: HBM / L2 for large tensors, latency for small ones, and close behind both the
 // FP64 units (two operations per SM and cycle), so entries are applied by kind: an MPO
@@ -14,7 +13,7 @@
 
 namespace ptn {
 
-constexpr int STAGE_Y = 128;     // threads of a CTA
+constexpr int STAGE_Y = 128;     // columns of a CTA, at least as many threads
 constexpr int STAGE_MAX = 64;    // largest P and Q
 
 enum { ENTRY_COMPLEX = 0, ENTRY_REAL = 1, ENTRY_ONE = 2 };
@@ -39,7 +38,7 @@ __device__ __forceinline__ double2 entry_fma(int kind, double2 v, double2 x, dou
 // M (given by strides into w) -> sval[q * P + p]
 __device__ __forceinline__ void stage_load_w(const double2* __restrict__ w, long ldq, long ldp,
                                              int P, int Q, double2* sval) {
-  for (int e = threadIdx.x; e < P * Q; e += STAGE_Y) sval[e] = w[(e / P) * ldq + (e % P) * ldp];
+  for (int e = threadIdx.x; e < P * Q; e += blockDim.x) sval[e] = w[(e / P) * ldq + (e % P) * ldp];
 }
 
 // row q of sval -> its nonzeros, their indices 4 * p + kind, their number

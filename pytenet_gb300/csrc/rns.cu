@@ -826,10 +826,12 @@ __global__ void __launch_bounds__(256) k_reconstruct(const ReconP g, double2 alp
 // ((x, p / pin), (p % pin, y)) is stage input (x, p, y), put together straight into the
 // shared-memory rows of the stage; the stage output goes to `out` and the exponents of the
 // rows it forms as the next operand to e2 (zeroed before). by_x false: rows (q % eq, y);
-// true: rows (x, q / eq). One CTA per (x, 128-wide y chunk). Saves writing and reading the
-// product in FP64 and a maximum pass over the stage output.
+// true: rows (x, q / eq). One CTA per (x, 128-wide y chunk), of STAGE_Y threads, or twice as
+// many where the CTAs alone leave too few warps in flight for the chain of loads and wide
+// integer sums. Saves writing and reading the product in FP64 and a maximum pass over the
+// stage output.
 template <int NM>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(2 * STAGE_Y)
     k_reconstruct_stage(const ReconP g, const double2* __restrict__ w, long ldq, long ldp, int P,
                         int pin, int Q, int Y, double2* __restrict__ out, int* __restrict__ e2,
                         int eq, int by_x) {
@@ -843,7 +845,7 @@ __global__ void __launch_bounds__(128)
   const int x = blockIdx.y, y0 = blockIdx.x * STAGE_Y, ty = threadIdx.x;
   stage_load_w(w, ldq, ldp, P, Q, sval);
   const int pair = 2 * (ty & 63);
-  for (int p = ty >> 6; p < P; p += 2) {
+  for (int p = ty >> 6; p < P; p += blockDim.x / 64) {
     const int y = y0 + pair;
     if (y < Y) {
       const int m = x * (P / pin) + p / pin, n = (p % pin) * Y + y;
@@ -858,14 +860,14 @@ __global__ void __launch_bounds__(128)
   __syncthreads();
   stage_compact(P, Q, sval, sidx, scount);
   __syncthreads();
-  const int y = y0 + ty;
+  const int yl = ty & (STAGE_Y - 1), y = y0 + yl;
   const int na = by_x ? Q / eq : eq, nb = by_x ? eq : Q / eq;
-  for (int a = 0; a < na; ++a) {
+  for (int a = ty / STAGE_Y; a < na; a += blockDim.x / STAGE_Y) {
     int E = 0;
     if (y < Y)
       for (int b = 0; b < nb; ++b) {
         const int q = by_x ? a * eq + b : b * eq + a;
-        const double2 z = stage_row(q, P, sin + ty, sval, sidx, scount);
+        const double2 z = stage_row(q, P, sin + yl, sval, sidx, scount);
         out[((long)x * Q + q) * Y + y] = z;
         E = max(E, max(biased_exp(z.x), biased_exp(z.y)));
       }
@@ -1147,7 +1149,10 @@ static ptn_status launch_stage(const ReconP& r, const RnsStage& s, cudaStream_t 
   });
   PTN_CUDA_TRY(attr);
   const dim3 grid((s.Y + STAGE_Y - 1) / STAGE_Y, s.X);
-  PTN_CUDA_TRY(launch(k_reconstruct_stage<NM>, dim3(grid), dim3(STAGE_Y), stage_smem(s.P, s.Q), st,
+  // measured, 250 x 256: 30 -> 22 us with 256 threads (500 CTAs); 1024 x 1024 (8192 CTAs):
+  // an environment step 2.09 -> 2.16 ms
+  const int threads = (long)grid.x * grid.y < 16L * num_sms() ? 2 * STAGE_Y : STAGE_Y;
+  PTN_CUDA_TRY(launch(k_reconstruct_stage<NM>, dim3(grid), dim3(threads), stage_smem(s.P, s.Q), st,
       r, s.w, s.ldq, s.ldp, s.P, s.pin, s.Q, s.Y, s.out, s.e2, s.eq, s.by_x ? 1 : 0));
   PTN_LAUNCH_CHECK();
   note_launches(1);
