@@ -202,11 +202,12 @@ struct Shape {
 //   bonds 250 x 256, chi 5   1207 + 1485 us -> 1201 + 1423 us (1.01 TF/s)
 //   bonds <= 28 (README run)   83 +  213 us ->    4 +    5 us, mean over a time step
 //   bonds <= 24, U(1) (DMRG)   87 +  289 us ->    4 +    5 us, mean over a sweep
-// PTN_TUNE_ZGEMM_SPLIT_WAVES 0 keeps K within a CTA, other values allow clusters.
+// PTN_TUNE_ZGEMM_SPLIT_WAVES 0 keeps K within a CTA where it has 128 entries or more; shorter
+// products are summed the same way whatever the knob.
 Shape choose_shape(int M, int N, int K, int batch) {
   const long subp = 4L * num_sms();
   const long steps = std::max(1, (K + 3) / 4);
-  const bool clusters = tune(PTN_TUNE_ZGEMM_SPLIT_WAVES) != 0;
+  const bool clusters = tune(PTN_TUNE_ZGEMM_SPLIT_WAVES) != 0 || K < 128;
   Shape best{1, 1, 0};
   double best_cost = -1.0;
   for (int kw : {1, 4})
