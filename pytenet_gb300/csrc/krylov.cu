@@ -21,6 +21,7 @@
 // to coefficients c_k and one combination pass out = sum_k c_k V[k].
 #include "ptn_common.cuh"
 #include "launch.cuh"
+#include "fp64_seed.cuh"
 #include "mlp_common.cuh"
 #include <cooperative_groups.h>
 #include <cfloat>
@@ -322,8 +323,8 @@ __global__ void __launch_bounds__(FT, 2) k_lanczos_fused(KState* st, double2* __
 // these sizes is the launches and the two-phase sums; here the vector stays in registers
 // (FS entries per thread) and the sums cross the cluster through distributed shared memory,
 // summed by every CTA in rank order. Above SMALL_MAX the FP64 work of 16 SMs outweighs it.
-// Measured (Lanczos step, graph replay): n = 512: 10.9 -> 7.7 us; n = 1568: 12.5 -> 10.3;
-// n = 16384: 13.1 -> 12.3.
+// Measured (Lanczos step, graph replay): n = 512: 10.9 -> 7.2 us; n = 1568: 12.5 -> 9.4;
+// n = 16384: 13.1 -> 11.2.
 constexpr int CT = 512;              // threads per CTA
 constexpr int FS = 2;                // entries per thread
 constexpr int CLUSTER_MAX = 16;
@@ -397,12 +398,15 @@ __global__ void __launch_bounds__(CT) k_lanczos_small(KState* st, double2* __res
       acc = fma(x[r].y, x[r].y, acc);
     }
   }
-  const double bnext = sqrt(cluster_sum(acc, sh, &part[1]));
+  const double b2 = cluster_sum(acc, sh, &part[1]);
+  const double inv = fast_rsqrt(b2);
+  double bnext = b2 * inv;
+  if (b2 > 0.0 && isfinite(b2)) bnext = fma(0.5 * inv, fma(-bnext, bnext, b2), bnext);
+  else bnext = sqrt(b2);
   // no CTA leaves while its partial sums are read
   if (cluster.num_blocks() > 1) cluster.sync();
   if (MODE == SMALL_START) {
     const bool ok = bnext > 0.0 && isfinite(bnext);
-    const double inv = ok ? 1.0 / bnext : 0.0;
     if (ok)
 #pragma unroll
       for (int r = 0; r < FS; ++r) {
@@ -429,7 +433,6 @@ __global__ void __launch_bounds__(CT) k_lanczos_small(KState* st, double2* __res
     }
     return;
   }
-  const double inv = 1.0 / bnext;
 #pragma unroll
   for (int r = 0; r < FS; ++r) {
     const long i = base + r * T;
@@ -507,87 +510,138 @@ __device__ void tridiag_ql(double* d, double* e, int n, double* z) {
 }
 
 // c = nrm exp(dt T) e_1 for the m x m symmetric tridiagonal T (diagonal alpha,
-// off-diagonal beta[0..m-2]), by one warp: lane l holds entries l and l + 32.
+// off-diagonal beta[0..m-2]), by one warp: lane l holds entries l and (HALVES = 2) l + 32.
 // Scaling and Taylor on the vector: with h = dt / 2^s and |h| |T|_1 <= 1/2, each of
-// the 2^s factors exp(h T) is summed to degree 16 (remainder below 2e-20 of the
-// vector). exp(dt T) e_1 is the same vector U exp(dt Lambda) U^T e_1 that
+// the 2^s factors exp(h T) is summed until the remainder is below 1e-20 of the vector (degree
+// 16 at most). exp(dt T) e_1 is the same vector U exp(dt Lambda) U^T e_1 that
 // expm_krylov forms from eigh (pytenet/krylov.py:133-136); here it costs a chain of
 // tridiagonal products instead of the serial FP64 sqrt / division chain of a QL
 // eigensolver. Writes out[0..m-1] when out != null; returns c_{m-1} to all lanes.
 // Beyond |dt| |T|_1 > 2^(EXPM_MAX_SCALE - 1) it does nothing and returns ok = false
 // (the caller then takes the eigen-decomposition route or the full depth).
+// What bounds it: FP64 instructions of the one warp, 64 cycles each. The usual case, s = 0
+// from the real start e_1, runs on real vectors: term k is dt^k / k! times the real T^k e_1,
+// so a term takes five instructions (dt real or imaginary) instead of twenty.
+// Measured (k_tridiag, m = 5): 22.0 us -> 6.9.
 constexpr int EXPM_MAX_SCALE = 12;
-__device__ double2 expm_e1_warp(const double* alpha, const double* beta, int m, double nrm,
-                                double dt_re, double dt_im, ptn_c128* out, bool& ok) {
+
+template <int HALVES>
+__device__ double2 expm_e1_halves(const double* alpha, const double* beta, int m, double nrm,
+                                  double dt_re, double dt_im, ptn_c128* out, bool& ok) {
   const int lane = threadIdx.x & 31;
-  double a[2], bl[2], br[2];   // diagonal, left and right off-diagonal of my rows
-  double tn = 0.0;
+  double a[HALVES], bl[HALVES], br[HALVES];   // diagonal, left and right off-diagonal of my rows
+  float tnf = 0.0f;
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
+  for (int q = 0; q < HALVES; ++q) {
     const int k = lane + 32 * q;
     a[q] = (k < m) ? alpha[k] : 0.0;
     bl[q] = (k < m && k > 0) ? beta[k - 1] : 0.0;
     br[q] = (k < m - 1) ? beta[k] : 0.0;
-    tn = fmax(tn, fabs(a[q]) + fabs(bl[q]) + fabs(br[q]));
+    const float t = __double2float_ru(fabs(a[q]) + fabs(bl[q]) + fabs(br[q]));
+    tnf = (t > tnf || t != t) ? t : tnf;
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) tn = fmax(tn, __shfl_xor_sync(0xffffffffu, tn, o));
-  const double dta = sqrt(dt_re * dt_re + dt_im * dt_im);
+  for (int o = 16; o > 0; o >>= 1) {
+    const float t = __shfl_xor_sync(0xffffffffu, tnf, o);
+    tnf = (t > tnf || t != t) ? t : tnf;
+  }
+  // a bound of |dt| |T|_1, rounded up
+  const double dta = dt_re == 0.0 ? fabs(dt_im)
+                                  : dt_im == 0.0 ? fabs(dt_re) : sqrt(dt_re * dt_re + dt_im * dt_im);
+  const float nt0 = __fmul_ru(__double2float_ru(dta), tnf);
   int sc = 0;
-  double nt = dta * tn;
-  while (nt > 0.5 && sc <= EXPM_MAX_SCALE) {
-    nt *= 0.5;
+  float nt = nt0;
+  while (nt > 0.5f && sc <= EXPM_MAX_SCALE) {
+    nt *= 0.5f;
     ++sc;
   }
   ok = (sc <= EXPM_MAX_SCALE) && (nt == nt);
   if (!ok) return make_double2(0.0, 0.0);
-  const double hs = ldexp(1.0, -sc);
-  const double hr = dt_re * hs, hi = dt_im * hs;
-  // v = e_1
-  double vr[2] = {lane == 0 ? 1.0 : 0.0, 0.0}, vi[2] = {0.0, 0.0};
-  const long reps = 1L << sc;
-  for (long rep = 0; rep < reps; ++rep) {
-    double yr[2] = {vr[0], vr[1]}, yi[2] = {vi[0], vi[1]};
-    double tr[2] = {vr[0], vr[1]}, ti[2] = {vi[0], vi[1]};
-    for (int k = 1; k <= 16; ++k) {
-      // neighbours: entry k-1 and k+1 of both halves
-      double pr[2], pi[2], nr[2], ni[2];
-      const double up_r0 = __shfl_up_sync(0xffffffffu, tr[0], 1), up_i0 = __shfl_up_sync(0xffffffffu, ti[0], 1);
-      const double up_r1 = __shfl_up_sync(0xffffffffu, tr[1], 1), up_i1 = __shfl_up_sync(0xffffffffu, ti[1], 1);
-      const double dn_r0 = __shfl_down_sync(0xffffffffu, tr[0], 1), dn_i0 = __shfl_down_sync(0xffffffffu, ti[0], 1);
-      const double dn_r1 = __shfl_down_sync(0xffffffffu, tr[1], 1), dn_i1 = __shfl_down_sync(0xffffffffu, ti[1], 1);
-      const double w31_r0 = __shfl_sync(0xffffffffu, tr[0], 31), w31_i0 = __shfl_sync(0xffffffffu, ti[0], 31);
-      const double w0_r1 = __shfl_sync(0xffffffffu, tr[1], 0), w0_i1 = __shfl_sync(0xffffffffu, ti[1], 0);
-      pr[0] = lane > 0 ? up_r0 : 0.0;
-      pi[0] = lane > 0 ? up_i0 : 0.0;
-      pr[1] = lane > 0 ? up_r1 : w31_r0;
-      pi[1] = lane > 0 ? up_i1 : w31_i0;
-      nr[0] = lane < 31 ? dn_r0 : w0_r1;
-      ni[0] = lane < 31 ? dn_i0 : w0_i1;
-      nr[1] = lane < 31 ? dn_r1 : 0.0;
-      ni[1] = lane < 31 ? dn_i1 : 0.0;
-      const double inv = 1.0 / (double)k;
+  double vr[HALVES], vi[HALVES];   // v = e_1
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        // u = T t (real T), then t <- (h / k) u
-        const double ur = fma(bl[q], pr[q], fma(a[q], tr[q], br[q] * nr[q]));
-        const double ui = fma(bl[q], pi[q], fma(a[q], ti[q], br[q] * ni[q]));
-        const double cr = hr * inv, ci = hi * inv;
-        tr[q] = fma(cr, ur, -ci * ui);
-        ti[q] = fma(cr, ui, ci * ur);
-        yr[q] += tr[q];
-        yi[q] += ti[q];
-      }
+  for (int q = 0; q < HALVES; ++q) {
+    vr[q] = (lane == 0 && q == 0) ? 1.0 : 0.0;
+    vi[q] = 0.0;
+  }
+  // neighbours k - 1 and k + 1 of a vector's entries
+  auto neighbours = [&](const double (&t)[HALVES], double (&p)[HALVES], double (&n)[HALVES]) {
+#pragma unroll
+    for (int q = 0; q < HALVES; ++q) {
+      p[q] = __shfl_up_sync(0xffffffffu, t[q], 1);
+      n[q] = __shfl_down_sync(0xffffffffu, t[q], 1);
     }
+    if constexpr (HALVES == 2) {
+      const double last = __shfl_sync(0xffffffffu, t[0], 31), first = __shfl_sync(0xffffffffu, t[1], 0);
+      if (lane == 0) p[1] = last;
+      if (lane == 31) n[0] = first;
+    }
+    // entry -1 and entry m meet zero off-diagonals
+  };
+  if (sc == 0 && (dt_re == 0.0 || dt_im == 0.0)) {
+    const double h = dt_re == 0.0 ? dt_im : dt_re;
+    double t[HALVES];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int kk = lane + 32 * q;
-      vr[q] = (kk < m) ? yr[q] : 0.0;
-      vi[q] = (kk < m) ? yi[q] : 0.0;
+    for (int q = 0; q < HALVES; ++q) {
+      a[q] *= h;
+      bl[q] *= h;
+      br[q] *= h;
+      t[q] = vr[q];
+    }
+    float rest = 1.0f;
+#pragma unroll
+    for (int k = 1; k <= 16; ++k) {
+      double p[HALVES], n[HALVES];
+      neighbours(t, p, n);
+#pragma unroll
+      for (int q = 0; q < HALVES; ++q) {
+        t[q] = fma(bl[q], p[q], fma(a[q], t[q], br[q] * n[q])) * (1.0 / (double)k);
+        if (dt_im == 0.0) vr[q] += t[q];                       // dt real: all terms add
+        else if ((k & 3) == 1) vi[q] += t[q];                  // i^k = i, -1, -i, 1
+        else if ((k & 3) == 2) vr[q] -= t[q];
+        else if ((k & 3) == 3) vi[q] -= t[q];
+        else vr[q] += t[q];
+      }
+      rest *= nt0 * (1.0f / (float)k);
+      if (rest < 1e-21f) break;   // uniform
+    }
+  } else {
+    const double hs = ldexp(1.0, -sc);
+    const double hr = dt_re * hs, hi = dt_im * hs;
+    const long reps = 1L << sc;
+    for (long rep = 0; rep < reps; ++rep) {
+      double yr[HALVES], yi[HALVES], tr[HALVES], ti[HALVES];
+#pragma unroll
+      for (int q = 0; q < HALVES; ++q) {
+        yr[q] = tr[q] = vr[q];
+        yi[q] = ti[q] = vi[q];
+      }
+#pragma unroll
+      for (int k = 1; k <= 16; ++k) {
+        double pr[HALVES], pi[HALVES], nr[HALVES], ni[HALVES];
+        neighbours(tr, pr, nr);
+        neighbours(ti, pi, ni);
+        const double cr = hr * (1.0 / (double)k), ci = hi * (1.0 / (double)k);
+#pragma unroll
+        for (int q = 0; q < HALVES; ++q) {
+          // u = T t (real T), then t <- (h / k) u
+          const double ur = fma(bl[q], pr[q], fma(a[q], tr[q], br[q] * nr[q]));
+          const double ui = fma(bl[q], pi[q], fma(a[q], ti[q], br[q] * ni[q]));
+          tr[q] = fma(cr, ur, -ci * ui);
+          ti[q] = fma(cr, ui, ci * ur);
+          yr[q] += tr[q];
+          yi[q] += ti[q];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < HALVES; ++q) {
+        const int kk = lane + 32 * q;
+        vr[q] = (kk < m) ? yr[q] : 0.0;
+        vi[q] = (kk < m) ? yi[q] : 0.0;
+      }
     }
   }
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
+  for (int q = 0; q < HALVES; ++q) {
     const int k = lane + 32 * q;
     if (out != nullptr && k < m) {
       out[k].re = nrm * vr[q];
@@ -595,9 +649,139 @@ __device__ double2 expm_e1_warp(const double* alpha, const double* beta, int m, 
     }
   }
   const int ql = (m - 1) >> 5, ll = (m - 1) & 31;
-  const double lr = __shfl_sync(0xffffffffu, ql ? vr[1] : vr[0], ll);
-  const double li = __shfl_sync(0xffffffffu, ql ? vi[1] : vi[0], ll);
+  const double lr = __shfl_sync(0xffffffffu, HALVES == 2 && ql ? vr[HALVES - 1] : vr[0], ll);
+  const double li = __shfl_sync(0xffffffffu, HALVES == 2 && ql ? vi[HALVES - 1] : vi[0], ll);
   return make_double2(nrm * lr, nrm * li);
+}
+
+__device__ double2 expm_e1_warp(const double* alpha, const double* beta, int m, double nrm,
+                                double dt_re, double dt_im, ptn_c128* out, bool& ok) {
+  return m <= 32 ? expm_e1_halves<1>(alpha, beta, m, nrm, dt_re, dt_im, out, ok)
+                 : expm_e1_halves<2>(alpha, beta, m, nrm, dt_re, dt_im, out, ok);
+}
+
+// Lowest eigenpair of T by one warp: an FP32 multisection (32 Sturm sequences at a time)
+// brackets the eigenvalue, then inverse iteration in FP64 with shifts just below it, where
+// T - shift is positive definite and the elimination needs no pivots; each solve squares the
+// error (shift = Rayleigh quotient minus twice the residual) until the residual is at
+// rounding level. A pivot that is not positive shows a shift above the eigenvalue and moves it
+// down. Returns false when that does not converge (the caller takes QL). The serial chain
+// of a solve is six FP64 instructions per row; QL takes some twenty per row, column and shift.
+// Measured (k_tridiag, m = 12): 255 us -> 26.7.
+__device__ bool lowest_pair_warp(const double* alpha, const double* beta, int m, double& eval,
+                                 double (&v)[2]) {
+  const int lane = threadIdx.x & 31;
+  __shared__ double s_a[PTN_KRYLOV_MAXITER], s_b[PTN_KRYLOV_MAXITER], s_l[PTN_KRYLOV_MAXITER],
+      s_r[PTN_KRYLOV_MAXITER], s_z[PTN_KRYLOV_MAXITER];
+  double a[2], bl[2], br[2];
+  float big = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int k = lane + 32 * q;
+    a[q] = k < m ? alpha[k] : 0.0;
+    bl[q] = (k < m && k > 0) ? beta[k - 1] : 0.0;
+    br[q] = k < m - 1 ? beta[k] : 0.0;
+    s_a[k] = a[q];
+    s_b[k] = br[q];
+    v[q] = k < m ? ((k & 1) ? -1.0 : 1.0) : 0.0;   // the signs of the lowest vector (beta > 0)
+    big = fmaxf(big, __double2float_ru(fabs(a[q]) + fabs(bl[q]) + fabs(br[q])));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+  __syncwarp();
+  if (!(big > 1e-30f && big < 1e30f)) return false;
+  if (m == 1) {
+    eval = a[0];
+    eval = __shfl_sync(0xffffffffu, eval, 0);
+    v[0] = lane == 0 ? 1.0 : 0.0;
+    v[1] = 0.0;
+    return true;
+  }
+  // ---- bracket: lo has no eigenvalue below it (as FP32 sees it)
+  const float inv = 1.0f / big;
+  float lo = -1.01f, hi = 1.01f;
+  for (int round = 0; round < 5; ++round) {
+    const float x = lo + (hi - lo) * (float)(lane + 1) * (1.0f / 33.0f);
+    float q = (float)s_a[0] * inv - x;
+    bool below = q < 0.0f;
+    for (int i = 1; i < m && !below; ++i) {
+      const float b = (float)s_b[i - 1] * inv;
+      q = (float)s_a[i] * inv - x - b * b / fmaxf(q, 1e-30f);
+      below = q < 0.0f;
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, below);
+    const int f = mask ? __ffs(mask) - 1 : 32;   // first point above the eigenvalue
+    const float w = (hi - lo) * (1.0f / 33.0f);
+    hi = f < 32 ? lo + w * (float)(f + 1) : hi;
+    lo = lo + w * (float)f;
+  }
+  const double scale = (double)big, eps = DBL_EPSILON;
+  double shift = ((double)lo - 4e-6) * scale, step = 1.6e-5 * scale;
+  double last = HUGE_VAL;
+  auto sum = [&](double x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  };
+  for (int it = 0; it < 16; ++it) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) s_z[lane + 32 * q] = v[q];
+    __syncwarp();
+    // ---- (T - shift) x = v, every lane the same
+    double d = s_a[0] - shift, z = s_z[0];
+    bool definite = d > 0.0;
+    double rd = fast_recip(d);
+    s_r[0] = rd;
+    for (int i = 1; i < m && definite; ++i) {
+      const double b = s_b[i - 1];
+      const double l = b * rd;
+      d = fma(-l, b, s_a[i] - shift);
+      z = fma(-l, z, s_z[i]);
+      definite = d > 0.0;
+      rd = fast_recip(d);
+      __syncwarp();
+      s_l[i] = l;
+      s_r[i] = rd;
+      s_z[i] = z;
+    }
+    __syncwarp();
+    if (!definite) {
+      shift -= step;
+      step *= 8.0;
+      continue;
+    }
+    double x = s_z[m - 1] * s_r[m - 1];
+    double mine[2] = {0.0, 0.0};
+    if (((m - 1) & 31) == lane) mine[(m - 1) >> 5] = x;
+    for (int i = m - 2; i >= 0; --i) {
+      x = fma(-s_l[i + 1], x, s_z[i] * s_r[i]);
+      if ((i & 31) == lane) mine[i >> 5] = x;
+    }
+    __syncwarp();
+    const double r = fast_rsqrt(sum(fma(mine[0], mine[0], mine[1] * mine[1])));
+#pragma unroll
+    for (int q = 0; q < 2; ++q) v[q] = mine[q] * r;
+    // ---- Rayleigh quotient and residual
+    double t[2];
+    {
+      const double up0 = __shfl_up_sync(0xffffffffu, v[0], 1), up1 = __shfl_up_sync(0xffffffffu, v[1], 1);
+      const double dn0 = __shfl_down_sync(0xffffffffu, v[0], 1), dn1 = __shfl_down_sync(0xffffffffu, v[1], 1);
+      const double e31 = __shfl_sync(0xffffffffu, v[0], 31), e32 = __shfl_sync(0xffffffffu, v[1], 0);
+      t[0] = fma(bl[0], up0, fma(a[0], v[0], br[0] * (lane < 31 ? dn0 : e32)));
+      t[1] = fma(bl[1], lane > 0 ? up1 : e31, fma(a[1], v[1], br[1] * dn1));
+    }
+    const double rho = sum(fma(t[0], v[0], t[1] * v[1]));
+    const double r0 = fma(-rho, v[0], t[0]), r1 = fma(-rho, v[1], t[1]);
+    const double res = sqrt(sum(fma(r0, r0, r1 * r1)));
+    eval = rho;
+    if (!(res == res)) return false;
+    // rounding level, or no more progress near it
+    if (res <= 4.0 * eps * scale || (res <= 64.0 * eps * scale && res >= 0.5 * last)) return true;
+    last = res;
+    shift = rho - 2.0 * res - 8.0 * eps * scale;
+    step = 8.0 * res;
+  }
+  return false;
 }
 
 // mode 0: expm coefficients c = nrm U exp(dt Lambda) U^T e_1;
@@ -621,6 +805,27 @@ __global__ void k_tridiag(KState* st, double dt_re, double dt_im, int mode) {
       st->s.iters_total += m;
     }
     return;
+  }
+  if (mode == 1) {
+    double ev, v[2];
+    if (lowest_pair_warp(st->s.alpha, st->s.beta, m, ev, v)) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int k = lane + 32 * q;
+        if (k < m) {
+          st->s.coef[k].re = v[q];
+          st->s.coef[k].im = 0.0;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) {
+        st->s.eval0 = ev;
+        const double c = st->s.coef[m - 1].re;
+        st->s.resid = st->s.beta_next * fabs(c) / st->s.nrm;
+        st->s.iters_total += m;
+      }
+      return;
+    }
   }
   double d[PTN_KRYLOV_MAXITER], e[PTN_KRYLOV_MAXITER], z[PTN_KRYLOV_MAXITER];
   for (int i = 0; i < m; ++i) {

@@ -21,6 +21,7 @@
 // (using T instead of T^H).
 #include "ptn_common.cuh"
 #include "launch.cuh"
+#include "fp64_seed.cuh"
 #include "rns.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -977,37 +978,6 @@ __global__ void __launch_bounds__(P6W * 32) qr_panel6_kernel(double2* __restrict
     }
   }
   cluster.sync();   // no CTA leaves while its shared memory may still be read
-}
-
-// 1 / sqrt(d) and 1 / d from an FP32 seed and one third-order step, seed and scaling by
-// integer work on the IEEE fields: five and three FP64 instructions (64 cycles each on this
-// part) where the division and square root sequences take several times that. Subnormal, zero and
-// non-finite arguments take the CUDA functions.
-__device__ __forceinline__ double seed_scale(float y, int e) {   // y 2^e for a normal float y
-  const unsigned b = __float_as_uint(y);
-  const int x = (int)(b >> 23) - 127 + 1023 + e;
-  return __longlong_as_double(((long long)x << 52) | ((long long)(b & 0x7FFFFFu) << 29));
-}
-
-__device__ __forceinline__ double fast_rsqrt(double d) {
-  const long long b = __double_as_longlong(d);
-  const int E = (int)((b >> 52) & 0x7FF);
-  if (b <= 0 || E == 0 || E == 0x7FF) return 1.0 / sqrt(d);
-  const int e = E - 1023, odd = e & 1;
-  const float m = __uint_as_float(((unsigned)(127 + odd) << 23) | ((unsigned)(b >> 29) & 0x7FFFFFu));
-  const double y = seed_scale(rsqrtf(m), -(e - odd) / 2);
-  const double r = fma(-(d * y), y, 1.0);
-  return fma(y * r, fma(r, 0.375, 0.5), y);
-}
-
-__device__ __forceinline__ double fast_recip(double d) {   // d > 0
-  const long long b = __double_as_longlong(d);
-  const int E = (int)((b >> 52) & 0x7FF);
-  if (b <= 0 || E < 2 || E > 2040) return 1.0 / d;
-  const float m = __uint_as_float(0x3F800000u | ((unsigned)(b >> 29) & 0x7FFFFFu));
-  const double y = seed_scale(__frcp_rn(m), -(E - 1023));
-  const double r = fma(-d, y, 1.0);
-  return fma(y, fma(r, r, r), y);
 }
 
 // Panel, default form: ONE cluster-wide reduction per column. The sums over the rows below

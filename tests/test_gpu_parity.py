@@ -383,3 +383,67 @@ def test_qr_in_wide_blocks(ptg, mn):
         assert np.abs(q.conj().T @ q - np.eye(k)).max() <= 1e-13 * (1 + k // 128)
         if not zero or m > n:
             assert np.abs(r - r_ref).max() <= 10 * tol and np.abs(q - q_ref).max() <= 1e-10
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 12, 31, 33, 60])
+@pytest.mark.parametrize("kind", ["random", "split", "degenerate", "scaled"])
+def test_lowest_pair_of_the_krylov_space(ptg, m, kind):
+    """Coefficients and energy of the Ritz step from the tridiagonal matrix in the Krylov state:
+    numpy's lowest eigenvalue to rounding, the residual at rounding level."""
+    import ctypes
+    import torch
+    from pytenet_gb300 import _lib
+    from pytenet_gb300.device import ptr, stream_ptr
+    L = _lib.load()
+    rng = np.random.default_rng(m)
+    a, b = rng.standard_normal(m) * 3, np.abs(rng.standard_normal(m)) + 0.1
+    if kind == "split" and m > 2:
+        b[m // 2 - 1] = 1e-13                      # two nearly uncoupled blocks
+    if kind == "degenerate":
+        a[:], b[:] = 1.0, 1e-9
+    if kind == "scaled":
+        a, b = a * 1e6 - 1e7, b * 1e6
+    st = _lib.KrylovState()
+    for i in range(m):
+        st.alpha[i], st.beta[i] = a[i], b[i]
+    st.m_used, st.status, st.nrm, st.beta_next = m, 0, 1.0, b[m - 1]
+    raw = np.zeros(L.ptn_krylov_state_bytes(), np.uint8)
+    raw[:ctypes.sizeof(st)] = np.frombuffer(bytes(st), np.uint8)
+    dev = torch.from_numpy(raw).to("cuda")
+    _lib.check(L.ptn_krylov_eigh_coef(ptr(dev), stream_ptr()))
+    out = _lib.KrylovState.from_buffer_copy(bytes(dev.cpu().numpy()[:ctypes.sizeof(st)]))
+    c = np.array([out.coef[i].re + 1j * out.coef[i].im for i in range(m)])
+    T = np.diag(a) + np.diag(b[:m - 1], 1) + np.diag(b[:m - 1], -1)
+    scale = np.abs(a).max() + 2 * np.abs(b).max()
+    eps = np.finfo(float).eps
+    assert abs(out.eval0 - np.linalg.eigvalsh(T)[0]) <= 16 * m * eps * scale
+    assert abs(np.linalg.norm(c) - 1) <= 16 * m * eps
+    assert np.linalg.norm(T @ c - out.eval0 * c) <= 64 * m * eps * scale
+
+
+@pytest.mark.parametrize("m", [1, 5, 31, 32, 33, 60])
+@pytest.mark.parametrize("dt", [-0.03j, 0.02, -0.4j, 0.01 - 0.05j, 0.0])
+def test_expm_coefficients_of_the_krylov_space(ptg, m, dt):
+    """exp(dt T) e_1 on one and two entries per lane, for real, imaginary and complex steps, with
+    and without scaling: numpy's eigh of T to 1e-13."""
+    import ctypes
+    import torch
+    from pytenet_gb300 import _lib
+    from pytenet_gb300.device import ptr, stream_ptr
+    L = _lib.load()
+    rng = np.random.default_rng(100 + m)
+    a, b = rng.standard_normal(m) * 3, np.abs(rng.standard_normal(m)) + 0.1
+    st = _lib.KrylovState()
+    for i in range(m):
+        st.alpha[i], st.beta[i] = a[i], b[i]
+    st.m_used, st.status, st.nrm, st.beta_next = m, 0, 1.7, b[m - 1]
+    raw = np.zeros(L.ptn_krylov_state_bytes(), np.uint8)
+    raw[:ctypes.sizeof(st)] = np.frombuffer(bytes(st), np.uint8)
+    dev = torch.from_numpy(raw).to("cuda")
+    dt = complex(dt)
+    _lib.check(L.ptn_krylov_expm_coef(ptr(dev), dt.real, dt.imag, stream_ptr()))
+    out = _lib.KrylovState.from_buffer_copy(bytes(dev.cpu().numpy()[:ctypes.sizeof(st)]))
+    c = np.array([out.coef[i].re + 1j * out.coef[i].im for i in range(m)])
+    w, u = np.linalg.eigh(np.diag(a) + np.diag(b[:m - 1], 1) + np.diag(b[:m - 1], -1))
+    ref = 1.7 * (u * np.exp(dt * w)) @ u[0]
+    assert np.abs(c - ref).max() <= 1e-13 * np.linalg.norm(ref)
