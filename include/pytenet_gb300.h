@@ -316,6 +316,21 @@ ptn_status ptn_eigh_site(ptn_c128* a, const ptn_c128* w, const ptn_c128* l, cons
 size_t ptn_qr_workspace_bytes(int m, int n);
 ptn_status ptn_qr(ptn_c128* a, int m, int n, ptn_c128* q, long ldq, ptn_c128* r, long ldr,
                   void* ws, size_t ws_bytes, void* stream);
+
+/* QR of blocks of a block-sparse matrix, all in one launch (pytenet/block_sparse_util.py:
+ * 106-180): block element (i, c) at src[src_row[i] + src_col[c]], its Q (m x k) and R (k x n),
+ * k = min(m, n), to q[q_row[i] + q_col[c]] and r[r_row[i] + r_col[c]]. `blocks` and the maps
+ * are device memory; a block has at most ptn_qr_blocks_max_columns() columns and
+ * ptn_qr_blocks_max_rows() rows (0 rows: not available under the present knobs), max_m is the
+ * largest row count among them. src must not alias q or r. */
+typedef struct {
+  int32_t m, n;
+  const int64_t *src_row, *src_col, *q_row, *q_col, *r_row, *r_col;
+} ptn_qr_block;
+int ptn_qr_blocks_max_columns(void);
+int ptn_qr_blocks_max_rows(void);
+ptn_status ptn_qr_blocks(const ptn_c128* src, ptn_c128* q, ptn_c128* r, const ptn_qr_block* blocks,
+                         int nblocks, int max_m, void* stream);
 /* dst[p*nc + c] = src[row_off[p] + col_off[c]] (gather one quantum-number block,
  * with any transposition folded into the offsets) */
 ptn_status ptn_gather(const ptn_c128* src, const int64_t* row_off, const int64_t* col_off,

@@ -130,6 +130,9 @@ _SIGS = {
     "ptn_diag_scale": (I, [P, L, L, L, P, I, P]),
     "ptn_qr_workspace_bytes": (S, [I, I]),
     "ptn_qr": (I, [P, I, I, P, L, P, L, P, S, P]),
+    "ptn_qr_blocks_max_columns": (I, []),
+    "ptn_qr_blocks_max_rows": (I, []),
+    "ptn_qr_blocks": (I, [P, P, P, P, I, I, P]),
     "ptn_gather": (I, [P, P, P, I, I, P, P]),
     "ptn_scatter": (I, [P, L, P, P, I, I, P, P]),
     "ptn_scale": (I, [P, P, L, c128, P]),

@@ -83,6 +83,25 @@ def _block_maps(plan, src_view, q_view, r_view):
     return maps
 
 
+def _small_blocks(plan, maps, key):
+    """Blocks narrow enough for the one-launch block QR: their indices, the largest row count
+    and the device table of ptn_qr_block, cached on the plan with the maps it points to."""
+    L = lib()
+    rows, cols = L.ptn_qr_blocks_max_rows(), L.ptn_qr_blocks_max_columns()
+    entry = plan.dev_cache.get((key, rows))
+    if entry is None:
+        small = [k for k, b in enumerate(plan.blocks) if len(b[1]) <= cols and len(b[0]) <= rows]
+        table = np.zeros((len(small), 7), np.int64)
+        for t, k in enumerate(small):
+            m, n = len(plan.blocks[k][0]), len(plan.blocks[k][1])
+            table[t, 0] = m | (n << 32)
+            table[t, 1:] = [ptr(x) for x in maps[k]]
+        max_m = max((len(plan.blocks[k][0]) for k in small), default=0)
+        entry = (frozenset(small), max_m, _dev_i64(table.reshape(-1)) if small else None)
+        plan.dev_cache[(key, rows)] = entry
+    return entry
+
+
 class QRScratch:
     """Device scratch of the block QR (grow-only)."""
 
@@ -91,6 +110,25 @@ class QRScratch:
         self.work = Workspace()
         self.qb = Workspace()
         self.rb = Workspace()
+
+    def reserve(self, mb, nb, kb):
+        L = lib()
+        wsb = L.ptn_qr_workspace_bytes(mb, nb)
+        return (self.work.get(mb * nb * 16), self.qb.get(mb * kb * 16), self.rb.get(kb * nb * 16),
+                self.ws.get(wsb), wsb)
+
+
+def _qr_block(block, maps, src, q_dst, r_dst, scratch, st):
+    """Gather, QR and scatter of one block on stream st."""
+    L = lib()
+    rows, cols, k0, kb = block
+    sro, sco, qro, qco, rro, rco = maps
+    mb, nb = len(rows), len(cols)
+    work, qb, rb, ws, wsb = scratch.reserve(mb, nb, kb)
+    call(L.ptn_gather, ptr(src), ptr(sro), ptr(sco), mb, nb, ptr(work), st)
+    call(L.ptn_qr, ptr(work), mb, nb, ptr(qb), kb, ptr(rb), nb, ptr(ws), wsb, st)
+    call(L.ptn_scatter, ptr(qb), kb, ptr(qro), ptr(qco), mb, kb, ptr(q_dst), st)
+    call(L.ptn_scatter, ptr(rb), nb, ptr(rro), ptr(rco), kb, nb, ptr(r_dst), st)
 
 
 def qr_execute(plan, src, src_view, q_dst, q_view, r_dst, r_view, scratch):
@@ -106,18 +144,13 @@ def qr_execute(plan, src, src_view, q_dst, q_view, r_dst, r_view, scratch):
         qro, qco = q_view.offsets([0], [0])
         q_dst.view(-1)[int(qro[0] + qco[0])] = 1.0
         return
-    for (rows, cols, k0, kb), (sro, sco, qro, qco, rro, rco) in zip(
-            plan.blocks, _block_maps(plan, src_view, q_view, r_view)):
-        mb, nb = len(rows), len(cols)
-        work = scratch.work.get(mb * nb * 16)
-        qb = scratch.qb.get(mb * kb * 16)
-        rb = scratch.rb.get(kb * nb * 16)
-        wsb = L.ptn_qr_workspace_bytes(mb, nb)
-        ws = scratch.ws.get(wsb)
-        call(L.ptn_gather, ptr(src), ptr(sro), ptr(sco), mb, nb, ptr(work), st)
-        call(L.ptn_qr, ptr(work), mb, nb, ptr(qb), kb, ptr(rb), nb, ptr(ws), wsb, st)
-        call(L.ptn_scatter, ptr(qb), kb, ptr(qro), ptr(qco), mb, kb, ptr(q_dst), st)
-        call(L.ptn_scatter, ptr(rb), nb, ptr(rro), ptr(rco), kb, nb, ptr(r_dst), st)
+    maps = _block_maps(plan, src_view, q_view, r_view)
+    small, max_m, table = _small_blocks(plan, maps, (src_view.key(), q_view.key(), r_view.key()))
+    if small:
+        call(L.ptn_qr_blocks, ptr(src), ptr(q_dst), ptr(r_dst), ptr(table), len(small), max_m, st)
+    for k in range(len(plan.blocks)):
+        if k not in small:
+            _qr_block(plan.blocks[k], maps[k], src, q_dst, r_dst, scratch, st)
 
 
 _SCRATCH = None

@@ -1001,10 +1001,35 @@ __global__ void __launch_bounds__(P6W * 32) qr_panel6_kernel(double2* __restrict
 constexpr int P8T = 256;
 constexpr int P8_ROWS = 768;   // most rows per CTA: 192 KB
 
-__global__ void __launch_bounds__(P8T) qr_panel8_kernel(double2* __restrict__ a, long lda, int m,
-                                                        int j0, int jb, double2* __restrict__ Tout,
-                                                        double2* __restrict__ V, long ldv) {
+// P8_FULL: the matrix is this panel alone (at most NB columns): Q = [I; 0] - V (T V1^H), V1
+// the top of V, and R are written here, in one launch instead of seven. P8_MAPS: the same for
+// the blocks of a block-sparse matrix, one cluster each, read and written through their
+// index maps, so that a whole block QR is one launch instead of four (gather, QR, two
+// scatters) per block.
+enum { P8_PANEL = 0, P8_FULL = 1, P8_MAPS = 2 };
+
+struct P8Args {
+  double2* a;              // panel / matrix, or the source of the blocks
+  long lda;
+  int m, ncol, j0, jb;     // rows, columns, first row and column, reflectors
+  double2* T;              // P8_PANEL: T, V
+  double2* V;
+  long ldv;
+  double2* q;              // the others: Q, R (P8_MAPS: the destinations of the blocks)
+  long ldq;
+  double2* r;
+  long ldr;
+  const ptn_qr_block* blocks;
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(P8T) qr_panel8_kernel(const P8Args g) {
+  constexpr bool FULL = MODE != P8_PANEL;
   grid_wait();
+  ptn_qr_block blk{};
+  if (MODE == P8_MAPS) blk = g.blocks[blockIdx.y];
+  const int m = MODE == P8_MAPS ? blk.m : g.m, ncol = MODE == P8_MAPS ? blk.n : g.ncol;
+  const int j0 = MODE == P8_MAPS ? 0 : g.j0, jb = MODE == P8_MAPS ? min(m, ncol) : g.jb;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), cs = (int)cluster.num_blocks();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1029,13 +1054,15 @@ __global__ void __launch_bounds__(P8T) qr_panel8_kernel(double2* __restrict__ a,
   const int nr = max(0, min(m, rb + chunk) - rb);   // its rows
   for (int e = tid; e < nr * NB; e += P8T) {
     const int c = e & (NB - 1);
-    xs[e] = c < jb ? a[(long)(rb + (e >> 4)) * lda + j0 + c] : c2(0.0, 0.0);
+    const int i = rb + (e >> 4);
+    if (MODE == P8_MAPS) xs[e] = c < ncol ? g.a[blk.src_row[i] + blk.src_col[c]] : c2(0.0, 0.0);
+    else xs[e] = c < ncol ? g.a[(long)i * g.lda + j0 + c] : c2(0.0, 0.0);
   }
   for (int e = tid; e < NB * (NB + 1); e += P8T) {
     (&s_S[0][0])[e] = c2(0.0, 0.0);
     (&s_T[0][0])[e] = c2(0.0, 0.0);
   }
-  const bool make_t = rank == cs - 1;   // the CTA with the fewest rows
+  const bool make_t = FULL || rank == cs - 1;   // the CTA with the fewest rows
   // column q of T from columns < q (threads 128 .. 255: eight per row)
   auto t_column = [&](int q) {
     const int t = tid - 128;
@@ -1186,20 +1213,65 @@ __global__ void __launch_bounds__(P8T) qr_panel8_kernel(double2* __restrict__ a,
     }
   }
   __syncthreads();
+  if (FULL) {
+    if (warp >= 4) t_column(jb - 1);
+    cluster.sync();
+    // V1 (unit lower triangular) into s_S, M = T V1^H
+    __shared__ double2 s_M[NB][NB + 1];
+    {
+      double2 v = c2(b16 == c16 ? 1.0 : 0.0, 0.0);
+      if (b16 > c16 && b16 < jb)
+        v = cluster.map_shared_rank(xs, b16 / chunk)[(b16 % chunk) * NB + c16];
+      s_S[b16][c16] = v;
+    }
+    __syncthreads();
+    {
+      double2 s = c2(0.0, 0.0);
+      for (int b = b16; b <= c16; ++b) s = cfma(s_T[b16][b], cconj(s_S[c16][b]), s);
+      s_M[b16][c16] = s;
+    }
+    __syncthreads();
+    // rows of R, then Q over the rows in place: a thread takes columns c and 15 - c of a row
+    for (int e = tid; e < nr * NB; e += P8T) {
+      const int i = rank * chunk + (e >> 4), c = e & (NB - 1);
+      if (i < jb && c < ncol)
+        g.r[MODE == P8_MAPS ? blk.r_row[i] + blk.r_col[c] : (long)i * g.ldr + c] =
+            c >= i ? xs[e] : c2(0.0, 0.0);
+    }
+    const int c = tid & 7, cc = NB - 1 - c;
+    for (int lr = tid >> 3; lr < nr; lr += P8T / 8) {
+      const int i = rank * chunk + lr;
+      const double2* row = xs + lr * NB;
+      double2 s = c2(0.0, 0.0), t = c2(0.0, 0.0);
+      const int top = min(i, jb - 1);   // entries of V in this row: k < i, and 1 at k = i
+      for (int k = 0; k <= min(cc, top); ++k) {
+        const double2 v = k == i ? c2(1.0, 0.0) : row[k];
+        t = cfma(v, s_M[k][cc], t);
+        if (k <= c) s = cfma(v, s_M[k][c], s);
+      }
+      const long at = MODE == P8_MAPS ? blk.q_row[i] : (long)i * g.ldq;
+      if (c < jb)
+        g.q[at + (MODE == P8_MAPS ? blk.q_col[c] : c)] = c2((i == c ? 1.0 : 0.0) - s.x, -s.y);
+      if (cc < jb)
+        g.q[at + (MODE == P8_MAPS ? blk.q_col[cc] : cc)] = c2((i == cc ? 1.0 : 0.0) - t.x, -t.y);
+    }
+    cluster.sync();   // no CTA leaves while its shared memory may still be read
+    return;
+  }
   // ---- the panel and the explicit V
   for (int e = tid; e < nr * NB; e += P8T) {
     const int c = e & (NB - 1);
     if (c < jb) {
       const int i = rb + (e >> 4), col = j0 + c;
       const double2 x = xs[e];
-      a[(long)i * lda + col] = x;
-      V[(long)i * ldv + col] = i < col ? c2(0.0, 0.0) : i == col ? c2(1.0, 0.0) : x;
+      g.a[(long)i * g.lda + col] = x;
+      g.V[(long)i * g.ldv + col] = i < col ? c2(0.0, 0.0) : i == col ? c2(1.0, 0.0) : x;
     }
   }
   if (make_t) {
     if (warp >= 4) t_column(jb - 1);
     __syncthreads();
-    Tout[tid] = s_T[b16][c16];
+    g.T[tid] = s_T[b16][c16];
   }
   cluster.sync();   // no CTA leaves while its shared memory may still be read
 }
@@ -1649,12 +1721,13 @@ int panel_cluster_size() {
   if (cudaFuncSetAttribute(qr_panel6_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
       cudaSuccess)
     cudaGetLastError();
-  if (cudaFuncSetAttribute(qr_panel8_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-      cudaSuccess)
-    cudaGetLastError();
-  if (cudaFuncSetAttribute(qr_panel8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           P8_ROWS * NB * (int)sizeof(double2)) != cudaSuccess)
-    cudaGetLastError();
+  for (auto f : {qr_panel8_kernel<P8_PANEL>, qr_panel8_kernel<P8_FULL>, qr_panel8_kernel<P8_MAPS>}) {
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+      cudaGetLastError();
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             P8_ROWS * NB * (int)sizeof(double2)) != cudaSuccess)
+      cudaGetLastError();
+  }
   for (int c : {16, 8}) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(c);
@@ -1863,6 +1936,9 @@ ptn_status qr(double2* a, int m, int n, double2* q, long ldq, double2* r, long l
   const int prof = prof_begin(st, PROF_QR, 2.0 * fq, 16.0 * 3.0 * m * n);
   const int cs_max = panel_cluster_size();
   const int cap = tune(PTN_TUNE_QR_CLUSTER);
+  // one panel of a small enough row count: Q and R come out of the panel kernel
+  const bool single = n <= NB && tune(PTN_TUNE_QR_PANEL) == 0 &&
+                      m <= P8_ROWS * std::min(cs_max, cap > 0 ? cap : cs_max);
   auto panel = [&](int j0, int p) -> ptn_status {
     const int jb = std::min(NB, k - j0);
     // cluster of the panel: at least 32 rows per CTA (power of two), at most the
@@ -1889,10 +1965,12 @@ ptn_status qr(double2* a, int m, int n, double2* q, long ldq, double2* r, long l
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       if (form == 0)
-        PTN_CUDA_TRY(launch_shape(qr_panel8_kernel,
+        PTN_CUDA_TRY(launch_shape(single ? qr_panel8_kernel<P8_FULL> : qr_panel8_kernel<P8_PANEL>,
                                   LaunchShape{cfg.gridDim, cfg.blockDim, cfg.dynamicSmemBytes,
                                               dim3(cs, 1, 1)},
-                                  st, a, lda, m, j0, jb, w.T + (long)p * NB * NB, w.V, (long)k));
+                                  st, P8Args{a, lda, m, single ? n : jb, j0, jb,
+                                             w.T + (long)p * NB * NB, w.V, (long)k, q, ldq, r, ldr,
+                                             nullptr}));
       else if (form == 3)
         PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, qr_panel6_kernel, a, lda, m, j0, jb,
                                         w.T + (long)p * NB * NB, w.V, (long)k));
@@ -1938,6 +2016,10 @@ ptn_status qr(double2* a, int m, int n, double2* q, long ldq, double2* r, long l
   const bool look_ahead = ss.ok && ss.device == dev && k > NB;
   bool pending = false;   // side-stream work not yet joined
   PTN_TRY(panel(0, 0));
+  if (single) {
+    prof_end(st, prof);
+    return PTN_OK;
+  }
   for (int j0 = 0, p = 0; j0 < k; j0 += NB, ++p) {
     const int jb = std::min(NB, k - j0);
     const int nc = n - j0 - jb;                               // trailing columns
@@ -1993,11 +2075,53 @@ ptn_status qr(double2* a, int m, int n, double2* q, long ldq, double2* r, long l
   return PTN_OK;
 }
 
+// The QR of every listed block (at most NB columns, max_m rows), one launch
+ptn_status qr_blocks(const double2* src, double2* q, double2* r, const ptn_qr_block* blocks,
+                     int nblocks, int max_m, cudaStream_t st) {
+  PTN_CHECK_ARG(max_m > 0 && nblocks >= 0 && nblocks <= 65535, "qr_blocks: bad sizes");
+  if (nblocks == 0) return PTN_OK;
+  const int cs_max = panel_cluster_size();
+  const int cap = tune(PTN_TUNE_QR_CLUSTER);
+  int cs = 1;
+  while (cs < cs_max && cs * 32 < max_m) cs *= 2;
+  if (cap > 0) cs = std::min(cs, cap);
+  const int chunk = (max_m + cs - 1) / cs;
+  PTN_CHECK_ARG(chunk <= P8_ROWS, "qr_blocks: blocks of %d rows are too tall", max_m);
+  P8Args g{};
+  g.a = const_cast<double2*>(src);
+  g.q = q;
+  g.r = r;
+  g.blocks = blocks;
+  const int prof = prof_begin(st, PROF_QR, 0.0, 0.0);
+  PTN_CUDA_TRY(launch_shape(qr_panel8_kernel<P8_MAPS>,
+                            LaunchShape{dim3(cs, nblocks), dim3(P8T),
+                                        (size_t)chunk * NB * sizeof(double2), dim3(cs, 1, 1)},
+                            st, g));
+  note_launches(1);
+  prof_end(st, prof);
+  return PTN_OK;
+}
+
 }  // namespace ptn
 
 extern "C" {
 
 size_t ptn_qr_workspace_bytes(int m, int n) { return ptn::qr_workspace_bytes(m, n); }
+
+int ptn_qr_blocks_max_columns(void) { return ptn::NB; }
+int ptn_qr_blocks_max_rows(void) {
+  const int cap = ptn::tune(PTN_TUNE_QR_CLUSTER);
+  if (ptn::tune(PTN_TUNE_QR_PANEL) != 0) return 0;   // another panel kernel is asked for
+  const int cs = ptn::panel_cluster_size();
+  return ptn::P8_ROWS * (cap > 0 ? std::min(cap, cs) : cs);
+}
+
+ptn_status ptn_qr_blocks(const ptn_c128* src, ptn_c128* q, ptn_c128* r, const ptn_qr_block* blocks,
+                         int nblocks, int max_m, void* stream) {
+  return ptn::qr_blocks(reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(q),
+                        reinterpret_cast<double2*>(r), blocks, nblocks, max_m,
+                        ptn::as_stream(stream));
+}
 
 ptn_status ptn_qr(ptn_c128* a, int m, int n, ptn_c128* q, long ldq, ptn_c128* r, long ldr,
                   void* ws, size_t ws_bytes, void* stream) {

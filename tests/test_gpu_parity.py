@@ -385,6 +385,26 @@ def test_qr_in_wide_blocks(ptg, mn):
             assert np.abs(r - r_ref).max() <= 10 * tol and np.abs(q - q_ref).max() <= 1e-10
 
 
+@pytest.mark.parametrize("mn", [(1, 1), (2, 1), (5, 5), (16, 16), (17, 16), (40, 9), (70, 16), (600, 13), (9000, 4)])
+def test_qr_of_one_panel(ptg, mn):
+    """At most 16 columns: Q and R come from the panel kernel, over one to sixteen CTAs, with
+    zero columns and an upper triangular matrix (reflectors that are the identity)."""
+    m, n = mn
+    rng = np.random.default_rng(m * 31 + n)
+    for kind in ("full", "zero", "triangular"):
+        a = orc.crandn((m, n), rng)
+        if kind == "zero":
+            a[:, n // 2] = 0
+        if kind == "triangular":
+            a = np.triu(a)
+            a[np.arange(n), np.arange(n)] = a[np.arange(n), np.arange(n)].real
+        q, r, _ = ptg.block_sparse_qr(a, np.zeros(m, int), np.zeros(n, int))
+        q_ref, r_ref = np.linalg.qr(a)
+        tol = 1e-13 * max(1.0, np.linalg.norm(a, 2))
+        assert np.abs(r - r_ref).max() <= tol and np.abs(q - q_ref).max() <= 1e-12, kind
+        assert np.all(np.tril(r, -1) == 0)
+
+
 @pytest.mark.parametrize("m", [1, 2, 3, 12, 31, 33, 60])
 @pytest.mark.parametrize("kind", ["random", "split", "degenerate", "scaled"])
 def test_lowest_pair_of_the_krylov_space(ptg, m, kind):
