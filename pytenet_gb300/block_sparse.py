@@ -103,13 +103,24 @@ def _small_blocks(plan, maps, key):
 
 
 class QRScratch:
-    """Device scratch of the block QR (grow-only)."""
+    """Device scratch of the block QR (grow-only), and of the blocks that run beside each
+    other on streams of their own."""
+
+    LANES = 4
 
     def __init__(self):
         self.ws = Workspace()
         self.work = Workspace()
         self.qb = Workspace()
         self.rb = Workspace()
+        self.streams = []
+        self.lanes = []
+
+    def lane(self, i):
+        while len(self.lanes) <= i:
+            self.lanes.append(QRScratch())
+            self.streams.append(torch.cuda.Stream())
+        return self.lanes[i], self.streams[i]
 
     def reserve(self, mb, nb, kb):
         L = lib()
@@ -148,9 +159,26 @@ def qr_execute(plan, src, src_view, q_dst, q_view, r_dst, r_view, scratch):
     small, max_m, table = _small_blocks(plan, maps, (src_view.key(), q_view.key(), r_view.key()))
     if small:
         call(L.ptn_qr_blocks, ptr(src), ptr(q_dst), ptr(r_dst), ptr(table), len(small), max_m, st)
-    for k in range(len(plan.blocks)):
-        if k not in small:
+    # the wide blocks are chains of small launches: beside each other, largest first
+    wide = sorted((k for k in range(len(plan.blocks)) if k not in small),
+                  key=lambda k: -len(plan.blocks[k][0]) * len(plan.blocks[k][1]) * plan.blocks[k][3])
+    lanes = min(len(wide), scratch.LANES)
+    if lanes < 2:
+        for k in wide:
             _qr_block(plan.blocks[k], maps[k], src, q_dst, r_dst, scratch, st)
+        return
+    main = torch.cuda.current_stream()
+    fork = main.record_event()
+    for i in range(lanes):
+        lane, stream = scratch.lane(i)
+        for k in wide[i::lanes]:   # no buffer is replaced while a block of this call uses it
+            rows, cols, _, kb = plan.blocks[k]
+            lane.reserve(len(rows), len(cols), kb)
+        stream.wait_event(fork)
+        for k in wide[i::lanes]:
+            _qr_block(plan.blocks[k], maps[k], src, q_dst, r_dst, lane, stream.cuda_stream)
+    for i in range(lanes):
+        main.wait_stream(scratch.streams[i])
 
 
 _SCRATCH = None
