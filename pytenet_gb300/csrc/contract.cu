@@ -102,19 +102,20 @@ GemmArgs gemm_args(char oa, char ob, int M, int N, int K, const double2* A, long
 // The FP64 form takes the residue planes where both GEMMs do (rns_wanted), the DMMA kernel
 // otherwise, or when the workspace is smaller than the query asks for; the mixed form takes
 // its (fewer) planes unless a product is too long for them.
-static int form(int prec, bool wanted, long k1, long k2) {
+static int form(int prec, bool wanted, long k1, long k2, int mixed) {
   if (prec == PTN_PREC_FP64) return wanted ? RNS_FP64 : 0;
-  return rns_bits(k1, RNS_MIXED) != 0 && rns_bits(k2, RNS_MIXED) != 0 ? RNS_MIXED : 0;
+  return rns_bits(k1, mixed) != 0 && rns_bits(k2, mixed) != 0 ? mixed : 0;
 }
 
 int heff_form(int prec, int Dl, int d, int Dr, int cl, int cr) {
   return form(prec, rns_wanted((long)Dl * d, (long)cr * Dr, Dr) &&
-                        rns_wanted(Dl, (long)d * Dr, (long)Dl * cl), Dr, (long)Dl * cl);
+                        rns_wanted(Dl, (long)d * Dr, (long)Dl * cl), Dr, (long)Dl * cl,
+              RNS_MIXED);
 }
 
 int bond_form(int prec, int Dl, int Dr, int chi) {
   return form(prec, rns_wanted(Dl, (long)chi * Dr, Dr) && rns_wanted(Dl, Dr, (long)Dl * chi), Dr,
-              (long)Dl * chi);
+              (long)Dl * chi, RNS_MIXED);
 }
 
 static int env_form(int prec, int Dl, int d, int Dr, int cl, int cr) {
@@ -123,7 +124,7 @@ static int env_form(int prec, int Dl, int d, int Dr, int cl, int cr) {
                   rns_wanted(Dr, (long)cr * Dr, (long)Dl * d) &&
                   rns_wanted((long)Dl * d, (long)cr * Dr, Dr) &&
                   rns_wanted((long)Dl * cl, Dl, (long)d * Dr),
-              std::max(Dl, Dr), (long)std::max(Dl, Dr) * d);
+              std::max(Dl, Dr), (long)std::max(Dl, Dr) * d, RNS_MIXED_ENV);
 }
 
 // ------------------------------------------------------------------ workspace layout

@@ -1074,9 +1074,11 @@ ptn_status rns_convert(const RnsView& v, const RnsOperand& d, bool have_exp, con
                        cudaStream_t st, int* clear, int nclear) {
   const int bits = rns_bits(d.kc, d.nm);
   PTN_CHECK_ARG(bits != 0, "rns_convert: products of %d terms are too long", d.kc);
-  return d.nm == RNS_FP64
-             ? convert<RNS_FP64>(v, d, have_exp, bits, clear, nclear, skip, st)
-             : convert<RNS_MIXED>(v, d, have_exp, bits, clear, nclear, skip, st);
+  switch (d.nm) {
+    case RNS_FP64: return convert<RNS_FP64>(v, d, have_exp, bits, clear, nclear, skip, st);
+    case RNS_MIXED_ENV: return convert<RNS_MIXED_ENV>(v, d, have_exp, bits, clear, nclear, skip, st);
+    default: return convert<RNS_MIXED>(v, d, have_exp, bits, clear, nclear, skip, st);
+  }
 }
 
 // the integer products of all planes -> res, and what their reconstruction needs
@@ -1130,11 +1132,9 @@ ptn_status rns_gemm(const RnsOperand& A, const RnsView& va, const RnsOperand& B,
   PTN_TRY(multiply(A, va, B, vb, res, skip, st, &r));
   const long pairs = (long)r.M * ((r.N + 1) / 2);
   const int blocks = (int)std::min<long>((pairs + 255) / 256, 16L * num_sms());
-  if (A.nm == RNS_FP64) PTN_CUDA_TRY(launch(k_reconstruct<RNS_FP64>, dim3(blocks), dim3(256), 0,
-      st, r, alpha, beta, out, ldc));
-  else PTN_CUDA_TRY(launch(k_reconstruct<RNS_MIXED>, dim3(blocks), dim3(256), 0, st, r, alpha,
-      beta, out, ldc));
-  PTN_LAUNCH_CHECK();
+  auto kernel = A.nm == RNS_FP64 ? k_reconstruct<RNS_FP64>
+                : A.nm == RNS_MIXED_ENV ? k_reconstruct<RNS_MIXED_ENV> : k_reconstruct<RNS_MIXED>;
+  PTN_CUDA_TRY(launch(kernel, dim3(blocks), dim3(256), 0, st, r, alpha, beta, out, ldc));
   note_launches(1);
   return PTN_OK;
 }
@@ -1167,7 +1167,11 @@ ptn_status rns_gemm_stage(const RnsOperand& A, const RnsView& va, const RnsOpera
   PTN_CHECK_ARG(s.X <= 65535, "MPO stage: X too large");
   ReconP r;
   PTN_TRY(multiply(A, va, B, vb, res, skip, st, &r));
-  return A.nm == RNS_FP64 ? launch_stage<RNS_FP64>(r, s, st) : launch_stage<RNS_MIXED>(r, s, st);
+  switch (A.nm) {
+    case RNS_FP64: return launch_stage<RNS_FP64>(r, s, st);
+    case RNS_MIXED_ENV: return launch_stage<RNS_MIXED_ENV>(r, s, st);
+    default: return launch_stage<RNS_MIXED>(r, s, st);
+  }
 }
 
 int rns_error_and_reset() {

@@ -7,9 +7,14 @@
 
 namespace ptn {
 
-// moduli of the FP64 form and of the mixed form
+// Moduli of the FP64 form and of the mixed form: its operators (40 bits and more) and its
+// environment steps (49 and more). Environments stay Hermitian to FP64 level that way: with 40
+// bits the chain ends, whose small Krylov spaces are exhausted, see residuals around the
+// breakdown threshold 100 n eps (2e-13 against 9e-14 at bond 2), and whether a run stops there
+// would depend on rounding.
 constexpr int RNS_FP64 = 14;
 constexpr int RNS_MIXED = 11;
+constexpr int RNS_MIXED_ENV = 13;
 
 // element (r, k) of a complex operand: src[r * sr + k * sk], conjugated if `conj`
 struct RnsView {
@@ -69,7 +74,7 @@ ptn_status rns_gemm_stage(const RnsOperand& A, const RnsView& va, const RnsOpera
                           const RnsView& vb, const RnsStage& s, void* res, const int* skip,
                           cudaStream_t st);
 
-// Contractions through residue planes (rns_ops.cu), nm = RNS_FP64 or RNS_MIXED. The views
+// Contractions through residue planes (rns_ops.cu), nm one of the counts above. The views
 // of an operator's l and r stay in use between prepare and the applies.
 size_t heff_workspace_bytes_rns(int nm, int Dl, int d, int Dr, int cl, int cr);
 ptn_status heff_prepare_rns(int nm, const double2* l, const double2* r, int Dl, int d, int Dr,
