@@ -23,16 +23,39 @@ inline size_t stage_smem(int P, int Q) {
   return (size_t)P * STAGE_Y * sizeof(double2) + (size_t)P * Q * (sizeof(double2) + sizeof(int));
 }
 
+// FP64 operations the compiler may not hoist out of their branch: computed for every entry
+// whatever its kind, they would cost 64 cycles of a sub-partition each
+__device__ __forceinline__ double mul_here(double a, double b) {
+  double r;
+  asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+}
+__device__ __forceinline__ double fma_here(double a, double b, double c) {
+  double r;
+  asm volatile("fma.rn.f64 %0, %1, %2, %3;" : "=d"(r) : "d"(a), "d"(b), "d"(c));
+  return r;
+}
+__device__ __forceinline__ double add_here(double a, double b) {
+  double r;
+  asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+}
+
+static __device__ __noinline__ double2 entry_complex(double2 v, double2 x, double2 acc, int first) {
+  return first ? cmul(v, x) : cfma(v, x, acc);
+}
+
 __device__ __forceinline__ double2 entry_mul(int kind, double2 v, double2 x) {
   if (kind == ENTRY_ONE) return x;
-  if (kind == ENTRY_REAL) return make_double2(v.x * x.x, v.x * x.y);
-  return cmul(v, x);
+  if (kind == ENTRY_REAL) return make_double2(mul_here(v.x, x.x), mul_here(v.x, x.y));
+  return entry_complex(v, x, x, 1);
 }
 
 __device__ __forceinline__ double2 entry_fma(int kind, double2 v, double2 x, double2 acc) {
-  if (kind == ENTRY_ONE) return cadd(acc, x);
-  if (kind == ENTRY_REAL) return make_double2(fma(v.x, x.x, acc.x), fma(v.x, x.y, acc.y));
-  return cfma(v, x, acc);
+  if (kind == ENTRY_ONE) return make_double2(add_here(acc.x, x.x), add_here(acc.y, x.y));
+  if (kind == ENTRY_REAL)
+    return make_double2(fma_here(v.x, x.x, acc.x), fma_here(v.x, x.y, acc.y));
+  return entry_complex(v, x, acc, 0);
 }
 
 // M (given by strides into w) -> sval[q * P + p]
