@@ -153,10 +153,34 @@ __constant__ ModTable c_mod = make_table();
 
 constexpr float MAGIC = 12582912.0f;   // 1.5 2^23: adding it rounds to an integer
 
-// v modulo p, centred, for an integer |v| <= 2^24 (off centre by one at most)
-__device__ __forceinline__ float reduce_mod(float v, float p, float inv) {
-  const float q = fmaf(v, inv, MAGIC) - MAGIC;
-  return fmaf(-q, p, v);
+// two FP32 operations in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<u64&>(d))
+      : "l"(reinterpret_cast<u64&>(a)), "l"(reinterpret_cast<u64&>(b)), "l"(reinterpret_cast<u64&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<u64&>(d))
+      : "l"(reinterpret_cast<u64&>(a)), "l"(reinterpret_cast<u64&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<u64&>(d))
+      : "l"(reinterpret_cast<u64&>(a)), "l"(reinterpret_cast<u64&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+
+// v modulo p, centred, for two integers |v| <= 2^24 (off centre by one at most)
+__device__ __forceinline__ float2 reduce_mod2(float2 v, float p, float inv) {
+  const float2 q = add2(fma2(v, both(inv), both(MAGIC)), both(-MAGIC));
+  return fma2(q, both(-p), v);
 }
 
 __device__ __forceinline__ int biased_exp(double x) {
@@ -191,8 +215,10 @@ __device__ __forceinline__ void pieces_of(double x, int E, int bits, float (&f)[
   }
 }
 
-// Residues of two neighbouring terms in all planes. 18 FP32 operations per term and
-// modulus: x and y as five pieces times small constants, two reductions.
+// Residues of two neighbouring terms in all planes: x and y as five pieces times small
+// constants, two reductions, the two terms side by side in packed FP32 operations (17 per
+// modulus instead of 36: H_eff at bond 512, mixed, 360 -> 340 us with the GEMM's epilogue in
+// the same form).
 template <int NM>
 __device__ __forceinline__ void convert_pair(const double2 (&z)[2], int E, int bits,
                                              bf16* __restrict__ row, long plane) {
@@ -203,24 +229,25 @@ __device__ __forceinline__ void convert_pair(const double2 (&z)[2], int E, int b
     pieces_of(z[q].x, E, bits, px[q]);
     pieces_of(z[q].y, E, bits, py[q]);
   }
+  float2 x[PIECES], y[PIECES];
+#pragma unroll
+  for (int t = 0; t < PIECES; ++t) {
+    x[t] = make_float2(px[0][t], px[1][t]);
+    y[t] = make_float2(py[0][t], py[1][t]);
+  }
 #pragma unroll
   for (int i = 0; i < NM; ++i) {
-    const float p = c.p[i], inv = c.inv[i];
-    float u[2], w[2];
+    float2 sx = x[0], sy = mul2(y[0], both(c.cy[i][0]));
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      float sx = px[q][0], sy = py[q][0] * c.cy[i][0];
-#pragma unroll
-      for (int t = 1; t < PIECES; ++t) {
-        sx = fmaf(px[q][t], c.cx[i][t], sx);
-        sy = fmaf(py[q][t], c.cy[i][t], sy);
-      }
-      u[q] = reduce_mod(sx + sy, p, inv);
-      w[q] = reduce_mod(sx - sy, p, inv);
+    for (int t = 1; t < PIECES; ++t) {
+      sx = fma2(x[t], both(c.cx[i][t]), sx);
+      sy = fma2(y[t], both(c.cy[i][t]), sy);
     }
-    *reinterpret_cast<__nv_bfloat162*>(row + (2L * i) * plane) = __floats2bfloat162_rn(u[0], u[1]);
+    const float2 u = reduce_mod2(add2(sx, sy), c.p[i], c.inv[i]);
+    const float2 w = reduce_mod2(fma2(sy, both(-1.0f), sx), c.p[i], c.inv[i]);
+    *reinterpret_cast<__nv_bfloat162*>(row + (2L * i) * plane) = __floats2bfloat162_rn(u.x, u.y);
     *reinterpret_cast<__nv_bfloat162*>(row + (2L * i + 1) * plane) =
-        __floats2bfloat162_rn(w[0], w[1]);
+        __floats2bfloat162_rn(w.x, w.y);
   }
 }
 
@@ -611,7 +638,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int n0 = (u % g.gx) * BN + half * T::COLS, pl = u / (g.gx * g.gy);
       const int row = ((u / g.gx) % g.gy) * BM + 32 * quad + lane;
       const float p = c_mod.p[pl >> 1], inv = c_mod.inv[pl >> 1];
-      float acc[T::COLS];
+      float2 acc[T::COLS / 2];
       for (int c = 0; c < nch; ++c, ++ch) {
         const int b = ch & 1;
         if (!mbar_wait(&tfull[b], (uint32_t)(ch >> 1) & 1u, abort_flag)) {
@@ -632,9 +659,11 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (lane == 0) mbar_arrive(&tempty[b]);
           }
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float r = reduce_mod(__uint_as_float(v[j]), p, inv);
-            acc[c0 + j] = c == 0 ? r : acc[c0 + j] + r;
+          for (int j = 0; j < 16; j += 2) {
+            const float2 r = reduce_mod2(
+                make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), p, inv);
+            float2& sum = acc[(c0 + j) >> 1];
+            sum = c == 0 ? r : add2(sum, r);
           }
         }
       }
@@ -647,14 +676,11 @@ __global__ void __launch_bounds__(THREADS, 1)
           unsigned q[4];
 #pragma unroll
           for (int j = 0; j < 8; j += 2) {
-            float r0 = acc[c0 + j], r1 = acc[c0 + j + 1];
-            if (nch > 1) {
-              r0 = reduce_mod(r0, p, inv);
-              r1 = reduce_mod(r1, p, inv);
-            }
+            float2 r = acc[(c0 + j) >> 1];
+            if (nch > 1) r = reduce_mod2(r, p, inv);
             // the low half of the magic sum's bits is the residue + 256
-            q[j >> 1] = __byte_perm(__float_as_uint(r0 + (MAGIC + 256.0f)),
-                                    __float_as_uint(r1 + (MAGIC + 256.0f)), 0x5410);
+            r = add2(r, both(MAGIC + 256.0f));
+            q[j >> 1] = __byte_perm(__float_as_uint(r.x), __float_as_uint(r.y), 0x5410);
           }
           *reinterpret_cast<uint4*>(dst + c0) = make_uint4(q[0], q[1], q[2], q[3]);
         }
@@ -790,17 +816,25 @@ __device__ __forceinline__ double2 element(const ReconP& g, int m, int n, int q,
   return z;
 }
 
-// alpha z; alpha = 1 matters to infinities and NaNs alone (0 * inf), as in the DMMA kernel
-__device__ __forceinline__ double2 scaled(double2 alpha, double2 z) {
-  const bool one = alpha.x == 1.0 && alpha.y == 0.0;
-  if (one && biased_exp(z.x) != 2047 && biased_exp(z.y) != 2047) return z;
-  return cmul(alpha, z);
+// alpha z + beta y as the DMMA kernel forms it. Not inlined: alpha = 1, beta = 0 needs it for
+// infinities and NaNs alone (0 * inf), and an FP64 operation that the compiler hoists out of
+// the rare branch costs every element 64 cycles of a sub-partition.
+__device__ __noinline__ double2 scale_add(double2 alpha, double2 z, double2 beta, const double2* y) {
+  z = cmul(alpha, z);
+  return y != nullptr ? cadd(z, cmul(beta, *y)) : z;
 }
 
-// Bound: the integer pipe (about 10 operations per residue pair), then reading 4 nm bytes
-// of residues per element, from L2 where the product fits it.
+__device__ __forceinline__ bool not_finite(double2 z) {
+  return biased_exp(z.x) == 2047 || biased_exp(z.y) == 2047;
+}
+
+// Bound: latency of the loads (all residues of a pair are fetched ahead: fewer in flight and
+// more warps was slower), then the integer pipe (about 10 operations per residue pair).
+// Measured, 1024 x 512, 11 moduli: 22 us while an alpha z was formed speculatively for every
+// element -> 14.
 template <int NM>
 __global__ void __launch_bounds__(256) k_reconstruct(const ReconP g, double2 alpha, double2 beta,
+                                                     int plain, int add,
                                                      double2* __restrict__ out, long ldc) {
   grid_wait();
   if (g.skip != nullptr && *g.skip != 0) return;
@@ -815,8 +849,7 @@ __global__ void __launch_bounds__(256) k_reconstruct(const ReconP g, double2 alp
       if (n + q >= g.N) break;
       double2 z = element<NM>(g, m, n + q, q, ru, rv);
       double2* o = out + (long)m * ldc + n + q;
-      z = scaled(alpha, z);
-      if (beta.x != 0.0 || beta.y != 0.0) z = cadd(z, cmul(beta, *o));
+      if (!plain || not_finite(z)) z = scale_add(alpha, z, beta, add ? o : nullptr);
       *o = z;
     }
   }
@@ -852,9 +885,13 @@ __global__ void __launch_bounds__(2 * STAGE_Y)
       unsigned ru[NM], rv[NM];
       load_residues<NM>(g.res + (long)m * g.ldr + n, g.rplane, y + 1 < Y, ru, rv);
       const double2 one = make_double2(1.0, 0.0);
-      sin[p * STAGE_Y + pair] = scaled(one, element<NM>(g, m, n, 0, ru, rv));
-      if (y + 1 < Y)
-        sin[p * STAGE_Y + pair + 1] = scaled(one, element<NM>(g, m, n + 1, 1, ru, rv));
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (y + q < Y) {
+          double2 z = element<NM>(g, m, n + q, q, ru, rv);
+          if (not_finite(z)) z = scale_add(one, z, one, nullptr);
+          sin[p * STAGE_Y + pair + q] = z;
+        }
     }
   }
   __syncthreads();
@@ -955,14 +992,16 @@ ptn_status launch_gemm(const RnsOperand& A, const RnsOperand& B, GemmP g, cudaSt
   return PTN_OK;
 }
 
-// cycles of a launch with N tiles of bn columns: whole turns of the SMs, the MMAs of a tile
-// (half a cycle per column and 16 terms, at least what reading the operands from shared
-// memory takes) and a fixed cost per tile
+// cycles of a launch with N tiles of bn columns: whole turns of the SMs; per tile and 16 terms
+// what the SM takes to read both operand tiles from L2 (64 bytes a cycle: 192, 128 and 96
+// cycles for 256, 128 and 64 columns; the MMAs themselves take half a cycle per column),
+// and a fixed cost per tile. Measured, M 2048, N 5120, K 1024: 300 us, 190 cycles per 16 terms
+// of a 128 x 256 tile.
 double tile_cost(int bn, long M, long N, long K, int planes) {
   const long units = ((N + bn - 1) / bn) * ((M + BM - 1) / BM) * planes;
   const long turns = (units + num_sms() - 1) / num_sms();
   const double k16 = (double)((K + 15) / 16);
-  return turns * (k16 * std::max(bn / 2.0, 32.0 + bn / 4.0) + 300.0 + bn);
+  return turns * (k16 * (64.0 + bn / 2.0) + 300.0 + bn);
 }
 
 constexpr double plog2(int nm) {
@@ -1029,13 +1068,12 @@ static ptn_status launch_convert(const RnsView& v, const RnsOperand& d, bool hav
                                 CR * (CK_MAX + 1) * (int)sizeof(double2));
   });
   PTN_CUDA_TRY(attr);
-  // terms per CTA: enough CTAs for the chip, multiples of 64, at most 8 CTAs to a row where
-  // the maxima are exchanged
+  // terms per CTA, multiples of 64: enough CTAs for the chip, and at most 256 terms (33 KB, six
+  // CTAs per SM: an environment step at bond 1024 takes 1.84 ms with up to 1024 terms and two
+  // CTAs per SM, 1.71 so), while at most 8 CTAs share a row where the maxima are exchanged
   const long groups = (d.rows + CR - 1) / CR;
-  const long want = std::max<long>(1, 2L * num_sms() / groups);
   const long blocks64 = (d.kc + 63) / 64;
-  long parts = std::min(want, blocks64);
-  parts = std::max(parts, ((long)d.kc + CK_MAX - 1) / CK_MAX);
+  long parts = std::max(std::min(2L * num_sms() / groups, blocks64), ((long)d.kc + 255) / 256);
   if (!have_exp) parts = std::min(parts, 8L);
   const long chunk = (blocks64 + parts - 1) / parts * 64;
   parts = (d.kc + chunk - 1) / chunk;
@@ -1134,7 +1172,9 @@ ptn_status rns_gemm(const RnsOperand& A, const RnsView& va, const RnsOperand& B,
   const int blocks = (int)std::min<long>((pairs + 255) / 256, 16L * num_sms());
   auto kernel = A.nm == RNS_FP64 ? k_reconstruct<RNS_FP64>
                 : A.nm == RNS_MIXED_ENV ? k_reconstruct<RNS_MIXED_ENV> : k_reconstruct<RNS_MIXED>;
-  PTN_CUDA_TRY(launch(kernel, dim3(blocks), dim3(256), 0, st, r, alpha, beta, out, ldc));
+  const int add = beta.x != 0.0 || beta.y != 0.0;
+  const int plain = !add && alpha.x == 1.0 && alpha.y == 0.0;
+  PTN_CUDA_TRY(launch(kernel, dim3(blocks), dim3(256), 0, st, r, alpha, beta, plain, add, out, ldc));
   note_launches(1);
   return PTN_OK;
 }
