@@ -11,10 +11,19 @@ from . import _lib
 CDT = torch.complex128
 
 
+_DEVICES = {}
+
+
 def device():
-    if not torch.cuda.is_available():
+    """The current CUDA device (asked for several times per call: availability is checked
+    once, the torch.device objects are kept)."""
+    if not _DEVICES and not torch.cuda.is_available():
         raise RuntimeError("pytenet_gb300 needs a CUDA GPU (GB300, sm_103a); no CPU fallback exists")
-    return torch.device("cuda", torch.cuda.current_device())
+    i = torch.cuda.current_device()
+    d = _DEVICES.get(i)
+    if d is None:
+        d = _DEVICES[i] = torch.device("cuda", i)
+    return d
 
 
 def lib():
@@ -32,6 +41,8 @@ def ptr(t):
 def to_dev(x):
     """Host array (or device tensor) -> contiguous complex128 device tensor."""
     if isinstance(x, torch.Tensor):
+        if x.dtype is CDT and x.is_cuda and x.get_device() == torch.cuda.current_device():
+            return x if x.is_contiguous() else x.contiguous()
         t = x.to(device=device(), dtype=CDT)
         return t.contiguous()
     a = np.ascontiguousarray(np.asarray(x), dtype=np.complex128)
