@@ -44,10 +44,13 @@ typedef enum {
 } ptn_status;
 
 typedef enum {
-  PTN_PREC_FP64 = 0,        /* plain complex128 (FP64 DMMA tensor cores) */
-  PTN_PREC_SPLIT_BF16 = 1   /* fixed-point BF16 digit products on tcgen05 (5 digits per
-                               row-scaled value, exact FP32 integer accumulation per digit
-                               level, FP64 recombination): ~2e-11 relative per contraction */
+  PTN_PREC_FP64 = 0,        /* plain complex128: FP64 DMMA, and for products of at least 32 in
+                               every dimension and 1e6 complex multiply-adds exact products of
+                               residues modulo 14 numbers on tcgen05 (rows as fixed-point
+                               numbers of 53-54 bits; errors below the DMMA kernel's) */
+  PTN_PREC_SPLIT_BF16 = 1   /* fewer moduli: 11 in the local operators (40-44 bits per
+                               row-scaled value, ~1e-12 relative per contraction), 13 in the
+                               environment steps (49-52 bits) */
 } ptn_precision;
 
 typedef struct { double re, im; } ptn_c128;
@@ -87,11 +90,13 @@ uint64_t ptn_launch_count(void);
 /* Tuning knobs (process-wide). They are read when an entry point chooses its
  * launch shape on the host, so a CUDA graph keeps the values it was captured
  * with; workspace queries read them too (query and call under the same values).
- *   PTN_TUNE_TC_SPLIT_WAVES    split-K of the tensor-core GEMM aims at this many
- *                              waves of CTAs (0..16, default 1; never fewer
- *                              splits than exact integer accumulation needs)
- *   PTN_TUNE_ZGEMM_SPLIT_WAVES split-K target of the FP64 GEMM (0..16, default 2;
- *                              0 = no split-K)
+ * The three PTN_TUNE_TC_* knobs concern the digit GEMM of ptn_zgemm_split_bf16; the residue
+ * products of the other entry points have no knobs.
+ *   PTN_TUNE_TC_SPLIT_WAVES    split-K of the digit GEMM aims at this many waves of
+ *                              CTAs (0..16, default 1; never fewer splits than exact
+ *                              integer accumulation needs)
+ *   PTN_TUNE_ZGEMM_SPLIT_WAVES split-K target of the FP64 DMMA GEMM (0..16, default 2;
+ *                              0 = no split-K; sums of fewer than 128 terms ignore it)
  *   PTN_TUNE_LARFB_TILE        QR block update: 0 register-tiled FMA-only kernels
  *                              (default); 1..5 the earlier three-pass kernels with
  *                              tile 1 16x16, 2 32x16, 3 32x32, 4 64x32 (rows x
@@ -102,15 +107,17 @@ uint64_t ptn_launch_count(void);
  *                              entries is one cooperative launch (dot, update, norm, scale
  *                              with two grid barriers, half the memory traffic); 0: three
  *                              launches. Runs that share the GPU with concurrent work on
- *                              other streams set 0.
- *   PTN_TUNE_QR_PANEL          QR panel kernel: 0 (default) two warps per 32-row group
- *                              (even / odd columns, one per SM sub-partition for 64-row
- *                              CTAs), select-free products summed through shared memory,
- *                              next pivot's norm published before the other updates;
- *                              3 the same layout with a shuffle reduce-scatter; 1 the
- *                              earlier one-warp-per-row-group panel; 2 that panel with
- *                              the reflector scalars and the cluster gather in one warp.
- *   PTN_TUNE_TC_PERSISTENT     0 (default): the tensor-core GEMM runs one CTA per (tile,
+ *                              other streams set 0. Vectors of at most 2^14 entries take
+ *                              one launch of a single cluster under either value.
+ *   PTN_TUNE_QR_PANEL          QR panel kernel: 0 (default) one cluster-wide reduction per
+ *                              column (dot products, Gram entries and the next pivot's
+ *                              norm together), rows in registers, and Q formed in blocks
+ *                              of 128 reflectors on the tensor cores where they are large;
+ *                              3 two warps per 32-row group with a shuffle reduce-scatter
+ *                              and two barriers per column; 1 the earlier
+ *                              one-warp-per-row-group panel; 2 that panel with the
+ *                              reflector scalars and the cluster gather in one warp.
+ *   PTN_TUNE_TC_PERSISTENT     0 (default): the digit GEMM runs one CTA per (tile,
  *                              K split) unit; 1: one CTA per SM over all units, the next
  *                              unit's loads and MMAs overlapping the current one's
  *                              epilogue (same results bit for bit; measured slower on
@@ -205,8 +212,9 @@ ptn_status ptn_zgemm(char opA, char opB, int M, int N, int K, ptn_c128 alpha,
                      int batch, void* ws, size_t ws_bytes, void* stream);
 
 /* C = A B for row-major complex A (M x K, leading dim lda) and B (K x N, ldb) on the
- * tensor cores: fixed-point BF16 digit products (the arithmetic of
- * PTN_PREC_SPLIT_BF16), FP64 output. */
+ * tensor cores: fixed-point BF16 digit products (5 digits per row-scaled value, exact FP32
+ * integer accumulation per digit level, FP64 recombination: ~2e-11 relative), FP64 output.
+ * The mixed form absorbs the bond matrix into the next site with it. */
 size_t ptn_zgemm_split_bf16_workspace_bytes(int M, int N, int K);
 ptn_status ptn_zgemm_split_bf16(const ptn_c128* A, long lda, const ptn_c128* B, long ldb,
                                 ptn_c128* C, long ldc, int M, int N, int K, void* ws,

@@ -1047,15 +1047,18 @@ int rns_bits(long K, int nm) {
   return bits >= (nm == RNS_FP64 ? 53 : 39) ? bits : 0;
 }
 
-// The fixed cost of the path (conversions, planes, reconstruction: about 33 us for a single
-// GEMM) meets the DMMA kernel's 1 TF/s near 4e6 complex products. Measured, the GEMMs of
-// H_eff at bond D and MPO bond 5 alone (DMMA -> residues):
-//   D = 64: 30.5 us;  80: 50 -> 34;  128: 184 -> 40;  256: 1416 -> 74;  512: 11269 -> 246
+// The fixed cost of the path (conversions, planes, reconstruction: 12 us for a single GEMM)
+// meets the DMMA kernel near 1e6 complex products. Measured, the GEMMs of H_eff at bond D
+// and MPO bond 5 alone (first / second, DMMA -> residues):
+//   D = 40: 9.7 -> 12.5, 12.9 -> 16.5 us;  48: 14.3 -> 12.4, 24.8 -> 16.8;  64: 30.3 -> 12.8,
+//   28.1 -> 17.8;  128: 184 -> 21, 217 -> 22;  256: 1419 -> 54, 1458 -> 45;  512: 11275 -> 188,
+//   11606 -> 159
 // and a Lanczos step (operands of the operator converted once):
-//   D = 80: 147 -> 86 us;  128: 436 -> 82;  256: 2924 -> 149;  512: 22967 -> 453
+//   D = 40: 43 -> 44 us;  48: 57 -> 42;  64: 77 -> 43;  128: 426 -> 59;  256: 2908 -> 119;
+//   512: 22961 -> 376
 bool rns_wanted(long M, long N, long K) {
   if (std::min(M, std::min(N, K)) < 32 || M > INT_MAX / 2 || N > INT_MAX / 2) return false;
-  return (double)M * N * K >= 4.0e6 && rns_bits(K, RNS_FP64) != 0;
+  return (double)M * N * K >= 1.0e6 && rns_bits(K, RNS_FP64) != 0;
 }
 
 template <int NM>

@@ -167,3 +167,14 @@ def test_mixed_contractions_in_residues(dims):
                          (ptg.contraction_operator_step_right, (a, b, w, r), None)):
         got, ref = fn(*args, precision="mixed"), fn(*args, precision="fp64")
         assert np.linalg.norm(got - ref) < 1e-11 * np.linalg.norm(ref), fn.__name__
+
+
+# around the smallest products that take the residue planes (a million complex multiply-adds)
+@pytest.mark.parametrize("mnk", [(32, 1000, 32), (33, 947, 33), (100, 100, 101), (1030, 32, 33),
+                                 (47, 235, 94), (64, 250, 64)])
+def test_smallest_products(mnk):
+    M, N, K = mnk
+    rng = np.random.default_rng(M + 3 * N + 7 * K)
+    A, B = crandn(rng, M, K), crandn(rng, K, N)
+    err, tol = errors(zgemm(A, B), A, B, rng)
+    assert np.all(err <= tol), (err / tol).max()
