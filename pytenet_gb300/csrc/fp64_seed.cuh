@@ -15,6 +15,11 @@ __device__ __forceinline__ double seed_scale(float y, int e) {   // y 2^e for a 
   return __longlong_as_double(((long long)x << 52) | ((long long)(b & 0x7FFFFFu) << 29));
 }
 
+// y / 2 of a normal y well above the subnormal range, without an FP64 instruction
+__device__ __forceinline__ double half_of(double y) {
+  return __longlong_as_double(__double_as_longlong(y) - (1LL << 52));
+}
+
 __device__ __forceinline__ double fast_rsqrt(double d) {
   const long long b = __double_as_longlong(d);
   const int E = (int)((b >> 52) & 0x7FF);

@@ -996,7 +996,9 @@ __global__ void __launch_bounds__(P6W * 32) qr_panel6_kernel(double2* __restrict
 // Newton steps on an FP32 seed.
 // Measured (panels of a 1024 x 512 matrix, 16 CTAs, mean over its 32): 127 us per 16 columns
 // with two reductions per column and the scaled vector multiplied -> 85 us; the whole QR
-// 8.25 -> 6.57 ms.
+// 8.25 -> 6.57 ms. Then 84 -> 70 us (the QR with Q in wide blocks 4.29 -> 4.02 ms) with one
+// component of a sum per lane, four warps (one per sub-partition) for the sums over warps and
+// over ranks, and the scalars, the row of R and the Gram entries in three warps.
 // Dynamic shared memory: xs[rows of the CTA][NB].
 constexpr int P8T = 256;
 constexpr int P8_ROWS = 768;   // most rows per CTA: 192 KB
@@ -1034,13 +1036,17 @@ __global__ void __launch_bounds__(P8T) qr_panel8_kernel(const P8Args g) {
   const int rank = (int)cluster.block_rank(), cs = (int)cluster.num_blocks();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int c16 = tid & 15, b16 = tid >> 4;
+  const int im = lane >> 4;                           // component of a lane that holds one
+  const int cc = 8 * (warp & 3) + (lane & 7), g4 = lane >> 3;   // sums: component, group
   extern __shared__ double2 dyn[];
   double2* xs = dyn;                        // xs[row * NB + c]
-  __shared__ double2 s_part[P8T / 32][NB];  // per-warp sums
-  __shared__ double2 s_pub[2][NB];          // this CTA's sums (read remotely), by column parity
+  // sums as doubles: real part of column c at c, imaginary part at NB + c
+  __shared__ double s_part[P8T / 32][2 * NB + 4];   // per-warp sums
+  __shared__ double s_pub[2][2 * NB];       // this CTA's sums (read remotely), by column parity
   __shared__ double2 s_row[2][NB];          // the pivot row, in its owner
-  __shared__ double2 s_gat[P8T / 32][NB];   // sums of two ranks per warp
+  __shared__ double s_tot[2 * NB];          // the cluster's sums
   __shared__ double2 s_prow[NB];
+  __shared__ double s_a2, s_ay2;            // |alpha|^2 of the pivot, its imaginary part squared
   __shared__ double2 s_r[NB], s_u[NB];      // row of R; scal times the update factors
   __shared__ double2 s_S[NB][NB + 1];       // Gram entries of the reflectors, [c][j], c < j
   __shared__ double2 s_T[NB][NB + 1];
@@ -1063,18 +1069,19 @@ __global__ void __launch_bounds__(P8T) qr_panel8_kernel(const P8Args g) {
     (&s_T[0][0])[e] = c2(0.0, 0.0);
   }
   const bool make_t = FULL || rank == cs - 1;   // the CTA with the fewest rows
-  // column q of T from columns < q (threads 128 .. 255: eight per row)
+  // column q of T from columns < q (warps 6 and 7, four threads per row: their sub-partitions
+  // are idle while warps 0 and 1 form the reflector scalars)
   auto t_column = [&](int q) {
-    const int t = tid - 128;
-    const int row = t >> 3, g = t & 7;
+    const int t = tid - 192;
+    const int row = t >> 2, g = t & 3;
     double2 s = c2(0.0, 0.0);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int k = g + 8 * h;
+    for (int h = 0; h < 4; ++h) {
+      const int k = g + 4 * h;
       if (k < q && k >= row) s = cfma(s_T[row][k], s_S[k][q], s);
     }
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
+    for (int o = 2; o > 0; o >>= 1) {
       s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
       s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
     }
@@ -1097,98 +1104,107 @@ __global__ void __launch_bounds__(P8T) qr_panel8_kernel(const P8Args g) {
       int lr = b16;
       if (lr < first) lr += (first - lr + 15) / 16 * 16;
       for (; lr < nr; lr += 16) s = cfma(cconj(xs[lr * NB + j]), xs[lr * NB + c16], s);
-      s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
-      s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
-      if (lane < 16) s_part[warp][c16] = s;
+      // one component per lane: the exchange costs one addition
+      const double o = __shfl_xor_sync(0xffffffffu, im ? s.x : s.y, 16);
+      s_part[warp][lane] = (im ? s.y : s.x) + o;
     }
     __syncthreads();
-    if (warp == 0) {
-      const int w = (lane >> 4) * 4;
-      double2 s = cadd(cadd(s_part[w][c16], s_part[w + 1][c16]),
-                       cadd(s_part[w + 2][c16], s_part[w + 3][c16]));
-      s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
-      s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
-      if (lane < 16) s_pub[par][c16] = s;
-    } else if (warp == 1 && rank == owner && lane < 16) {
+    // eight sums per warp, four lanes each
+    if (warp < 4) {
+      double s = s_part[2 * g4][cc] + s_part[2 * g4 + 1][cc];
+      s += __shfl_xor_sync(0xffffffffu, s, 8);
+      s += __shfl_xor_sync(0xffffffffu, s, 16);
+      if (lane < 8) s_pub[par][cc] = s;
+    } else if (warp == 4 && rank == owner && lane < 16) {
       s_row[par][c16] = xs[(j0 + j - rb) * NB + c16];
     }
     cluster.sync();
-    // ---- gather: thread (column, rank)
-    {
-      double2 s = c2(0.0, 0.0);
-      if (b16 < cs) s = cluster.map_shared_rank(&s_pub[par][0], b16)[c16];
-      if (cs > 1) {
-        s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
-        s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
+    // ---- gather: four ranks per lane
+    if (warp < 4) {
+      auto of = [&](int r) {
+        return r < cs ? cluster.map_shared_rank(&s_pub[par][0], r)[cc] : 0.0;
+      };
+      double s = of(4 * g4);
+      if (cs > 2) {
+        const double s1 = of(4 * g4 + 1), s2 = of(4 * g4 + 2), s3 = of(4 * g4 + 3);
+        s = (s + s1) + (s2 + s3);
+      } else if (cs > 1) {
+        s += of(4 * g4 + 1);
       }
-      if (lane < 16) s_gat[warp][c16] = s;
-      if (warp == 7 && lane >= 16) s_prow[c16] = cluster.map_shared_rank(&s_row[par][0], owner)[c16];
+      if (cs > 4) {
+        s += __shfl_xor_sync(0xffffffffu, s, 8);
+        s += __shfl_xor_sync(0xffffffffu, s, 16);
+      }
+      if (lane < 8) s_tot[cc] = s;
+    } else if (warp == 4 && lane < 16) {
+      const double2 a = cluster.map_shared_rank(&s_row[par][0], owner)[c16];
+      s_prow[c16] = a;
+      const double ay2 = a.y * a.y, a2 = fma(a.x, a.x, ay2);
+      if (c16 == j) {
+        s_a2 = a2;
+        s_ay2 = ay2;
+      }
     }
     __syncthreads();
-    if (warp < 2) {
-      // all sums, in the lane of their column (both warps, to save an exchange)
-      const int w = (lane >> 4) * 4;
-      double2 tot = s_gat[w][c16];
-      if (cs > 2) {
-        tot = cadd(cadd(tot, s_gat[w + 1][c16]), cadd(s_gat[w + 2][c16], s_gat[w + 3][c16]));
-        tot.x += __shfl_xor_sync(0xffffffffu, tot.x, 16);
-        tot.y += __shfl_xor_sync(0xffffffffu, tot.y, 16);
-      } else {
-        tot.x = __shfl_sync(0xffffffffu, tot.x, c16);
-        tot.y = __shfl_sync(0xffffffffu, tot.y, c16);
-      }
-      const double2 prow = s_prow[c16];
+    if (warp < 3) {
       const double2 alpha = s_prow[j];
-      const double xn2 = __shfl_sync(0xffffffffu, tot.x, j);
+      const double xn2 = s_tot[j];
       const bool apply = !(xn2 == 0.0 && alpha.y == 0.0);
+      // this lane's component of its column, and the other one
+      const double own = s_tot[lane], other = s_tot[lane ^ 16];
+      const double2 prow = s_prow[c16];
+      const double p_own = im ? prow.y : prow.x, p_other = im ? prow.x : prow.y;
       if (warp == 0) {
-        // reflector scalars (every lane the same)
-        double beta = alpha.x, ib = 0.0;
-        double2 tau = c2(0.0, 0.0), scal = c2(0.0, 0.0);
+        // reflector scalars (every lane the same): 16 FP64 instructions up to scal
+        double beta = alpha.x, ib = 0.0, nrm = 0.0, n2 = 0.0;
         if (apply) {
-          const double n2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn2));
+          n2 = xn2 + s_a2;
           const double y = fast_rsqrt(n2);
-          double nrm = n2 * y;
-          nrm = fma(0.5 * y, fma(-nrm, nrm, n2), nrm);
-          beta = -copysign(nrm, alpha.x);
           ib = -copysign(y, alpha.x);
+          nrm = n2 * y;
+          nrm = fma(half_of(y), fma(-nrm, nrm, n2), nrm);
+          beta = -copysign(nrm, alpha.x);
         }
         if (lane == 0) {
           s_ib = ib;
           s_beta = beta;
           s_apply = apply ? 1 : 0;
         }
-        asm volatile("bar.sync 1, 64;" ::: "memory");
+        asm volatile("bar.sync 1, 96;" ::: "memory");
+        double dx = 0.0;
         if (apply) {
-          const double dx = alpha.x - beta;
-          const double id2 = fast_recip(fma(dx, dx, alpha.y * alpha.y));
-          scal = c2(dx * id2, -alpha.y * id2);
-          tau = c2((beta - alpha.x) * ib, -alpha.y * ib);
+          dx = alpha.x - beta;
+          const double id2 = fast_recip(fma(dx, dx, s_ay2));
+          if (lane == 0) s_scal = c2(dx * id2, -alpha.y * id2);
+        } else if (lane == 0) {
+          s_scal = c2(0.0, 0.0);
         }
-        if (lane == 0) {
-          s_scal = scal;
-          s_tau[j] = tau;
-        }
-        asm volatile("bar.sync 1, 64;" ::: "memory");
-        // Gram entries v_c^H v_j, c < j
-        if (lane < j) s_S[lane][j] = cadd(cmul(cconj(tot), scal), cconj(prow));
-      } else {
+        asm volatile("bar.sync 1, 96;" ::: "memory");
+        if (lane == 0) s_tau[j] = c2(-dx * ib, -alpha.y * ib);
+      } else if (warp == 1) {
         // row of R and the update factors
-        const double2 t = cfma(cconj(alpha), prow, tot);
-        asm volatile("bar.sync 1, 64;" ::: "memory");
-        const double ib = s_ib;
-        const double2 r = c2(t.x * ib, t.y * ib);
-        const double2 w = csub(prow, r);
-        asm volatile("bar.sync 1, 64;" ::: "memory");
+        const double t = fma(im ? -alpha.y : alpha.y, p_other, fma(alpha.x, p_own, own));
+        asm volatile("bar.sync 1, 96;" ::: "memory");
+        const double r = t * s_ib;
+        const double w = p_own - r;
+        const double w_other = __shfl_xor_sync(0xffffffffu, w, 16);
+        reinterpret_cast<double*>(&s_r[c16])[im] =
+            apply ? (c16 > j ? r : c16 == j ? (im ? 0.0 : s_beta) : p_own) : p_own;
+        asm volatile("bar.sync 1, 96;" ::: "memory");
+        // column j takes scal x_j, the columns behind it x - x_j (scal w)
         const double2 scal = s_scal;
-        if (lane < 16) {
-          s_r[c16] = apply ? (c16 > j ? r : c16 == j ? c2(s_beta, 0.0) : prow) : prow;
-          // column j takes scal x_j, the columns behind it x - x_j (scal w)
-          const double2 u = cmul(scal, w);
-          s_u[c16] = c16 == j ? scal : c2(-u.x, -u.y);
-        }
+        const double u = fma(im ? scal.y : -scal.y, w_other, scal.x * w);
+        reinterpret_cast<double*>(&s_u[c16])[im] = c16 == j ? (im ? scal.y : scal.x) : -u;
+      } else {
+        // Gram entries v_c^H v_j = conj(sum) scal + conj(pivot row), c < j
+        asm volatile("bar.sync 1, 96;" ::: "memory");
+        asm volatile("bar.sync 1, 96;" ::: "memory");
+        const double2 scal = s_scal;
+        const double g = fma(im ? scal.y : scal.x, im ? other : own,
+                             fma(im ? -scal.x : scal.y, im ? own : other, im ? -p_own : p_own));
+        if (c16 < j) reinterpret_cast<double*>(&s_S[c16][j])[im] = g;
       }
-    } else if (warp >= 4 && make_t && j > 0) {
+    } else if (warp >= 6 && make_t && j > 0) {
       t_column(j - 1);
     }
     __syncthreads();
@@ -1214,7 +1230,7 @@ __global__ void __launch_bounds__(P8T) qr_panel8_kernel(const P8Args g) {
   }
   __syncthreads();
   if (FULL) {
-    if (warp >= 4) t_column(jb - 1);
+    if (warp >= 6) t_column(jb - 1);
     cluster.sync();
     // V1 (unit lower triangular) into s_S, M = T V1^H
     __shared__ double2 s_M[NB][NB + 1];
