@@ -377,12 +377,11 @@ __global__ void svd_first_order_kernel(const double2* __restrict__ G, int r, dou
     const int i = (int)(e / r), j = (int)(e % r);
     double2 y = c2(i == j ? 1.0 : 0.0, 0.0);
     if (i != j) {
-      const double2 g = G[e];
+      // both elements of a pair from the one above the diagonal: G is Hermitian up to rounding
+      // only, and where singular values repeat its off-diagonal part is nothing but rounding
+      const double2 t = i < j ? G[e] : cconj(G[(long)j * r + i]);
       const double d = G[(long)j * r + j].x - G[(long)i * r + i].x;
-      // both pairs (i, j) and (j, i) decide alike: G is Hermitian bit for bit only up to
-      // rounding, so the test is made on the element above the diagonal
-      const double2 t = i < j ? g : G[(long)j * r + i];
-      if (fabs(t.x) + fabs(t.y) <= xmax * fabs(d) && d != 0.0) y = c2(g.x / d, g.y / d);
+      if (fabs(t.x) + fabs(t.y) <= xmax * fabs(d) && d != 0.0) y = c2(t.x / d, t.y / d);
     }
     Y[e] = y;
   }

@@ -278,3 +278,19 @@ def test_svd_from_fp32_start(mn, kind):
     keep = s > 1e-13 * s[0]
     for x in (u[:, keep], vh[keep].conj().T):
         assert np.abs(x.conj().T @ x - np.eye(keep.sum())).max() <= tol * np.sqrt(r)
+
+
+@pytest.mark.parametrize("m", [32, 40, 57])
+@pytest.mark.parametrize("seed", range(6))
+def test_svd_of_repeated_values(m, seed):
+    """A multiple of a unitary matrix but for three values: the Gram matrix of the refinement
+    holds nothing but rounding off its diagonal."""
+    rng = np.random.default_rng(seed)
+    u, _, vh = np.linalg.svd(orc.crandn((m, m), rng))
+    a = (u * np.r_[np.full(m - 3, 2.0), 1.0, 1.0, 0.5]) @ vh
+    u, s, vh, sweeps = dev_svd(a)
+    tol = 16 * m * np.finfo(float).eps
+    assert np.abs(s - np.linalg.svd(a, compute_uv=False)).max() <= 2 * tol
+    assert np.linalg.norm((u * s) @ vh - a) <= tol * np.linalg.norm(a) * np.sqrt(m)
+    for x in (u, vh.conj().T):
+        assert np.abs(x.conj().T @ x - np.eye(m)).max() <= tol * np.sqrt(m)
