@@ -24,8 +24,8 @@
 // two more Newton-Schulz steps make it unitary. The FP64 sweeps, whose stopping rule and so
 // whose accuracy stay as they are, then mostly verify: one sweep instead of nine or ten.
 // What bounds the iteration: an FP64 instruction of a warp takes 64 cycles of its
-// sub-partition; the FP32 sweeps cost only their rounds' latency (L2 round trip, cluster
-// barrier).
+// sub-partition; the FP32 sweeps cost only their rounds' latency (sums, rotation,
+// cluster barrier).
 //
 // Singular vectors of one singular value are unique only up to a phase (or a
 // unitary mix for repeated values): they need not equal LAPACK's, while the
@@ -33,9 +33,10 @@
 // truncated split agree to rounding.
 //
 // One cluster of up to 16 CTAs per matrix: a round's pairs are spread over the CTAs, four
-// warps to a pair; the columns stay in global memory (L2), a cluster barrier ends a round.
-// Measured, 128 x 96: 75.6 ms (one CTA, FP64 sweeps only) -> 2.45 ms (FP32 sweeps 1.57,
-// GEMMs 0.25, FP64 sweeps 0.57).
+// warps to a pair; the columns stay in global memory (L2), in the FP32 sweeps in shared memory
+// where they fit; a cluster barrier ends a round.
+// Measured, 128 x 96: 75.6 ms (one CTA, FP64 sweeps only) -> 2.40 ms with FP32 sweeps through
+// L2 (1.53 of it) -> 1.83 ms (FP32 sweeps 0.96, GEMMs 0.25, FP64 sweeps 0.57).
 #include "ptn_common.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -97,7 +98,14 @@ struct Rot {
   int on;
 };
 
-// off: |c| / sqrt(a b) as far as FP32 tells. FP32 form.
+__device__ __forceinline__ float fast_sqrt(float x) {
+  float y;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// off: |c| / sqrt(a b) as far as FP32 tells. FP32 form, with approximate divisions and square
+// roots (a few units of the last place, which V32 is off unitary by anyway).
 __device__ __forceinline__ Rot<float> rotation(float aa, float bb, float cr, float ci, float tol,
                                                float& off) {
   Rot<float> R;
@@ -106,16 +114,17 @@ __device__ __forceinline__ Rot<float> rotation(float aa, float bb, float cr, flo
   // columns below 1e-15 of the largest entry: beyond what FP32 resolves (and their products
   // near the end of its range)
   if (!(aa > 1e-30f && bb > 1e-30f)) return R;
-  const float mx = fmaxf(fabsf(cr), fabsf(ci)), ab = sqrtf(aa) * sqrtf(bb);
+  const float mx = fmaxf(fabsf(cr), fabsf(ci)), ab = fast_sqrt(aa) * fast_sqrt(bb);
   if (!(mx > 0.5f * tol * ab)) return R;
-  const float ur = cr / mx, ui = ci / mx, ul = rsqrtf(ur * ur + ui * ui);
-  const float ac = mx / ul;
-  off = ac / ab;
+  const float im = __fdividef(1.0f, mx), ur = cr * im, ui = ci * im;
+  const float u2 = ur * ur + ui * ui, ul = rsqrtf(u2);
+  const float ac = mx * u2 * ul;
+  off = __fdividef(ac, ab);
   R.on = ac > tol * ab;
   if (!R.on) return R;
   const float pr = ur * ul, pi = -ui * ul;
-  const float z = (bb - aa) / (2.0f * ac);
-  const float t = copysignf(1.0f, z) / (fabsf(z) + sqrtf(1.0f + z * z));
+  const float z = __fdividef(bb - aa, 2.0f * ac);
+  const float t = __fdividef(copysignf(1.0f, z), fabsf(z) + fast_sqrt(1.0f + z * z));
   R.cs = rsqrtf(1.0f + t * t);
   R.sn = R.cs * t;
   R.gr = R.sn * pr;
@@ -387,6 +396,114 @@ __global__ void svd_first_order_kernel(const double2* __restrict__ G, int r, dou
   }
 }
 
+// The FP32 sweeps with the columns of W and V in shared memory, for matrices whose two copies
+// fit the cluster (SHARED_MAX a CTA; others stay in L2, above). Pair t of a round lives in CTA
+// t / S; in the circle order a pair's first column goes to pair t - 1 for the next round and
+// its second to pair t + 1, so a rotation writes its columns where the next round reads them,
+// into the other copy, mostly in the same CTA. Every warp forms its group's rotation itself.
+// What bounds it: latency of a round (sums over the group, the rotation, the cluster barrier).
+// Measured, 128 x 96: 1525 us through L2 -> 956 us (no integer division in a round, approximate
+// FP32 divisions and roots in the rotation: 1320 us without these two).
+constexpr long SHARED_MAX = 192 * 1024;
+constexpr long pre_pairs(long r, long cs) { return ((r + 1) / 2 + cs - 1) / cs; }   // S
+constexpr long pre_bytes(long p, long r, long cs) {
+  return pre_pairs(r, cs) * 2 * 2 * (p + r) * (long)sizeof(float2);
+}
+
+__device__ void sweeps_shared(float2* sh, const double2* __restrict__ a, long lda, bool wide, int p,
+                              int r, int ex, float tol, float last, int max_sweeps,
+                              double2* __restrict__ Vd) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int g = tid / GROUP, gt = tid % GROUP, gw = gt >> 5;
+  __shared__ float s_sum[NGROUP][2][4][4];
+  __shared__ int s_off[2];
+  if (tid < 2) s_off[tid] = 0;
+  const int T = (r + 1) / 2, ring = 2 * T - 1;   // pairs, columns in the circle
+  const int S = (int)pre_pairs(r, cs), len = p + r;
+  const int mine = max(0, min(S, T - rank * S));
+  auto first_of = [&](int q, int t) { return t == 0 ? 0 : 1 + (q + t) % ring; };
+  auto second_of = [&](int q, int t) { return 1 + (q + ring - t) % ring; };
+  for (int e = tid; e < mine * 2 * len; e += ST) {
+    const int h = e / len, i = e % len, t = rank * S + (h >> 1);
+    const int c = h & 1 ? second_of(0, t) : first_of(0, t);
+    float2 v = make_float2(i - p == c ? 1.0f : 0.0f, 0.0f);
+    if (i < p && c < r) {   // the column that makes an odd count even is zero
+      double2 z = wide ? a[(long)c * lda + i] : a[(long)i * lda + c];
+      if (wide) z.y = -z.y;
+      v = make_float2(scaled_float(z.x, ex - 1022), scaled_float(z.y, ex - 1022));
+    }
+    sh[e] = v;
+  }
+  cluster.sync();
+  int b = 0, par = 0;
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    int worst = 0;
+    for (int q = 0; q < ring; ++q) {
+      for (int s = g; s < mine; s += NGROUP) {
+        const int t = rank * S + s;
+        const float2* x = sh + (b * S + s) * 2 * len;
+        const float2* y = x + len;
+        auto place = [&](int by, int side) {   // in pair t + by; no divisions in here
+          const int to = s + by, rk = rank + (to < 0 ? -1 : to == S ? 1 : 0);
+          const int sl = to < 0 ? S - 1 : to == S ? 0 : to;
+          return cluster.map_shared_rank(sh, rk) + ((b ^ 1) * S + sl) * 2 * len + side * len;
+        };
+        float2* nx = place(t == 0 ? 0 : -1, t == 1 ? 1 : 0);
+        float2* ny = t == T - 1 ? place(0, 0) : place(1, 1);
+        Rot<float> R;
+        R.on = 0;
+        if (r == ring + 1 || max(first_of(q, t), second_of(q, t)) < r) {
+          float aa = 0.0f, bb = 0.0f, cr = 0.0f, ci = 0.0f;
+          for (int i = gt; i < p; i += GROUP) {
+            const float2 u = x[i], v = y[i];
+            aa = fmaf(u.x, u.x, fmaf(u.y, u.y, aa));
+            bb = fmaf(v.x, v.x, fmaf(v.y, v.y, bb));
+            cr = fmaf(u.x, v.x, fmaf(u.y, v.y, cr));   // conj(u) v
+            ci = fmaf(u.x, v.y, fmaf(-u.y, v.x, ci));
+          }
+          const float sum = warp_sum4(aa, bb, cr, ci);
+          float(*part)[4] = s_sum[g][par];
+          par ^= 1;   // a warp may be one pair ahead of the others
+          if (lane < 4) part[gw][lane] = sum;
+          group_sync(g);
+          float v[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v[k] = (part[0][k] + part[1][k]) + (part[2][k] + part[3][k]);
+          float off;
+          R = rotation(v[0], v[1], v[2], v[3], tol, off);
+          if (R.on) worst = max(worst, __float_as_int(off));
+        }
+        for (int i = gt; i < len; i += GROUP) {
+          float2 u = x[i], v = y[i];
+          if (R.on) rotate(R, u, v);
+          nx[i] = u;
+          ny[i] = v;
+        }
+      }
+      cluster.sync();
+      b ^= 1;
+    }
+    // the largest off-orthogonality of the sweep, over the cluster
+    if (worst > 0 && lane == 0)
+      for (int c = 0; c < cs; ++c) atomicMax(cluster.map_shared_rank(&s_off[sweep & 1], c), worst);
+    if (tid == 0) s_off[(sweep + 1) & 1] = 0;
+    cluster.sync();
+    if (__int_as_float(s_off[sweep & 1]) <= last) break;
+    // everyone has read it before the next but one sweep clears it
+  }
+  // a whole sweep brings every column back to its first place
+  for (int e = tid; e < mine * 2 * r; e += ST) {
+    const int h = e / r, i = e % r, t = rank * S + (h >> 1);
+    const int c = h & 1 ? second_of(0, t) : first_of(0, t);
+    if (c < r) {
+      const float2 v = sh[((long)b * S * 2 + h) * len + p + i];
+      Vd[(long)c * r + i] = c2(v.x, v.y);
+    }
+  }
+}
+
 // FP32 sweeps on A scaled to entries below 1: V32 as FP64 to Vd (column-major), identities
 // to the NS buffers G (for the Newton-Schulz steps), *bad = 1 when A holds an infinity or NaN (the
 // GEMMs and the FP64 sweeps then start from A itself).
@@ -395,7 +512,8 @@ __global__ void __launch_bounds__(ST) svd_pre_kernel(const double2* __restrict__
                                                      float2* __restrict__ V,
                                                      double2* __restrict__ Vd,
                                                      double2* __restrict__ G,
-                                                     int* __restrict__ bad) {
+                                                     int* __restrict__ bad, bool shared) {
+  extern __shared__ float2 columns[];
   cg::cluster_group cluster = cg::this_cluster();
   const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x;
@@ -404,7 +522,9 @@ __global__ void __launch_bounds__(ST) svd_pre_kernel(const double2* __restrict__
   const long step = (long)cs * ST, first = rank * (long)ST + tid;
   const int e = largest_exponent(a, m, n, lda);
   if (rank == 0 && tid == 0) *bad = e == 2047 ? 1 : 0;
-  if (e != 2047) {
+  if (e != 2047 && shared) {
+    sweeps_shared(columns, a, lda, wide, p, r, e, 1e-6f, 3e-4f, PRE_SWEEPS, Vd);
+  } else if (e != 2047) {
     for (long q = first; q < (long)p * r; q += step) {
       const int j = (int)(q / p), i = (int)(q % p);
       double2 z = wide ? a[(long)j * lda + i] : a[(long)i * lda + j];
@@ -420,7 +540,7 @@ __global__ void __launch_bounds__(ST) svd_pre_kernel(const double2* __restrict__
     const double2 one = c2(q / r == q % r ? 1.0 : 0.0, 0.0);
 #pragma unroll
     for (int t = 0; t < NS; ++t) G[(long)t * r * r + q] = one;
-    if (e != 2047) {
+    if (e != 2047 && !shared) {
       const float2 v = __ldcg(V + q);
       Vd[q] = c2(v.x, v.y);
     }
@@ -527,8 +647,10 @@ inline size_t al(size_t b) { return (b + 255) & ~size_t(255); }
 }  // namespace
 
 // largest cluster the kernels can be launched with (16, else 8, else 1); decided once
-static int svd_cluster_max() {
+// and whether the FP32 kernel fits with its columns in shared memory
+static int svd_cluster_max(bool* shared = nullptr) {
   static int best = 1;
+  static bool fits = false;
   static std::once_flag once;
   std::call_once(once, [] {
     for (const void* f : {(const void*)svd_pre_kernel, (const void*)svd_jacobi_kernel})
@@ -550,11 +672,18 @@ static int svd_cluster_max() {
           cudaOccupancyMaxActiveClusters(&nb, svd_jacobi_kernel, &cfg) == cudaSuccess && na > 0 &&
           nb > 0) {
         best = c;
+        if (cudaFuncSetAttribute(svd_pre_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)SHARED_MAX) == cudaSuccess) {
+          cfg.dynamicSmemBytes = SHARED_MAX;
+          fits = cudaOccupancyMaxActiveClusters(&na, svd_pre_kernel, &cfg) == cudaSuccess && na > 0;
+        }
+        if (!fits) cudaGetLastError();
         break;
       }
       cudaGetLastError();
     }
   });
+  if (shared != nullptr) *shared = fits;
   return best;
 }
 
@@ -619,8 +748,13 @@ ptn_status svd(const double2* a, int m, int n, long lda, double2* u, long ldu, d
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (pre) {
+    bool shared = false;
+    svd_cluster_max(&shared);
+    shared = shared && pre_bytes(p, r, cs) <= SHARED_MAX;
+    cfg.dynamicSmemBytes = shared ? pre_bytes(p, r, cs) : 0;
     PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, svd_pre_kernel, a, m, n, lda, w.W32, w.V32, w.V0, w.G,
-                                    w.bad));
+                                    w.bad, shared));
+    cfg.dynamicSmemBytes = 0;
     note_launches(1);
     // the buffers hold V^T and W^T row-major (V and W column by column)
     double2* V = w.V0;

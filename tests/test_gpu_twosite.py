@@ -294,3 +294,19 @@ def test_svd_of_repeated_values(m, seed):
     assert np.linalg.norm((u * s) @ vh - a) <= tol * np.linalg.norm(a) * np.sqrt(m)
     for x in (u, vh.conj().T):
         assert np.abs(x.conj().T @ x - np.eye(m)).max() <= tol * np.sqrt(m)
+
+
+# the largest matrices whose FP32 sweeps keep the columns in shared memory, and the smallest
+# beyond; more pairs than thread groups in a CTA
+@pytest.mark.parametrize("mn", [(310, 300), (330, 300), (256, 257), (131, 131)])
+def test_svd_columns_in_shared_memory(mn):
+    m, n = mn
+    a = orc.crandn((m, n), np.random.default_rng(m + n))
+    u, s, vh, sweeps = dev_svd(a)
+    assert sweeps < 60
+    s_ref = np.linalg.svd(a, compute_uv=False)
+    tol = 16 * max(m, n) * np.finfo(float).eps
+    assert np.abs(s - s_ref).max() <= tol * s_ref[0]
+    assert np.linalg.norm((u * s) @ vh - a) <= tol * np.linalg.norm(a) * np.sqrt(min(m, n))
+    for x in (u, vh.conj().T):
+        assert np.abs(x.conj().T @ x - np.eye(min(m, n))).max() <= tol * np.sqrt(min(m, n))
