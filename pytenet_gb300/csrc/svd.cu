@@ -22,7 +22,8 @@
 // G = W^H W, W = A V, the first-order rotation V (I + X), X_ij = G_ij / (G_jj - G_ii), leaves
 // the square of the off-diagonal part (pairs too close for that are left to the sweeps), and
 // two more Newton-Schulz steps make it unitary. The FP64 sweeps, whose stopping rule and so
-// whose accuracy stay as they are, then mostly verify: one sweep instead of nine or ten.
+// whose accuracy stay as they are, then run only if the Gram matrix of the result shows a pair
+// that the rule would rotate: none or one sweep instead of nine or ten.
 // What bounds the iteration: an FP64 instruction of a warp takes 64 cycles of its
 // sub-partition; the FP32 sweeps cost only their rounds' latency (sums, rotation,
 // cluster barrier).
@@ -36,7 +37,8 @@
 // warps to a pair; the columns stay in global memory (L2), in the FP32 sweeps in shared memory
 // where they fit; a cluster barrier ends a round.
 // Measured, 128 x 96: 75.6 ms (one CTA, FP64 sweeps only) -> 2.40 ms with FP32 sweeps through
-// L2 (1.53 of it) -> 1.83 ms (FP32 sweeps 0.96, GEMMs 0.25, FP64 sweeps 0.57).
+// L2 (1.53 of it) -> 1.83 ms (FP32 sweeps 0.96, GEMMs 0.25, one FP64 sweep 0.57) -> 1.45 ms
+// (the last check on a Gram matrix).
 #include "ptn_common.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -550,6 +552,33 @@ __global__ void __launch_bounds__(ST) svd_pre_kernel(const double2* __restrict__
 
 // W (p x r) and V (r x r) are column-major scratch; u, vh row-major outputs. `pre`: W and V
 // hold the start of the sweeps unless *bad.
+// whether a pair of the Gram matrix H = W^H W is further from orthogonal than tol, by the
+// cluster: the test that a sweep makes pair by pair, with its exceptions (columns near the
+// lower end of the range are left to it)
+__device__ bool pair_left(const double2* __restrict__ H, int r, float tol) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  __shared__ int s_left;
+  if (threadIdx.x == 0) s_left = 0;
+  cluster.sync();
+  bool left = false;
+  for (long e = rank * (long)ST + threadIdx.x; e < (long)r * r; e += (long)cs * ST) {
+    const int i = (int)(e / r), j = (int)(e % r);
+    if (i >= j) continue;
+    const double2 h = H[e];
+    const double aa = H[(long)i * r + i].x, bb = H[(long)j * r + j].x;
+    const int ea = exp_of(aa), eb = exp_of(bb), sh = (ea + eb) >> 1;
+    if (ea == 1024 || eb == 1024) continue;
+    const float fr = scaled_float(h.x, sh), fi = scaled_float(h.y, sh);
+    const float ab = scaled_float(aa, ea) * scaled_float(bb, eb) * ((ea + eb) & 1 ? 2.0f : 1.0f);
+    left |= ea < -960 || eb < -960 || !(fr * fr + fi * fi <= tol * tol * ab);
+  }
+  if (__any_sync(0xffffffffu, left) && (threadIdx.x & 31) == 0)
+    for (int c = 0; c < cs; ++c) *cluster.map_shared_rank(&s_left, c) = 1;
+  cluster.sync();
+  return s_left != 0;
+}
+
 __global__ void __launch_bounds__(ST) svd_jacobi_kernel(const double2* __restrict__ a, int m, int n,
                                                        long lda, double2* __restrict__ W,
                                                        double2* __restrict__ V,
@@ -558,7 +587,8 @@ __global__ void __launch_bounds__(ST) svd_jacobi_kernel(const double2* __restric
                                                        long ldu, double* __restrict__ s,
                                                        double2* __restrict__ vh, long ldvh,
                                                        int* __restrict__ sweeps_out, int pre,
-                                                       const int* __restrict__ bad) {
+                                                       const int* __restrict__ bad,
+                                                       const double2* __restrict__ H) {
   cg::cluster_group cluster = cg::this_cluster();
   const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = tid & 31;
@@ -584,7 +614,9 @@ __global__ void __launch_bounds__(ST) svd_jacobi_kernel(const double2* __restric
   }
   cluster.sync();
   const double tol = (double)p * 2.220446049250313e-16;
-  const int sweep = sweeps<double>(W, V, p, r, tol, 0.0f, MAX_SWEEPS);
+  int sweep = 0;
+  if (!pre || *bad != 0 || shift != 0 || pair_left(H, r, (float)tol))
+    sweep = sweeps<double>(W, V, p, r, tol, 0.0f, MAX_SWEEPS);
   // singular values, their order, the outputs
   for (int j = warp; j < r; j += nwarp) {
     const double2* wj = W + (long)j * p;
@@ -794,10 +826,11 @@ ptn_status svd(const double2* a, int m, int n, long lda, double2* u, long ldu, d
       PTN_TRY(newton_schulz(2 * t + 2));
       PTN_TRY(times_a());
     }
+    PTN_TRY(mult('C', 'T', r, r, p, w.W, p, w.W, p, w.H, 1.0, 0.0));   // for the last check
     w.V = V;
   }
   PTN_CUDA_TRY(cudaLaunchKernelEx(&cfg, svd_jacobi_kernel, a, m, n, lda, w.W, w.V, w.sig, w.pos, u,
-                                  ldu, s, vh, ldvh, sweeps, pre ? 1 : 0, (const int*)w.bad));
+                                  ldu, s, vh, ldvh, sweeps, pre ? 1 : 0, (const int*)w.bad, (const double2*)w.H));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;
