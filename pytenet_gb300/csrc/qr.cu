@@ -1285,7 +1285,7 @@ __global__ void __launch_bounds__(P8T) qr_panel8_kernel(const P8Args g) {
     }
   }
   if (make_t) {
-    if (warp >= 4) t_column(jb - 1);
+    if (warp >= 6) t_column(jb - 1);
     __syncthreads();
     g.T[tid] = s_T[b16][c16];
   }
