@@ -12,9 +12,9 @@ explicit L2 flush is needed between steps.
   python bench.py [--gpus N] [--steps K] [--warmup W] [--form learned|mixed|fp64] [--no-graph]
 
 Forms: "fp64" = complex128 everywhere, fixed Lanczos depth (the reference's
-method); "mixed" = tensor-core contractions from five fixed-point BF16 digits per
-row-scaled value (exact integer accumulation of the leading digit levels, FP64
-recombination) with FP64 Krylov / QR, fixed depth; "learned" (default) = "mixed" plus the
+method); "mixed" = tensor-core contractions of row-scaled fixed-point values by
+residues (11 moduli in the operators, 13 in the environments; the FP64 form takes 14)
+with FP64 Krylov / QR, fixed depth; "learned" (default) = "mixed" plus the
 learned Lanczos depth (trained MLP, residual-guarded early exit, falling back to the full
 depth); "residual" = "mixed" with the same residual estimate tested after every iteration
 from depth 2 and no network (the baseline the learned depth is measured against). Each timed step is replayed as a captured CUDA graph unless --no-graph.
@@ -294,7 +294,7 @@ def replica_value(world, site_updates, steps, ms_max):
 
 
 def kern_key(form):
-    return "zgemm_dmma" if form == "fp64" else "tc_gemm"
+    return "rns_gemm_fp64" if form == "fp64" else "rns_gemm"
 
 
 def capture_traffic(kernel, D):
@@ -365,7 +365,8 @@ def our_arm(a):
     clocks = ClockSampler(local)
     clocks.start()
     launches0 = L.ptn_launch_count()
-    dominant = 0 if a.form == "fp64" else 1
+    # products below the tensor-core rule (bonds under about 80 in the FP64 form) are DMMA
+    dominant = 0 if a.form == "fp64" and a.D < 80 else 1
     ks0 = run.chain.krylov_state()
     L.ptn_prof_start((1 << dominant) | (1 << 3) | (1 << 4))
     e0 = torch.cuda.Event(enable_timing=True)
@@ -433,7 +434,7 @@ def our_arm(a):
                     else "bf16 sustained of fallback")
         achieved = k_fl / (k_ms / 1e3) / 1e12 if k_ms > 0 else None
         unit = "TFLOP/s"
-        kern = "tcgen05 BF16-digit complex GEMM (5 digits)"
+        kern = "tcgen05 residue complex GEMM (BF16 residues, FP32 exact)"
     else:
         # FP64 tensor (DMMA) peak: measured on this machine's GB300 with a DMMA-only kernel
         peak = 1.047
@@ -448,7 +449,9 @@ def our_arm(a):
                 "unit": unit, "frac": (achieved / peak) if achieved else None, "traffic": traffic,
                 "traffic_unit": "bytes per launch" if traffic else None,
                 "traffic_source": traffic_src,
-                "digit_product_tflops": (achieved * 15.0) if (achieved and dominant == 1) else None,
+                # two real products per modulus: 14 moduli (FP64) or at least 11 (mixed)
+                "residue_product_tflops": (achieved * (7.0 if a.form == "fp64" else 5.5))
+                if (achieved and dominant == 1) else None,
                 "peak_source": peak_src, "launches_timed": k_n,
                 "kernel_share_of_step": (k_ms / prof_ms) if prof_ms > 0 else None,
                 "qr_share_of_step": (q_ms / prof_ms) if prof_ms > 0 else None,
@@ -493,7 +496,7 @@ def our_arm(a):
         out = {"metric": METRIC, "value": value, "unit": "site-updates/s", "n_gpus": world,
                "steps": a.steps, "warmup": a.warmup, "ms_per_step": ms_max / a.steps,
                "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-               "dtype": "c128" if a.form == "fp64" else "bf16 digits (5 x 8-bit fixed point, tcgen05) + f64",
+               "dtype": "c128" if a.form == "fp64" else "bf16 residues (fixed point of 40-52 bits, tcgen05) + f64",
                "data": "synthetic",
                "config": {"workload": workload_desc(a), "form": a.form, "L": a.L, "D": a.D,
                           "numiter_lanczos": a.m, "delta": delta, "graph": a.graph,
@@ -598,13 +601,13 @@ def batch_arm(a):
                 "the first 32768 timed launches"
     launches_step = L.ptn_launch_count() - launches0
     kinds = {}
-    for k, name in enumerate(["zgemm_dmma (FP64 GEMM)", "tc_gemm (tcgen05 digit GEMM)",
+    for k, name in enumerate(["zgemm_dmma (FP64 GEMM)", "rns_gemm (tcgen05 residue GEMM)",
                               "mpo_stage", "qr", "krylov"]):
         tot, fl, by, n = ctypes.c_double(), ctypes.c_double(), ctypes.c_double(), ctypes.c_long()
         _lib.check(L.ptn_prof_read(k, ctypes.byref(tot), ctypes.byref(fl), ctypes.byref(by),
                                    ctypes.byref(n)))
         kinds[name] = {"ms": tot.value, "flops": fl.value, "bytes": by.value, "launches": n.value}
-    dom = "tc_gemm (tcgen05 digit GEMM)" if prec == "mixed" else "zgemm_dmma (FP64 GEMM)"
+    dom = max(list(kinds)[:2], key=lambda k: kinds[k]["ms"])
     kd = kinds[dom]
     achieved = kd["flops"] / (kd["ms"] / 1e3) / 1e12 if kd["ms"] > 0 else None
     peaks = {}
@@ -612,11 +615,11 @@ def batch_arm(a):
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
     except Exception:
         pass
-    peak = peaks.get("bf16_tflops", 1900.0) if prec == "mixed" else 1.047
+    peak = peaks.get("bf16_tflops", 1900.0) if dom.startswith("rns") else 1.047
     eager_total = sum(v["ms"] for v in kinds.values())
     roofline = {"bound": "tensor", "kernel": dom, "achieved": achieved, "peak": peak,
                 "unit": "TFLOP/s", "frac": achieved / peak if achieved else None, "traffic": None,
-                "peak_source": ("bf16_tflops of measured" if prec == "mixed" else
+                "peak_source": ("bf16_tflops of measured" if dom.startswith("rns") else
                                 "FP64 DMMA m8n8k4 throughput measured on GB300 (1.047 TFLOP/s)"),
                 "measured_on": prof_note,
                 "kind_ms_eager_step": {k: v["ms"] for k, v in kinds.items()},
@@ -659,7 +662,7 @@ def batch_arm(a):
     out = {"metric": BATCH_METRIC, "value": value, "unit": "site-updates/s", "n_gpus": 1,
            "steps": a.steps, "warmup": a.warmup, "ms_per_step": ms / a.steps,
            "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-           "dtype": "c128" if prec == "fp64" else "bf16 digits (5 x 8-bit fixed point, tcgen05) + f64",
+           "dtype": "c128" if prec == "fp64" else "bf16 residues (fixed point of 40-52 bits, tcgen05) + f64",
            "data": "synthetic",
            "config": {"workload": batch_desc(a), "form": prec, "instances": a.batch_count,
                       "site_updates_per_step": site_updates, "d_caps": dmix,
@@ -796,7 +799,7 @@ def precision_arm(a):
     out = {"metric": PREC_METRIC, "value": value, "unit": "site-updates/s", "n_gpus": 1,
            "steps": a.steps, "warmup": a.acc_steps + warm, "ms_per_step": ms / a.steps,
            "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-           "dtype": "bf16 digits (5 x 8-bit fixed point, tcgen05) + f64", "data": "synthetic",
+           "dtype": "bf16 residues (fixed point of 40-52 bits, tcgen05) + f64", "data": "synthetic",
            "config": {"workload": f"XXZ L={L} D={D} J=1 Delta=0.8 h=-0.1 (seed {a.seed}), "
                                   f"dt=0.02j, numiter_lanczos={m}; TDVP steps timed after "
                                   f"{a.acc_steps} accuracy steps",
@@ -854,7 +857,7 @@ def accuracy_vs_fp64(a, ptg, h, psi_host0, qb0, depth_model=None):
         fp64 = {"value": (2 * a.L - 1) / (ms / 1e3), "unit": "site-updates/s",
                 "ms_per_step": ms, "steps_timed": len(fp64_ms), "warmup": 1,
                 "graph": a.graph,
-                "what": "plain complex128 form (FP64 DMMA contractions, FP64 Krylov and QR, "
+                "what": "plain complex128 form (residue contractions at FP64 accuracy, FP64 Krylov and QR, "
                         "fixed depth numiter_lanczos) on the same chain and initial state; the "
                         "first step (graph capture) untimed"}
     return out, fp64

@@ -6,8 +6,8 @@ streams the batch is spread over.
 Knobs (include/pytenet_gb300.h), plus "mmb", the smallest bond on which the mixed form
 uses the tensor cores (a tensor-core GEMM CTA takes a whole SM's shared memory and
 tensor memory, so in a batch small problems may overlap better on the FP64 path):
-  PTN_TUNE_TC_SPLIT_WAVES    split-K target of the tensor-core digit GEMM
-  PTN_TUNE_ZGEMM_SPLIT_WAVES split-K target of the FP64 GEMM
+  PTN_TUNE_TC_SPLIT_WAVES    split-K target of the digit GEMM (bond-matrix absorption, mixed)
+  PTN_TUNE_ZGEMM_SPLIT_WAVES split-K target of the FP64 DMMA GEMM
   PTN_TUNE_LARFB_TILE        block-update tile of the QR
   PTN_TUNE_QR_CLUSTER        cluster size cap of the QR panel
 Each bucket is tuned on its most expensive instance by coordinate descent: one

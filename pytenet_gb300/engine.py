@@ -125,9 +125,9 @@ class DeviceMPS:
         return c
 
     def _gemm(self, M, N, K, a, b, out, mixed):
-        """out (M x N) = a (M x K) b (K x N), row-major complex: FP64 DMMA, or with
-        mixed=True the tensor-core digit GEMM (the contraction arithmetic of the
-        mixed form)."""
+        """out (M x N) = a (M x K) b (K x N), row-major complex: FP64 form, or with
+        mixed=True the tensor-core digit GEMM. (Residue products here would save 1 %
+        of the mixed step and move its states by 1e-9; the digits stay.)"""
         L, st = lib(), stream_ptr()
         if mixed:
             wsb = L.ptn_zgemm_split_bf16_workspace_bytes(M, N, K)
@@ -267,9 +267,9 @@ class Chain(DeviceMPS):
         self.depth = depth
 
     def prec_for(self, Dl, Dr):
-        """Arithmetic of one local problem. The mixed form runs the tensor-core digit
-        GEMMs only where both bonds reach mixed_min_bond (MIXED_MIN_BOND unless set):
-        below that the contractions are too small to fill a 128 x 96 tile, and the
+        """Arithmetic of one local problem. The mixed form runs with fewer moduli
+        only where both bonds reach mixed_min_bond (MIXED_MIN_BOND unless set):
+        below that the contractions are too small to fill a 128 x 64 tile, and the
         Krylov space of a small problem can be exhausted (a Lanczos breakdown at
         beta < 100 n eps), which only the FP64 operator detects the way the reference
         does. The batched driver raises it per bucket: a tensor-core GEMM CTA takes a

@@ -14,8 +14,8 @@ class TDVPRun:
     """Device-resident TDVP run: upload once, step many times, download when
     asked. `tdvp_singlesite` is this class driven for `numsteps` steps.
 
-    precision: "fp64" (plain complex128) or "mixed" (fixed-point BF16 digit
-    contractions on the tensor cores, FP64 Krylov / QR).
+    precision: "fp64" (plain complex128) or "mixed" (tensor-core
+    contractions of rows with 40 to 52 bits, FP64 Krylov / QR).
     depth_model: a trained learned.DepthModel; numiter_lanczos is then the full
     depth the run falls back to whenever the residual estimate at the predicted
     depth exceeds depth_tol. depth_model="residual" tests the same estimate after
