@@ -46,8 +46,13 @@ typedef enum {
 typedef enum {
   PTN_PREC_FP64 = 0,        /* plain complex128: FP64 DMMA, and for products of at least 32 in
                                every dimension and 1e6 complex multiply-adds exact products of
-                               residues modulo 14 numbers on tcgen05 (rows as fixed-point
-                               numbers of 53-54 bits; errors below the DMMA kernel's) */
+                               residues modulo 14 numbers on tcgen05. Rows are fixed-point numbers
+                               of 53-54 bits there, after a scaling of the summed index taken from
+                               one operand (B): error of (m, n) per term 2^-53 of the largest
+                               |A[m, k] B[n', k]| over k and n', less where B's column n is below
+                               the others; row, column and index scalings cancel. A result far
+                               below the others of its row keeps that error, where DMMA sums of
+                               |A[m, k] B[n, k]| alone bound it */
   PTN_PREC_SPLIT_BF16 = 1   /* fewer moduli: 11 in the local operators (40-44 bits per
                                row-scaled value, ~1e-12 relative per contraction), 13 in the
                                environment steps (49-52 bits) */

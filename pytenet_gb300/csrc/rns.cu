@@ -3,7 +3,9 @@
 // C = A B over complex FP64 is computed exactly in integers and rounded once:
 //   - every row of A and every column of B is scaled by its own power of two and rounded
 //     to Gaussian integers of `bits` bits (53 or 54 in the FP64 form, 40 and more in the
-//     mixed form);
+//     mixed form); in the FP64 form the terms are scaled before by powers of two that cancel
+//     in the product (RnsTerms in rns.cuh), so that operands which grow and decay against
+//     each other along the terms lose nothing;
 //   - the integer product is formed modulo nm small pairwise coprime numbers p and put
 //     together by the Chinese remainder theorem (Ozaki, Uchino and Imamura, "Ozaki Scheme
 //     II", 2025, use it for real matrices). All prime factors of the moduli are 1 mod 4,
@@ -18,12 +20,12 @@
 //     s_p = u + v or u - v and w_p a 96-bit constant, so the reconstruction is a sum of
 //     small times wide integers that wraps by itself, one 64 x 64 product by P and one
 //     rounding. Error of a result before that rounding: 2^-bits max|A row| max|B column|
-//     per term, from the rounding of the operands alone.
+//     per term (of the scaled operands), from the rounding of the operands alone.
 //
 // Why: the FP64 units of this part do two FMAs per SM and cycle (1.0 TF/s measured for
 // the DMMA kernel, zgemm_f64.cu); 28 BF16 products at the tensor cores' rate are some 40
-// times faster. Rows that hold an infinity or NaN, or numbers near the ends of the FP64
-// range, are multiplied entry by entry in FP64 by the reconstruction kernel.
+// times faster. Rows that hold an infinity or NaN, and results outside the normal FP64 range,
+// are multiplied entry by entry in FP64 by the reconstruction kernel.
 #include "rns.cuh"
 #include "launch.cuh"
 #include "mpo_stage.cuh"
@@ -184,28 +186,174 @@ __device__ __forceinline__ float2 reduce_mod2(float2 v, float p, float inv) {
 }
 
 __device__ __forceinline__ int biased_exp(double x) {
-  const long long b = __double_as_longlong(x);
-  const int E = (int)((b >> 52) & 0x7FF);
-  return E != 0 ? E : ((b << 1) != 0 ? 1 : 0);   // subnormals count as exponent 1
+  return (int)((__double_as_longlong(x) >> 52) & 0x7FF);
 }
 
-// rows whose products are formed in FP64 entry by entry: infinities, NaNs, numbers so
-// small that entries of the row or products may be subnormal
-constexpr int EXP_TINY = 200;
-__device__ __forceinline__ bool special(int E) { return E == 2047 || (E != 0 && E < EXP_TINY); }
+// ------------------------------------------------------------------ exponents
+// A component x != 0 has the exponent e with 2^(e - 1023) <= |x| < 2^(e - 1022), subnormal
+// ones below 1. Rows keep the largest e + s of their entries, s the scaling of the term, plus
+// EXP_BASE: positive, so that 0 can mean a row without entries.
+constexpr int EXP_BASE = 1 << 13;
+constexpr int EXP_SPECIAL = 1 << 20;   // the row holds an infinity or NaN: products in FP64
+constexpr int EXP_NONE = -(1 << 20);   // no entry
+constexpr int TERM_DROP = -(1 << 16);  // scaling of a term that meets zeros alone
 
-// ------------------------------------------------------------------ conversion
-// pieces of T = round(x 2^(bits - e)), |x| < 2^e = 2^(E - 1022), as signed floats
+__device__ __forceinline__ int entry_exp(double2 z) {
+  const int E = max(biased_exp(z.x), biased_exp(z.y));
+  const u64 x = (u64)__double_as_longlong(z.x), y = (u64)__double_as_longlong(z.y);
+  const u64 m = (x | y) & ((1ULL << 52) - 1);   // its top bit is that of the larger component
+  const int sub = m != 0 ? 12 - __clzll((long long)m) : EXP_NONE;
+  return E != 0 ? E : sub;
+}
+
+// an entry's part of its row's exponent
+__device__ __forceinline__ int row_exp(double2 z, int s) {
+  const int e = entry_exp(z);
+  return e == 2047 ? EXP_SPECIAL : max(e + s + EXP_BASE, 0);
+}
+
+// Largest finite exponent of every term of an operand (EXP_NONE: zeros); terms k = (o, i), i <
+// in, in > 1: f[o], the largest of its terms, and be[k] relative to it. A view whose rows are
+// next to each other: `wpt` warps take a term, or a CTA the terms of an o; otherwise (in = 1) a
+// lane takes a term and the warps of the CTA share its rows. Two operands in one launch. Bound:
+// memory (the operand read once), latency where it is small.
+struct TermJob {
+  RnsView v;
+  int rows, kc, in;
+  int *be, *f;
+  int wpt, ctas;
+};
+
+__global__ void __launch_bounds__(256) k_term_exp(const TermJob j0, const TermJob j1, const int* skip) {
+  grid_wait();
+  if (skip != nullptr && *skip != 0) return;
+  __shared__ int s_max[8][32];
+  const bool second = (int)blockIdx.x >= j0.ctas;
+  const TermJob j = second ? j1 : j0;
+  const int b = second ? (int)blockIdx.x - j0.ctas : (int)blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int m = EXP_NONE;
+  // entries first, first + step, ... < rows, `stride` apart: eight loads in flight
+  auto take = [&](const double2* src, long stride, int first, int step) {
+    for (int r = first; r < j.rows; r += 8 * step) {
+      double2 z[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        z[q] = r + q * step < j.rows ? src[(r + q * step) * stride] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const bool fx = biased_exp(z[q].x) != 2047, fy = biased_exp(z[q].y) != 2047;
+        m = max(m, entry_exp(make_double2(fx ? z[q].x : 0.0, fy ? z[q].y : 0.0)));
+      }
+    }
+  };
+  if (j.in > 1) {
+    __shared__ int s_be[RNS_INNER_MAX];
+    for (int i = warp; i < j.in; i += 8) {
+      const double2* src = j.v.src + ((long)b * j.in + i) * j.v.sk;
+      m = EXP_NONE;
+      take(src, 1, lane, 32);
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) s_be[i] = m;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      m = EXP_NONE;
+      for (int i = lane; i < j.in; i += 32) m = max(m, s_be[i]);
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) j.f[b] = m;
+      for (int i = lane; i < j.in; i += 32)
+        j.be[b * j.in + i] = s_be[i] != EXP_NONE ? s_be[i] - m : EXP_NONE;
+    }
+  } else if (j.wpt > 0) {
+    const int k = b * (8 / j.wpt) + warp / j.wpt;
+    if (k < j.kc) {
+      const double2* src = j.v.src + (long)k * j.v.sk;
+      take(src, 1, (warp % j.wpt) * 32 + lane, 32 * j.wpt);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) s_max[warp][0] = m;
+    __syncthreads();
+    if (lane == 0 && warp % j.wpt == 0 && k < j.kc) {
+      for (int w = 1; w < j.wpt; ++w) m = max(m, s_max[warp + w][0]);
+      j.be[k] = m;
+    }
+  } else {
+    const int k = b * 32 + lane;
+    if (k < j.kc) {
+      const double2* src = j.v.src + (long)k * j.v.sk;
+      take(src, j.v.sr, warp, 8);
+    }
+    s_max[warp][lane] = m;
+    __syncthreads();
+    if (warp == 0 && k < j.kc) {
+      for (int w = 1; w < 8; ++w) m = max(m, s_max[w][lane]);
+      j.be[k] = m;
+    }
+  }
+}
+
+// What a conversion does to the terms of its operand: nothing (t null), forms the scaling t
+// from be and f and applies its inverse (`source`, the operand that they were taken from), or
+// applies t (the other one).
+struct TermScale {
+  const int *be, *f;
+  int* t;
+  int in;
+  bool source;
+};
+
+// whole pairs of bits below the largest: terms of about the same size (a factor of four) stay
+// as they are
+__device__ __forceinline__ int in_pairs(int below) { return below & ~1; }
+
+// powers of two that the terms [k0, k0 + kn) of the operand take, to sh (shared memory, behind a
+// barrier of the caller's); the `writer` CTA of these terms leaves t for the other operand
+template <int NT>
+__device__ __forceinline__ void term_shifts(const TermScale& ts, int K, int k0, int kn, int* sh,
+                                            bool writer) {
+  if (!ts.source) {
+    for (int k = threadIdx.x; k < kn; k += NT) sh[k] = ts.t[k0 + k];
+    return;
+  }
+  __shared__ int s_top[NT / 32], s_g[RNS_INNER_MAX];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int no = K / ts.in;
+  const int* f = ts.in > 1 ? ts.f : ts.be;
+  int top = EXP_NONE;
+  for (int o = threadIdx.x; o < no; o += NT) top = max(top, f[o]);
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) s_top[warp] = top;
+  if (ts.in > 1)
+    for (int i = warp; i < ts.in; i += NT / 32) {
+      int g = EXP_NONE;
+      for (int o = lane; o < no; o += 32) g = max(g, ts.be[o * ts.in + i]);
+      g = __reduce_max_sync(0xffffffffu, g);
+      if (lane == 0) s_g[i] = g;
+    }
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < NT / 32; ++w) top = max(top, s_top[w]);
+  for (int q = threadIdx.x; q < kn; q += NT) {
+    const int k = k0 + q, o = k / ts.in;
+    const int t = ts.be[k] == EXP_NONE ? TERM_DROP
+                  : -in_pairs(top - f[o]) - (ts.in > 1 ? in_pairs(-s_g[k - o * ts.in]) : 0);
+    sh[q] = -t;
+    if (writer) ts.t[k] = t;
+  }
+}
+
+// pieces of T = round(x 2^(bits - e)), |x| < 2^e, e = E - 1022, as signed floats (0 where x is
+// too small for one bit)
 __device__ __forceinline__ void pieces_of(double x, int E, int bits, float (&f)[PIECES]) {
   const long long b = __double_as_longlong(x);
   const int Ex = (int)((b >> 52) & 0x7FF);
   u64 T = 0;
-  if (Ex != 0) {
-    const u64 mant = ((u64)b & ((1ULL << 52) - 1)) | (1ULL << 52);
-    const int rs = E - Ex + 53 - bits;
-    if (rs <= 0) T = mant << (-rs);
-    else if (rs < 55) T = (mant + (1ULL << (rs - 1))) >> rs;
-  }
+  const u64 frac = (u64)b & ((1ULL << 52) - 1);
+  const u64 mant = Ex != 0 ? frac | (1ULL << 52) : frac;
+  const int rs = E - max(Ex, 1) + 53 - bits;
+  if (rs > 0) T = rs < 55 ? (mant + (1ULL << (rs - 1))) >> rs : 0;
+  else if (mant != 0) T = mant << (-rs);
   const unsigned sign = (unsigned)((u64)b >> 32) & 0x80000000u;
 #pragma unroll
   for (int i = 0; i < PIECES; ++i) {
@@ -220,14 +368,14 @@ __device__ __forceinline__ void pieces_of(double x, int E, int bits, float (&f)[
 // modulus instead of 36: H_eff at bond 512, mixed, 360 -> 340 us with the GEMM's epilogue in
 // the same form).
 template <int NM>
-__device__ __forceinline__ void convert_pair(const double2 (&z)[2], int E, int bits,
+__device__ __forceinline__ void convert_pair(const double2 (&z)[2], const int (&E)[2], int bits,
                                              bf16* __restrict__ row, long plane) {
   constexpr RnsConst<NM> c = make_const<NM>();
   float px[2][PIECES], py[2][PIECES];
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
-    pieces_of(z[q].x, E, bits, px[q]);
-    pieces_of(z[q].y, E, bits, py[q]);
+    pieces_of(z[q].x, E[q], bits, px[q]);
+    pieces_of(z[q].y, E[q], bits, py[q]);
   }
   float2 x[PIECES], y[PIECES];
 #pragma unroll
@@ -251,6 +399,14 @@ __device__ __forceinline__ void convert_pair(const double2 (&z)[2], int E, int b
   }
 }
 
+// one entry to shared memory, asynchronously; zero (and no read) where `on` is false
+__device__ __forceinline__ void load_async(double2* dst, const double2* src, bool on) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(on ? 16 : 0)
+               : "memory");
+}
+
 // Residue planes of a view with any strides: a CTA takes 8 rows (128 contiguous bytes per
 // term of a transposed view) and part of the terms into shared memory; the CTAs of a
 // cluster share the rows' terms and exchange the row maxima, so the view is read once and
@@ -266,13 +422,15 @@ __global__ void __launch_bounds__(256) k_convert(const RnsView v, int R, int K, 
                                                  int* __restrict__ e, int have_exp, int bits,
                                                  bf16* __restrict__ dst, long Kp, long plane,
                                                  int* __restrict__ clear, int nclear,
-                                                 const int* skip) {
+                                                 const TermScale ts, const int* skip) {
   grid_wait();
   if (skip != nullptr && *skip != 0) return;   // uniform over the launch
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* tile = reinterpret_cast<double2*>(smem_raw);   // [CR][chunk + 1]
+  int* shift = reinterpret_cast<int*>(tile + CR * (chunk + 1));   // of the terms
   __shared__ int s_max[CR];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool scaled = NM == RNS_FP64 && ts.t != nullptr;
   const int r0 = blockIdx.x * CR, k0 = blockIdx.y * chunk, ld = chunk + 1;
   const int kn = min(chunk, K - k0);           // terms of this CTA (the last may have fewer)
   for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * 256 + tid; i < nclear;
@@ -282,13 +440,14 @@ __global__ void __launch_bounds__(256) k_convert(const RnsView v, int R, int K, 
   if (v.sk == 1) {
     const int r = r0 + warp;
     for (int k = lane; k < chunk; k += 32)
-      tile[warp * ld + k] = (r < R && k < kn) ? v.src[(long)r * v.sr + k0 + k] : make_double2(0.0, 0.0);
+      load_async(&tile[warp * ld + k], v.src + (long)r * v.sr + k0 + k, r < R && k < kn);
   } else {
     const int rr = tid & 7, r = r0 + rr;
     for (int k = tid >> 3; k < chunk; k += 32)
-      tile[rr * ld + k] = (r < R && k < kn) ? v.src[(long)r * v.sr + (long)(k0 + k) * v.sk]
-                                            : make_double2(0.0, 0.0);
+      load_async(&tile[rr * ld + k], v.src + (long)r * v.sr + (long)(k0 + k) * v.sk, r < R && k < kn);
   }
+  if (scaled) term_shifts<256>(ts, K, k0, kn, shift, blockIdx.x == 0);   // meanwhile
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   const double2* row = tile + warp * ld;
   const int r = r0 + warp;
@@ -297,7 +456,7 @@ __global__ void __launch_bounds__(256) k_convert(const RnsView v, int R, int K, 
     E = r < R ? e[r] : 0;
   } else {
     E = 0;
-    for (int k = lane; k < kn; k += 32) E = max(E, max(biased_exp(row[k].x), biased_exp(row[k].y)));
+    for (int k = lane; k < kn; k += 32) E = max(E, row_exp(row[k], scaled ? shift[k] : 0));
     E = __reduce_max_sync(0xffffffffu, E);
     if (gridDim.y > 1) {
       cg::cluster_group cluster = cg::this_cluster();
@@ -310,20 +469,23 @@ __global__ void __launch_bounds__(256) k_convert(const RnsView v, int R, int K, 
     if (lane == 0 && blockIdx.y == 0 && r < R) e[r] = E;
   }
   if (r >= R) return;
-  const bool live = E != 0 && !special(E);
+  const bool live = E != 0 && E != EXP_SPECIAL;
   const int kend = (int)min((long)chunk, Kp - k0);
   for (int k = 2 * lane; k < kend; k += 64) {
     double2 z[2];
+    int ez[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       z[q] = live ? row[k + q] : make_double2(0.0, 0.0);
       if (v.conj) z[q].y = -z[q].y;
+      ez[q] = E - EXP_BASE - (scaled && k + q < kn ? shift[k + q] : 0);
     }
-    convert_pair<NM>(z, E, bits, dst + (long)r * Kp + k0 + k, plane);
+    convert_pair<NM>(z, ez, bits, dst + (long)r * Kp + k0 + k, plane);
   }
 }
 
-// The exponents alone, for rows too long for a cluster (e zeroed before).
+// The exponents alone, for rows too long for a cluster (e zeroed before). Rows of the mixed
+// form alone are that long: no scaling of the terms.
 __global__ void __launch_bounds__(256) k_row_exp(const RnsView v, int R, int K, int* __restrict__ e,
                                                  const int* skip) {
   if (skip != nullptr && *skip != 0) return;
@@ -337,7 +499,7 @@ __global__ void __launch_bounds__(256) k_row_exp(const RnsView v, int R, int K, 
   if (r < R)
     for (long k = blockIdx.y * (long)CK_MAX + kk; k < min((long)K, (blockIdx.y + 1) * (long)CK_MAX); k += 32) {
       const double2 z = v.src[(long)r * v.sr + k * v.sk];
-      m = max(m, max(biased_exp(z.x), biased_exp(z.y)));
+      m = max(m, row_exp(z, 0));
     }
   atomicMax(&s_max[rr], m);
   __syncthreads();
@@ -355,30 +517,42 @@ __global__ void __launch_bounds__(128) k_convert_rows(const RnsView v, int R, in
                                                       int* __restrict__ e, int bits,
                                                       bf16* __restrict__ dst, long Kp, long plane,
                                                       int* __restrict__ clear, int nclear,
-                                                      const int* skip) {
+                                                      const TermScale ts, const int* skip) {
   grid_wait();
   if (skip != nullptr && *skip != 0) return;
+  __shared__ int shift[NM == RNS_FP64 ? ROW_MAX : 1];
+  const bool scaled = NM == RNS_FP64 && ts.t != nullptr;
+  if (scaled) {
+    term_shifts<128>(ts, K, 0, K, shift, blockIdx.x == 0);
+    __syncthreads();
+  }
   for (int i = blockIdx.x * 128 + threadIdx.x; i < nclear; i += gridDim.x * 128) clear[i] = 0;
   const int lane = threadIdx.x & 31;
   const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (r >= R) return;
   const double2* src = v.src + (long)r * v.sr;
   int E = 0;
-  for (int k = lane; k < K; k += 32) {
-    const double2 z = src[k];
-    E = max(E, max(biased_exp(z.x), biased_exp(z.y)));
+  for (int k0 = lane; k0 < K; k0 += 128) {   // four loads in flight
+    double2 z[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) z[q] = k0 + 32 * q < K ? src[k0 + 32 * q] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      E = max(E, row_exp(z[q], scaled && k0 + 32 * q < K ? shift[k0 + 32 * q] : 0));
   }
   E = __reduce_max_sync(0xffffffffu, E);
   if (lane == 0) e[r] = E;
-  const bool live = E != 0 && !special(E);
+  const bool live = E != 0 && E != EXP_SPECIAL;
   for (int k = 2 * lane; k < Kp; k += 64) {
     double2 z[2];
+    int ez[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       z[q] = (live && k + q < K) ? src[k + q] : make_double2(0.0, 0.0);
       if (v.conj) z[q].y = -z[q].y;
+      ez[q] = E - EXP_BASE - (scaled && k + q < K ? shift[k + q] : 0);
     }
-    convert_pair<NM>(z, E, bits, dst + (long)r * Kp + k, plane);
+    convert_pair<NM>(z, ez, bits, dst + (long)r * Kp + k, plane);
   }
 }
 
@@ -739,7 +913,7 @@ struct ReconP {
   const unsigned short* res;
   long ldr, rplane;
   const int *ea, *eb;
-  int sh0;                // -2 bits - 2 * 1022
+  int sh0;                // -2 bits - 2 (1022 + EXP_BASE)
   RnsView va, vb;
   const int* skip;
 };
@@ -805,7 +979,7 @@ __device__ __forceinline__ double2 element(const ReconP& g, int m, int n, int q,
   u64 xh = x1 + ((u64)x2 << 32), yh = y1 + ((u64)y2 << 32);
   xh -= c.off_x_hi + (xl < c.off_x_lo ? 1ULL : 0ULL);
   yh -= c.off_y_hi + (yl < c.off_y_lo ? 1ULL : 0ULL);
-  bool ok = !special(Ea) && !special(Eb);
+  bool ok = Ea != EXP_SPECIAL && Eb != EXP_SPECIAL;
   double2 z = make_double2(0.0, 0.0);
   if (ok && Ea != 0 && Eb != 0) {
     const int sh = Ea + Eb + g.sh0;
@@ -859,7 +1033,7 @@ __global__ void __launch_bounds__(256) k_reconstruct(const ReconP g, double2 alp
 // ((x, p / pin), (p % pin, y)) is stage input (x, p, y), put together straight into the
 // shared-memory rows of the stage; the stage output goes to `out` and the exponents of the
 // rows it forms as the next operand to e2 (zeroed before). by_x false: rows (q % eq, y);
-// true: rows (x, q / eq). One CTA per (x, 128-wide y chunk), of STAGE_Y threads, or twice as
+// true: rows (x, q / eq). t2 (or null): the scaling of that operand's terms. One CTA per (x, 128-wide y chunk), of STAGE_Y threads, or twice as
 // many where the CTAs alone leave too few warps in flight for the chain of loads and wide
 // integer sums. Saves writing and reading the product in FP64 and a maximum pass over the
 // stage output.
@@ -867,7 +1041,7 @@ template <int NM>
 __global__ void __launch_bounds__(2 * STAGE_Y)
     k_reconstruct_stage(const ReconP g, const double2* __restrict__ w, long ldq, long ldp, int P,
                         int pin, int Q, int Y, double2* __restrict__ out, int* __restrict__ e2,
-                        int eq, int by_x) {
+                        const int* __restrict__ t2, int eq, int by_x) {
   grid_wait();
   if (g.skip != nullptr && *g.skip != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -876,6 +1050,10 @@ __global__ void __launch_bounds__(2 * STAGE_Y)
   int* sidx = reinterpret_cast<int*>(sval + (size_t)P * Q);
   __shared__ int scount[STAGE_MAX];
   const int x = blockIdx.y, y0 = blockIdx.x * STAGE_Y, ty = threadIdx.x;
+  const int na = by_x ? Q / eq : eq, nb = by_x ? eq : Q / eq;
+  const bool scaled = NM == RNS_FP64 && t2 != nullptr;
+  __shared__ int s_t2[STAGE_MAX];
+  if (scaled && !by_x && ty < nb) s_t2[ty] = t2[(long)x * nb + ty];
   stage_load_w(w, ldq, ldp, P, Q, sval);
   const int pair = 2 * (ty & 63);
   for (int p = ty >> 6; p < P; p += blockDim.x / 64) {
@@ -898,7 +1076,6 @@ __global__ void __launch_bounds__(2 * STAGE_Y)
   stage_compact(P, Q, sval, sidx, scount);
   __syncthreads();
   const int yl = ty & (STAGE_Y - 1), y = y0 + yl;
-  const int na = by_x ? Q / eq : eq, nb = by_x ? eq : Q / eq;
   for (int a = ty / STAGE_Y; a < na; a += blockDim.x / STAGE_Y) {
     int E = 0;
     if (y < Y)
@@ -906,7 +1083,7 @@ __global__ void __launch_bounds__(2 * STAGE_Y)
         const int q = by_x ? a * eq + b : b * eq + a;
         const double2 z = stage_row(q, P, sin + yl, sval, sidx, scount);
         out[((long)x * Q + q) * Y + y] = z;
-        E = max(E, max(biased_exp(z.x), biased_exp(z.y)));
+        E = max(E, row_exp(z, !scaled ? 0 : by_x ? t2[(long)b * Y + y] : s_t2[b]));
       }
     if (by_x) {
       E = __reduce_max_sync(0xffffffffu, E);
@@ -1063,12 +1240,13 @@ bool rns_wanted(long M, long N, long K) {
 
 template <int NM>
 static ptn_status launch_convert(const RnsView& v, const RnsOperand& d, bool have_exp, int bits,
-                                 int* clear, int nclear, const int* skip, cudaStream_t st) {
+                                 int* clear, int nclear, const TermScale& ts, const int* skip,
+                                 cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [] {
     attr = cudaFuncSetAttribute(k_convert<NM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                CR * (CK_MAX + 1) * (int)sizeof(double2));
+                                CR * (CK_MAX + 1) * (int)sizeof(double2) + CK_MAX * (int)sizeof(int));
   });
   PTN_CUDA_TRY(attr);
   // terms per CTA, multiples of 64: enough CTAs for the chip, and at most 256 terms (33 KB, six
@@ -1084,42 +1262,71 @@ static ptn_status launch_convert(const RnsView& v, const RnsOperand& d, bool hav
     PTN_CUDA_TRY(cudaMemsetAsync(d.e, 0, (size_t)d.rows * sizeof(int), st));
     const dim3 ge((unsigned)groups, (unsigned)((d.kc + CK_MAX - 1) / CK_MAX));
     PTN_CHECK_ARG(ge.y <= 65535, "rns_convert: too many columns");
+    PTN_CHECK_ARG(ts.t == nullptr, "rns_convert: rows too long for scaled terms");
     k_row_exp<<<ge, 256, 0, st>>>(v, d.rows, d.kc, d.e, skip);
     PTN_LAUNCH_CHECK();
     note_launches(1);
-    return launch_convert<NM>(v, d, true, bits, clear, nclear, skip, st);
+    return launch_convert<NM>(v, d, true, bits, clear, nclear, ts, skip, st);
   }
   PTN_CHECK_ARG(parts <= 65535, "rns_convert: too many columns");
   LaunchShape shape{dim3((unsigned)groups, (unsigned)parts), dim3(256),
-                    CR * (size_t)(chunk + 1) * sizeof(double2)};
+                    CR * (size_t)(chunk + 1) * sizeof(double2) + chunk * sizeof(int)};
   if (!have_exp) shape.cluster = dim3(1, (unsigned)parts, 1);
   PTN_CUDA_TRY(launch_shape(k_convert<NM>, shape, st, v, d.rows, d.kc, (int)chunk, d.e,
-                            have_exp ? 1 : 0, bits, d.p, d.Kp, d.plane(), clear, nclear, skip));
+                            have_exp ? 1 : 0, bits, d.p, d.Kp, d.plane(), clear, nclear, ts, skip));
   note_launches(1);
   return PTN_OK;
 }
 
 template <int NM>
 static ptn_status convert(const RnsView& v, const RnsOperand& d, bool have_exp, int bits,
-                          int* clear, int nclear, const int* skip, cudaStream_t st) {
+                          int* clear, int nclear, const TermScale& ts, const int* skip,
+                          cudaStream_t st) {
   if (v.sk != 1 || have_exp || d.kc > ROW_MAX)
-    return launch_convert<NM>(v, d, have_exp, bits, clear, nclear, skip, st);
+    return launch_convert<NM>(v, d, have_exp, bits, clear, nclear, ts, skip, st);
   PTN_CUDA_TRY(launch(k_convert_rows<NM>, dim3((d.rows + 3) / 4), dim3(128), 0, st, v, d.rows,
-      d.kc, d.e, bits, d.p, d.Kp, d.plane(), clear, nclear, skip));
+      d.kc, d.e, bits, d.p, d.Kp, d.plane(), clear, nclear, ts, skip));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;
 }
 
 ptn_status rns_convert(const RnsView& v, const RnsOperand& d, bool have_exp, const int* skip,
-                       cudaStream_t st, int* clear, int nclear) {
+                       cudaStream_t st, int* clear, int nclear, const RnsTerms* terms, bool source) {
   const int bits = rns_bits(d.kc, d.nm);
   PTN_CHECK_ARG(bits != 0, "rns_convert: products of %d terms are too long", d.kc);
+  TermScale ts{};
+  if (terms != nullptr) ts = TermScale{terms->be, terms->f, terms->t, terms->in, source};
   switch (d.nm) {
-    case RNS_FP64: return convert<RNS_FP64>(v, d, have_exp, bits, clear, nclear, skip, st);
-    case RNS_MIXED_ENV: return convert<RNS_MIXED_ENV>(v, d, have_exp, bits, clear, nclear, skip, st);
-    default: return convert<RNS_MIXED>(v, d, have_exp, bits, clear, nclear, skip, st);
+    case RNS_FP64: return convert<RNS_FP64>(v, d, have_exp, bits, clear, nclear, ts, skip, st);
+    case RNS_MIXED_ENV:
+      return convert<RNS_MIXED_ENV>(v, d, have_exp, bits, clear, nclear, ts, skip, st);
+    default: return convert<RNS_MIXED>(v, d, have_exp, bits, clear, nclear, ts, skip, st);
   }
+}
+
+ptn_status rns_term_exps(const RnsTermsOf* of, int n, const int* skip, cudaStream_t st) {
+  TermJob j[2] = {};
+  int ctas = 0;
+  for (int i = 0; i < n; ++i) {
+    j[i].v = of[i].v;
+    j[i].rows = of[i].rows;
+    j[i].kc = of[i].kc;
+    j[i].be = of[i].terms->be;
+    j[i].f = of[i].terms->f;
+    j[i].in = of[i].terms->in;
+    PTN_CHECK_ARG(j[i].in == 1 || (of[i].v.sr == 1 && of[i].kc % j[i].in == 0),
+                  "rns_term_exps: bad layout");
+    // warps of a term: up to four rows per lane
+    j[i].wpt = of[i].v.sr != 1 ? 0 : of[i].rows <= 128 ? 1 : of[i].rows <= 256 ? 2
+                                   : of[i].rows <= 512 ? 4 : 8;
+    const int per = j[i].in > 1 ? j[i].in : j[i].wpt == 0 ? 32 : 8 / j[i].wpt;
+    j[i].ctas = (of[i].kc + per - 1) / per;
+    ctas += j[i].ctas;
+  }
+  PTN_CUDA_TRY(launch(k_term_exp, dim3(ctas), dim3(256), 0, st, j[0], j[1], skip));
+  note_launches(1);
+  return PTN_OK;
 }
 
 // the integer products of all planes -> res, and what their reconstruction needs
@@ -1159,7 +1366,7 @@ static ptn_status multiply(const RnsOperand& A, const RnsView& va, const RnsOper
   r->rplane = g.rplane;
   r->ea = A.e;
   r->eb = B.e;
-  r->sh0 = -2 * bits - 2 * 1022;
+  r->sh0 = -2 * bits - 2 * (1022 + EXP_BASE);
   r->va = va;
   r->vb = vb;
   r->skip = skip;
@@ -1196,7 +1403,7 @@ static ptn_status launch_stage(const ReconP& r, const RnsStage& s, cudaStream_t 
   // an environment step 2.09 -> 2.16 ms
   const int threads = (long)grid.x * grid.y < 16L * num_sms() ? 2 * STAGE_Y : STAGE_Y;
   PTN_CUDA_TRY(launch(k_reconstruct_stage<NM>, dim3(grid), dim3(threads), stage_smem(s.P, s.Q), st,
-      r, s.w, s.ldq, s.ldp, s.P, s.pin, s.Q, s.Y, s.out, s.e2, s.eq, s.by_x ? 1 : 0));
+      r, s.w, s.ldq, s.ldp, s.P, s.pin, s.Q, s.Y, s.out, s.e2, s.t2, s.eq, s.by_x ? 1 : 0));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;

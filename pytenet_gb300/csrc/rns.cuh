@@ -24,8 +24,8 @@ struct RnsView {
 };
 
 // a complex operand with `rows` rows and kc columns as 2 * nm residue planes
-// [plane][rows][Kp] (BF16, Kp a multiple of 8), and the biased exponent of the largest
-// component of every row (0: no non-zero entry)
+// [plane][rows][Kp] (BF16, Kp a multiple of 8), and the exponent of the largest component of
+// every row (as rns.cu keeps it; 0: no non-zero entry)
 struct RnsOperand {
   __nv_bfloat16* p;
   int* e;
@@ -33,6 +33,35 @@ struct RnsOperand {
   long Kp;
   long plane() const { return (long)rows * Kp; }
 };
+
+// Powers of two on the terms of a product (FP64 form): A[m, k] 2^t[k] and B[n, k] 2^-t[k] have
+// the same product. Rows are fixed-point numbers, so operands that grow and decay against each
+// other along k (the two sides of a bond in a gauge A D, D^-1 B) would lose the bits of the
+// entries that count. With t from the largest entry of B in every term, B is of one size along
+// k; the error of a result (m, n) is then 2^-bits per term of the largest |A[m, k] B[n', k]| over
+// k and n', and further down by what B's row n lies below the others: scalings of the terms, of
+// the rows of A and of those of B cancel. Terms k = (o, i) of a bond o and an MPO bond i < in
+// take t = f[o] + g[i]: in a channel as sparse as the identity a term of its own size says
+// nothing about its bond. Relative error (Frobenius norm, scalings taken out) of A D times
+// D^-1 R D^-1 at bond 64, |D| spread over 1e6 / 1e12: 1.0e-11 / 7.2e-6 without, 3.3e-16 / 3.5e-16
+// with it (DMMA 2.7e-16 / 3.0e-16). The exponents are a launch of their own: H_eff at bonds
+// 250 x 256 110 -> 116 us, an environment step at 187 x 300 85.0 -> 88.7, at bonds of 1024 1 %.
+// be, f: exponents of the terms of the operand that t comes from. Null t: no scaling.
+constexpr int RNS_INNER_MAX = 64;
+struct RnsTerms {
+  int *be, *f, *t;
+  int in;
+};
+
+// an operand whose terms' exponents are wanted
+struct RnsTermsOf {
+  RnsView v;
+  int rows, kc;
+  const RnsTerms* terms;
+};
+
+// of one or two operands, one launch
+ptn_status rns_term_exps(const RnsTermsOf* of, int n, const int* skip, cudaStream_t st);
 
 // bytes of the planes / exponents / GEMM residues, each to be 256-byte aligned
 size_t rns_plane_bytes(long rows, long kc, int nm);
@@ -47,12 +76,14 @@ int rns_bits(long K, int nm);
 bool rns_wanted(long M, long N, long K);
 
 // view -> residue planes for products over all kc terms. `have_exp`: the row exponents are
-// in d.e already (from rns_gemm_stage). Also zeroes clear[0 .. nclear).
+// in d.e already (from rns_gemm_stage). Also zeroes clear[0 .. nclear). `source`: the operand
+// that terms->be was taken from, which also forms terms->t (before the other one reads it).
 ptn_status rns_convert(const RnsView& v, const RnsOperand& d, bool have_exp, const int* skip,
-                       cudaStream_t st, int* clear = nullptr, int nclear = 0);
+                       cudaStream_t st, int* clear = nullptr, int nclear = 0,
+                       const RnsTerms* terms = nullptr, bool source = false);
 
 // out[m * ldc + n] = alpha sum_k A[m, k] B[n, k] + beta out[m * ldc + n]; va / vb are the
-// views the operands came from (rows with infinities, NaNs or numbers near the ends of the
+// views the operands came from (rows with infinities or NaNs and results outside the normal
 // FP64 range are multiplied from them directly), res the residue buffer
 ptn_status rns_gemm(const RnsOperand& A, const RnsView& va, const RnsOperand& B, const RnsView& vb,
                     double2 alpha, double2 beta, double2* out, long ldc, void* res,
@@ -60,13 +91,15 @@ ptn_status rns_gemm(const RnsOperand& A, const RnsView& va, const RnsOperand& B,
 
 // MPO stage on a product: out[x, q, y] = sum_p W[q, p] in[x, p, y] (W at w[q * ldq + p * ldp]),
 // in[x, p, y] = element ((x, p / pin), (p % pin, y)) of the product. e2 (zeroed before) takes
-// the row exponents of the output as an operand with rows (q % eq, y), or (x, q / eq) if by_x.
+// the row exponents of the output as an operand with rows (q % eq, y), or (x, q / eq) if by_x,
+// under the scaling t2 of its terms (x, q / eq), or (q % eq, y) (null: none).
 struct RnsStage {
   const double2* w;
   long ldq, ldp;
   int X, P, pin, Q, Y;
   double2* out;
   int* e2;
+  const int* t2;
   int eq;
   bool by_x;
 };

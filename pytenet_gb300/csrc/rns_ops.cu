@@ -4,7 +4,8 @@
 //
 // Data flow of H_eff . x (site tensors (Dl, d, Dr), MPO bonds cl / cr); an operand is a set
 // of residue planes, rows x terms:
-//   prepare (once per local step):  R -> rows (wr, r2), terms r0;  L -> rows l2, terms (l0, wl)
+//   prepare (once per local step):  R -> rows (wr, r2), terms r0;  L -> rows l2, terms (l0, wl);
+//           in the FP64 form the scaling of both GEMMs' terms comes from them (RnsTerms)
 //   apply:  x -> rows (l0, t), terms r0
 //           GEMM 1 T1[(l0,t)][(wr,r2)], reconstructed inside the MPO stage, which writes
 //           T2[l0,(wl,s),r2] in FP64 with the exponents of its rows as the next operand
@@ -38,6 +39,16 @@ struct Carver {
     void* e = take((size_t)rows * sizeof(int));
     return rns_operand(p, e, rows, kc, nm);
   }
+  // kc = outer * inner terms
+  RnsTerms terms(long outer, int inner, int nm) {
+    RnsTerms t{nullptr, nullptr, nullptr, 1};
+    if (nm != RNS_FP64) return t;
+    if (inner <= RNS_INNER_MAX) t.in = inner;
+    t.be = static_cast<int*>(take((size_t)outer * inner * sizeof(int)));
+    t.f = static_cast<int*>(take((size_t)outer * sizeof(int)));
+    t.t = static_cast<int*>(take((size_t)outer * inner * sizeof(int)));
+    return t;
+  }
 };
 
 #define RNS_CHECK_WS(layout)                                                     \
@@ -49,6 +60,7 @@ struct Carver {
 
 struct HeffWs {
   RnsOperand r, l, x, t2;
+  RnsTerms tr, tl;        // from R and L
   double2* T2;
   void* res;
 };
@@ -59,6 +71,8 @@ HeffWs heff_ws(Carver& c, int nm, int Dl, int d, int Dr, int cl, int cr) {
   w.l = c.operand(Dl, (long)Dl * cl, nm);
   w.x = c.operand((long)Dl * d, Dr, nm);
   w.t2 = c.operand((long)d * Dr, (long)Dl * cl, nm);
+  w.tr = c.terms(Dr, 1, nm);
+  w.tl = c.terms(Dl, cl, nm);
   w.T2 = static_cast<double2*>(c.take((size_t)Dl * cl * d * Dr * sizeof(double2)));
   w.res = c.take(std::max(rns_out_bytes((long)Dl * d, (long)cr * Dr, nm),
                           rns_out_bytes(Dl, (long)d * Dr, nm)));
@@ -67,6 +81,7 @@ HeffWs heff_ws(Carver& c, int nm, int Dl, int d, int Dr, int cl, int cr) {
 
 struct BondWs {
   RnsOperand r, l, x, t1;
+  RnsTerms tr, tl;
   double2* T1;
   void* res;
 };
@@ -77,6 +92,8 @@ BondWs bond_ws(Carver& c, int nm, int Dl, int Dr, int chi) {
   w.l = c.operand(Dl, (long)Dl * chi, nm);
   w.x = c.operand(Dl, Dr, nm);
   w.t1 = c.operand(Dr, (long)Dl * chi, nm);
+  w.tr = c.terms(Dr, 1, nm);
+  w.tl = c.terms(Dl, chi, nm);
   w.T1 = static_cast<double2*>(c.take((size_t)Dl * chi * Dr * sizeof(double2)));
   w.res = c.take(std::max(rns_out_bytes(Dl, (long)chi * Dr, nm), rns_out_bytes(Dl, Dr, nm)));
   return w;
@@ -85,6 +102,7 @@ BondWs bond_ws(Carver& c, int nm, int Dl, int Dr, int chi) {
 // a1 b1: first GEMM, a2 b2: second one
 struct EnvWs {
   RnsOperand a1, b1, a2, b2;
+  RnsTerms t1, t2;        // scaling of their terms, from the site tensors
   double2* T2;
   void* res;
 };
@@ -95,6 +113,8 @@ EnvWs env_left_ws(Carver& c, int nm, int Dl, int d, int Dr, int cl, int cr) {
   w.b1 = c.operand((long)d * Dr, Dl, nm);              // conj(B), rows (t, rb), terms l2
   w.a2 = c.operand(Dr, (long)Dl * d, nm);              // A, rows ra, terms (l0, s)
   w.b2 = c.operand((long)cr * Dr, (long)Dl * d, nm);   // T2, rows (wr, rb), terms (l0, s)
+  w.t1 = c.terms(Dl, 1, nm);
+  w.t2 = c.terms((long)Dl * d, 1, nm);
   w.T2 = static_cast<double2*>(c.take((size_t)Dl * d * cr * Dr * sizeof(double2)));
   w.res = c.take(std::max(rns_out_bytes((long)Dl * cl, (long)d * Dr, nm),
                           rns_out_bytes(Dr, (long)cr * Dr, nm)));
@@ -107,10 +127,20 @@ EnvWs env_right_ws(Carver& c, int nm, int Dl, int d, int Dr, int cl, int cr) {
   w.b1 = c.operand((long)cr * Dr, Dr, nm);             // R, rows (wr, r2), terms r0
   w.a2 = c.operand((long)Dl * cl, (long)d * Dr, nm);   // T2, rows (l0, wl), terms (t, r2)
   w.b2 = c.operand(Dl, (long)d * Dr, nm);              // conj(B), rows lb, terms (t, r2)
+  w.t1 = c.terms(Dr, 1, nm);
+  w.t2 = c.terms((long)d * Dr, 1, nm);
   w.T2 = static_cast<double2*>(c.take((size_t)Dl * cl * d * Dr * sizeof(double2)));
   w.res = c.take(std::max(rns_out_bytes((long)Dl * d, (long)cr * Dr, nm),
                           rns_out_bytes((long)Dl * cl, Dl, nm)));
   return w;
+}
+
+// exponents of the terms of the two operands that the scalings come from
+ptn_status term_exps(const RnsView& v1, const RnsOperand& o1, const RnsTerms& t1, const RnsView& v2,
+                     const RnsOperand& o2, const RnsTerms& t2, cudaStream_t st) {
+  if (t1.t == nullptr) return PTN_OK;
+  const RnsTermsOf of[2] = {{v1, o1.rows, o1.kc, &t1}, {v2, o2.rows, o2.kc, &t2}};
+  return rns_term_exps(of, 2, nullptr, st);
 }
 
 }  // namespace
@@ -131,8 +161,10 @@ ptn_status heff_prepare_rns(int nm, const double2* l, const double2* r, int Dl, 
   RNS_CHECK_WS(layout);
   Carver c(ws);
   const HeffWs h = layout(c);
-  PTN_TRY(rns_convert(view_r(r, Dr, cr), h.r, false, nullptr, st));
-  return rns_convert(view_l(l, Dl), h.l, false, nullptr, st);
+  const RnsView vr = view_r(r, Dr, cr), vl = view_l(l, Dl);
+  PTN_TRY(term_exps(vr, h.r, h.tr, vl, h.l, h.tl, st));
+  PTN_TRY(rns_convert(vr, h.r, false, nullptr, st, nullptr, 0, &h.tr, true));
+  return rns_convert(vl, h.l, false, nullptr, st, nullptr, 0, &h.tl, true);
 }
 
 ptn_status heff_apply_rns(int nm, const double2* x, double2* y, const double2* w, const double2* l,
@@ -141,11 +173,12 @@ ptn_status heff_apply_rns(int nm, const double2* x, double2* y, const double2* w
   Carver c(ws);
   const HeffWs h = heff_ws(c, nm, Dl, d, Dr, cl, cr);
   const RnsView vx{x, Dr, 1, 0}, vt{h.T2, 1, (long)d * Dr, 0};
-  PTN_TRY(rns_convert(vx, h.x, false, skip, st, h.t2.e, h.t2.rows));
+  PTN_TRY(rns_convert(vx, h.x, false, skip, st, h.t2.e, h.t2.rows, &h.tr));
   // T2[l0,(wl,s),r2] = sum_(t,wr) W[(wl,s),(t,wr)] T1[l0,(t,wr),r2]
-  const RnsStage s{w, (long)d * cr, 1, Dl, d * cr, cr, cl * d, Dr, h.T2, h.t2.e, d, false};
+  const RnsStage s{w, (long)d * cr, 1, Dl, d * cr, cr, cl * d, Dr, h.T2, h.t2.e, h.tl.t, d,
+                   false};
   PTN_TRY(rns_gemm_stage(h.x, vx, h.r, view_r(r, Dr, cr), s, h.res, skip, st));
-  PTN_TRY(rns_convert(vt, h.t2, true, skip, st));
+  PTN_TRY(rns_convert(vt, h.t2, true, skip, st, nullptr, 0, &h.tl));
   return rns_gemm(h.l, view_l(l, Dl), h.t2, vt, ONE, ZERO, y, (long)d * Dr, h.res, skip, st);
 }
 
@@ -162,8 +195,10 @@ ptn_status bond_prepare_rns(int nm, const double2* l, const double2* r, int Dl, 
   RNS_CHECK_WS(layout);
   Carver c(ws);
   const BondWs b = layout(c);
-  PTN_TRY(rns_convert(view_r(r, Dr, chi), b.r, false, nullptr, st));
-  return rns_convert(view_l(l, Dl), b.l, false, nullptr, st);
+  const RnsView vr = view_r(r, Dr, chi), vl = view_l(l, Dl);
+  PTN_TRY(term_exps(vr, b.r, b.tr, vl, b.l, b.tl, st));
+  PTN_TRY(rns_convert(vr, b.r, false, nullptr, st, nullptr, 0, &b.tr, true));
+  return rns_convert(vl, b.l, false, nullptr, st, nullptr, 0, &b.tl, true);
 }
 
 ptn_status bond_apply_rns(int nm, const double2* x, double2* y, const double2* l, const double2* r,
@@ -171,12 +206,12 @@ ptn_status bond_apply_rns(int nm, const double2* x, double2* y, const double2* l
   Carver c(ws);
   const BondWs b = bond_ws(c, nm, Dl, Dr, chi);
   const RnsView vx{x, Dr, 1, 0}, vt{b.T1, 1, Dr, 0};
-  PTN_TRY(rns_convert(vx, b.x, false, skip, st));
+  PTN_TRY(rns_convert(vx, b.x, false, skip, st, nullptr, 0, &b.tr));
   // T1[l0][(w, r2)]
   PTN_TRY(rns_gemm(b.x, vx, b.r, view_r(r, Dr, chi), ONE, ZERO, b.T1, (long)chi * Dr, b.res, skip,
                    st));
   // rows r2, terms (l0, w)
-  PTN_TRY(rns_convert(vt, b.t1, false, skip, st));
+  PTN_TRY(rns_convert(vt, b.t1, false, skip, st, nullptr, 0, &b.tl));
   return rns_gemm(b.l, view_l(l, Dl), b.t1, vt, ONE, ZERO, y, Dr, b.res, skip, st);
 }
 
@@ -198,13 +233,15 @@ ptn_status env_left_rns(int nm, const double2* a, const double2* b, const double
   const EnvWs e = layout(c);
   const RnsView v1{l, Dl, 1, 0}, v2{b, 1, (long)d * Dr, 1}, v3{a, 1, Dr, 0},
       v4{e.T2, 1, (long)cr * Dr, 0};
-  PTN_TRY(rns_convert(v1, e.a1, false, nullptr, st, e.b2.e, e.b2.rows));
-  PTN_TRY(rns_convert(v2, e.b1, false, nullptr, st));
-  PTN_TRY(rns_convert(v3, e.a2, false, nullptr, st));
+  PTN_TRY(term_exps(v2, e.b1, e.t1, v3, e.a2, e.t2, st));
+  PTN_TRY(rns_convert(v2, e.b1, false, nullptr, st, e.b2.e, e.b2.rows, &e.t1, true));
+  PTN_TRY(rns_convert(v1, e.a1, false, nullptr, st, nullptr, 0, &e.t1));
+  PTN_TRY(rns_convert(v3, e.a2, false, nullptr, st, nullptr, 0, &e.t2, true));
   // T2[l0,(s,wr),rb] = sum_(wl,t) W[wl,t,s,wr] T1[l0,(wl,t),rb]   (stage matrix W^T)
-  const RnsStage s{w, 1, (long)d * cr, Dl, cl * d, d, d * cr, Dr, e.T2, e.b2.e, cr, false};
+  const RnsStage s{w, 1, (long)d * cr, Dl, cl * d, d, d * cr, Dr, e.T2, e.b2.e, e.t2.t, cr,
+                   false};
   PTN_TRY(rns_gemm_stage(e.a1, v1, e.b1, v2, s, e.res, nullptr, st));
-  PTN_TRY(rns_convert(v4, e.b2, true, nullptr, st));
+  PTN_TRY(rns_convert(v4, e.b2, true, nullptr, st, nullptr, 0, &e.t2));
   return rns_gemm(e.a2, v3, e.b2, v4, ONE, ZERO, lnext, (long)cr * Dr, e.res, nullptr, st);
 }
 
@@ -218,13 +255,15 @@ ptn_status env_right_rns(int nm, const double2* a, const double2* b, const doubl
   const EnvWs e = layout(c);
   const RnsView v1{a, Dr, 1, 0}, v2 = view_r(r, Dr, cr), v3{e.T2, (long)d * Dr, 1, 0},
       v4{b, (long)d * Dr, 1, 1};
-  PTN_TRY(rns_convert(v1, e.a1, false, nullptr, st, e.a2.e, e.a2.rows));
-  PTN_TRY(rns_convert(v2, e.b1, false, nullptr, st));
-  PTN_TRY(rns_convert(v4, e.b2, false, nullptr, st));
+  PTN_TRY(term_exps(v1, e.a1, e.t1, v4, e.b2, e.t2, st));
+  PTN_TRY(rns_convert(v1, e.a1, false, nullptr, st, e.a2.e, e.a2.rows, &e.t1, true));
+  PTN_TRY(rns_convert(v2, e.b1, false, nullptr, st, nullptr, 0, &e.t1));
+  PTN_TRY(rns_convert(v4, e.b2, false, nullptr, st, nullptr, 0, &e.t2, true));
   // T2[l0,(wl,t),r2] = sum_(s,wr) W[(wl,t),(s,wr)] T1[l0,(s,wr),r2]
-  const RnsStage s{w, (long)d * cr, 1, Dl, d * cr, cr, cl * d, Dr, e.T2, e.a2.e, d, true};
+  const RnsStage s{w, (long)d * cr, 1, Dl, d * cr, cr, cl * d, Dr, e.T2, e.a2.e, e.t2.t, d,
+                   true};
   PTN_TRY(rns_gemm_stage(e.a1, v1, e.b1, v2, s, e.res, nullptr, st));
-  PTN_TRY(rns_convert(v3, e.a2, true, nullptr, st));
+  PTN_TRY(rns_convert(v3, e.a2, true, nullptr, st, nullptr, 0, &e.t2));
   return rns_gemm(e.a2, v3, e.b2, v4, ONE, ZERO, rnext, Dl, e.res, nullptr, st);
 }
 
@@ -233,6 +272,7 @@ size_t zgemm_rns_workspace_bytes(int nm, long M, long N, long K) {
   Carver c(nullptr);
   c.operand(M, K, nm);
   c.operand(N, K, nm);
+  c.terms(K, 1, nm);
   c.take(rns_out_bytes(M, N, nm));
   return c.off + 256;
 }
@@ -241,14 +281,23 @@ ptn_status zgemm_rns(int nm, const GemmArgs& g, void* ws, cudaStream_t st) {
   Carver c(reinterpret_cast<void*>(al(reinterpret_cast<uintptr_t>(ws))));
   const RnsOperand A = c.operand(g.M, g.K, nm);
   const RnsOperand B = c.operand(g.N, g.K, nm);
+  const RnsTerms terms = c.terms(g.K, 1, nm);
   void* res = c.take(0);
   // op(A) by rows, op(B) by columns
   const bool ta = g.opA == 'T' || g.opA == 'H', tb = g.opB == 'T' || g.opB == 'H';
   const bool ca = g.opA == 'C' || g.opA == 'H', cb = g.opB == 'C' || g.opB == 'H';
   const RnsView va = ta ? RnsView{g.A, 1, g.lda, ca} : RnsView{g.A, g.lda, 1, ca};
   const RnsView vb = tb ? RnsView{g.B, g.ldb, 1, cb} : RnsView{g.B, 1, g.ldb, cb};
-  PTN_TRY(rns_convert(va, A, false, g.skip, st));
-  PTN_TRY(rns_convert(vb, B, false, g.skip, st));
+  // the scaling of the terms from the operand whose rows are next to each other, or that has
+  // fewer of them
+  const bool from_b = (va.sr == 1) != (vb.sr == 1) ? vb.sr == 1 : g.N <= g.M;
+  if (terms.t != nullptr) {
+    const RnsTermsOf of{from_b ? vb : va, from_b ? g.N : g.M, g.K, &terms};
+    PTN_TRY(rns_term_exps(&of, 1, g.skip, st));
+  }
+  if (from_b) PTN_TRY(rns_convert(vb, B, false, g.skip, st, nullptr, 0, &terms, true));
+  PTN_TRY(rns_convert(va, A, false, g.skip, st, nullptr, 0, &terms, !from_b));
+  if (!from_b) PTN_TRY(rns_convert(vb, B, false, g.skip, st, nullptr, 0, &terms));
   return rns_gemm(A, va, B, vb, g.alpha, g.beta, g.C, g.ldc, res, g.skip, st);
 }
 

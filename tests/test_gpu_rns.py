@@ -178,3 +178,106 @@ def test_smallest_products(mnk):
     A, B = crandn(rng, M, K), crandn(rng, K, N)
     err, tol = errors(zgemm(A, B), A, B, rng)
     assert np.all(err <= tol), (err / tol).max()
+
+
+def spread(rng, n, width):
+    """n factors between 1 / width and 1, both ends among them, in random order."""
+    s = 10.0 ** -(rng.uniform(0, 1, n) * np.log10(width))
+    s[rng.permutation(n)[:2]] = 1.0, 1.0 / width
+    return s
+
+
+# Operands that grow and decay against each other along the summed index: the products are of
+# one size, so FP64 has them to rounding. Tolerance: the form's 1e-12 per contraction, in the
+# norm without the scalings (rounding alone is below 1e-14 at these sizes).
+GAUGES = [1e3, 1e6, 1e9, 1e12]
+
+
+@pytest.mark.parametrize("width", GAUGES)
+@pytest.mark.parametrize("ops", ["NN", "TN", "NT", "HC"])
+@pytest.mark.parametrize("mnk", [(128, 130, 96), (40, 300, 700), (310, 36, 1100)])
+def test_products_of_opposite_scalings(mnk, ops, width):
+    """A D times D^-1 B, with rows of A and columns of B scaled too."""
+    M, N, K = mnk
+    rng = np.random.default_rng(M + K + int(np.log10(width)))
+    s, x, y = spread(rng, K, width), spread(rng, M, width), spread(rng, N, 1e3)
+    A = x[:, None] * crandn(rng, M, K) * s
+    B = crandn(rng, K, N) / s[:, None] * y
+    g = {"N": lambda z: z, "T": lambda z: z.T, "C": np.conj, "H": lambda z: z.conj().T}
+    got = zgemm(np.ascontiguousarray(g[ops[0]](A)), np.ascontiguousarray(g[ops[1]](B)), *ops)
+    rows, cols = rng.integers(0, M, 30), rng.integers(0, N, 30)
+    ref = exact(A, B, rows, cols)
+    free = x[rows][:, None] * y[cols][None, :]
+    err = np.linalg.norm(((got[np.ix_(rows, cols)] - ref) / free).astype(complex))
+    assert err < 1e-12 * np.linalg.norm((ref / free).astype(complex))
+
+
+@pytest.mark.parametrize("channel", ["dense", "identity"])
+@pytest.mark.parametrize("width", GAUGES)
+def test_contractions_in_a_scaled_gauge(width, channel):
+    """A site tensor in the gauge X a Y with the environments of that gauge: both products of
+    every contraction sum over an index that the two operands scale against each other."""
+    import pytenet_gb300 as ptg
+    Dl, d, Dr, cl, cr = 72, 2, 76, 3, 4
+    rng = np.random.default_rng(int(np.log10(width)))
+    x, y = spread(rng, Dl, width), spread(rng, Dr, width)
+    a, b = crandn(rng, Dl, d, Dr), crandn(rng, Dl, d, Dr)
+    w = rng.standard_normal((cl, d, d, cr)) + 0j
+    l, r, c = crandn(rng, Dl, cl, Dl), crandn(rng, Dr, cr, Dr), crandn(rng, Dl, Dr)
+    r2 = crandn(rng, Dr, cl, Dr)
+    if channel == "identity":
+        l[:, 0], r[:, 0], r2[:, 0] = np.eye(Dl), np.eye(Dr), np.eye(Dr)
+    # X a Y, X^-1 l X^-1, Y^-1 r Y^-1
+    up = lambda t: x[:, None, None] * t * y[None, None, :]
+    lx = l / (x[:, None, None] * x[None, None, :])
+    ry, ry2 = (t / (y[:, None, None] * y[None, None, :]) for t in (r, r2))
+    q = lambda t: t.astype(np.clongdouble)
+
+    def close(got, ref, free):
+        free = np.broadcast_to(free, got.shape)
+        err = np.linalg.norm(((got - ref) * free).astype(complex))
+        assert err < 1e-12 * np.linalg.norm((ref * free).astype(complex))
+
+    A, B, W, L, R = (q(t) for t in (up(a), up(b), w, lx, ry))
+    t1 = np.tensordot(A, R, ([2], [0]))                                  # l0 t wr r2
+    t2 = np.tensordot(W, t1, ([2, 3], [1, 2]))                           # wl s l0 r2
+    close(ptg.apply_local_hamiltonian(up(a), w, lx, ry), np.tensordot(L, t2, ([0, 1], [2, 0])),
+          x[:, None, None] * y[None, None, :])
+    cx = x[:, None] * c * y[None, :]
+    ref = np.tensordot(L, np.tensordot(q(cx), q(ry2), ([1], [0])), ([0, 1], [0, 1]))
+    close(ptg.apply_local_bond_contraction(cx, lx, ry2), ref, x[:, None] * y[None, :])
+    t = np.tensordot(L, B.conj(), ([2], [0]))                            # l0 wl t rb
+    t = np.tensordot(W, t, ([0, 1], [1, 2]))                             # s wr l0 rb
+    ref = np.tensordot(A, t, ([0, 1], [2, 0]))                           # ra wr rb
+    close(ptg.contraction_operator_step_left(up(a), up(b), w, lx), ref,
+          1 / (y[:, None, None] * y[None, None, :]))
+    t = np.tensordot(t1, W, ([1, 2], [2, 3]))                            # l0 r2 wl t
+    ref = np.tensordot(t, B.conj(), ([3, 1], [1, 2]))                    # la wl lb
+    close(ptg.contraction_operator_step_right(up(a), up(b), w, ry), ref,
+          1 / (x[:, None, None] * x[None, None, :]))
+
+
+def test_terms_that_meet_zeros_or_subnormals():
+    """Terms without entries in one operand drop out whatever the other one holds there (but
+    for infinities and NaNs), and subnormal entries count where their term is large."""
+    rng = np.random.default_rng(11)
+    M, N, K = 140, 150, 96
+    A, B = crandn(rng, M, K), crandn(rng, K, N)
+    B[5] = 0
+    A[:, 5] *= 1e200
+    A[:, 9] *= 2.0 ** -1050
+    B[9] *= 2.0 ** 1000
+    B[11] *= 2.0 ** -1060
+    A[:, 11] *= 2.0 ** 1010
+    got = zgemm(A, B)
+    keep = np.arange(K) != 5
+    err, tol = errors(got, np.delete(A, 5, 1) * 1.0, np.delete(B, 5, 0) * 1.0, rng)
+    # rows and columns without the scalings, as bounds of the terms
+    s = np.ones(K)
+    s[9], s[11] = 2.0 ** 1000, 2.0 ** -1010
+    As, Bs = (A * s)[:, keep], (B / s[:, None])[keep]
+    bound = 32 * K * 2.0 ** -53 * np.abs(As).max() * np.abs(Bs).max()
+    assert np.isfinite(got).all() and float(err.max()) < bound
+    A[3, 5] = np.inf
+    bad = zgemm(A, B)
+    assert not np.isfinite(bad[3]).any() and np.isfinite(np.delete(bad, 3, 0)).all()
