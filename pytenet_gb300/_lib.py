@@ -102,7 +102,9 @@ _SIGS = {
                       P]),
     "ptn_zgemm_split_bf16_workspace_bytes": (S, [I, I, I]),
     "ptn_zgemm_split_bf16": (I, [P, L, P, L, P, L, I, I, I, P, S, P]),
+    "ptn_device_error": (I, [P]),
     "ptn_tc_error": (I, []),
+    "ptn_device_error_inject": (I, [I, P]),
     "ptn_krylov_state_bytes": (S, []),
     "ptn_krylov_stop_flag": (P, [P]),
     "ptn_krylov_start": (I, [P, P, P, L, I, P]),

@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .device import call, empty, lib, ptr, stream_ptr, to_dev, to_host, Workspace
+from .device import call, empty, lib, ptr, stream_ptr, to_dev, to_host, to_host_all, Workspace
 from .qnumber import qr_plan, is_qsparse
 
 __all__ = ["RowMajor", "ColMajor", "Flip3", "qr_execute", "block_sparse_qr", "svd_execute",
@@ -206,7 +206,7 @@ def block_sparse_qr(a, q0, q1):
         _SCRATCH = QRScratch()
     qr_execute(plan, src, RowMajor(n), q, RowMajor(plan.K), r, RowMajor(n), _SCRATCH)
     if host:
-        return to_host(q), to_host(r), plan.qinterm.copy()
+        return (*to_host_all([q, r]), plan.qinterm.copy())
     return q, r, plan.qinterm.copy()
 
 
@@ -285,7 +285,7 @@ def block_sparse_svd(a, q0, q1):
     u, s, vh = svd_execute(plan, src, RowMajor(a.shape[1]), _svd_scratch())
     q = plan.qinterm.copy()
     if host:
-        return to_host(u), s.cpu().numpy(), to_host(vh), q
+        return (*to_host_all([u, s, vh]), q)
     return u, s, vh, q
 
 
@@ -297,7 +297,7 @@ def split_block_sparse_matrix_svd(a, q0, q1, tol):
     from .bond_ops import retained_bond_indices
     host = not isinstance(a, torch.Tensor)
     u, s, vh, q = block_sparse_svd(to_dev(a) if host else a, q0, q1)
-    s_host = s.cpu().numpy()
+    s_host = to_host(s)
     idx = retained_bond_indices(s_host, tol)
     u, vh = take_singular(u, vh, idx)
     s_keep = s_host[idx]

@@ -8,7 +8,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .device import Workspace, call, device, empty, lib, ptr, stream_ptr, to_dev, to_host
+from .device import Workspace, call, device, empty, lib, ptr, stream_ptr, to_dev, to_host, to_host_all, scalar
 
 __all__ = ["apply_local_hamiltonian", "apply_local_bond_contraction",
            "contraction_operator_step_left", "contraction_operator_step_right",
@@ -132,7 +132,7 @@ def mpo_inner_product(chi, op, psi):
     for i in reversed(range(len(A))):
         t = contraction_operator_step_right(to_dev(A[i]), to_dev(B[i]), to_dev(W[i]), t)
     assert tuple(t.shape) == (1, 1, 1)
-    return complex(t.reshape(-1)[0].item())
+    return complex(scalar(t))
 
 
 def mpo_average(psi, op):
@@ -169,7 +169,7 @@ def mps_vdot(chi, psi):
         _zgemm(b"N", b"H", Dl, El, d * Er, u, d * Er, b, d * Er, tn, El)
         t = tn
     assert tuple(t.shape) == (1, 1)
-    return complex(t.reshape(-1)[0].item())
+    return complex(scalar(t))
 
 
 def mps_norm(psi):
@@ -224,7 +224,7 @@ def apply_mpo(op, psi):
         ocols = (kc * Dl * Dr + kr).reshape(-1)
         t = gather(x, orows, ocols, cl * Dl * d, cr * Dr)
         tensors.append(t.view(cl * Dl, d, cr * Dr))
-    out.a = [to_host(t).copy() for t in tensors]
+    out.a = [t.copy() for t in to_host_all(tensors)]
     for i in range(n):
         assert is_qsparse(out.a[i], [out.qbonds[i], out.qsite, -out.qbonds[i + 1]]), \
             "sparsity pattern of MPS tensor does not match quantum numbers"

@@ -19,7 +19,7 @@ import torch
 from . import _lib
 from .block_sparse import RowMajor, svd_execute, take_singular, _svd_scratch
 from .bond_ops import retained_bond_indices
-from .device import Workspace, call, device, empty, lib, ptr, stream_ptr, to_dev, to_host
+from .device import Workspace, call, device, empty, lib, ptr, stream_ptr, to_dev, to_host, to_host_all
 from .qnumber import is_qsparse, qnumber_flatten, qr_plan
 
 __all__ = ["compress_svd", "compress_density"]
@@ -30,7 +30,7 @@ def _split(x, rows, cols, q0, q1, tol):
     u (rows x k), s (k, host and device), vh (k x cols), q (k,)."""
     plan = qr_plan(q0, q1)
     u, s, vh = svd_execute(plan, x, RowMajor(cols), _svd_scratch())
-    s_host = s.cpu().numpy()
+    s_host = to_host(s)
     idx = retained_bond_indices(s_host, tol)
     u, vh = take_singular(u, vh, idx)
     sk = s_host[idx]
@@ -106,7 +106,7 @@ def compress_svd(psi, tol, direction="left"):
                 t = complex(to_host(u).reshape(-1)[0])
                 call(L.ptn_scale, ptr(a[i]), ptr(a[i]), a[i].numel(), _lib.cval(t / abs(t)), st)
                 scale = abs(t)
-    psi.a = [to_host(x).copy() for x in a]
+    psi.a = [x.copy() for x in to_host_all(a)]
     psi.qbonds = qb
     return nrm, scale
 
@@ -175,7 +175,7 @@ def compress_density(psi, tol):
         plan = qr_plan(qr, qr)
         uu, s, vh = svd_execute(plan, rho, RowMajor(d * Ku), _svd_scratch())
         perm = _eigh_order(plan, qr)
-        ev = s.cpu().numpy()[perm]
+        ev = to_host(s)[perm]
         idx = retained_bond_indices(ev, tol)
         keep = perm[idx]
         k = len(keep)
@@ -195,6 +195,6 @@ def compress_density(psi, tol):
     s0 = float(torch.linalg.vector_norm(b3).item())
     call(L.ptn_scale, ptr(b3), ptr(b3), b3.numel(), _lib.cval(1.0 / s0), st)
     a[0] = b3
-    psi.a = [to_host(x).copy() for x in a]
+    psi.a = [x.copy() for x in to_host_all(a)]
     psi.qbonds = qb
     return nrm, s0 / nrm

@@ -4,6 +4,7 @@
 // the (2,1,0) transpose of the right-to-left sweep (pytenet/tdvp.py:95,104) and
 // scaling.
 #include "ptn_common.cuh"
+#include <mutex>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -187,9 +188,52 @@ ptn_status transpose210(const double2* in, double2* out, int n0, int n1, int n2,
 
 }  // namespace ptn
 
+namespace ptn {
+
+__device__ int g_device_err;
+
+int* device_error_word() {
+  static int* word = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* a = nullptr;
+    if (cudaGetSymbolAddress(&a, g_device_err) == cudaSuccess) word = static_cast<int*>(a);
+  });
+  return word;
+}
+
+}  // namespace ptn
+
 using namespace ptn;
 
 extern "C" {
+
+// The copies go to the given stream: nothing here touches the legacy stream, which a thread
+// that captures a graph forbids to all others.
+int ptn_device_error(void* stream) {
+  int* word = device_error_word();
+  int v = 0;
+  if (word == nullptr ||
+      cudaMemcpyAsync(&v, word, sizeof(int), cudaMemcpyDeviceToHost, as_stream(stream)) != cudaSuccess ||
+      cudaStreamSynchronize(as_stream(stream)) != cudaSuccess)
+    return -1;
+  if (v != 0 && (cudaMemsetAsync(word, 0, sizeof(int), as_stream(stream)) != cudaSuccess ||
+                 cudaStreamSynchronize(as_stream(stream)) != cudaSuccess))
+    return -1;
+  return v;
+}
+
+int ptn_tc_error(void) {
+  return cudaDeviceSynchronize() == cudaSuccess ? ptn_device_error(nullptr) : -1;
+}
+
+ptn_status ptn_device_error_inject(int code, void* stream) {
+  int* word = device_error_word();
+  PTN_CHECK_ARG(word != nullptr, "device_error_inject: error word lookup failed");
+  PTN_CUDA_TRY(cudaMemcpyAsync(word, &code, sizeof(int), cudaMemcpyHostToDevice, as_stream(stream)));
+  PTN_CUDA_TRY(cudaStreamSynchronize(as_stream(stream)));
+  return PTN_OK;
+}
 
 int ptn_abi_version(void) { return PTN_ABI_VERSION; }
 const char* ptn_version(void) { return "pytenet_gb300 0.1 (sm_103a)"; }

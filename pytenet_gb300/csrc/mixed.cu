@@ -18,7 +18,6 @@
 namespace ptn {
 
 void note_launches(int n);
-int rns_error_and_reset();
 ptn_status tc_gemm(const void* Aslices, long aplane, const int* ea, const void* Bslices, long bplane,
                    const int* eb, int M, int Nc, int Kc, long Kp, double2* out, long ldm, long ldn,
                    bool accumulate, void* ws, size_t ws_bytes, const int* skip, cudaStream_t st,
@@ -270,13 +269,6 @@ ptn_status ptn_zgemm_split_bf16(const ptn_c128* A, long lda, const ptn_c128* B, 
   return ptn::zgemm_split(reinterpret_cast<const double2*>(A), lda,
                           reinterpret_cast<const double2*>(B), ldb, reinterpret_cast<double2*>(C),
                           ldc, M, N, K, ws, ws_bytes, ptn::as_stream(stream));
-}
-
-int ptn_tc_error(void) {
-  extern int tc_gemm_error_and_reset_c(void);
-  const int e = tc_gemm_error_and_reset_c();
-  const int r = ptn::rns_error_and_reset();
-  return e != 0 ? e : r;
 }
 
 }  // extern "C"

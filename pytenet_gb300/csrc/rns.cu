@@ -688,7 +688,8 @@ struct GemmP {
 // two accumulators in tensor memory while warps 2..9 (warp w: lanes 32 (w % 4).., half of
 // the columns) read the other one, reduce it modulo p and add it up in registers, so the
 // drain of a chunk hides behind the next chunk's MMAs, across tiles too. Every wait is
-// bounded: on expiry an error code is set, the copies in flight land and TMEM is freed.
+// bounded: on expiry an error code is set, the copies in flight land and TMEM is freed; the
+// reconstruction gives NaN while the code stands (ptn_device_error).
 template <int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     k_rns_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -915,6 +916,7 @@ struct ReconP {
   const int *ea, *eb;
   int sh0;                // -2 bits - 2 (1022 + EXP_BASE)
   RnsView va, vb;
+  const int* err;         // device_error_word(): residues may be missing once it is set
   const int* skip;
 };
 
@@ -979,6 +981,7 @@ __device__ __forceinline__ double2 element(const ReconP& g, int m, int n, int q,
   u64 xh = x1 + ((u64)x2 << 32), yh = y1 + ((u64)y2 << 32);
   xh -= c.off_x_hi + (xl < c.off_x_lo ? 1ULL : 0ULL);
   yh -= c.off_y_hi + (yl < c.off_y_lo ? 1ULL : 0ULL);
+  if (*g.err != 0) return make_double2(__longlong_as_double(-1LL), __longlong_as_double(-1LL));
   bool ok = Ea != EXP_SPECIAL && Eb != EXP_SPECIAL;
   double2 z = make_double2(0.0, 0.0);
   if (ok && Ea != 0 && Eb != 0) {
@@ -1127,19 +1130,6 @@ bool make_map(CUtensorMap* out, const RnsOperand& o, int box_rows) {
   return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, o.p, dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// sticky error code of the kernels (bounded waits that expired)
-__device__ int g_rns_err;
-
-int* err_flag() {
-  static int* flag = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* a = nullptr;
-    if (cudaGetSymbolAddress(&a, g_rns_err) == cudaSuccess) flag = static_cast<int*>(a);
-  });
-  return flag;
 }
 
 long residue_ld(long N) { return (N + 7) / 8 * 8; }
@@ -1345,7 +1335,7 @@ static ptn_status multiply(const RnsOperand& A, const RnsView& va, const RnsOper
   g.res = static_cast<unsigned short*>(res);
   g.ldr = residue_ld(N);
   g.rplane = (long)M * g.ldr;
-  g.err = err_flag();
+  g.err = device_error_word();
   g.skip = skip;
   PTN_CHECK_ARG(g.err != nullptr, "rns_gemm: error flag lookup failed");
   const int planes = 2 * A.nm;
@@ -1369,6 +1359,7 @@ static ptn_status multiply(const RnsOperand& A, const RnsView& va, const RnsOper
   r->sh0 = -2 * bits - 2 * (1022 + EXP_BASE);
   r->va = va;
   r->vb = vb;
+  r->err = g.err;
   r->skip = skip;
   return PTN_OK;
 }
@@ -1422,16 +1413,6 @@ ptn_status rns_gemm_stage(const RnsOperand& A, const RnsView& va, const RnsOpera
     case RNS_MIXED_ENV: return launch_stage<RNS_MIXED_ENV>(r, s, st);
     default: return launch_stage<RNS_MIXED>(r, s, st);
   }
-}
-
-int rns_error_and_reset() {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_rns_err, sizeof(int)) != cudaSuccess) return -1;
-  if (v != 0) {
-    const int zero = 0;
-    cudaMemcpyToSymbol(g_rns_err, &zero, sizeof(int));
-  }
-  return v;
 }
 
 }  // namespace ptn

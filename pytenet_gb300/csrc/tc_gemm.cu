@@ -913,19 +913,6 @@ bool make_map(CUtensorMap* out, const void* ptr, long rows, long K, long Kp, lon
   return true;
 }
 
-// sticky error code of the tensor-core kernels (bounded waits that expired)
-__device__ int g_tc_err;
-
-int* err_flag() {
-  static int* flag = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* a = nullptr;
-    if (cudaGetSymbolAddress(&a, g_tc_err) == cudaSuccess) flag = static_cast<int*>(a);
-  });
-  return flag;
-}
-
 }  // namespace
 
 // K splits: at least what the accuracy bound needs (MAX_K_SPLIT reals per split), at most enough CTAs for twice PTN_TUNE_TC_SPLIT_WAVES waves (one CTA per SM);
@@ -1014,7 +1001,7 @@ ptn_status tc_gemm(const void* Aslices, long aplane, const int* ea, const void* 
   a.ldn = ldn;
   a.accumulate = accumulate ? 1 : 0;
   a.part = splits > 1 ? static_cast<double*>(ws) : nullptr;
-  a.err = err_flag();
+  a.err = device_error_word();
   a.skip = skip;
   const bool flags = fa != nullptr && fb != nullptr;
   PTN_CHECK_ARG(!flags || fk == a.nkb, "tc_gemm: flag rows of %d K blocks for %d", fk, a.nkb);
@@ -1048,17 +1035,4 @@ ptn_status tc_gemm(const void* Aslices, long aplane, const int* ea, const void* 
   return PTN_OK;
 }
 
-// host read of the sticky error flag (0 = fine); resets it
-int tc_gemm_error_and_reset() {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_tc_err, sizeof(int)) != cudaSuccess) return -1;
-  if (v != 0) {
-    const int zero = 0;
-    cudaMemcpyToSymbol(g_tc_err, &zero, sizeof(int));
-  }
-  return v;
-}
-
 }  // namespace ptn
-
-extern "C" int tc_gemm_error_and_reset_c(void) { return ptn::tc_gemm_error_and_reset(); }

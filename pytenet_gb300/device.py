@@ -49,8 +49,32 @@ def to_dev(x):
     return torch.from_numpy(a).to(device(), non_blocking=False)
 
 
+def check_device():
+    """Raise if a kernel on the device gave up on a bounded wait since the last check (results
+    since then are NaN or incomplete). Waits for the current stream: for places that read a
+    result anyway."""
+    code = lib().ptn_device_error(stream_ptr())
+    if code != 0:
+        raise _lib.PtnError(_lib.PTN_TIMEOUT if code > 0 else _lib.PTN_CUDA_ERROR,
+                            f"a bounded wait of a device kernel expired (code {code})"
+                            if code > 0 else "the device's error word cannot be read")
+
+
+def to_host_all(tensors):
+    """Device tensors -> NumPy arrays; raises if a kernel before them did not finish."""
+    out = [t.detach().cpu().numpy() for t in tensors]
+    if any(t.is_cuda for t in tensors):
+        check_device()
+    return out
+
+
 def to_host(t):
-    return t.detach().cpu().numpy()
+    return to_host_all([t])[0]
+
+
+def scalar(t):
+    """The first entry of a device tensor as a Python number, checked like to_host."""
+    return to_host(t.reshape(-1)[:1])[0].item()
 
 
 def empty(shape):

@@ -20,7 +20,7 @@ import torch
 
 from . import _lib
 from .block_sparse import ColMajor, Flip3, QRScratch, RowMajor, qr_execute
-from .device import CDT, Workspace, call, device, empty, lib, ptr, stream_ptr, to_dev, to_host
+from .device import CDT, Workspace, call, device, empty, lib, ptr, stream_ptr, to_dev, to_host_all
 from .qnumber import is_qsparse, qnumber_flatten, qr_plan
 
 PREC = {"fp64": _lib.PREC_FP64, "plain": _lib.PREC_FP64, "mixed": _lib.PREC_SPLIT_BF16,
@@ -68,8 +68,8 @@ class DeviceMPS:
         return self.buf[i][: s[0] * s[1] * s[2]].view(s)
 
     def download(self, psi):
-        for i in range(self.nsites):
-            psi.a[i] = to_host(self.site(i)).copy()
+        for i, x in enumerate(to_host_all([self.site(i) for i in range(self.nsites)])):
+            psi.a[i] = x.copy()
         psi.qbonds = [q.copy() for q in self.qbonds]
 
     # ---------------------------------------------------------------- QR steps

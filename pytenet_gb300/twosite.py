@@ -22,7 +22,7 @@ from . import _lib
 from .block_sparse import Flip3, QRScratch, RowMajor, ColMajor, qr_execute, svd_execute, \
     take_singular, _svd_scratch
 from .bond_ops import retained_bond_indices
-from .device import Workspace, call, device, empty, lib, ptr, stream_ptr, to_dev, to_host
+from .device import Workspace, call, device, empty, lib, ptr, stream_ptr, to_dev, to_host, to_host_all
 from .engine import MIXED_MIN_BOND, prec_code
 from .qnumber import is_qsparse, qnumber_flatten, qr_plan
 
@@ -71,7 +71,7 @@ class TwoSiteRun:
         self.qbonds = [np.asarray(q).copy() for q in psi.qbonds]
 
     def download(self, psi):
-        psi.a = [to_host(x).copy() for x in self.a]
+        psi.a = [x.copy() for x in to_host_all(self.a)]
         psi.qbonds = [q.copy() for q in self.qbonds]
 
     def prec_for(self, Dl, Dr):
@@ -176,7 +176,7 @@ class TwoSiteRun:
         q1 = qnumber_flatten([-self.qsite, self.qbonds[i + 2]])
         plan = qr_plan(q0, q1)
         u, s, vh = svd_execute(plan, x, RowMajor(d * Dr), _svd_scratch())
-        s_host = s.cpu().numpy()          # the truncation is an integer decision
+        s_host = to_host(s)               # the truncation is an integer decision
         idx = retained_bond_indices(s_host, tol)
         u, vh = take_singular(u, vh, idx)
         k = len(idx)
@@ -297,4 +297,4 @@ def dmrg_twosite(hamiltonian, psi, numsweeps, numiter_lanczos=25, tol_split=0,
         run.dmrg_sweep(en, k, tol_split)
     run.download(psi)
     _warn(run)
-    return en.cpu().numpy()
+    return to_host(en)
