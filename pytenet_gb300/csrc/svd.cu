@@ -65,6 +65,8 @@ constexpr int NS = 5;             // Newton-Schulz steps: one, and two after eac
 constexpr int REFINE = 2;
 constexpr double X_NORM[REFINE] = {0.1, 1e-3};
 constexpr int REG = 4;            // column entries a thread keeps in registers
+constexpr int RANGE = 200;        // binary orders of the largest entry that need no shift: its square, and those of
+                                  // columns 2^300 below it, are normal numbers
 
 template <typename T>
 struct Cplx;
@@ -159,17 +161,18 @@ __device__ __forceinline__ double inv_norm(double x, double y) {
   return fma(s * e, fma(e, 0.375, 0.5), s);
 }
 
-// FP64 throughout: columns of very different size, or near the lower end of the range
+// FP64 throughout: columns of very different size, or near the lower end of the range. The
+// Gram entries are squares already: nothing here squares them again.
 __device__ __noinline__ Rot<double> rotation_fp64(double aa, double bb, double cr, double ci,
                                                   double tol, float& off) {
   Rot<double> R;
-  const double ac = sqrt(cr * cr + ci * ci), ab = sqrt(aa) * sqrt(bb);
+  const double ac = hypot(cr, ci), ab = sqrt(aa) * sqrt(bb);
   R.on = ac > 0.0 && ac > tol * ab;
   off = R.on ? (float)fmax(ac / ab, 1e-30) : 0.0f;
   if (!R.on) return R;
   const double pr = cr / ac, pi = -ci / ac;
   const double z = (bb - aa) / (2.0 * ac);
-  const double t = copysign(1.0, z) / (fabs(z) + sqrt(1.0 + z * z));
+  const double t = copysign(1.0, z) / (fabs(z) + hypot(1.0, z));
   R.cs = 1.0 / sqrt(1.0 + t * t);
   R.sn = R.cs * t;
   R.gr = R.sn * pr;
@@ -507,8 +510,9 @@ __device__ void sweeps_shared(float2* sh, const double2* __restrict__ a, long ld
 }
 
 // FP32 sweeps on A scaled to entries below 1: V32 as FP64 to Vd (column-major), identities
-// to the NS buffers G (for the Newton-Schulz steps), *bad = 1 when A holds an infinity or NaN (the
-// GEMMs and the FP64 sweeps then start from A itself).
+// to the NS buffers G (for the Newton-Schulz steps), *bad = 1 when A holds an infinity or NaN, or
+// entries whose squares would leave the range in the Gram matrices (the GEMMs are skipped and the
+// FP64 sweeps start from A itself).
 __global__ void __launch_bounds__(ST) svd_pre_kernel(const double2* __restrict__ a, int m, int n,
                                                      long lda, float2* __restrict__ W,
                                                      float2* __restrict__ V,
@@ -523,10 +527,11 @@ __global__ void __launch_bounds__(ST) svd_pre_kernel(const double2* __restrict__
   const int p = wide ? n : m, r = wide ? m : n;
   const long step = (long)cs * ST, first = rank * (long)ST + tid;
   const int e = largest_exponent(a, m, n, lda);
-  if (rank == 0 && tid == 0) *bad = e == 2047 ? 1 : 0;
-  if (e != 2047 && shared) {
+  const bool skip = e > 1023 + RANGE;
+  if (rank == 0 && tid == 0) *bad = skip ? 1 : 0;
+  if (!skip && shared) {
     sweeps_shared(columns, a, lda, wide, p, r, e, 1e-6f, 3e-4f, PRE_SWEEPS, Vd);
-  } else if (e != 2047) {
+  } else if (!skip) {
     for (long q = first; q < (long)p * r; q += step) {
       const int j = (int)(q / p), i = (int)(q % p);
       double2 z = wide ? a[(long)j * lda + i] : a[(long)i * lda + j];
@@ -542,7 +547,7 @@ __global__ void __launch_bounds__(ST) svd_pre_kernel(const double2* __restrict__
     const double2 one = c2(q / r == q % r ? 1.0 : 0.0, 0.0);
 #pragma unroll
     for (int t = 0; t < NS; ++t) G[(long)t * r * r + q] = one;
-    if (e != 2047 && !shared) {
+    if (!skip && !shared) {
       const float2 v = __ldcg(V + q);
       Vd[q] = c2(v.x, v.y);
     }
@@ -598,7 +603,7 @@ __global__ void __launch_bounds__(ST) svd_jacobi_kernel(const double2* __restric
   const long step = (long)cs * ST, first = rank * (long)ST + tid;
   // entries whose squares would leave the FP64 range: W carries a power of two
   const int ea = largest_exponent(a, m, n, lda);
-  const int shift = (ea != 0 && ea != 2047 && abs(ea - 1023) > 400) ? 1023 - ea : 0;
+  const int shift = (ea != 0 && ea != 2047 && abs(ea - 1023) > RANGE) ? 1023 - ea : 0;
   if (!pre || *bad != 0) {
     for (long e = first; e < (long)p * r; e += step) {
       const int j = (int)(e / p), i = (int)(e % p);

@@ -310,3 +310,30 @@ def test_svd_columns_in_shared_memory(mn):
     assert np.linalg.norm((u * s) @ vh - a) <= tol * np.linalg.norm(a) * np.sqrt(min(m, n))
     for x in (u, vh.conj().T):
         assert np.abs(x.conj().T @ x - np.eye(min(m, n))).max() <= tol * np.sqrt(min(m, n))
+
+
+@pytest.mark.parametrize("top", [-390, -300, 254, 300, 398, 401, 402, 510, 600, 980])
+@pytest.mark.parametrize("mn", [(32, 32), (70, 45), (40, 90)])
+def test_svd_over_the_range_of_scales(mn, top):
+    """Graded matrices whose entries, squares or fourth powers leave the FP64 range: as for the
+    matrix of order one."""
+    m, n = mn
+    r = min(m, n)
+    rng = np.random.default_rng(m + n)
+    u, _, vh = np.linalg.svd(orc.crandn((m, n), rng), full_matrices=False)
+    a = (u * 2.0 ** -np.linspace(0, 40, r)) @ vh
+    for steep in (False, True):   # and a few columns far below the others
+        if steep:
+            a[:, 3:6] *= 2.0 ** -120
+        big = a * 2.0 ** top
+        u, s, vh, sweeps = dev_svd(big)
+        assert sweeps < 60
+        s = s * 2.0 ** -top
+        s_ref = np.linalg.svd(a, compute_uv=False)
+        tol = 16 * max(m, n) * np.finfo(float).eps
+        assert np.all(np.diff(s) <= 0)
+        assert np.abs(s - s_ref).max() <= tol * s_ref[0]
+        assert np.linalg.norm((u * s) @ vh - a) <= tol * np.linalg.norm(a) * np.sqrt(r)
+        keep = s > 1e-13 * s[0]
+        for x in (u[:, keep], vh[keep].conj().T):
+            assert np.abs(x.conj().T @ x - np.eye(keep.sum())).max() <= tol * np.sqrt(r)
