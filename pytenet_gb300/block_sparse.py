@@ -169,16 +169,21 @@ def qr_execute(plan, src, src_view, q_dst, q_view, r_dst, r_view, scratch):
         return
     main = torch.cuda.current_stream()
     fork = main.record_event()
-    for i in range(lanes):
-        lane, stream = scratch.lane(i)
-        for k in wide[i::lanes]:   # no buffer is replaced while a block of this call uses it
-            rows, cols, _, kb = plan.blocks[k]
-            lane.reserve(len(rows), len(cols), kb)
-        stream.wait_event(fork)
-        for k in wide[i::lanes]:
-            _qr_block(plan.blocks[k], maps[k], src, q_dst, r_dst, lane, stream.cuda_stream)
-    for i in range(lanes):
-        main.wait_stream(scratch.streams[i])
+    forked = []
+    try:
+        for i in range(lanes):
+            lane, stream = scratch.lane(i)
+            for k in wide[i::lanes]:   # no buffer is replaced while a block of this call uses it
+                rows, cols, _, kb = plan.blocks[k]
+                lane.reserve(len(rows), len(cols), kb)
+            stream.wait_event(fork)
+            forked.append(stream)
+            for k in wide[i::lanes]:
+                _qr_block(plan.blocks[k], maps[k], src, q_dst, r_dst, lane, stream.cuda_stream)
+    finally:
+        # after an error too: the caller may let go of the tensors that the lanes still use
+        for stream in forked:
+            main.wait_stream(stream)
 
 
 _SCRATCH = None

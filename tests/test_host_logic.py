@@ -206,3 +206,71 @@ def test_is_qsparse_without_constraints_and_with_violations():
     assert not is_qsparse(a, qn) and not orc.is_qsparse(a, qn)
     enforce_qsparsity(a, qn)
     assert is_qsparse(a, qn) and orc.is_qsparse(a, qn)
+
+
+@pytest.mark.parametrize("fails_at", [None, 0, 3, 6, 9])
+def test_qr_lanes_join_after_an_error(monkeypatch, fails_at):
+    """The streams that a block QR forked are waited for whatever call raises in between."""
+    from pytenet_gb300 import block_sparse as bs
+
+    class Stream:
+        def __init__(self, name):
+            self.cuda_stream = name
+            self.waits = []
+
+        def wait_event(self, e):
+            self.waits.append(e)
+
+        def wait_stream(self, s):
+            self.waits.append(s)
+
+        def record_event(self):
+            return "fork"
+
+    class Lib:
+        ptn_gather = ptn_qr = ptn_scatter = ptn_qr_blocks = staticmethod(lambda *a: 0)
+        ptn_qr_workspace_bytes = staticmethod(lambda m, n: 256)
+
+    class Buffer:
+        def get(self, n):
+            return None
+
+    main, made, calls = Stream("main"), [], []
+
+    class Scratch(bs.QRScratch):
+        def __init__(self):
+            super().__init__()
+            self.ws = self.work = self.qb = self.rb = Buffer()
+
+        def lane(self, i):
+            while len(self.lanes) <= i:
+                self.lanes.append(Scratch())
+                self.streams.append(Stream(f"lane {i}"))
+                made.append(self.streams[-1])
+            return self.lanes[i], self.streams[i]
+
+    def call(fn, *args):
+        calls.append(fn)
+        if fails_at is not None and len(calls) > fails_at:
+            raise RuntimeError("a call that fails")
+
+    plan = bs.qr_plan(np.repeat([0, 1, 2], 40), np.repeat([0, 1, 2], 20))
+    monkeypatch.setattr(bs, "lib", Lib)
+    monkeypatch.setattr(bs, "stream_ptr", lambda: "main")
+    monkeypatch.setattr(bs, "call", call)
+    monkeypatch.setattr(bs, "ptr", lambda x: 0)
+    monkeypatch.setattr(bs, "_block_maps", lambda *a: [(None,) * 6] * len(plan.blocks))
+    monkeypatch.setattr(bs, "_small_blocks", lambda *a: (frozenset(), 0, None))
+    monkeypatch.setattr(bs.torch.cuda, "current_stream", lambda: main)
+    dst = np.zeros(1)
+    dst_like = type("T", (), {"zero_": lambda self: None})()
+    run = lambda: bs.qr_execute(plan, dst, bs.RowMajor(60), dst_like, bs.RowMajor(60), dst_like,
+                                bs.RowMajor(60), Scratch())
+    if fails_at is None:
+        run()
+        assert len(made) == 3
+    else:
+        with pytest.raises(RuntimeError):
+            run()
+    forked = [s for s in made if s.waits == ["fork"]]
+    assert len(forked) == len(made) > 0 and main.waits == forked
