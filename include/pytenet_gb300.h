@@ -54,8 +54,9 @@ typedef enum {
                                below the others of its row keeps that error, where DMMA sums of
                                |A[m, k] B[n, k]| alone bound it */
   PTN_PREC_SPLIT_BF16 = 1   /* fewer moduli: 11 in the local operators (40-44 bits per
-                               row-scaled value, ~1e-12 relative per contraction), 13 in the
-                               environment steps (49-52 bits) */
+                               row-scaled value, 39 in sums of more than 16384 terms; ~1e-12
+                               relative per contraction), 13 in the environment steps (49-53
+                               bits, 48 in sums of more than 8192 terms) */
 } ptn_precision;
 
 typedef struct { double re, im; } ptn_c128;

@@ -2,7 +2,7 @@
 //
 // C = A B over complex FP64 is computed exactly in integers and rounded once:
 //   - every row of A and every column of B is scaled by its own power of two and rounded
-//     to Gaussian integers of `bits` bits (53 or 54 in the FP64 form, 40 and more in the
+//     to Gaussian integers of `bits` bits (53 or 54 in the FP64 form, 39 and more in the
 //     mixed form); in the FP64 form the terms are scaled before by powers of two that cancel
 //     in the product (RnsTerms in rns.cuh), so that operands which grow and decay against
 //     each other along the terms lose nothing;

@@ -7,8 +7,9 @@
 
 namespace ptn {
 
-// Moduli of the FP64 form and of the mixed form: its operators (40 bits and more) and its
-// environment steps (49 and more). Environments stay Hermitian to FP64 level that way: with 40
+// Moduli of the FP64 form (53 bits and more, else the DMMA kernels: 8192 terms) and of the mixed
+// form: its operators (40 bits and more up to 16384 terms, 39 beyond) and its environment steps
+// (49 and more up to 8192 terms, 48 beyond). Environments stay Hermitian to FP64 level: with 40
 // bits the chain ends, whose small Krylov spaces are exhausted, see residuals around the
 // breakdown threshold 100 n eps (2e-13 against 9e-14 at bond 2), and whether a run stops there
 // would depend on rounding.

@@ -281,3 +281,28 @@ def test_terms_that_meet_zeros_or_subnormals():
     A[3, 5] = np.inf
     bad = zgemm(A, B)
     assert not np.isfinite(bad[3]).any() and np.isfinite(np.delete(bad, 3, 0)).all()
+
+
+# Rows longer than a cluster converts (8192 terms): their exponents come from a pass of their
+# own, 11 moduli leave 40 bits up to 16384 terms and 39 beyond, 13 moduli 49 and 48, and the
+# FP64 form keeps to the DMMA kernels (fewer than 53 bits). Tolerance: rows of Gaussian entries
+# reach 8, so an entry of order one is off by 2^(3 - bits) at most, in either operand, and the
+# errors of the terms add up like the terms: twice 2^(3 - 39) and 2^(3 - 48).
+@pytest.mark.parametrize("op,chi,tol", [("bond", 300, 2 * 2.0 ** -36), ("bond", 520, 2 * 2.0 ** -36),
+                                        ("env", 3, 2 * 2.0 ** -45)])
+def test_mixed_contractions_of_long_rows(op, chi, tol):
+    import torch
+    import pytenet_gb300 as ptg
+    gen = torch.Generator(device="cuda").manual_seed(chi)
+    c = lambda *s: torch.randn(*s, dtype=torch.complex128, device="cuda", generator=gen)
+    if op == "bond":
+        dl, dr = 33, 40
+        args, fn = (c(dl, dr), c(dl, chi, dl), c(dr, chi, dr)), ptg.apply_local_bond_contraction
+    else:
+        dl, dr = 33, 4100
+        w = torch.randn(chi, 2, 2, chi, dtype=torch.complex128, device="cuda", generator=gen)
+        args = (c(dl, 2, dr), c(dl, 2, dr), w, c(dr, chi, dr))
+        fn = ptg.contraction_operator_step_right
+    got, ref = fn(*args, precision="mixed"), fn(*args, precision="fp64")
+    err = float(torch.linalg.vector_norm(got - ref) / torch.linalg.vector_norm(ref))
+    assert 0 < err < tol, err
