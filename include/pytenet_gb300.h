@@ -53,10 +53,13 @@ typedef enum {
                                the others; row, column and index scalings cancel. A result far
                                below the others of its row keeps that error, where DMMA sums of
                                |A[m, k] B[n, k]| alone bound it */
-  PTN_PREC_SPLIT_BF16 = 1   /* fewer moduli: 11 in the local operators (40-44 bits per
+  PTN_PREC_SPLIT_BF16 = 1,  /* fewer moduli: 11 in the local operators (40-44 bits per
                                row-scaled value, 39 in sums of more than 16384 terms; ~1e-12
                                relative per contraction), 13 in the environment steps (49-53
                                bits, 48 in sums of more than 8192 terms) */
+  PTN_PREC_FP64_DMMA = 2    /* FP64 with the DMMA kernels at every size: the error of a result is
+                               bounded by its own sum of |A[m, k] B[n, k]|, and the workspace is
+                               the smallest (the two intermediates of a contraction) */
 } ptn_precision;
 
 typedef struct { double re, im; } ptn_c128;
@@ -157,7 +160,10 @@ void ptn_prof_stop(void);
 ptn_status ptn_prof_read(int kind, double* total_ms, double* flops, double* bytes,
                          long* launches);
 
-/* ----------------------------------------------------------- contractions */
+/* ----------------------------------------------------------- contractions
+ * Workspaces: with PTN_PREC_FP64 a workspace smaller than the query asks for, down to the size
+ * of PTN_PREC_FP64_DMMA, is taken too, and leaves the DMMA kernels where the residues have no
+ * room. */
 
 /* a1: out = H_eff . a, out[l2, s, r2] = sum L[l0,wl,l2] W[wl,s,t,wr] a[l0,t,r0] R[r0,wr,r2].
  * Replaces apply_local_hamiltonian, pytenet/chain_ops.py:237-279. */
@@ -167,7 +173,7 @@ ptn_status ptn_heff_apply(const ptn_c128* a, const ptn_c128* w, const ptn_c128* 
                           int chil, int chir, int prec, void* ws, size_t ws_bytes,
                           void* stream);
 
-/* H_eff . a exactly as ptn_heff_apply with prec = PTN_PREC_FP64, but without a
+/* H_eff . a as ptn_heff_apply with prec = PTN_PREC_FP64 on a small workspace, but without a
  * workspace argument, for callers that cannot allocate device memory (an FFI host
  * without a CUDA allocator, a process whose device memory belongs to another
  * framework's pool, code running where allocation is forbidden). No counterpart
@@ -333,6 +339,8 @@ ptn_status ptn_eigh_site(ptn_c128* a, const ptn_c128* w, const ptn_c128* l, cons
  * `a` (m x n, row-major, lda = n) is overwritten. Q is m x k, R is k x n,
  * k = min(m, n), written with leading dimensions ldq / ldr. */
 size_t ptn_qr_workspace_bytes(int m, int n);
+/* the least that ptn_qr takes: without the room for Q in wide blocks */
+size_t ptn_qr_least_workspace_bytes(int m, int n);
 ptn_status ptn_qr(ptn_c128* a, int m, int n, ptn_c128* q, long ldq, ptn_c128* r, long ldr,
                   void* ws, size_t ws_bytes, void* stream);
 

@@ -16,7 +16,7 @@ ABI_VERSION = 3
 KRYLOV_MAXITER = 64
 
 PTN_OK, PTN_BAD_SHAPE, PTN_BREAKDOWN, PTN_NAN, PTN_TIMEOUT, PTN_CUDA_ERROR, PTN_UNSUPPORTED = range(7)
-PREC_FP64, PREC_SPLIT_BF16 = 0, 1
+PREC_FP64, PREC_SPLIT_BF16, PREC_FP64_DMMA = 0, 1, 2
 TUNE_TC_SPLIT_WAVES, TUNE_ZGEMM_SPLIT_WAVES, TUNE_LARFB_TILE, TUNE_QR_CLUSTER = 0, 1, 2, 3
 TUNE_KRYLOV_FUSED = 4
 TUNE_QR_PANEL = 5
@@ -131,6 +131,7 @@ _SIGS = {
     "ptn_svd": (I, [P, I, I, L, P, L, P, P, L, P, P, S, P]),
     "ptn_diag_scale": (I, [P, L, L, L, P, I, P]),
     "ptn_qr_workspace_bytes": (S, [I, I]),
+    "ptn_qr_least_workspace_bytes": (S, [I, I]),
     "ptn_qr": (I, [P, I, I, P, L, P, L, P, S, P]),
     "ptn_qr_blocks_max_columns": (I, []),
     "ptn_qr_blocks_max_rows": (I, []),

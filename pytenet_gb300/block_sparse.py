@@ -124,9 +124,9 @@ class QRScratch:
 
     def reserve(self, mb, nb, kb):
         L = lib()
-        wsb = L.ptn_qr_workspace_bytes(mb, nb)
         return (self.work.get(mb * nb * 16), self.qb.get(mb * kb * 16), self.rb.get(kb * nb * 16),
-                self.ws.get(wsb), wsb)
+                *self.ws.room(L.ptn_qr_workspace_bytes(mb, nb),
+                              lambda: L.ptn_qr_least_workspace_bytes(mb, nb)))
 
 
 def _qr_block(block, maps, src, q_dst, r_dst, scratch, st):

@@ -39,9 +39,9 @@ def apply_local_hamiltonian(a, w, l, r, precision="fp64"):
     out = empty((Dl, d, Dr))
     p = prec_code(precision)
     L = lib()
-    wsb = L.ptn_heff_workspace_bytes(Dl, d, Dr, cl, cr, p)
+    ws, wsb, p = _WS.for_precision(lambda q: L.ptn_heff_workspace_bytes(Dl, d, Dr, cl, cr, q), p)
     call(L.ptn_heff_apply, ptr(A), ptr(W), ptr(Lt), ptr(R), ptr(out), Dl, d, Dr, cl, cr, p,
-         ptr(_WS.get(wsb)), wsb, stream_ptr())
+         ptr(ws), wsb, stream_ptr())
     return _ret(out, host)
 
 
@@ -57,9 +57,9 @@ def apply_local_bond_contraction(c, l, r, precision="fp64"):
     out = empty((Dl, Dr))
     p = prec_code(precision)
     L = lib()
-    wsb = L.ptn_bond_workspace_bytes(Dl, Dr, chi, p)
-    call(L.ptn_bond_apply, ptr(Cm), ptr(Lt), ptr(R), ptr(out), Dl, Dr, chi, p, ptr(_WS.get(wsb)),
-         wsb, stream_ptr())
+    ws, wsb, p = _WS.for_precision(lambda q: L.ptn_bond_workspace_bytes(Dl, Dr, chi, q), p)
+    call(L.ptn_bond_apply, ptr(Cm), ptr(Lt), ptr(R), ptr(out), Dl, Dr, chi, p, ptr(ws), wsb,
+         stream_ptr())
     return _ret(out, host)
 
 
@@ -76,9 +76,9 @@ def contraction_operator_step_left(a, b, w, l, precision="fp64"):
     A, B, W, Lt = (to_dev(x) for x in (a, b, w, l))
     out = empty((Dr, cr, Dr))
     L = lib()
-    wsb = L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, p)
+    ws, wsb, p = _WS.for_precision(lambda q: L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, q), p)
     call(L.ptn_env_step_left, ptr(A), ptr(B), ptr(W), ptr(Lt), ptr(out), Dl, d, Dr, cl, cr, p,
-         ptr(_WS.get(wsb)), wsb, stream_ptr())
+         ptr(ws), wsb, stream_ptr())
     return _ret(out, host)
 
 
@@ -95,9 +95,9 @@ def contraction_operator_step_right(a, b, w, r, precision="fp64"):
     A, B, W, R = (to_dev(x) for x in (a, b, w, r))
     out = empty((Dl, cl, Dl))
     L = lib()
-    wsb = L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, p)
+    ws, wsb, p = _WS.for_precision(lambda q: L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, q), p)
     call(L.ptn_env_step_right, ptr(A), ptr(B), ptr(W), ptr(R), ptr(out), Dl, d, Dr, cl, cr, p,
-         ptr(_WS.get(wsb)), wsb, stream_ptr())
+         ptr(ws), wsb, stream_ptr())
     return _ret(out, host)
 
 
@@ -142,9 +142,9 @@ def mpo_average(psi, op):
 
 def _zgemm(opa, opb, M, N, K, A, lda, B, ldb, Cout, ldc):
     L = lib()
-    wsb = L.ptn_zgemm_workspace_bytes(M, N, K, 1)
+    ws, wsb = _WS.room(L.ptn_zgemm_workspace_bytes(M, N, K, 1), lambda: 0)
     call(L.ptn_zgemm, opa, opb, M, N, K, _lib.cval(1), ptr(A), lda, 0, ptr(B), ldb, 0,
-         _lib.cval(0), ptr(Cout), ldc, 0, 1, ptr(_WS.get(wsb)), wsb, stream_ptr())
+         _lib.cval(0), ptr(Cout), ldc, 0, 1, ptr(ws), wsb, stream_ptr())
 
 
 def mps_vdot(chi, psi):

@@ -41,8 +41,7 @@ def _gemm(M, N, K, a, b, out, ws, opa="N", opb="N"):
     """out (M x N) = op(a) op(b) on the FP64 tensor cores; a is stored M x K for
     "N" / "C" and K x M for "T" / "H", b likewise (row-major)."""
     L = lib()
-    wsb = L.ptn_zgemm_workspace_bytes(M, N, K, 1)
-    w = ws.get(wsb)
+    w, wsb = ws.room(L.ptn_zgemm_workspace_bytes(M, N, K, 1), lambda: 0)
     lda = K if opa in "NC" else M
     ldb = N if opb in "NC" else K
     call(L.ptn_zgemm, opa.encode(), opb.encode(), M, N, K, _lib.cval(1), ptr(a), lda, 0, ptr(b),

@@ -101,8 +101,9 @@ GemmArgs gemm_args(char oa, char ob, int M, int N, int K, const double2* A, long
 // ------------------------------------------------------------------ choice of kernels
 // The FP64 form takes the residue planes where both GEMMs do (rns_wanted), the DMMA kernel
 // otherwise, or when the workspace is smaller than the query asks for; the mixed form takes
-// its (fewer) planes unless a product is too long for them.
+// its (fewer) planes unless a product is too long for them; PTN_PREC_FP64_DMMA takes none.
 static int form(int prec, bool wanted, long k1, long k2, int mixed) {
+  if (prec == PTN_PREC_FP64_DMMA) return 0;
   if (prec == PTN_PREC_FP64) return wanted ? RNS_FP64 : 0;
   return rns_bits(k1, mixed) != 0 && rns_bits(k2, mixed) != 0 ? mixed : 0;
 }
@@ -145,9 +146,14 @@ static size_t heff_gemm_ws(int Dl, int d, int Dr, int chil, int chir) {
                   zgemm_workspace_bytes(Dl, d * Dr, Dl * chil, 1));
 }
 
+// the two intermediates alone: the least that the FP64 forms run on, and all of
+// PTN_PREC_FP64_DMMA
+size_t heff_workspace_bytes_dmma(int Dl, int d, int Dr, int chil, int chir) {
+  return 2 * align256(heff_t_elems(Dl, d, Dr, chil, chir) * sizeof(double2));
+}
+
 size_t heff_workspace_bytes_f64(int Dl, int d, int Dr, int chil, int chir) {
-  const size_t t = align256(heff_t_elems(Dl, d, Dr, chil, chir) * sizeof(double2));
-  return 2 * t + align256(heff_gemm_ws(Dl, d, Dr, chil, chir));
+  return heff_workspace_bytes_dmma(Dl, d, Dr, chil, chir) + align256(heff_gemm_ws(Dl, d, Dr, chil, chir));
 }
 
 static ContractWs carve(void* ws, size_t t_elems, size_t ws_bytes) {
@@ -164,7 +170,7 @@ static ContractWs carve(void* ws, size_t t_elems, size_t ws_bytes) {
 ptn_status heff_apply_f64(const double2* a, const double2* w, const double2* l, const double2* r,
                           double2* out, int Dl, int d, int Dr, int chil, int chir, void* ws,
                           size_t ws_bytes, const int* skip, cudaStream_t st) {
-  PTN_CHECK_ARG(ws_bytes >= 2 * align256(heff_t_elems(Dl, d, Dr, chil, chir) * sizeof(double2)),
+  PTN_CHECK_ARG(ws_bytes >= heff_workspace_bytes_dmma(Dl, d, Dr, chil, chir),
                 "heff: workspace too small");
   ContractWs c = carve(ws, heff_t_elems(Dl, d, Dr, chil, chir), ws_bytes);
   // T1[(l0,t),(wr,r2)] = A[(l0,t), r0] R[r0, (wr,r2)]
@@ -178,18 +184,20 @@ ptn_status heff_apply_f64(const double2* a, const double2* w, const double2* l, 
   return PTN_OK;
 }
 
+size_t bond_workspace_bytes_dmma(int Dl, int Dr, int chi) {
+  return 2 * align256((size_t)Dl * chi * Dr * sizeof(double2));
+}
+
 size_t bond_workspace_bytes_f64(int Dl, int Dr, int chi) {
-  const size_t t = align256((size_t)Dl * chi * Dr * sizeof(double2));
   const size_t g = std::max(zgemm_workspace_bytes(Dl, chi * Dr, Dr, 1),
                             zgemm_workspace_bytes(Dl, Dr, Dl * chi, 1));
-  return 2 * t + align256(g);
+  return bond_workspace_bytes_dmma(Dl, Dr, chi) + align256(g);
 }
 
 ptn_status bond_apply_f64(const double2* cm, const double2* l, const double2* r, double2* out,
                           int Dl, int Dr, int chi, void* ws, size_t ws_bytes, const int* skip,
                           cudaStream_t st) {
-  PTN_CHECK_ARG(ws_bytes >= 2 * align256((size_t)Dl * chi * Dr * sizeof(double2)),
-                "bond: workspace too small");
+  PTN_CHECK_ARG(ws_bytes >= bond_workspace_bytes_dmma(Dl, Dr, chi), "bond: workspace too small");
   ContractWs c = carve(ws, (size_t)Dl * chi * Dr, ws_bytes);
   // T1[l0,(w,r2)] = C[l0,r0] R[r0,(w,r2)]
   PTN_TRY(zgemm(gemm_args('N', 'N', Dl, chi * Dr, Dr, cm, Dr, r, (long)chi * Dr, c.t1,
@@ -200,20 +208,26 @@ ptn_status bond_apply_f64(const double2* cm, const double2* l, const double2* r,
   return PTN_OK;
 }
 
+static size_t env_t_elems(int Dl, int d, int Dr, int chil, int chir) {
+  return (size_t)Dl * d * Dr * std::max(chil, chir);
+}
+
+size_t env_workspace_bytes_dmma(int Dl, int d, int Dr, int chil, int chir) {
+  return 2 * align256(env_t_elems(Dl, d, Dr, chil, chir) * sizeof(double2));
+}
+
 size_t env_workspace_bytes_f64(int Dl, int d, int Dr, int chil, int chir) {
-  const size_t te = (size_t)std::max(Dl * chil * d * Dr, Dl * d * chir * Dr);
-  const size_t t = align256(te * sizeof(double2));
   size_t g = zgemm_workspace_bytes(Dl * chil, d * Dr, Dl, 1);
   g = std::max(g, zgemm_workspace_bytes(Dr, chir * Dr, Dl * d, 1));
   g = std::max(g, zgemm_workspace_bytes(Dl * d, chir * Dr, Dr, 1));
   g = std::max(g, zgemm_workspace_bytes(Dl * chil, Dl, d * Dr, 1));
-  return 2 * t + align256(g);
+  return env_workspace_bytes_dmma(Dl, d, Dr, chil, chir) + align256(g);
 }
 
 ptn_status env_left_f64(const double2* a, const double2* b, const double2* w, const double2* l,
                         double2* lnext, int Dl, int d, int Dr, int chil, int chir, void* ws,
                         size_t ws_bytes, cudaStream_t st) {
-  const size_t te = (size_t)std::max(Dl * chil * d * Dr, Dl * d * chir * Dr);
+  const size_t te = env_t_elems(Dl, d, Dr, chil, chir);
   PTN_CHECK_ARG(ws_bytes >= 2 * align256(te * sizeof(double2)), "env_left: workspace too small");
   ContractWs c = carve(ws, te, ws_bytes);
   // T1[(l0,wl),(t,rb)] = sum_l2 L[(l0,wl), l2] conj(B)[l2,(t,rb)]
@@ -230,7 +244,7 @@ ptn_status env_left_f64(const double2* a, const double2* b, const double2* w, co
 ptn_status env_right_f64(const double2* a, const double2* b, const double2* w, const double2* r,
                          double2* rnext, int Dl, int d, int Dr, int chil, int chir, void* ws,
                          size_t ws_bytes, cudaStream_t st) {
-  const size_t te = (size_t)std::max(Dl * chil * d * Dr, Dl * d * chir * Dr);
+  const size_t te = env_t_elems(Dl, d, Dr, chil, chir);
   PTN_CHECK_ARG(ws_bytes >= 2 * align256(te * sizeof(double2)), "env_right: workspace too small");
   ContractWs c = carve(ws, te, ws_bytes);
   // T1[(l0,s),(wr,r2)] = A[(l0,s),r0] R[r0,(wr,r2)]
@@ -257,22 +271,28 @@ extern "C" {
 size_t ptn_heff_workspace_bytes(int Dl, int d, int Dr, int chil, int chir, int prec) {
   const int nm = heff_form(prec, Dl, d, Dr, chil, chir);
   return nm != 0 ? heff_workspace_bytes_rns(nm, Dl, d, Dr, chil, chir)
-                 : heff_workspace_bytes_f64(Dl, d, Dr, chil, chir);
+         : prec == PTN_PREC_FP64_DMMA ? heff_workspace_bytes_dmma(Dl, d, Dr, chil, chir)
+                                      : heff_workspace_bytes_f64(Dl, d, Dr, chil, chir);
 }
 
 size_t ptn_bond_workspace_bytes(int Dl, int Dr, int chi, int prec) {
   const int nm = bond_form(prec, Dl, Dr, chi);
-  return nm != 0 ? bond_workspace_bytes_rns(nm, Dl, Dr, chi) : bond_workspace_bytes_f64(Dl, Dr, chi);
+  return nm != 0 ? bond_workspace_bytes_rns(nm, Dl, Dr, chi)
+         : prec == PTN_PREC_FP64_DMMA ? bond_workspace_bytes_dmma(Dl, Dr, chi)
+                                      : bond_workspace_bytes_f64(Dl, Dr, chi);
 }
 
 size_t ptn_env_workspace_bytes(int Dl, int d, int Dr, int chil, int chir, int prec) {
   const int nm = env_form(prec, Dl, d, Dr, chil, chir);
   return nm != 0 ? env_workspace_bytes_rns(nm, Dl, d, Dr, chil, chir)
-                 : env_workspace_bytes_f64(Dl, d, Dr, chil, chir);
+         : prec == PTN_PREC_FP64_DMMA ? env_workspace_bytes_dmma(Dl, d, Dr, chil, chir)
+                                      : env_workspace_bytes_f64(Dl, d, Dr, chil, chir);
 }
 
-// the FP64 form falls back to the DMMA kernels on a workspace smaller than the query's
-static int fitting(int nm, int prec, size_t ws_bytes, size_t need) {
+// the FP64 form falls back to the DMMA kernels on a workspace smaller than the query's; the
+// DMMA form uses no more than its own (the rest would go to residues of single products)
+static int fitting(int nm, int prec, size_t& ws_bytes, size_t need) {
+  if (prec == PTN_PREC_FP64_DMMA) ws_bytes = std::min(ws_bytes, need);
   return prec == PTN_PREC_FP64 && ws_bytes < need ? 0 : nm;
 }
 

@@ -2123,6 +2123,7 @@ ptn_status qr_blocks(const double2* src, double2* q, double2* r, const ptn_qr_bl
 extern "C" {
 
 size_t ptn_qr_workspace_bytes(int m, int n) { return ptn::qr_workspace_bytes(m, n); }
+size_t ptn_qr_least_workspace_bytes(int m, int n) { return ptn::qr_base_bytes(m, n); }
 
 int ptn_qr_blocks_max_columns(void) { return ptn::NB; }
 int ptn_qr_blocks_max_rows(void) {

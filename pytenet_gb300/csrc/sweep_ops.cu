@@ -60,9 +60,14 @@ struct LocalOp {
 
   ptn_status apply(const double2* x, double2* y, const int* skip, cudaStream_t st) const {
     const int nm = form();
-    if (nm == 0)
-      return site ? heff_apply_f64(x, w, l, r, y, Dl, d, Dr, chil, chir, ws, ws_bytes, skip, st)
-                  : bond_apply_f64(x, l, r, y, Dl, Dr, chil, ws, ws_bytes, skip, st);
+    if (nm == 0) {
+      // the DMMA form keeps to its own workspace: residues of single products would use the rest
+      const size_t wsb = prec != PTN_PREC_FP64_DMMA ? ws_bytes
+          : std::min(ws_bytes, site ? ptn_heff_workspace_bytes(Dl, d, Dr, chil, chir, prec)
+                                    : ptn_bond_workspace_bytes(Dl, Dr, chil, prec));
+      return site ? heff_apply_f64(x, w, l, r, y, Dl, d, Dr, chil, chir, ws, wsb, skip, st)
+                  : bond_apply_f64(x, l, r, y, Dl, Dr, chil, ws, wsb, skip, st);
+    }
     return site ? heff_apply_rns(nm, x, y, w, l, r, Dl, d, Dr, chil, chir, ws, skip, st)
                 : bond_apply_rns(nm, x, y, l, r, Dl, Dr, chil, ws, skip, st);
   }
@@ -106,14 +111,11 @@ using namespace ptn;
 extern "C" {
 
 size_t ptn_site_step_workspace_bytes(int Dl, int d, int Dr, int chil, int chir, int prec) {
-  const int nm = heff_form(prec, Dl, d, Dr, chil, chir);
-  return nm != 0 ? heff_workspace_bytes_rns(nm, Dl, d, Dr, chil, chir)
-                 : heff_workspace_bytes_f64(Dl, d, Dr, chil, chir);
+  return ptn_heff_workspace_bytes(Dl, d, Dr, chil, chir, prec);
 }
 
 size_t ptn_bond_step_workspace_bytes(int Dl, int Dr, int chi, int prec) {
-  const int nm = bond_form(prec, Dl, Dr, chi);
-  return nm != 0 ? bond_workspace_bytes_rns(nm, Dl, Dr, chi) : bond_workspace_bytes_f64(Dl, Dr, chi);
+  return ptn_bond_workspace_bytes(Dl, Dr, chi, prec);
 }
 
 ptn_status ptn_expm_site(ptn_c128* a, const ptn_c128* w, const ptn_c128* l, const ptn_c128* r,

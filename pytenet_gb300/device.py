@@ -3,6 +3,8 @@ Device plumbing: PyTorch is used only for device memory, streams and graph
 capture. All arithmetic happens in the CUDA kernels of libptn_gb300.so.
 """
 
+import warnings
+
 import numpy as np
 import torch
 
@@ -90,12 +92,45 @@ class Workspace:
 
     def __init__(self):
         self.buf = None
+        self.refused = None   # the smallest size that the device had no memory for
 
-    def get(self, nbytes):
+    def get(self, nbytes, least=None):
+        """A buffer of nbytes, or where the device has no memory for that, of at least least()
+        (None: nbytes); then use what fits, min(nbytes, buf.numel())."""
         nbytes = max(int(nbytes), 256)
-        if self.buf is None or self.buf.numel() < nbytes:
-            self.buf = torch.empty(nbytes, dtype=torch.uint8, device=device())
+        if self.buf is not None and self.buf.numel() >= nbytes:
+            return self.buf
+        if least is None or self.refused is None or nbytes < self.refused:
+            try:
+                self.buf = torch.empty(nbytes, dtype=torch.uint8, device=device())
+                return self.buf
+            except torch.cuda.OutOfMemoryError:
+                if least is None:
+                    raise
+                self.refused = nbytes
+        low = max(int(least()), 256)
+        if self.buf is None or self.buf.numel() < low:
+            self.buf = None
+            self.buf = torch.empty(low, dtype=torch.uint8, device=device())
         return self.buf
+
+    def room(self, nbytes, least):
+        """(buffer, bytes of it to use) of get(nbytes, least)."""
+        nbytes = max(int(nbytes), 256)
+        buf = self.get(nbytes, least)
+        return buf, min(nbytes, buf.numel())
+
+    def for_precision(self, query, prec):
+        """Workspace of a contraction: (buffer, bytes, precision to call it with), `query` the
+        size as a function of the precision. Where the device has no memory for it the FP64
+        form takes the DMMA kernels, and the mixed form becomes the FP64 form on those."""
+        need = query(prec)
+        buf, n = self.room(need, lambda: query(_lib.PREC_FP64_DMMA))
+        if n < need and prec == _lib.PREC_SPLIT_BF16:
+            warnings.warn(f"no device memory for the {need / 2**30:.1f} GB workspace of the mixed "
+                          "form: FP64 kernels", RuntimeWarning, stacklevel=3)
+            prec = _lib.PREC_FP64
+        return buf, n, prec
 
     def ptr(self, nbytes):
         return self.get(nbytes).data_ptr(), max(int(nbytes), 256)

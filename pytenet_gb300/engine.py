@@ -24,7 +24,7 @@ from .device import CDT, Workspace, call, device, empty, lib, ptr, stream_ptr, t
 from .qnumber import is_qsparse, qnumber_flatten, qr_plan
 
 PREC = {"fp64": _lib.PREC_FP64, "plain": _lib.PREC_FP64, "mixed": _lib.PREC_SPLIT_BF16,
-        "split-bf16": _lib.PREC_SPLIT_BF16}
+        "split-bf16": _lib.PREC_SPLIT_BF16, "fp64-dmma": _lib.PREC_FP64_DMMA}
 # smallest bond dimension (both sides) at which the mixed form uses the tensor cores
 MIXED_MIN_BOND = 32
 
@@ -61,6 +61,7 @@ class DeviceMPS:
         self.scratch = QRScratch()
         self.nrm_dev = torch.zeros(1, dtype=torch.float64, device=device())
         self.one = torch.ones(1, dtype=CDT, device=device())
+        self.dmma = False   # products by the DMMA kernels at every size
 
     # ---------------------------------------------------------------- views
     def site(self, i):
@@ -84,8 +85,8 @@ class DeviceMPS:
         c = self.cbuf[: K * n].view(K, n)
         a = self.buf[i]
         if plan.dense:
-            wsb = L.ptn_qr_workspace_bytes(m, n)
-            ws = self.qr_ws.get(wsb)
+            ws, wsb = self.qr_ws.room(L.ptn_qr_workspace_bytes(m, n),
+                                      lambda: L.ptn_qr_least_workspace_bytes(m, n))
             call(L.ptn_qr, ptr(a), m, n, ptr(a), K, ptr(c), n, ptr(ws), wsb, st)
         else:
             src = self.tmp[: m * n]
@@ -109,8 +110,8 @@ class DeviceMPS:
         if plan.dense:
             work = self.work[: m * n]
             call(L.ptn_transpose_210, ptr(a), ptr(work), Dl, d, Dr, st)
-            wsb = L.ptn_qr_workspace_bytes(m, n)
-            ws = self.qr_ws.get(wsb)
+            ws, wsb = self.qr_ws.room(L.ptn_qr_workspace_bytes(m, n),
+                                      lambda: L.ptn_qr_least_workspace_bytes(m, n))
             r = self.rbuf[: K * n]
             call(L.ptn_qr, ptr(work), m, n, ptr(work), K, ptr(r), n, ptr(ws), wsb, st)
             call(L.ptn_transpose_210, ptr(work), ptr(a), Dr, d, K, st)
@@ -135,8 +136,8 @@ class DeviceMPS:
             call(L.ptn_zgemm_split_bf16, ptr(a), K, ptr(b), N, ptr(out), N, M, N, K, ptr(ws),
                  wsb, st)
             return
-        wsb = L.ptn_zgemm_workspace_bytes(M, N, K, 1)
-        ws = self.gemm_ws.get(wsb)
+        wsb = 0 if self.dmma else L.ptn_zgemm_workspace_bytes(M, N, K, 1)
+        ws, wsb = self.gemm_ws.room(wsb, lambda: 0)
         call(L.ptn_zgemm, b"N", b"N", M, N, K, _lib.cval(1), ptr(a), K, 0, ptr(b), N, 0,
              _lib.cval(0), ptr(out), N, 0, 1, ptr(ws), wsb, st)
 
@@ -234,6 +235,7 @@ class Chain(DeviceMPS):
         assert len(op.a) == len(psi.a)
         super().__init__(psi)
         self.prec = prec_code(precision)
+        self.dmma = self.prec == _lib.PREC_FP64_DMMA
         self.mixed_min_bond = MIXED_MIN_BOND if mixed_min_bond is None else int(mixed_min_bond)
         self.numiter = int(numiter)
         if not 1 <= self.numiter < _lib.KRYLOV_MAXITER:
@@ -253,17 +255,22 @@ class Chain(DeviceMPS):
         self.state = torch.zeros(lib().ptn_krylov_state_bytes(), dtype=torch.uint8, device=device())
         self.cws = Workspace()
         L = lib()
-        need = 0
-        for i in range(Lx):
-            Dl, d, Dr = self.shape[i]
-            cl, cr = self.chi[i], self.chi[i + 1]
-            for p in {self.prec, _lib.PREC_FP64}:
-                need = max(need, L.ptn_site_step_workspace_bytes(Dl, d, Dr, cl, cr, p),
-                           L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, p),
-                           L.ptn_bond_step_workspace_bytes(Dr, Dr, cr, p),
-                           L.ptn_bond_step_workspace_bytes(Dl, Dl, cl, p))
-        self.cws_bytes = need
-        self.cws.get(need)
+
+        def need(prec):
+            """The largest workspace of a local step or environment at this precision."""
+            forms = {prec, _lib.PREC_FP64} if prec == _lib.PREC_SPLIT_BF16 else {prec}
+            n = 0
+            for i in range(Lx):
+                Dl, d, Dr = self.shape[i]
+                cl, cr = self.chi[i], self.chi[i + 1]
+                for p in forms:
+                    n = max(n, L.ptn_site_step_workspace_bytes(Dl, d, Dr, cl, cr, p),
+                            L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, p),
+                            L.ptn_bond_step_workspace_bytes(Dr, Dr, cr, p),
+                            L.ptn_bond_step_workspace_bytes(Dl, Dl, cl, p))
+            return n
+
+        _, self.cws_bytes, self.prec = self.cws.for_precision(need, self.prec)
         self.depth = depth
 
     def prec_for(self, Dl, Dr):
@@ -275,7 +282,7 @@ class Chain(DeviceMPS):
         does. The batched driver raises it per bucket: a tensor-core GEMM CTA takes a
         whole SM's shared memory and tensor memory, so small problems of concurrent
         instances overlap better on the FP64 path."""
-        if self.prec != _lib.PREC_FP64 and min(Dl, Dr) < self.mixed_min_bond:
+        if self.prec == _lib.PREC_SPLIT_BF16 and min(Dl, Dr) < self.mixed_min_bond:
             return _lib.PREC_FP64
         return self.prec
 
@@ -381,7 +388,7 @@ class Chain(DeviceMPS):
     def mixed_absorb(self, c, i):
         """Whether absorbing the bond matrix c into site i runs on the tensor cores:
         the mixed form, with every dimension of the product at least mixed_min_bond."""
-        if self.prec == _lib.PREC_FP64:
+        if self.prec != _lib.PREC_SPLIT_BF16:
             return False
         Dl, d, Dr = self.shape[i]
         return min(c.shape[0], c.shape[1], Dl, Dr) >= self.mixed_min_bond

@@ -75,7 +75,7 @@ class TwoSiteRun:
         psi.qbonds = [q.copy() for q in self.qbonds]
 
     def prec_for(self, Dl, Dr):
-        if self.prec != _lib.PREC_FP64 and min(Dl, Dr) < MIXED_MIN_BOND:
+        if self.prec == _lib.PREC_SPLIT_BF16 and min(Dl, Dr) < MIXED_MIN_BOND:
             return _lib.PREC_FP64
         return self.prec
 
@@ -103,9 +103,8 @@ class TwoSiteRun:
         Dl, d, Dr = self.a[i].shape
         cl, cr = self.chi[i], self.chi[i + 1]
         out = empty((Dr, cr, Dr))
-        prec = self.prec_for(Dl, Dr)
-        wsb = L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, prec)
-        ws = self.ws.get(wsb)
+        ws, wsb, prec = self.ws.for_precision(
+            lambda p: L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, p), self.prec_for(Dl, Dr))
         call(L.ptn_env_step_left, ptr(self.a[i]), ptr(self.a[i]), ptr(self.w[i]),
              ptr(self.lenv[i]), ptr(out), Dl, d, Dr, cl, cr, prec, ptr(ws), wsb, st)
         self.lenv[i + 1] = out
@@ -116,9 +115,8 @@ class TwoSiteRun:
         Dl, d, Dr = self.a[i].shape
         cl, cr = self.chi[i], self.chi[i + 1]
         out = empty((Dl, cl, Dl))
-        prec = self.prec_for(Dl, Dr)
-        wsb = L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, prec)
-        ws = self.ws.get(wsb)
+        ws, wsb, prec = self.ws.for_precision(
+            lambda p: L.ptn_env_workspace_bytes(Dl, d, Dr, cl, cr, p), self.prec_for(Dl, Dr))
         call(L.ptn_env_step_right, ptr(self.a[i]), ptr(self.a[i]), ptr(self.w[i]),
              ptr(self.renv[i]), ptr(out), Dl, d, Dr, cl, cr, prec, ptr(ws), wsb, st)
         self.renv[i - 1] = out
@@ -133,9 +131,8 @@ class TwoSiteRun:
         L, st = lib(), stream_ptr()
         Dl, dd, Dr = x.shape
         z = -complex(dt)
-        prec = self.prec_for(Dl, Dr)
-        wsb = L.ptn_site_step_workspace_bytes(Dl, dd, Dr, cl, cr, prec)
-        ws = self.ws.get(wsb)
+        ws, wsb, prec = self.ws.for_precision(
+            lambda p: L.ptn_site_step_workspace_bytes(Dl, dd, Dr, cl, cr, p), self.prec_for(Dl, Dr))
         V = self._krylov_buffers(Dl * dd * Dr)
         call(L.ptn_expm_site, ptr(x), ptr(w), ptr(l), ptr(r), Dl, dd, Dr, cl, cr, z.real, z.imag,
              self.numiter, prec, ptr(V), ptr(self.state), ptr(ws), wsb, st)
@@ -144,9 +141,8 @@ class TwoSiteRun:
         """x <- lowest Ritz vector of H_eff (_minimize_local_energy, dmrg.py:181-189)."""
         L, st = lib(), stream_ptr()
         Dl, dd, Dr = x.shape
-        prec = self.prec_for(Dl, Dr)
-        wsb = L.ptn_site_step_workspace_bytes(Dl, dd, Dr, cl, cr, prec)
-        ws = self.ws.get(wsb)
+        ws, wsb, prec = self.ws.for_precision(
+            lambda p: L.ptn_site_step_workspace_bytes(Dl, dd, Dr, cl, cr, p), self.prec_for(Dl, Dr))
         V = self._krylov_buffers(Dl * dd * Dr)
         call(L.ptn_eigh_site, ptr(x), ptr(w), ptr(l), ptr(r), Dl, dd, Dr, cl, cr, self.numiter,
              prec, ptr(V), ptr(self.state), ptr(ws), wsb, st)
@@ -159,8 +155,8 @@ class TwoSiteRun:
         assert Dm == Dm2
         out = empty((Dl, d0 * d1, Dr))
         M, N, K = Dl * d0, d1 * Dr, Dm
-        wsb = L.ptn_zgemm_workspace_bytes(M, N, K, 1)
-        ws = self.gws.get(wsb)
+        wsb = 0 if self.prec == _lib.PREC_FP64_DMMA else L.ptn_zgemm_workspace_bytes(M, N, K, 1)
+        ws, wsb = self.gws.room(wsb, lambda: 0)
         call(L.ptn_zgemm, b"N", b"N", M, N, K, _lib.cval(1), ptr(self.a[i]), K, 0,
              ptr(self.a[i + 1]), N, 0, _lib.cval(0), ptr(out), N, 0, 1, ptr(ws), wsb, st)
         return out
