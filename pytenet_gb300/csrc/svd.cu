@@ -40,6 +40,7 @@
 // L2 (1.53 of it) -> 1.83 ms (FP32 sweeps 0.96, GEMMs 0.25, one FP64 sweep 0.57) -> 1.31 ms
 // (the last check on a Gram matrix).
 #include "ptn_common.cuh"
+#include "fp64_seed.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
 #include <mutex>
@@ -150,15 +151,6 @@ __device__ __forceinline__ float scaled_float(double x, int h) {
   if (((b >> 52) & 0x7FF) == 0 || e <= 0) return __uint_as_float(sign);
   if (e >= 255) return __uint_as_float(sign | 0x7F800000u);
   return __uint_as_float(sign | ((unsigned)e << 23) | ((unsigned)(b >> 29) & 0x7FFFFFu));
-}
-
-// 1 / sqrt(x^2 + y^2) to FP64 accuracy from an FP32 seed (one third-order step), for sums
-// near 1 .. 2
-__device__ __forceinline__ double inv_norm(double x, double y) {
-  const double d = fma(x, x, y * y);
-  const double s = (double)rsqrtf((float)d);
-  const double e = fma(-d * s, s, 1.0);
-  return fma(s * e, fma(e, 0.375, 0.5), s);
 }
 
 // FP64 throughout: columns of very different size, or near the lower end of the range. The
