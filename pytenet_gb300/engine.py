@@ -59,6 +59,9 @@ class DeviceMPS:
         self.qr_ws = Workspace()
         self.gemm_ws = Workspace()
         self.scratch = QRScratch()
+        # plans of the last QR at every site and side: kernels read their device maps, so a
+        # captured graph needs them for as long as it lives, whatever the plan cache drops
+        self.plans = {}
         self.nrm_dev = torch.zeros(1, dtype=torch.float64, device=device())
         self.one = torch.ones(1, dtype=CDT, device=device())
         self.dmma = False   # products by the DMMA kernels at every size
@@ -81,6 +84,7 @@ class DeviceMPS:
         Dl, d, Dr = self.shape[i]
         m, n = Dl * d, Dr
         plan = qr_plan(qnumber_flatten((self.qbonds[i], self.qsite)), self.qbonds[i + 1])
+        self.plans[i, "left"] = plan
         K = plan.K
         c = self.cbuf[: K * n].view(K, n)
         a = self.buf[i]
@@ -104,6 +108,7 @@ class DeviceMPS:
         Dl, d, Dr = self.shape[i]
         m, n = Dr * d, Dl
         plan = qr_plan(qnumber_flatten((-self.qbonds[i + 1], self.qsite)), -self.qbonds[i])
+        self.plans[i, "right"] = plan
         K = plan.K
         c = self.cbuf[: n * K].view(n, K)
         a = self.buf[i]

@@ -48,6 +48,7 @@ class TDVPRun:
         self.use_graph = graph
         self.graph = None
         self.graph_dt = None
+        self.graph_plans = None
         self.steps_done = 0
 
     def _state_key(self):
@@ -78,6 +79,7 @@ class TDVPRun:
             assert self._state_key() == before
             self.graph = g
             self.graph_dt = dt
+            self.graph_plans = dict(self.chain.plans)   # read by the graph's kernels
 
     def download(self):
         self.chain.download(self.psi)

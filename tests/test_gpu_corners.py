@@ -166,3 +166,34 @@ def test_infinities_and_nans_through_contractions(bad, where):
         fx, fy = (np.isfinite(t.real) & np.isfinite(t.imag) for t in (x, y))
         assert np.array_equal(fx, fy)
         assert np.linalg.norm(x[fx] - y[fy]) <= 1e-13 * np.linalg.norm(y[fy])
+
+
+def test_graph_keeps_the_plans_it_reads():
+    """The kernels of a captured step read index maps that belong to QR plans: a plan cache that
+    is emptied (as it is when it is full) must not free them, nor steps with another dt."""
+    import gc
+    import weakref
+    import pytenet_gb300 as ptg
+    from pytenet_gb300 import qnumber
+    rng = np.random.default_rng(5)
+    h = ptg.heisenberg_xxz_1d_mpo(10, 1.0, 0.8, -0.1)
+    psi = u1_state(ptg, h, 10, 24, rng)
+    psi.orthonormalize(mode="left")
+    run = ptg.TDVPRun(h, psi, numiter_lanczos=4, graph=True)
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        run.step(0.02j)
+        assert run.graph is not None
+        captured = list(run.chain.plans.values())
+        maps = [m[0].data_ptr() for p in captured for e in p.dev_cache.values()
+                if isinstance(e, list) for m in e]
+        alive = [weakref.ref(p) for p in captured]
+        del captured
+        qnumber._PLANS.clear()
+        run.use_graph = False
+        run.step(0.01j)   # by new plans
+        run.use_graph = True
+        gc.collect()
+        assert maps and all(r() is not None for r in alive)
+        run.step(0.02j)   # the graph again
+    assert all(np.isfinite(x).all() for x in run.download().a)
