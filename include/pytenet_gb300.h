@@ -46,13 +46,13 @@ typedef enum {
 typedef enum {
   PTN_PREC_FP64 = 0,        /* plain complex128: FP64 DMMA, and for products of at least 32 in
                                every dimension and 1e6 complex multiply-adds exact products of
-                               residues modulo 14 numbers on tcgen05. Rows are fixed-point numbers
-                               of 53-54 bits there, after a scaling of the summed index taken from
-                               one operand (B): error of (m, n) per term 2^-53 of the largest
-                               |A[m, k] B[n', k]| over k and n', less where B's column n is below
-                               the others; row, column and index scalings cancel. A result far
-                               below the others of its row keeps that error, where DMMA sums of
-                               |A[m, k] B[n, k]| alone bound it */
+                               residues modulo 14 numbers on tcgen05. Rows of A and columns of B
+                               are fixed-point numbers of 53-54 bits there, after a scaling of
+                               the summed index by powers of two. Scalings of rows, columns and
+                               index cancel; otherwise the error is normwise (2^-53 per term of
+                               the largest |A[m, k] B[n, k]| of the row or of the product): a
+                               result far below the others keeps their error, where the DMMA
+                               kernel's is bounded by its own sum of |A[m, k] B[n, k]| */
   PTN_PREC_SPLIT_BF16 = 1,  /* fewer moduli: 11 in the local operators (40-44 bits per
                                row-scaled value, 39 in sums of more than 16384 terms; ~1e-12
                                relative per contraction), 13 in the environment steps (49-53

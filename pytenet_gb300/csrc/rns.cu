@@ -215,8 +215,9 @@ __device__ __forceinline__ int row_exp(double2 z, int s) {
 // Largest finite exponent of every term of an operand (EXP_NONE: zeros); terms k = (o, i), i <
 // in, in > 1: f[o], the largest of its terms, and be[k] relative to it. A view whose rows are
 // next to each other: `wpt` warps take a term, or a CTA the terms of an o; otherwise (in = 1) a
-// lane takes a term and the warps of the CTA share its rows. Two operands in one launch. Bound:
-// memory (the operand read once), latency where it is small.
+// CTA takes TERM_COLS terms (64 bytes of a row). Several operands in one launch.
+// Bound: memory (the operands read once), latency where they are small.
+constexpr int TERM_COLS = 4;
 struct TermJob {
   RnsView v;
   int rows, kc, in;
@@ -224,13 +225,22 @@ struct TermJob {
   int wpt, ctas;
 };
 
-__global__ void __launch_bounds__(256) k_term_exp(const TermJob j0, const TermJob j1, const int* skip) {
+struct TermJobs {
+  TermJob j[RNS_TERM_JOBS];
+};
+
+__global__ void __launch_bounds__(256) k_term_exp(const TermJobs jobs, const int* skip) {
   grid_wait();
   if (skip != nullptr && *skip != 0) return;
-  __shared__ int s_max[8][32];
-  const bool second = (int)blockIdx.x >= j0.ctas;
-  const TermJob j = second ? j1 : j0;
-  const int b = second ? (int)blockIdx.x - j0.ctas : (int)blockIdx.x;
+  __shared__ int s_max[8][TERM_COLS];
+  int b = blockIdx.x;
+  TermJob j = jobs.j[0];
+#pragma unroll
+  for (int i = 1; i < RNS_TERM_JOBS; ++i)
+    if (b >= j.ctas) {
+      b -= j.ctas;
+      j = jobs.j[i];
+    }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int m = EXP_NONE;
   // entries first, first + step, ... < rows, `stride` apart: eight loads in flight
@@ -279,14 +289,15 @@ __global__ void __launch_bounds__(256) k_term_exp(const TermJob j0, const TermJo
       j.be[k] = m;
     }
   } else {
-    const int k = b * 32 + lane;
-    if (k < j.kc) {
-      const double2* src = j.v.src + (long)k * j.v.sk;
-      take(src, j.v.sr, warp, 8);
-    }
-    s_max[warp][lane] = m;
+    const int k = b * TERM_COLS + (lane & (TERM_COLS - 1));
+    if (k < j.kc)
+      take(j.v.src + (long)k * j.v.sk, j.v.sr, warp * (32 / TERM_COLS) + lane / TERM_COLS,
+           256 / TERM_COLS);
+#pragma unroll
+    for (int o = TERM_COLS; o < 32; o *= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane < TERM_COLS) s_max[warp][lane] = m;
     __syncthreads();
-    if (warp == 0 && k < j.kc) {
+    if (warp == 0 && lane < TERM_COLS && k < j.kc) {
       for (int w = 1; w < 8; ++w) m = max(m, s_max[w][lane]);
       j.be[k] = m;
     }
@@ -294,21 +305,21 @@ __global__ void __launch_bounds__(256) k_term_exp(const TermJob j0, const TermJo
 }
 
 // What a conversion does to the terms of its operand: nothing (t null), forms the scaling t
-// from be and f and applies its inverse (`source`, the operand that they were taken from), or
-// applies t (the other one).
+// and applies its inverse (`source`), or applies t (the other operand).
 struct TermScale {
-  const int *be, *f;
+  const int *be, *f, *o;
   int* t;
-  int in;
+  int in, odiv, omod;
   bool source;
 };
 
-// whole pairs of bits below the largest: terms of about the same size (a factor of four) stay
-// as they are
-__device__ __forceinline__ int in_pairs(int below) { return below & ~1; }
-
-// powers of two that the terms [k0, k0 + kn) of the operand take, to sh (shared memory, behind a
-// barrier of the caller's); the `writer` CTA of these terms leaves t for the other operand
+// Powers of two that the terms [k0, k0 + kn) of the operand take, to sh (shared memory, behind a
+// barrier of the caller's); the `writer` CTA of these terms leaves t for the other operand.
+//   The other operand's sizes o known: largest entries a_k (other) and b_k (source) meet in a
+// product of 2^S at most, S = max (a_k + b_k); the rows lose the bits by which max a + max b
+// exceeds S. Every t with b_k - H <= t_k <= G - a_k, G + H = S, loses none: the one nearest to 0, so
+// that operands which do not grow against each other stay as they are.
+//   Not known: t from the source alone, whole pairs of bits below its largest terms.
 template <int NT>
 __device__ __forceinline__ void term_shifts(const TermScale& ts, int K, int k0, int kn, int* sh,
                                             bool writer) {
@@ -316,16 +327,52 @@ __device__ __forceinline__ void term_shifts(const TermScale& ts, int K, int k0, 
     for (int k = threadIdx.x; k < kn; k += NT) sh[k] = ts.t[k0 + k];
     return;
   }
-  __shared__ int s_top[NT / 32], s_g[RNS_INNER_MAX];
+  constexpr int NW = NT / 32;
+  __shared__ int s_top[3][NW], s_g[RNS_INNER_MAX];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (ts.o != nullptr) {
+    auto other = [&](int k) { return ts.o[(k / ts.odiv) % ts.omod]; };
+    int a = EXP_NONE, b = EXP_NONE, both = 2 * EXP_NONE;
+    for (int k = threadIdx.x; k < K; k += NT) {
+      const int ok = other(k), bk = ts.be[k];
+      a = max(a, ok);
+      b = max(b, bk);
+      both = max(both, ok + bk);
+    }
+    a = __reduce_max_sync(0xffffffffu, a);
+    b = __reduce_max_sync(0xffffffffu, b);
+    both = __reduce_max_sync(0xffffffffu, both);
+    if (lane == 0) {
+      s_top[0][warp] = a;
+      s_top[1][warp] = b;
+      s_top[2][warp] = both;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      a = max(a, s_top[0][w]);
+      b = max(b, s_top[1][w]);
+      both = max(both, s_top[2][w]);
+    }
+    const int loss = both > EXP_NONE / 2 ? a + b - both : 0;   // no common term: nothing to lose
+    const int ga = a - loss / 2, hb = b - (loss - loss / 2);   // G, H
+    for (int q = threadIdx.x; q < kn; q += NT) {
+      const int k = k0 + q, ok = other(k), bk = ts.be[k];
+      const int t = loss < 2 ? 0 : max(bk - hb, min(ga - ok, 0));
+      sh[q] = ok == EXP_NONE ? TERM_DROP : -t;
+      if (writer) ts.t[k] = bk == EXP_NONE ? TERM_DROP : t;
+    }
+    return;
+  }
   const int no = K / ts.in;
   const int* f = ts.in > 1 ? ts.f : ts.be;
+  auto in_pairs = [](int below) { return below & ~1; };
   int top = EXP_NONE;
   for (int o = threadIdx.x; o < no; o += NT) top = max(top, f[o]);
   top = __reduce_max_sync(0xffffffffu, top);
-  if (lane == 0) s_top[warp] = top;
+  if (lane == 0) s_top[0][warp] = top;
   if (ts.in > 1)
-    for (int i = warp; i < ts.in; i += NT / 32) {
+    for (int i = warp; i < ts.in; i += NW) {
       int g = EXP_NONE;
       for (int o = lane; o < no; o += 32) g = max(g, ts.be[o * ts.in + i]);
       g = __reduce_max_sync(0xffffffffu, g);
@@ -333,7 +380,7 @@ __device__ __forceinline__ void term_shifts(const TermScale& ts, int K, int k0, 
     }
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < NT / 32; ++w) top = max(top, s_top[w]);
+  for (int w = 0; w < NW; ++w) top = max(top, s_top[0][w]);
   for (int q = threadIdx.x; q < kn; q += NT) {
     const int k = k0 + q, o = k / ts.in;
     const int t = ts.be[k] == EXP_NONE ? TERM_DROP
@@ -1286,7 +1333,9 @@ ptn_status rns_convert(const RnsView& v, const RnsOperand& d, bool have_exp, con
   const int bits = rns_bits(d.kc, d.nm);
   PTN_CHECK_ARG(bits != 0, "rns_convert: products of %d terms are too long", d.kc);
   TermScale ts{};
-  if (terms != nullptr) ts = TermScale{terms->be, terms->f, terms->t, terms->in, source};
+  if (terms != nullptr)
+    ts = TermScale{terms->be, terms->f, terms->o, terms->t, terms->in, terms->odiv, terms->omod,
+                   source};
   switch (d.nm) {
     case RNS_FP64: return convert<RNS_FP64>(v, d, have_exp, bits, clear, nclear, ts, skip, st);
     case RNS_MIXED_ENV:
@@ -1296,25 +1345,19 @@ ptn_status rns_convert(const RnsView& v, const RnsOperand& d, bool have_exp, con
 }
 
 ptn_status rns_term_exps(const RnsTermsOf* of, int n, const int* skip, cudaStream_t st) {
-  TermJob j[2] = {};
+  TermJobs jobs = {};
   int ctas = 0;
   for (int i = 0; i < n; ++i) {
-    j[i].v = of[i].v;
-    j[i].rows = of[i].rows;
-    j[i].kc = of[i].kc;
-    j[i].be = of[i].terms->be;
-    j[i].f = of[i].terms->f;
-    j[i].in = of[i].terms->in;
-    PTN_CHECK_ARG(j[i].in == 1 || (of[i].v.sr == 1 && of[i].kc % j[i].in == 0),
-                  "rns_term_exps: bad layout");
+    TermJob& j = jobs.j[i];
+    j = TermJob{of[i].v, of[i].rows, of[i].kc, of[i].in, of[i].be, of[i].f, 0, 0};
+    PTN_CHECK_ARG(j.in == 1 || (j.v.sr == 1 && j.kc % j.in == 0), "rns_term_exps: bad layout");
     // warps of a term: up to four rows per lane
-    j[i].wpt = of[i].v.sr != 1 ? 0 : of[i].rows <= 128 ? 1 : of[i].rows <= 256 ? 2
-                                   : of[i].rows <= 512 ? 4 : 8;
-    const int per = j[i].in > 1 ? j[i].in : j[i].wpt == 0 ? 32 : 8 / j[i].wpt;
-    j[i].ctas = (of[i].kc + per - 1) / per;
-    ctas += j[i].ctas;
+    j.wpt = j.v.sr != 1 ? 0 : j.rows <= 128 ? 1 : j.rows <= 256 ? 2 : j.rows <= 512 ? 4 : 8;
+    const int per = j.in > 1 ? j.in : j.wpt == 0 ? TERM_COLS : 8 / j.wpt;
+    j.ctas = (j.kc + per - 1) / per;
+    ctas += j.ctas;
   }
-  PTN_CUDA_TRY(launch(k_term_exp, dim3(ctas), dim3(256), 0, st, j[0], j[1], skip));
+  PTN_CUDA_TRY(launch(k_term_exp, dim3(ctas), dim3(256), 0, st, jobs, skip));
   note_launches(1);
   return PTN_OK;
 }

@@ -38,30 +38,35 @@ struct RnsOperand {
 // Powers of two on the terms of a product (FP64 form): A[m, k] 2^t[k] and B[n, k] 2^-t[k] have
 // the same product. Rows are fixed-point numbers, so operands that grow and decay against each
 // other along k (the two sides of a bond in a gauge A D, D^-1 B) would lose the bits of the
-// entries that count. With t from the largest entry of B in every term, B is of one size along
-// k; the error of a result (m, n) is then 2^-bits per term of the largest |A[m, k] B[n', k]| over
-// k and n', and further down by what B's row n lies below the others: scalings of the terms, of
-// the rows of A and of those of B cancel. Terms k = (o, i) of a bond o and an MPO bond i < in
-// take t = f[o] + g[i]: in a channel as sparse as the identity a term of its own size says
-// nothing about its bond. Relative error (Frobenius norm, scalings taken out) of A D times
-// D^-1 R D^-1 at bond 64, |D| spread over 1e6 / 1e12: 1.0e-11 / 7.2e-6 without, 3.3e-16 / 3.5e-16
-// with it (DMMA 2.7e-16 / 3.0e-16). The exponents are a launch of their own: H_eff at bonds
-// 250 x 256 110 -> 116 us, an environment step at 187 x 300 85.0 -> 88.7, at bonds of 1024 1 %.
-// be, f: exponents of the terms of the operand that t comes from. Null t: no scaling.
+// entries that count: relative error (Frobenius norm, scalings taken out) of A D times
+// D^-1 R D^-1 at bond 64, |D| spread over 1e6 / 1e12: 1.0e-11 / 7.2e-6 without, 3e-16 with
+// it (DMMA 3e-16). Where the sizes of both operands are known beforehand (o: of the other
+// one), t is what keeps the error at 2^-bits per term of the largest |A[m, k] B[n, k]|, and 0
+// where nothing is lost. An operator's planes are made before its vectors: t then comes
+// from the operator alone, which it brings to one size along k, so that the error of (m, n) is
+// 2^-bits per term of the largest |A[m, k] B[n', k]| over k and n', and further down by what
+// B's row n lies below the others. Either way scalings of the terms, of the rows of A and of those
+// of B cancel. Terms k = (o, i) of a bond o and an MPO bond i < in take t = f[o] + g[i]: in a
+// channel as sparse as the identity a term of its own size says nothing about its bond.
+// The exponents are a launch of their own: H_eff at bonds 250 x 256 110 -> 117 us, an
+// environment step at 187 x 300 85 -> 90, at bonds of 1024 1 %.
+// be, f, o: exponents of the terms of the operand that t comes from and of the other one (term k
+// at o[(k / odiv) % omod]; null: not known). Null t: no scaling.
 constexpr int RNS_INNER_MAX = 64;
+constexpr int RNS_TERM_JOBS = 4;
 struct RnsTerms {
-  int *be, *f, *t;
-  int in;
+  int *be, *f, *o, *t;
+  int in, odiv, omod;
 };
 
-// an operand whose terms' exponents are wanted
+// an operand whose terms' exponents are wanted (in > 1: be relative to f)
 struct RnsTermsOf {
   RnsView v;
-  int rows, kc;
-  const RnsTerms* terms;
+  int rows, kc, in;
+  int *be, *f;
 };
 
-// of one or two operands, one launch
+// of up to RNS_TERM_JOBS operands, one launch
 ptn_status rns_term_exps(const RnsTermsOf* of, int n, const int* skip, cudaStream_t st);
 
 // bytes of the planes / exponents / GEMM residues, each to be 256-byte aligned

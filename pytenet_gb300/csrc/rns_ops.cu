@@ -39,14 +39,23 @@ struct Carver {
     void* e = take((size_t)rows * sizeof(int));
     return rns_operand(p, e, rows, kc, nm);
   }
-  // kc = outer * inner terms
+  // scaling of outer * inner terms from one operand
   RnsTerms terms(long outer, int inner, int nm) {
-    RnsTerms t{nullptr, nullptr, nullptr, 1};
+    RnsTerms t{nullptr, nullptr, nullptr, nullptr, 1, 1, 1};
     if (nm != RNS_FP64) return t;
     if (inner <= RNS_INNER_MAX) t.in = inner;
     t.be = static_cast<int*>(take((size_t)outer * inner * sizeof(int)));
     t.f = static_cast<int*>(take((size_t)outer * sizeof(int)));
     t.t = static_cast<int*>(take((size_t)outer * inner * sizeof(int)));
+    return t;
+  }
+  // from both, the other one's term k at (k / odiv) % omod
+  RnsTerms terms_of_both(long kc, int odiv, int omod, int nm) {
+    RnsTerms t = terms(kc, 1, nm);
+    if (nm != RNS_FP64) return t;
+    t.o = static_cast<int*>(take((size_t)omod * sizeof(int)));
+    t.odiv = odiv;
+    t.omod = omod;
     return t;
   }
 };
@@ -102,7 +111,7 @@ BondWs bond_ws(Carver& c, int nm, int Dl, int Dr, int chi) {
 // a1 b1: first GEMM, a2 b2: second one
 struct EnvWs {
   RnsOperand a1, b1, a2, b2;
-  RnsTerms t1, t2;        // scaling of their terms, from the site tensors
+  RnsTerms t1, t2;        // scaling of their terms; of T2 the sizes that L (R) gives its terms
   double2* T2;
   void* res;
 };
@@ -113,8 +122,8 @@ EnvWs env_left_ws(Carver& c, int nm, int Dl, int d, int Dr, int cl, int cr) {
   w.b1 = c.operand((long)d * Dr, Dl, nm);              // conj(B), rows (t, rb), terms l2
   w.a2 = c.operand(Dr, (long)Dl * d, nm);              // A, rows ra, terms (l0, s)
   w.b2 = c.operand((long)cr * Dr, (long)Dl * d, nm);   // T2, rows (wr, rb), terms (l0, s)
-  w.t1 = c.terms(Dl, 1, nm);
-  w.t2 = c.terms((long)Dl * d, 1, nm);
+  w.t1 = c.terms_of_both(Dl, 1, Dl, nm);
+  w.t2 = c.terms_of_both((long)Dl * d, d, Dl, nm);
   w.T2 = static_cast<double2*>(c.take((size_t)Dl * d * cr * Dr * sizeof(double2)));
   w.res = c.take(std::max(rns_out_bytes((long)Dl * cl, (long)d * Dr, nm),
                           rns_out_bytes(Dr, (long)cr * Dr, nm)));
@@ -127,20 +136,21 @@ EnvWs env_right_ws(Carver& c, int nm, int Dl, int d, int Dr, int cl, int cr) {
   w.b1 = c.operand((long)cr * Dr, Dr, nm);             // R, rows (wr, r2), terms r0
   w.a2 = c.operand((long)Dl * cl, (long)d * Dr, nm);   // T2, rows (l0, wl), terms (t, r2)
   w.b2 = c.operand(Dl, (long)d * Dr, nm);              // conj(B), rows lb, terms (t, r2)
-  w.t1 = c.terms(Dr, 1, nm);
-  w.t2 = c.terms((long)d * Dr, 1, nm);
+  w.t1 = c.terms_of_both(Dr, 1, Dr, nm);
+  w.t2 = c.terms_of_both((long)d * Dr, 1, Dr, nm);
   w.T2 = static_cast<double2*>(c.take((size_t)Dl * cl * d * Dr * sizeof(double2)));
   w.res = c.take(std::max(rns_out_bytes((long)Dl * d, (long)cr * Dr, nm),
                           rns_out_bytes((long)Dl * cl, Dl, nm)));
   return w;
 }
 
-// exponents of the terms of the two operands that the scalings come from
-ptn_status term_exps(const RnsView& v1, const RnsOperand& o1, const RnsTerms& t1, const RnsView& v2,
-                     const RnsOperand& o2, const RnsTerms& t2, cudaStream_t st) {
-  if (t1.t == nullptr) return PTN_OK;
-  const RnsTermsOf of[2] = {{v1, o1.rows, o1.kc, &t1}, {v2, o2.rows, o2.kc, &t2}};
-  return rns_term_exps(of, 2, nullptr, st);
+RnsTermsOf source_terms(const RnsView& v, const RnsOperand& o, const RnsTerms& t) {
+  return {v, o.rows, o.kc, t.in, t.be, t.f};
+}
+
+// the other operand's, `rows` of them to each of t.omod terms
+RnsTermsOf other_terms(const RnsView& v, long rows, const RnsTerms& t) {
+  return {v, (int)rows, t.omod, 1, t.o, nullptr};
 }
 
 }  // namespace
@@ -162,7 +172,10 @@ ptn_status heff_prepare_rns(int nm, const double2* l, const double2* r, int Dl, 
   Carver c(ws);
   const HeffWs h = layout(c);
   const RnsView vr = view_r(r, Dr, cr), vl = view_l(l, Dl);
-  PTN_TRY(term_exps(vr, h.r, h.tr, vl, h.l, h.tl, st));
+  if (h.tr.t != nullptr) {
+    const RnsTermsOf of[2] = {source_terms(vr, h.r, h.tr), source_terms(vl, h.l, h.tl)};
+    PTN_TRY(rns_term_exps(of, 2, nullptr, st));
+  }
   PTN_TRY(rns_convert(vr, h.r, false, nullptr, st, nullptr, 0, &h.tr, true));
   return rns_convert(vl, h.l, false, nullptr, st, nullptr, 0, &h.tl, true);
 }
@@ -196,7 +209,10 @@ ptn_status bond_prepare_rns(int nm, const double2* l, const double2* r, int Dl, 
   Carver c(ws);
   const BondWs b = layout(c);
   const RnsView vr = view_r(r, Dr, chi), vl = view_l(l, Dl);
-  PTN_TRY(term_exps(vr, b.r, b.tr, vl, b.l, b.tl, st));
+  if (b.tr.t != nullptr) {
+    const RnsTermsOf of[2] = {source_terms(vr, b.r, b.tr), source_terms(vl, b.l, b.tl)};
+    PTN_TRY(rns_term_exps(of, 2, nullptr, st));
+  }
   PTN_TRY(rns_convert(vr, b.r, false, nullptr, st, nullptr, 0, &b.tr, true));
   return rns_convert(vl, b.l, false, nullptr, st, nullptr, 0, &b.tl, true);
 }
@@ -233,7 +249,13 @@ ptn_status env_left_rns(int nm, const double2* a, const double2* b, const double
   const EnvWs e = layout(c);
   const RnsView v1{l, Dl, 1, 0}, v2{b, 1, (long)d * Dr, 1}, v3{a, 1, Dr, 0},
       v4{e.T2, 1, (long)cr * Dr, 0};
-  PTN_TRY(term_exps(v2, e.b1, e.t1, v3, e.a2, e.t2, st));
+  if (e.t1.t != nullptr) {
+    // T2's terms (l0, s) are as large as L at l0
+    const RnsTermsOf of[4] = {source_terms(v2, e.b1, e.t1), other_terms(v1, e.a1.rows, e.t1),
+                              source_terms(v3, e.a2, e.t2),
+                              other_terms({l, 1, (long)cl * Dl, 0}, (long)cl * Dl, e.t2)};
+    PTN_TRY(rns_term_exps(of, 4, nullptr, st));
+  }
   PTN_TRY(rns_convert(v2, e.b1, false, nullptr, st, e.b2.e, e.b2.rows, &e.t1, true));
   PTN_TRY(rns_convert(v1, e.a1, false, nullptr, st, nullptr, 0, &e.t1));
   PTN_TRY(rns_convert(v3, e.a2, false, nullptr, st, nullptr, 0, &e.t2, true));
@@ -255,7 +277,13 @@ ptn_status env_right_rns(int nm, const double2* a, const double2* b, const doubl
   const EnvWs e = layout(c);
   const RnsView v1{a, Dr, 1, 0}, v2 = view_r(r, Dr, cr), v3{e.T2, (long)d * Dr, 1, 0},
       v4{b, (long)d * Dr, 1, 1};
-  PTN_TRY(term_exps(v1, e.a1, e.t1, v4, e.b2, e.t2, st));
+  if (e.t1.t != nullptr) {
+    // T2's terms (t, r2) are as large as R at r2
+    const RnsTermsOf of[4] = {source_terms(v1, e.a1, e.t1), other_terms(v2, e.b1.rows, e.t1),
+                              source_terms(v4, e.b2, e.t2),
+                              other_terms({r, Dr, 1, 0}, (long)Dr * cr, e.t2)};
+    PTN_TRY(rns_term_exps(of, 4, nullptr, st));
+  }
   PTN_TRY(rns_convert(v1, e.a1, false, nullptr, st, e.a2.e, e.a2.rows, &e.t1, true));
   PTN_TRY(rns_convert(v2, e.b1, false, nullptr, st, nullptr, 0, &e.t1));
   PTN_TRY(rns_convert(v4, e.b2, false, nullptr, st, nullptr, 0, &e.t2, true));
@@ -272,7 +300,7 @@ size_t zgemm_rns_workspace_bytes(int nm, long M, long N, long K) {
   Carver c(nullptr);
   c.operand(M, K, nm);
   c.operand(N, K, nm);
-  c.terms(K, 1, nm);
+  c.terms_of_both(K, 1, (int)K, nm);
   c.take(rns_out_bytes(M, N, nm));
   return c.off + 256;
 }
@@ -281,19 +309,19 @@ ptn_status zgemm_rns(int nm, const GemmArgs& g, void* ws, cudaStream_t st) {
   Carver c(reinterpret_cast<void*>(al(reinterpret_cast<uintptr_t>(ws))));
   const RnsOperand A = c.operand(g.M, g.K, nm);
   const RnsOperand B = c.operand(g.N, g.K, nm);
-  const RnsTerms terms = c.terms(g.K, 1, nm);
+  const RnsTerms terms = c.terms_of_both(g.K, 1, g.K, nm);
   void* res = c.take(0);
   // op(A) by rows, op(B) by columns
   const bool ta = g.opA == 'T' || g.opA == 'H', tb = g.opB == 'T' || g.opB == 'H';
   const bool ca = g.opA == 'C' || g.opA == 'H', cb = g.opB == 'C' || g.opB == 'H';
   const RnsView va = ta ? RnsView{g.A, 1, g.lda, ca} : RnsView{g.A, g.lda, 1, ca};
   const RnsView vb = tb ? RnsView{g.B, g.ldb, 1, cb} : RnsView{g.B, 1, g.ldb, cb};
-  // the scaling of the terms from the operand whose rows are next to each other, or that has
-  // fewer of them
-  const bool from_b = (va.sr == 1) != (vb.sr == 1) ? vb.sr == 1 : g.N <= g.M;
+  // which operand forms the scaling of the terms makes no difference: the shorter one
+  const bool from_b = g.N <= g.M;
   if (terms.t != nullptr) {
-    const RnsTermsOf of{from_b ? vb : va, from_b ? g.N : g.M, g.K, &terms};
-    PTN_TRY(rns_term_exps(&of, 1, g.skip, st));
+    const RnsTermsOf of[2] = {source_terms(from_b ? vb : va, from_b ? B : A, terms),
+                              other_terms(from_b ? va : vb, from_b ? g.M : g.N, terms)};
+    PTN_TRY(rns_term_exps(of, 2, g.skip, st));
   }
   if (from_b) PTN_TRY(rns_convert(vb, B, false, g.skip, st, nullptr, 0, &terms, true));
   PTN_TRY(rns_convert(va, A, false, g.skip, st, nullptr, 0, &terms, !from_b));
