@@ -119,8 +119,8 @@ uint64_t ptn_launch_count(void);
  *                              other streams set 0. Vectors of at most 2^14 entries take
  *                              one launch of a single cluster under either value.
  *   PTN_TUNE_QR_PANEL          QR panel kernel: 0 (default) one cluster-wide reduction per
- *                              column (dot products, Gram entries and the next pivot's
- *                              norm together), rows in registers, and Q formed in blocks
+ *                              column (dot products, Gram entries and the pivot's norm
+ *                              together), rows in shared memory, and Q formed in blocks
  *                              of 128 reflectors on the tensor cores where they are large;
  *                              3 two warps per 32-row group with a shuffle reduce-scatter
  *                              and two barriers per column; 1 the earlier

@@ -13,12 +13,13 @@
 // A breakdown sets state->stopped: all later passes (and the operator launches,
 // which test the same flag) return immediately, m_used keeps the truncated size,
 // exactly the early return of krylov.py:44-50.
-// The tridiagonal eigenproblem (eigh_tridiag, krylov.py:142-150) is solved by one
-// warp with the implicit QL algorithm with Wilkinson shifts (Bowdler, Martin,
-// Reinsch, Wilkinson 1968); lane k carries row k of the eigenvector matrix, every
-// lane runs the same scalar recurrence, so no synchronisation is needed.
-// expm_krylov (krylov.py:122-136) and eigh_krylov (krylov.py:110-119) then reduce
-// to coefficients c_k and one combination pass out = sum_k c_k V[k].
+// expm_krylov (krylov.py:122-136) and the lowest pair of eigh_krylov (krylov.py:110-119)
+// reduce to coefficients c_k and one combination pass out = sum_k c_k V[k]. One warp forms
+// them: scaled Taylor on the vector for the exponential, bisection and inverse iteration for
+// the lowest pair. The whole tridiagonal eigenproblem (eigh_tridiag, krylov.py:142-150), and
+// what those two hand on, is solved by the implicit QL algorithm with Wilkinson shifts (Bowdler,
+// Martin, Reinsch, Wilkinson 1968); lane k carries row k of the eigenvector matrix, every lane
+// runs the same scalar recurrence, so no synchronisation is needed.
 #include "ptn_common.cuh"
 #include "launch.cuh"
 #include "fp64_seed.cuh"

@@ -547,8 +547,6 @@ __global__ void __launch_bounds__(ST) svd_pre_kernel(const double2* __restrict__
   cluster.sync();
 }
 
-// W (p x r) and V (r x r) are column-major scratch; u, vh row-major outputs. `pre`: W and V
-// hold the start of the sweeps unless *bad.
 // whether a pair of the Gram matrix H = W^H W is further from orthogonal than tol, by the
 // cluster: the test that a sweep makes pair by pair, with its exceptions (columns near the
 // lower end of the range are left to it)
@@ -576,6 +574,8 @@ __device__ bool pair_left(const double2* __restrict__ H, int r, float tol) {
   return s_left != 0;
 }
 
+// W (p x r) and V (r x r) are column-major scratch; u, vh row-major outputs. `pre`: W and V
+// hold the start of the sweeps unless *bad.
 __global__ void __launch_bounds__(ST) svd_jacobi_kernel(const double2* __restrict__ a, int m, int n,
                                                        long lda, double2* __restrict__ W,
                                                        double2* __restrict__ V,
