@@ -1261,15 +1261,15 @@ int rns_bits(long K, int nm) {
   return bits >= (nm == RNS_FP64 ? 53 : 39) ? bits : 0;
 }
 
-// The fixed cost of the path (conversions, planes, reconstruction: 12 us for a single GEMM)
-// meets the DMMA kernel near 1e6 complex products. Measured, the GEMMs of H_eff at bond D
-// and MPO bond 5 alone (first / second, DMMA -> residues):
-//   D = 40: 9.7 -> 12.5, 12.9 -> 16.5 us;  48: 14.3 -> 12.4, 24.8 -> 16.8;  64: 30.3 -> 12.8,
-//   28.1 -> 17.8;  128: 184 -> 21, 217 -> 22;  256: 1419 -> 54, 1458 -> 45;  512: 11275 -> 188,
-//   11606 -> 159
-// and a Lanczos step (operands of the operator converted once):
-//   D = 40: 43 -> 44 us;  48: 57 -> 42;  64: 77 -> 43;  128: 426 -> 59;  256: 2908 -> 119;
-//   512: 22961 -> 376
+// The fixed cost of the path (exponents, conversions, planes, reconstruction: 16 us for a single
+// GEMM) meets the DMMA kernel between 1e6 and 2e6 complex products, that of a Lanczos step
+// (operands of the operator converted once) at 1e6. Measured, the GEMMs of H_eff at bond D and
+// MPO bond 5 alone (first / second, DMMA -> residues):
+//   D = 48: 14.2 -> 16.3, 24.9 -> 20.8 us;  56: 20.2 -> 16.6, 24.2 -> 22.6;  64: 30.1 -> 16.8,
+//   28.3 -> 22.7;  128: 184 -> 26, 217 -> 27;  256: 1417 -> 58, 1456 -> 52
+// whole calls: H_eff at D = 48 44.5 -> 40.5 us, 64 64.7 -> 42.5; environment steps at 48 37.3 ->
+// 40.4, 56 47.5 -> 42; and a Lanczos step:
+//   D = 48: 56 -> 42 us;  64: 77 -> 44;  128: 425 -> 59;  256: 2908 -> 120
 bool rns_wanted(long M, long N, long K) {
   if (std::min(M, std::min(N, K)) < 32 || M > INT_MAX / 2 || N > INT_MAX / 2) return false;
   return (double)M * N * K >= 1.0e6 && rns_bits(K, RNS_FP64) != 0;
