@@ -15,7 +15,7 @@ __all__ = ["apply_local_hamiltonian", "apply_local_bond_contraction",
            "compute_right_operator_blocks", "mpo_average", "mpo_inner_product",
            "mps_vdot", "mps_norm"]
 
-_WS = Workspace()
+_WS = Workspace(remember=False)
 
 
 def _is_host(*xs):

@@ -88,11 +88,14 @@ def zeros(shape):
 
 
 class Workspace:
-    """Grow-only device scratch buffer (bytes)."""
+    """Grow-only device scratch buffer (bytes). A run's buffer remembers a size that the device
+    had no memory for (asking again is slow, and not possible while a graph is captured); with
+    remember=False every call asks again."""
 
-    def __init__(self):
+    def __init__(self, remember=True):
         self.buf = None
-        self.refused = None   # the smallest size that the device had no memory for
+        self.remember = remember
+        self.refused = None   # the smallest size that was refused
 
     def get(self, nbytes, least=None):
         """A buffer of nbytes, or where the device has no memory for that, of at least least()
@@ -107,7 +110,8 @@ class Workspace:
             except torch.cuda.OutOfMemoryError:
                 if least is None:
                     raise
-                self.refused = nbytes
+                if self.remember:
+                    self.refused = nbytes
         low = max(int(least()), 256)
         if self.buf is None or self.buf.numel() < low:
             self.buf = None

@@ -42,6 +42,10 @@ def test_workspace_takes_what_there_is(monkeypatch):
     assert w.room(0, lambda: 0)[1] == 256
     with pytest.raises(torch.cuda.OutOfMemoryError):
         w.room(9000, lambda: 6000)
+    w = device.Workspace(remember=False)
+    for _ in range(2):
+        asked.clear()
+        assert w.room(9000, lambda: 2000)[1] == 2000 and asked[0] == 9000   # asked every time
     size = {_lib.PREC_FP64: 8000, _lib.PREC_SPLIT_BF16: 7000, _lib.PREC_FP64_DMMA: 3000}
     for prec, runs in ((_lib.PREC_FP64, _lib.PREC_FP64), (_lib.PREC_SPLIT_BF16, _lib.PREC_FP64),
                        (_lib.PREC_FP64_DMMA, _lib.PREC_FP64_DMMA)):
