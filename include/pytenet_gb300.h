@@ -231,8 +231,9 @@ size_t ptn_zgemm_split_bf16_workspace_bytes(int M, int N, int K);
 ptn_status ptn_zgemm_split_bf16(const ptn_c128* A, long lda, const ptn_c128* B, long ldb,
                                 ptn_c128* C, long ldc, int M, int N, int K, void* ws,
                                 size_t ws_bytes, void* stream);
-/* Error word of the device: 0, or the code of a bounded wait that expired in a tensor-core
- * kernel (1 producer, 2 MMA, 3 epilogue), -1 if it cannot be read. It stands until it is read
+/* Error word of the device: 0, or the code of a bounded wait that expired, in a tensor-core
+ * kernel (1 producer, 2 MMA, 3 epilogue) or at a grid barrier of a Lanczos step whose local step
+ * was therefore left out (4), -1 if it cannot be read. It stands until it is read
  * (which resets it), and while it stands every residue product gives NaN, so that no result of
  * an unfinished product passes for one. ptn_device_error waits for `stream`, ptn_tc_error for
  * the device. ptn_device_error_inject sets the word, for tests of what happens then. */

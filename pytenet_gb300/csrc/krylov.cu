@@ -207,7 +207,7 @@ __device__ __forceinline__ double reduce_partials_cg(const double* part, int nb,
 }
 
 // grid-wide barrier over co-resident CTAs (cooperative launch); bounded: on expiry
-// it reports false (the step then stops with PTN_TIMEOUT instead of waiting on)
+// it reports false (the step then stops with PTN_TIMEOUT instead of waiting on, see k_tridiag)
 __device__ bool grid_barrier(KState* st) {
   __shared__ int s_ok;
   __syncthreads();
@@ -787,10 +787,15 @@ __device__ bool lowest_pair_warp(const double* alpha, const double* beta, int m,
 
 // mode 0: expm coefficients c = nrm U exp(dt Lambda) U^T e_1;
 // mode 1: lowest Ritz vector coefficients c = U[:, argmin], eval0 = min eigenvalue.
-__global__ void k_tridiag(KState* st, double dt_re, double dt_im, int mode) {
+// A run that a grid barrier gave up on leaves its vector as it was: the device's error word
+// (code 4) says so, since the next run starts the state afresh.
+__global__ void k_tridiag(KState* st, double dt_re, double dt_im, int mode, int* err) {
   grid_wait();
   const int lane = threadIdx.x;  // one warp
-  if (st->s.status != PTN_OK) return;
+  if (st->s.status != PTN_OK) {
+    if (st->s.status == PTN_TIMEOUT && lane == 0) atomicExch(err, 4);
+    return;
+  }
   const int m = st->s.m_used;
   bool ok = true;
   if (mode == 0 && !st->coef_ready)
@@ -1238,8 +1243,10 @@ ptn_status krylov_last(void* state, const double2* V, const double2* w, long n, 
 }
 
 ptn_status krylov_coef(void* state, double dt_re, double dt_im, int mode, cudaStream_t st) {
+  int* err = device_error_word();
+  PTN_CHECK_ARG(err != nullptr, "krylov: error word lookup failed");
   PTN_CUDA_TRY(launch(k_tridiag, dim3(1), dim3(32), 0, st, static_cast<KState*>(state), dt_re,
-      dt_im, mode));
+      dt_im, mode, err));
   PTN_LAUNCH_CHECK();
   note_launches(1);
   return PTN_OK;

@@ -37,7 +37,10 @@ class _Run:
 
     def read_state(self):
         raw = self.state[: _lib.C.sizeof(_lib.KrylovState)].cpu().numpy().tobytes()
-        return _lib.KrylovState.from_buffer_copy(raw)
+        s = _lib.KrylovState.from_buffer_copy(raw)
+        if s.status == _lib.PTN_TIMEOUT:
+            raise _lib.PtnError(s.status, "a grid barrier of a Lanczos step gave up")
+        return s
 
     def apply(self, afunc, j, out_row):
         x = self.V[j]

@@ -108,3 +108,30 @@ def test_a_run_raises_instead_of_returning_tensors(graph):
     with pytest.raises(_lib.PtnError):
         run.download()
     assert all(np.array_equal(x, y) for x, y in zip(before, psi.a))   # nothing was handed out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["expm", "eigh", "python"])
+def test_a_lanczos_run_that_timed_out_is_reported(mode):
+    """The state of a Lanczos step whose grid barrier gave up, as that step leaves it."""
+    import torch
+    from pytenet_gb300 import _lib, krylov
+    from pytenet_gb300.device import check_device, ptr, stream_ptr, to_dev, to_host
+    rng = np.random.default_rng(3)
+    r = krylov._Run(to_dev(rng.standard_normal(300) + 0j), 4)
+    check_device()
+    at = _lib.KrylovState.status.offset
+    r.state[at:at + 4].view(torch.int32).fill_(_lib.PTN_TIMEOUT)
+    L = _lib.load()
+    if mode == "python":
+        with pytest.raises(_lib.PtnError):
+            r.read_state()
+        return
+    if mode == "expm":
+        _lib.check(L.ptn_krylov_expm_coef(ptr(r.state), 0.0, -0.1, stream_ptr()))
+    else:
+        _lib.check(L.ptn_krylov_eigh_coef(ptr(r.state), stream_ptr()))
+    with pytest.raises(_lib.PtnError) as e:
+        to_host(r.V)
+    assert e.value.status == _lib.PTN_TIMEOUT and "code 4" in str(e.value)
+    check_device()
