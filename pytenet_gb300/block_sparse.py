@@ -122,24 +122,50 @@ class QRScratch:
             self.streams.append(torch.cuda.Stream())
         return self.lanes[i], self.streams[i]
 
-    def reserve(self, mb, nb, kb):
+    def reserve(self, work, qb, rb, ws, ws_least):
+        """The buffers of one block after the other, and the bytes of the QR's own scratch."""
+        buf, n = self.ws.room(ws, lambda: ws_least)
+        return self.work.get(work), self.qb.get(qb), self.rb.get(rb), buf, n
+
+
+def _wide_blocks(plan, small, count, key):
+    """The blocks too wide for the one-launch QR, largest first, dealt to `count` lanes: their
+    indices and the buffer sizes of each lane, cached on the plan."""
+    lanes = plan.dev_cache.get((key, "lanes"))
+    if lanes is None:
         L = lib()
-        return (self.work.get(mb * nb * 16), self.qb.get(mb * kb * 16), self.rb.get(kb * nb * 16),
-                *self.ws.room(L.ptn_qr_workspace_bytes(mb, nb),
-                              lambda: L.ptn_qr_least_workspace_bytes(mb, nb)))
+        wide = sorted((k for k in range(len(plan.blocks)) if k not in small),
+                      key=lambda k: -len(plan.blocks[k][0]) * len(plan.blocks[k][1]) * plan.blocks[k][3])
+        count = max(1, min(len(wide), count))
+        lanes = []
+        for i in range(count):
+            need = [0] * 5
+            for k in wide[i::count]:
+                rows, cols, _, kb = plan.blocks[k]
+                mb, nb = len(rows), len(cols)
+                sizes = (mb * nb * 16, mb * kb * 16, kb * nb * 16, L.ptn_qr_workspace_bytes(mb, nb),
+                         L.ptn_qr_least_workspace_bytes(mb, nb))
+                need = [max(x, y) for x, y in zip(need, sizes)]
+            lanes.append((wide[i::count], need))
+        plan.dev_cache[(key, "lanes")] = lanes
+    return lanes
 
 
-def _qr_block(block, maps, src, q_dst, r_dst, scratch, st):
-    """Gather, QR and scatter of one block on stream st."""
+def _qr_lane(plan, blocks, need, maps, src, q_dst, r_dst, scratch, st):
+    """Gather, QR and scatter of the blocks, one after the other on stream st."""
     L = lib()
-    rows, cols, k0, kb = block
-    sro, sco, qro, qco, rro, rco = maps
-    mb, nb = len(rows), len(cols)
-    work, qb, rb, ws, wsb = scratch.reserve(mb, nb, kb)
-    call(L.ptn_gather, ptr(src), ptr(sro), ptr(sco), mb, nb, ptr(work), st)
-    call(L.ptn_qr, ptr(work), mb, nb, ptr(qb), kb, ptr(rb), nb, ptr(ws), wsb, st)
-    call(L.ptn_scatter, ptr(qb), kb, ptr(qro), ptr(qco), mb, kb, ptr(q_dst), st)
-    call(L.ptn_scatter, ptr(rb), nb, ptr(rro), ptr(rco), kb, nb, ptr(r_dst), st)
+    # all buffers before the first launch: none is replaced while a block uses it
+    work, qb, rb, ws, wsb = scratch.reserve(*need)
+    work, qb, rb, ws = ptr(work), ptr(qb), ptr(rb), ptr(ws)
+    src, q_dst, r_dst = ptr(src), ptr(q_dst), ptr(r_dst)
+    for k in blocks:
+        rows, cols, _, kb = plan.blocks[k]
+        sro, sco, qro, qco, rro, rco = (ptr(x) for x in maps[k])
+        mb, nb = len(rows), len(cols)
+        call(L.ptn_gather, src, sro, sco, mb, nb, work, st)
+        call(L.ptn_qr, work, mb, nb, qb, kb, rb, nb, ws, wsb, st)
+        call(L.ptn_scatter, qb, kb, qro, qco, mb, kb, q_dst, st)
+        call(L.ptn_scatter, rb, nb, rro, rco, kb, nb, r_dst, st)
 
 
 def qr_execute(plan, src, src_view, q_dst, q_view, r_dst, r_view, scratch):
@@ -156,30 +182,26 @@ def qr_execute(plan, src, src_view, q_dst, q_view, r_dst, r_view, scratch):
         q_dst.view(-1)[int(qro[0] + qco[0])] = 1.0
         return
     maps = _block_maps(plan, src_view, q_view, r_view)
-    small, max_m, table = _small_blocks(plan, maps, (src_view.key(), q_view.key(), r_view.key()))
+    key = (src_view.key(), q_view.key(), r_view.key())
+    small, max_m, table = _small_blocks(plan, maps, key)
     if small:
         call(L.ptn_qr_blocks, ptr(src), ptr(q_dst), ptr(r_dst), ptr(table), len(small), max_m, st)
-    # the wide blocks are chains of small launches: beside each other, largest first
-    wide = sorted((k for k in range(len(plan.blocks)) if k not in small),
-                  key=lambda k: -len(plan.blocks[k][0]) * len(plan.blocks[k][1]) * plan.blocks[k][3])
-    lanes = min(len(wide), scratch.LANES)
-    if lanes < 2:
-        for k in wide:
-            _qr_block(plan.blocks[k], maps[k], src, q_dst, r_dst, scratch, st)
+    if len(small) == len(plan.blocks):
+        return
+    # the wide blocks are chains of small launches: beside each other
+    lanes = _wide_blocks(plan, small, scratch.LANES, len(small))
+    if len(lanes) < 2:
+        _qr_lane(plan, *lanes[0], maps, src, q_dst, r_dst, scratch, st)
         return
     main = torch.cuda.current_stream()
     fork = main.record_event()
     forked = []
     try:
-        for i in range(lanes):
+        for i, (blocks, need) in enumerate(lanes):
             lane, stream = scratch.lane(i)
-            for k in wide[i::lanes]:   # no buffer is replaced while a block of this call uses it
-                rows, cols, _, kb = plan.blocks[k]
-                lane.reserve(len(rows), len(cols), kb)
             stream.wait_event(fork)
             forked.append(stream)
-            for k in wide[i::lanes]:
-                _qr_block(plan.blocks[k], maps[k], src, q_dst, r_dst, lane, stream.cuda_stream)
+            _qr_lane(plan, blocks, need, maps, src, q_dst, r_dst, lane, stream.cuda_stream)
     finally:
         # after an error too: the caller may let go of the tensors that the lanes still use
         for stream in forked:

@@ -229,12 +229,12 @@ def test_qr_lanes_join_after_an_error(monkeypatch, fails_at):
 
     class Lib:
         ptn_gather = ptn_qr = ptn_scatter = ptn_qr_blocks = staticmethod(lambda *a: 0)
-        ptn_qr_workspace_bytes = staticmethod(lambda m, n: 256)
+        ptn_qr_workspace_bytes = ptn_qr_least_workspace_bytes = staticmethod(lambda m, n: 256)
 
     main, made, calls = Stream("main"), [], []
 
     class Scratch(bs.QRScratch):
-        def reserve(self, mb, nb, kb):
+        def reserve(self, *sizes):
             return (None,) * 4 + (0,)
 
         def lane(self, i):
